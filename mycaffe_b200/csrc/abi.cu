@@ -4,6 +4,7 @@
 // ids listed in mycaffe_attn.h, and nothing else of that DLL.
 #include <dlfcn.h>
 
+#include <chrono>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -128,14 +129,25 @@ struct Kernel {
   std::string last_detail;
   float* stage = nullptr;  // grow-only fp32 staging buffer for float <-> bf16 transfers
   size_t stage_count = 0;
-  int* h_answer = nullptr; // eight pinned words for small device answers the host has to wait for (a mask's class in
-                           // [0], an attention handle's class + status words in [2..6])
+  bool synced = false;     // the call being dispatched has already synchronised the stream behind its last launch
+  bool fail_words = false; // this device's kernels raise the process's failure words (see g_fail_words)
+  int* h_answer = nullptr; // pinned words for small device answers: a mask's class in [0], written by the kernel that finds it
   int* answer_words() {
-    if (h_answer == nullptr && cudaMallocHost((void**)&h_answer, 8 * sizeof(int)) != cudaSuccess) {
-      cudaGetLastError();
-      h_answer = nullptr;
+    if (h_answer == nullptr) {
+      if (cudaMallocHost((void**)&h_answer, 8 * sizeof(int)) != cudaSuccess) {
+        cudaGetLastError();
+        h_answer = nullptr;
+      } else {
+        h_answer[0] = -1;
+      }
     }
     return h_answer;
+  }
+
+  int class_tag = 0;       // even; tags the last classification whose answer goes to h_answer[0] (tag + class)
+  int answered_class() const {   // -1: that answer has not arrived yet
+    const int w = *reinterpret_cast<const volatile int*>(h_answer) - class_tag;
+    return w == 0 || w == 1 ? w : -1;
   }
 
   float* staging(size_t count) {
@@ -157,6 +169,49 @@ struct Kernel {
 
 Kernel* g_kernels[kMaxKernels];
 std::mutex g_table_lock;
+
+// McaFailWord array in pinned host memory, raised by the kernels of every device: behind a stream synchronisation one
+// host load says whether any device status word is worth reading.  A raised MCA_FAIL_TC word stays raised (it stands for
+// every attention handle's own status words, and a bounded wait giving up is no ordinary event); the other two families
+// have one status array per device and their word is lowered before that array is read.
+int* g_fail_words = nullptr;
+uint64_t g_fail_words_devices = 0;   // devices whose kernels know the address
+
+bool arm_fail_words(int dev) {   // under g_table_lock, with dev current
+  if (dev >= 64) return false;
+  if (g_fail_words == nullptr) {
+    if (cudaHostAlloc((void**)&g_fail_words, MCA_FAIL_WORDS * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+      cudaGetLastError();
+      g_fail_words = nullptr;
+      return false;
+    }
+    for (int i = 0; i < MCA_FAIL_WORDS; ++i) g_fail_words[i] = 0;
+  }
+  if (!(g_fail_words_devices >> dev & 1)) {
+    if (mca_set_fail_words_fwd(g_fail_words) || mca_set_fail_words_bwd(g_fail_words) || mca_set_fail_words_probe(g_fail_words) ||
+        mca_set_fail_words_decode(g_fail_words) || mca_set_fail_words_proj(g_fail_words)) {
+      cudaGetLastError();
+      return false;
+    }
+    g_fail_words_devices |= 1ull << dev;
+  }
+  return true;
+}
+
+bool may_have_failed(const Kernel* k, McaFailWord family) {
+  return !k->fail_words || *reinterpret_cast<volatile int*>(g_fail_words + family) != 0;
+}
+void lower_fail_word(const Kernel* k, McaFailWord family) {
+  if (k->fail_words) *reinterpret_cast<volatile int*>(g_fail_words + family) = 0;
+}
+
+// The one synchronisation of a synchronous call.
+long sync_call(Kernel* k) {
+  if (k->synced) return 0;
+  const cudaError_t ce = cudaStreamSynchronize(0);
+  k->synced = ce == cudaSuccess;
+  return (long)ce;
+}
 
 const char* error_name(long e) {
   switch (e) {
@@ -219,7 +274,7 @@ long set_out(float v, MCA_LONG* plOutput, float** ppOutput) {
 
 long finish(Kernel* k, long err) {
   if (err) return err;
-  if (!k->async) return (long)cudaStreamSynchronize(0);  // the reference blocks after every op (attn.cu:601)
+  if (!k->async) return sync_call(k);  // the reference blocks after every op (attn.cu:601)
   return 0;
 }
 
@@ -423,7 +478,12 @@ long resolve_mask(Kernel* k, AttnHandle& a, long hMask, bool batch_mask, int T, 
   *mask = m;
   if (batch_mask) { *mode = MCA_MASK_BATCH; return 0; }
   *mode = MCA_MASK_TT;
-  if ((e = mca_classify_causal_mask_ws(m, T, a.causal_flag, a.causal_flag + 6, 0))) return e;
+  // The class goes to a pinned host word as well, tagged with this classification's number.
+  if (need_host_answer && k->answer_words() == nullptr) return ERROR_MEMORY_OUT;
+  k->class_tag = (k->class_tag + 2) & 0x3ffffffe;
+  k->synced = false;
+  if ((e = mca_classify_causal_mask_ws(m, T, a.causal_flag, need_host_answer ? k->h_answer : nullptr, k->class_tag, a.causal_flag + 6, 0)))
+    return e;
   if (need_host_answer && may_speculate && !k->async && a.spec_allowed && a.spec_class >= 0) {
     a.spec_pending = true;
     a.spec_assumed = a.spec_class;
@@ -431,14 +491,18 @@ long resolve_mask(Kernel* k, AttnHandle& a, long hMask, bool batch_mask, int T, 
     return 0;
   }
   if (need_host_answer) {
-    // into pinned memory on the stream, then one stream synchronisation: a third of the latency of a blocking copy
-    // into pageable memory
-    if (k->answer_words() == nullptr) return ERROR_MEMORY_OUT;
-    cudaError_t ce = cudaMemcpyAsync(k->h_answer, a.causal_flag, sizeof(int), cudaMemcpyDeviceToHost, 0);
-    if (ce == cudaSuccess) ce = cudaStreamSynchronize(0);
-    if (ce != cudaSuccess) return ce;
-    if (*k->h_answer == 1) *mode = MCA_MASK_CAUSAL;
-    a.spec_class = *k->h_answer == 1 ? 1 : 0;
+    // Poll the word: it arrives a microsecond after the kernel has written it, where a copy back and a stream
+    // synchronisation left the GPU idle for twenty.  The polling is bounded; a long queue ahead of the classification
+    // is waited for by a synchronisation.
+    const auto t0 = std::chrono::steady_clock::now();
+    while (k->answered_class() < 0 && std::chrono::steady_clock::now() - t0 < std::chrono::milliseconds(2)) {
+    }
+    if (k->answered_class() < 0) {
+      const cudaError_t ce = cudaStreamSynchronize(0);
+      if (ce != cudaSuccess) return ce;
+    }
+    a.spec_class = k->answered_class() == 1 ? 1 : 0;
+    if (a.spec_class == 1) *mode = MCA_MASK_CAUSAL;
   }
   return 0;
 }
@@ -478,17 +542,16 @@ long ensure_mask_ws(AttnHandle& a) {
 // attention handle at the next call that synchronises (CUDA_FN_SYNCHRONIZEDEVICE).
 long read_status(Kernel* k, AttnHandle& a) {
   if (!a.causal_flag) return 0;
-  // into pinned words on the stream, then one stream synchronisation (a blocking copy into pageable memory takes
-  // several microseconds longer, on every call of the synchronous mode)
-  if (k->answer_words() == nullptr) return ERROR_MEMORY_OUT;
-  int* w = k->h_answer + 2;
-  cudaError_t ce = cudaMemcpyAsync(w, a.causal_flag, 5 * sizeof(int), cudaMemcpyDeviceToHost, 0);
-  if (ce == cudaSuccess) ce = cudaStreamSynchronize(0);
-  if (ce != cudaSuccess) return ce;
-  const int* st = w + 1;
+  long e = sync_call(k);
+  if (e) return e;
+  int st[4] = {0, 0, 0, 0};
+  if (may_have_failed(k, MCA_FAIL_TC)) {
+    const cudaError_t ce = cudaMemcpy(st, a.causal_flag + 1, sizeof(st), cudaMemcpyDeviceToHost);
+    if (ce != cudaSuccess) return ce;
+  }
   if (a.spec_pending) {   // the class this call's kernels were chosen on, against what its classification found
     a.spec_pending = false;
-    const int actual = w[0] == 1 ? 1 : 0;
+    const int actual = k->answered_class() == 1 ? 1 : 0;
     const bool matters = a.spec_assumed == 1 && actual == 0;   // the other way round the result is right, only slower
     a.spec_class = actual;
     if (matters && st[0] == 0) return kMaskClassMiss;
@@ -508,8 +571,8 @@ long tc_status(Kernel* k, AttnHandle& a) {
   return read_status(k, a);
 }
 long sync_and_collect_status(Kernel* k) {
-  cudaError_t ce = cudaStreamSynchronize(0);
-  if (ce != cudaSuccess) return ce;
+  const long se = sync_call(k);
+  if (se) return se;
   long first = 0;
   for (auto& kv : k->attn) {
     if (!kv.second.status_pending) continue;
@@ -536,6 +599,7 @@ long attn_fwd(Kernel* k, long llInput, MCA_LONGLONG* pl, int layout) {
   if (e != kMaskClassMiss) return e;
   AttnHandle& a = k->attn.find((long)pl[1])->second;   // the handle exists: the first pass ran its kernels
   a.spec_allowed = false;                              // this time the class is read before the kernels are chosen
+  k->synced = false;
   e = attn_fwd_once(k, llInput, pl, layout);
   a.spec_allowed = true;
   return e;
@@ -892,8 +956,8 @@ long decode_step(Kernel* k, long llInput, MCA_LONGLONG* pl) {
   if (e || k->async) return e;
   // synchronous mode: a position outside [0, maxLen) was refused on the device (that sequence's output is zero,
   // its cache untouched); report it instead of returning success
-  cudaError_t ce = cudaStreamSynchronize(0);
-  if (ce != cudaSuccess) return ce;
+  if ((e = sync_call(k)) || !may_have_failed(k, MCA_FAIL_DECODE)) return e;
+  lower_fail_word(k, MCA_FAIL_DECODE);
   int st[3] = {0, 0, 0};
   if ((e = mca_decode_status(st))) return e;
   if (st[0] != 0) {
@@ -910,8 +974,8 @@ long decode_step(Kernel* k, long llInput, MCA_LONGLONG* pl) {
 // up inside that kernel is reported here instead of returning success.
 long proj_result(Kernel* k, long e, long B) {
   if (e || k->async || B <= 8) return e;
-  cudaError_t ce = cudaStreamSynchronize(0);
-  if (ce != cudaSuccess) return ce;
+  if ((e = sync_call(k)) || !may_have_failed(k, MCA_FAIL_PROJ)) return e;
+  lower_fail_word(k, MCA_FAIL_PROJ);
   int st[4] = {0, 0, 0, 0};
   if ((e = mca_proj_tc_status(st))) return e;
   if (st[0] != 0) {
@@ -1170,15 +1234,16 @@ long kernel_init(float* pInput, long lInput, long* idx_out) {
   cudaError_t ce = cudaGetDeviceCount(&count);
   if (ce != cudaSuccess) { cudaGetLastError(); return ce; }
   if (dev < 0 || dev >= count) return ERROR_PARAM_OUT_OF_RANGE;
-  cudaDeviceProp prop;
-  if ((ce = cudaGetDeviceProperties(&prop, dev)) != cudaSuccess) return ce;
-  if (prop.major != 10) return ERROR_ATTN_NOT_B200;  // sm_100a code only: fail loudly elsewhere
+  int major = 0;   // one attribute: the full property query takes several milliseconds
+  if ((ce = cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev)) != cudaSuccess) return ce;
+  if (major != 10) return ERROR_ATTN_NOT_B200;  // sm_100a code only: fail loudly elsewhere
   if ((ce = cudaSetDevice(dev)) != cudaSuccess) return ce;
   std::lock_guard<std::mutex> lock(g_table_lock);
   for (int i = 1; i < kMaxKernels; ++i) {
     if (!g_kernels[i]) {
       g_kernels[i] = new Kernel();
       g_kernels[i]->device = dev;
+      g_kernels[i]->fail_words = arm_fail_words(dev);
       *idx_out = i;
       return 0;
     }
@@ -1213,6 +1278,7 @@ long run(Kernel* k, long fn, float* pf, long lInput, MCA_LONGLONG* pl, long llIn
   cudaError_t ce = cudaSetDevice(k->device);
   if (ce != cudaSuccess) return ce;
   k->last_detail.clear();
+  k->synced = false;
   long e;
   switch (fn) {
     case CUDA_FN_SETDEVICE: return 0;

@@ -425,7 +425,7 @@ __global__ void set_int_kernel(int* p, int v) { *p = v; }
 // The same answer from one launch: a warp per row (16-byte loads when T allows), the blocks' mismatch counts and a
 // ticket in two scratch words that are zero before and after; the last block to finish writes the flag.
 __global__ void __launch_bounds__(256) classify_causal_rows_kernel(const float* __restrict__ mask, int T, int* __restrict__ flag,
-                                                                   int* __restrict__ scratch) {
+                                                                   int* __restrict__ host_flag, int host_base, int* __restrict__ scratch) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   bool bad = false;
   for (int i = blockIdx.x * 8 + warp; i < T; i += gridDim.x * 8) {
@@ -446,7 +446,9 @@ __global__ void __launch_bounds__(256) classify_causal_rows_kernel(const float* 
     __threadfence();
     if (atomicAdd(scratch + 1, 1) == (int)gridDim.x - 1) {
       __threadfence();
-      *flag = atomicExch(scratch, 0) == 0 ? 1 : 0;
+      const int causal = atomicExch(scratch, 0) == 0 ? 1 : 0;
+      *flag = causal;
+      if (host_flag != nullptr) *host_flag = host_base + causal;   // pinned host memory: read behind the next stream synchronisation
       scratch[1] = 0;
     }
   }
@@ -463,11 +465,11 @@ template <typename F> int set_smem(F kernel, size_t bytes) {
 
 }  // namespace
 
-int mca_classify_causal_mask_ws(const float* mask, int T, int* flag, int* scratch, void* stream) {
+int mca_classify_causal_mask_ws(const float* mask, int T, int* flag, int* host_flag, int host_base, int* scratch, void* stream) {
   if (!mask || !flag || !scratch) return ERROR_PARAM_NULL;
   if (T <= 0) return ERROR_PARAM_OUT_OF_RANGE;
   const int blocks = std::min(1184, (T + 7) / 8);
-  classify_causal_rows_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(mask, T, flag, scratch);
+  classify_causal_rows_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(mask, T, flag, host_flag, host_base, scratch);
   return mca_launch_status();
 }
 

@@ -781,11 +781,15 @@ int launch_shape(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap
   dim3 grid(mca_ceil_div(T, SH::QT * BLK), B * H);
   if constexpr (MODE != MODE_TF32) {
     if (masked) {
-      MCA_CUDA_TRY(cudaFuncSetAttribute(sdpa_fwd_tc_kernel<HD, MODE, true, NARROW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      static std::atomic<uint64_t> done{0};
+      const int e = mca_smem_once(done, sdpa_fwd_tc_kernel<HD, MODE, true, NARROW>, smem);
+      if (e) return e;
       return mca_launch_pdl(sdpa_fwd_tc_kernel<HD, MODE, true, NARROW>, grid, dim3(SH::THREADS), smem, st, mq, mk, mv, p);
     }
   }
-  MCA_CUDA_TRY(cudaFuncSetAttribute(sdpa_fwd_tc_kernel<HD, MODE, false, NARROW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  static std::atomic<uint64_t> done{0};
+  const int e = mca_smem_once(done, sdpa_fwd_tc_kernel<HD, MODE, false, NARROW>, smem);
+  if (e) return e;
   return mca_launch_pdl(sdpa_fwd_tc_kernel<HD, MODE, false, NARROW>, grid, dim3(SH::THREADS), smem, st, mq, mk, mv, p);
 }
 
@@ -1048,3 +1052,5 @@ int mca_mask_pack(const float* mask, int mask_mode, int B, int T, uint32_t* bits
                                                                                mask_mode == MCA_MASK_TT ? bits_t : nullptr);
   return mca_launch_status();
 }
+
+int mca_set_fail_words_fwd(int* words) { return (int)cudaMemcpyToSymbol(tc::g_fail_words, &words, sizeof(words)); }

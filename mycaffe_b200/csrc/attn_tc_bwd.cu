@@ -477,7 +477,7 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   uint32_t dyn_bytes;
   asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_bytes));
   if (smem_base + PL::NEED_KV > smem_u32(smem_raw) + dyn_bytes) {
-    if (tid == 0 && atomicCAS(p.status, 0, 2) == 0) { p.status[1] = 299; p.status[2] = (int)(smem_base - smem_u32(smem_raw)); }
+    if (tid == 0 && atomicCAS(p.status, 0, 2) == 0) { p.status[1] = 299; p.status[2] = (int)(smem_base - smem_u32(smem_raw)); raise_failure(); }
     return;
   }
   volatile int* s_abort = reinterpret_cast<volatile int*>(smem_gen + PL::OFF_FLAG_KV);
@@ -815,11 +815,14 @@ int launch_bwd_pair(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensor
                     void* dq, void* dk, void* dv, int B, int H, int T, cudaStream_t st) {
   using PL = BwdPlan<SPLIT ? 128 : HD>;
   const size_t smem_kv = PL::BYTES_KV, smem_dq = PL::BYTES_DQ;
-  MCA_CUDA_TRY(cudaFuncSetAttribute(sdpa_bwd_dkdv_tc_kernel<HD, SPLIT, MASKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_kv));
-  MCA_CUDA_TRY(cudaFuncSetAttribute(sdpa_bwd_dq_tc_kernel<HD, SPLIT, MASKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_dq));
+  static std::atomic<uint64_t> done_kv{0}, done_dq{0};
+  int e;
+  if ((e = mca_smem_once(done_kv, sdpa_bwd_dkdv_tc_kernel<HD, SPLIT, MASKED>, smem_kv)) ||
+      (e = mca_smem_once(done_dq, sdpa_bwd_dq_tc_kernel<HD, SPLIT, MASKED>, smem_dq)))
+    return e;
   dim3 grid(mca_ceil_div(T, BLK), B * H);
   p.out0 = dk; p.out1 = dv;
-  int e = mca_launch_pdl(sdpa_bwd_dkdv_tc_kernel<HD, SPLIT, MASKED>, grid, dim3(BW_THREADS), smem_kv, st, mq, mk, mv, mdo, p);
+  e = mca_launch_pdl(sdpa_bwd_dkdv_tc_kernel<HD, SPLIT, MASKED>, grid, dim3(BW_THREADS), smem_kv, st, mq, mk, mv, mdo, p);
   if (e) return e;
   p.out0 = dq; p.out1 = nullptr;
   return mca_launch_pdl(sdpa_bwd_dq_tc_kernel<HD, SPLIT, MASKED>, grid, dim3(BW_THREADS), smem_dq, st, mq, mk, mv, mdo, p);
@@ -975,3 +978,5 @@ int mca_sdpa_backward_f32_tc_masked(const float* dy, const float* y_copy, const 
   }
   return ERROR_ATTN_UNSUPPORTED_SHAPE;
 }
+
+int mca_set_fail_words_bwd(int* words) { return (int)cudaMemcpyToSymbol(tc::g_fail_words, &words, sizeof(words)); }

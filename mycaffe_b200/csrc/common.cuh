@@ -1,6 +1,7 @@
 // Shared declarations for the attention library (sm_100a only).
 #pragma once
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstdlib>
 #include <cuda_bf16.h>
 #include <stdint.h>
@@ -87,6 +88,13 @@ static inline int mca_launch_status() {
 
 __host__ __device__ static inline int mca_ceil_div(int a, int b) { return (a + b - 1) / b; }
 
+// Failure words in pinned host memory (one array per process, visible to every device): a kernel that writes a failure
+// into its device status words also raises the word of its family here, so that a synchronous call learns from a plain
+// host load behind its one stream synchronisation that nothing failed.  (Copying the status words back after every call
+// cost a 3 us transfer and its launch on each.)  Each family's device code holds the array's address in a symbol of its
+// own translation unit, set when a kernel index is initialised; null (raw callers) means no word is raised.
+enum McaFailWord : int { MCA_FAIL_TC = 0, MCA_FAIL_DECODE = 1, MCA_FAIL_PROJ = 2, MCA_FAIL_WORDS = 4 };
+
 // Programmatic dependent launch.  A kernel launched with mca_launch_pdl may start while the
 // previous kernel of the stream is still running (once every CTA of that kernel has executed
 // mca_pdl_launch_dependents or exited); what it does before mca_pdl_wait() must depend on nothing
@@ -100,6 +108,26 @@ __device__ __forceinline__ void mca_cp_async16(uint32_t dst_smem, const void* sr
 }
 __device__ __forceinline__ void mca_cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void mca_cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+__device__ __forceinline__ void mca_raise_fail_word(int* words, int family) {
+  if (words != nullptr) {
+    *reinterpret_cast<volatile int*>(words + family) = 1;
+    __threadfence_system();
+  }
+}
+
+// Opt a kernel into `bytes` of dynamic shared memory, once per device (the attribute call costs more than the launch's
+// own host work when it is repeated).  done: a static of the instantiation that launches this kernel with this size.
+template <typename F>
+static inline int mca_smem_once(std::atomic<uint64_t>& done, F kern, size_t bytes) {
+  int dev = 0;
+  MCA_CUDA_TRY(cudaGetDevice(&dev));
+  const uint64_t bit = 1ull << (dev & 63);
+  if (dev < 64 && (done.load(std::memory_order_acquire) & bit)) return 0;
+  MCA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  if (dev < 64) done.fetch_or(bit, std::memory_order_release);
+  return 0;
+}
 
 __device__ __forceinline__ void mca_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void mca_pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

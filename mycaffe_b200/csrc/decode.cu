@@ -45,6 +45,7 @@ template <typename CT, int HS> struct Epl {
 // Status words of the decode kernels: [0] number of sequences whose position was outside [0, max_len) since the
 // last read, [1] the first such sequence, [2] its position.  Such a sequence is not attended and its output is zero.
 __device__ int g_decode_status[4];
+__device__ int* g_fail_words;   // the process's failure words (McaFailWord), or null
 
 struct DecodeParams {
   const float* q;        // (B, n_heads*HS): projection of the new token (before RoPE when fr != null)
@@ -170,9 +171,13 @@ __global__ void __launch_bounds__(DEC_THREADS, KVM == 1 ? 2 : 1) decode_split_ke
     // A position outside the cache (or beyond the planned splits) is not followed: nothing of this sequence is
     // read or appended, its output is zero, and the status words say which sequence it was.
     if (split == 0) {
-      if (blockIdx.y == 0 && threadIdx.x == 0 && atomicAdd(&g_decode_status[0], 1) == 0) {
-        g_decode_status[1] = b;
-        g_decode_status[2] = pos;
+      if (blockIdx.y == 0 && threadIdx.x == 0) {
+        if (atomicAdd(&g_decode_status[0], 1) == 0) {
+          g_decode_status[1] = b;
+          g_decode_status[2] = pos;
+        }
+        __threadfence();
+        mca_raise_fail_word(g_fail_words, MCA_FAIL_DECODE);
       }
       if (p.nsplit == 1)
         for (int i = threadIdx.x; i < KVM * HS; i += DEC_THREADS) p.out[(int64_t)b * p.n_heads * HS + (int64_t)h0 * HS + i] = 0.f;
@@ -487,9 +492,11 @@ int launch_decode(const DecodeParams& p, int B, cudaStream_t st) {
   dim3 grid(p.nsplit, p.n_heads / kvmt, B);
   const size_t smem = sizeof(CT) == 2 ? DecRing<Epl<CT, HS>::value / 8>::BYTES : 0;   // the bf16 path's cp.async ring
   if (smem) {
-    MCA_CUDA_TRY(cudaFuncSetAttribute(decode_split_kernel<CT, HS, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    MCA_CUDA_TRY(cudaFuncSetAttribute(decode_split_kernel<CT, HS, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    MCA_CUDA_TRY(cudaFuncSetAttribute(decode_split_kernel<CT, HS, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static std::atomic<uint64_t> done1{0}, done2{0}, done4{0};
+    int e;
+    if ((e = mca_smem_once(done1, decode_split_kernel<CT, HS, 1>, smem)) || (e = mca_smem_once(done2, decode_split_kernel<CT, HS, 2>, smem)) ||
+        (e = mca_smem_once(done4, decode_split_kernel<CT, HS, 4>, smem)))
+      return e;
   }
   // Up to eight sequences the kernel is launched ahead of the one before it (resident and waiting when that one
   // finishes: the step is short and the launch latency shows, + 6 % at one sequence).  With more sequences the
@@ -682,3 +689,5 @@ int mca_decode_exchange(const float* src, float* const* dst, int* const* flag_ds
   const int blocks = std::max(1, std::min(148, (total + 255) / 256));
   return mca_launch_pdl(decode_exchange_kernel, dim3(blocks), dim3(256), 0, (cudaStream_t)stream, p);
 }
+
+int mca_set_fail_words_decode(int* words) { return (int)cudaMemcpyToSymbol(g_fail_words, &words, sizeof(words)); }

@@ -355,11 +355,22 @@ int run_proj_tc(const GemvParams& p, cudaStream_t st) {
   if (tiles > proj::MAX_TILES) return -1;
   int dev = 0, sms = 148;
   MCA_CUDA_TRY(cudaGetDevice(&dev));
-  MCA_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   uint16_t* pieces = nullptr;
   float* xscale = nullptr;
-  MCA_CUDA_TRY(cudaGetSymbolAddress(reinterpret_cast<void**>(&pieces), proj::g_x_pieces));
-  MCA_CUDA_TRY(cudaGetSymbolAddress(reinterpret_cast<void**>(&xscale), proj::g_x_scale));
+  {
+    // the SM count and the arrays' addresses are looked up once per device
+    static std::mutex lock;
+    static struct { int sms; uint16_t* pieces; float* xscale; } known[64];
+    if (dev < 0 || dev >= 64) return ERROR_PARAM_OUT_OF_RANGE;
+    std::lock_guard<std::mutex> g(lock);
+    auto& c = known[dev];
+    if (c.sms == 0) {
+      MCA_CUDA_TRY(cudaGetSymbolAddress(reinterpret_cast<void**>(&c.pieces), proj::g_x_pieces));
+      MCA_CUDA_TRY(cudaGetSymbolAddress(reinterpret_cast<void**>(&c.xscale), proj::g_x_scale));
+      MCA_CUDA_TRY(cudaDeviceGetAttribute(&c.sms, cudaDevAttrMultiProcessorCount, dev));
+    }
+    sms = c.sms; pieces = c.pieces; xscale = c.xscale;
+  }
   q.n_mats = p.n_mats; q.B = p.B; q.Bp = Bp; q.n = p.n; q.accumulate = p.accumulate; q.swiglu = p.swiglu;
   q.tiles = tiles; q.kchunks = mca_ceil_div(p.n, proj::KC);
   q.slices = proj::pick_slices(tiles, q.kchunks, sms);
@@ -376,14 +387,15 @@ int run_proj_tc(const GemvParams& p, cudaStream_t st) {
                              (int64_t)PL::PIECES * Bp, p.n, proj::KC, Bp, CU_TENSOR_MAP_SWIZZLE_128B)))
     return e;
   auto pre = proj::x_pieces_kernel<BF>;
-  MCA_CUDA_TRY(cudaFuncSetAttribute(pre, cudaFuncAttributeMaxDynamicSharedMemorySize, proj::MAX_N * 4));
+  static std::atomic<uint64_t> pre_done{0}, kern_done{0};
+  if ((e = mca_smem_once(pre_done, pre, proj::MAX_N * 4))) return e;
   // both kernels are launched programmatically dependent: the pre-pass's launch overlaps the tail of whatever runs
   // before it (it waits for that before it reads or writes anything), the contraction's set-up overlaps the pre-pass
   if ((e = mca_launch_pdl(pre, dim3(Bp), dim3(256), sizeof(float) * (size_t)p.n, st, p.x, p.norm_w, p.eps, p.n, p.B, Bp, pieces, xscale)))
     return e;
   const size_t smem = proj::smem_bytes<WT>();
   auto kern = proj::proj_tc_kernel<WT>;
-  MCA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if ((e = mca_smem_once(kern_done, kern, smem))) return e;
   const int items = tiles * q.slices;
   // programmatic dependent launch: set-up and the first weight tiles overlap the pre-pass
   return mca_launch_pdl(kern, dim3(std::min(items, sms)), dim3(proj::THREADS), smem, st, mw[0], mw[1], mw[2], mx, q);
@@ -519,3 +531,5 @@ int mca_proj_tc_status(int* status4) {
   }
   return 0;
 }
+
+int mca_set_fail_words_proj(int* words) { return (int)cudaMemcpyToSymbol(tc::g_fail_words, &words, sizeof(words)); }

@@ -25,6 +25,7 @@
 // The activation pieces, per-sequence scales, partial sums and tickets live in arrays that are part of the library
 // image (about 24 MB per device): nothing is allocated, but two of these products must not overlap on one device.
 #pragma once
+#define MCA_TU_FAIL_FAMILY MCA_FAIL_PROJ
 #include "tc_common.cuh"
 
 namespace proj {

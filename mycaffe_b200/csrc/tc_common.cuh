@@ -48,6 +48,14 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
   return t;
 }
 
+// Address of the process's failure words (see McaFailWord); one copy per translation unit that includes this header.
+// MCA_TU_FAIL_FAMILY: which of the words this translation unit's kernels raise.
+#ifndef MCA_TU_FAIL_FAMILY
+#define MCA_TU_FAIL_FAMILY MCA_FAIL_TC
+#endif
+static __device__ int* g_fail_words;
+static __device__ __noinline__ void raise_failure() { mca_raise_fail_word(g_fail_words, MCA_TU_FAIL_FAMILY); }
+
 // Bounded wait.  Returns false after limit_ns (or as soon as another CTA reported a
 // failure) and records {code, stage, block, iteration} in status[0..3].
 static __device__ __noinline__ bool mbar_wait_limited(uint32_t bar, uint32_t parity, int* status, int stage, int iter,
@@ -63,6 +71,7 @@ static __device__ __noinline__ bool mbar_wait_limited(uint32_t bar, uint32_t par
           status[2] = (int)(blockIdx.x + gridDim.x * blockIdx.y);
           status[3] = iter;
           __threadfence();
+          raise_failure();
         }
         return false;
       }

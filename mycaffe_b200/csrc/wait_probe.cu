@@ -29,3 +29,5 @@ int mca_wait_probe(int* status, int limit_us, void* stream) {
   wait_probe_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(status, (unsigned long long)limit_us * 1000ull);
   return mca_launch_status();
 }
+
+int mca_set_fail_words_probe(int* words) { return (int)cudaMemcpyToSymbol(tc::g_fail_words, &words, sizeof(words)); }

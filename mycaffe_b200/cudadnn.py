@@ -11,6 +11,7 @@ packed float / long arrays the C# code builds.
 from __future__ import annotations
 
 import ctypes as C
+import threading
 
 import numpy as np
 
@@ -25,11 +26,23 @@ class CudaDnnError(RuntimeError):
         self.native_message = message
 
 
+class _ErrorText(threading.local):
+    """This thread's buffer for the native error message."""
+
+    def __init__(self):
+        self.buf = C.create_string_buffer(1024)
+
+
+_error_text = _ErrorText()
+_LONGS = [C.c_int64 * n for n in range(20)]
+
+
 class CudaDnn:
     """One instance == one native kernel index (CudaDnn.cs:1693-1735)."""
 
     def __init__(self, device_id: int = 0):
         self._lib = _lib.load()
+        self._invoke_void = self._lib.DLL_InvokeFloatEx2
         self._kernel = 0
         out = self._invoke(ids.CUDA_DLL_INITIALIZE, [float(device_id), 0.0], None)
         self._kernel = int(out[0])
@@ -59,6 +72,22 @@ class CudaDnn:
             lib.DLL_InvokeFloat(self._kernel, ids.CUDA_DLL_FREEMEM, pp, 0, None, None, err, 1024)
             return res
         return out_buf[:n]
+
+    def _call(self, fn, longs, floats=None):
+        """A function id that returns nothing: the arguments are packed by ctypes alone and no result buffer is made
+        (2 us of host time where _invoke takes 8, on calls whose kernels last a few microseconds)."""
+        n = len(longs)
+        try:
+            packed = _LONGS[n](*longs)
+        except TypeError:        # whole numbers held in floats
+            packed = _LONGS[n](*[int(v) for v in longs])
+        err = _error_text.buf
+        if floats is None:
+            rc = self._invoke_void(self._kernel, fn, None, 0, packed, n, None, None, err, 1024)
+        else:
+            rc = self._invoke_void(self._kernel, fn, (C.c_float * len(floats))(*floats), len(floats), packed, n, None, None, err, 1024)
+        if rc != 0:
+            raise CudaDnnError(rc, err.value.decode(errors="replace"))
 
     def _finish(self, rc, err, pp, n_out, out_buf):
         if rc != 0:
@@ -174,7 +203,7 @@ class CudaDnn:
         return int(self._invoke(ids.MCA_FN_ALLOCMEM_BF16, packed, [data.size])[0])
 
     def FreeMemory(self, h):
-        self._invoke(ids.CUDA_FN_FREEMEM, None, [int(h)])
+        self._call(ids.CUDA_FN_FREEMEM, [int(h)])
 
     def GetMemory(self, h, count=-1) -> np.ndarray:
         cap = int(count) if count and count > 0 else 1
@@ -203,7 +232,7 @@ class CudaDnn:
         self.SetMemory(h, np.ascontiguousarray(data, np.int32).view(np.float32))
 
     def ConvertMemory(self, hSrc, hDst, count):
-        self._invoke(ids.MCA_FN_CONVERT, None, [int(hSrc), int(hDst), int(count)])
+        self._call(ids.MCA_FN_CONVERT, [int(hSrc), int(hDst), int(count)])
 
     def GetPointer(self, h) -> int:
         p = C.c_void_p()
@@ -243,11 +272,11 @@ class CudaDnn:
         self._invoke(ids.CUDNN_FN_ATTN_SET, [float(fDropout)], longs)
 
     def AttnScaledDotProductForward(self, hCuDnn, hAttn, nBlockSize, hQ, hK, hV, hMask, hY, bBatchMask=False):
-        self._invoke(ids.CUDNN_FN_ATTN_FWD, None,
+        self._call(ids.CUDNN_FN_ATTN_FWD,
                      [hCuDnn, hAttn, nBlockSize, hQ, hK, hV, hMask, hY, 1 if bBatchMask else 0])
 
     def AttnScaledDotProductBackward(self, hCuDnn, hAttn, hQ, hdQ, hK, hdK, hV, hdV, hMask, hY, hdY):
-        self._invoke(ids.CUDNN_FN_ATTN_BWD, None, [hCuDnn, hAttn, hQ, hdQ, hK, hdK, hV, hdV, hMask, hY, hdY])
+        self._call(ids.CUDNN_FN_ATTN_BWD, [hCuDnn, hAttn, hQ, hdQ, hK, hdK, hV, hdV, hMask, hY, hdY])
 
     # ------------------------------------------------------------------ LayerNorm (CudaDnn.cs:6307-6360)
     def CreateLayerNorm(self, nGpuID, nCount, nOuterNum, nChannels, nInnerNum, fEps=1e-10) -> int:
@@ -258,19 +287,19 @@ class CudaDnn:
         self._invoke(ids.CUDA_FN_FREE_LAYERNORM, [float(h)])
 
     def LayerNormForward(self, hLayerNorm, hXdata, hYdata):
-        self._invoke(ids.CUDA_FN_LAYERNORM_FWD, None, [hLayerNorm, hXdata, hYdata])
+        self._call(ids.CUDA_FN_LAYERNORM_FWD, [hLayerNorm, hXdata, hYdata])
 
     def LayerNormBackward(self, hLayerNorm, hYdata, hYdiff, hXdiff):
-        self._invoke(ids.CUDA_FN_LAYERNORM_BWD, None, [hLayerNorm, hYdata, hYdiff, hXdiff])
+        self._call(ids.CUDA_FN_LAYERNORM_BWD, [hLayerNorm, hYdata, hYdiff, hXdiff])
 
     # ------------------------------------------------------------------ RMSNorm layer (RMSNormLayer.cs:156-231)
     def RmsNormForward(self, hX, hW, hY, hInvRms, nRows, nInner, fEps=1e-5):
         """y = w * x / sqrt(mean(x^2) + eps) in one pass; hW = 0 for a layer without weights."""
-        self._invoke(ids.MCA_FN_RMSNORM_FWD, [float(fEps)], [hX, hW, hY, hInvRms, nRows, nInner])
+        self._call(ids.MCA_FN_RMSNORM_FWD, [hX, hW, hY, hInvRms, nRows, nInner], [float(fEps)])
 
     def RmsNormBackward(self, hX, hW, hdY, hInvRms, hdX, hdW, nRows, nInner):
         """dx (and dw unless hdW = 0) from dy and the 1/rms the forward saved."""
-        self._invoke(ids.MCA_FN_RMSNORM_BWD, None, [hX, hW, hdY, hInvRms, hdX, hdW, nRows, nInner])
+        self._call(ids.MCA_FN_RMSNORM_BWD, [hX, hW, hdY, hInvRms, hdX, hdW, nRows, nInner])
 
     # ------------------------------------------------------------------ RoPE (CudaDnn.cs:6375-6431)
     def CreateRope(self, nSharedIndex, nGpuID, nCount, nBatch, nSeqLen, nHeads, nDim, fTheta=10000.0) -> int:
@@ -281,10 +310,10 @@ class CudaDnn:
         self._invoke(ids.CUDA_FN_FREE_ROPE, [float(h)])
 
     def RopeForward(self, hRope, n, hX, hY, nFreqOffset=-1):
-        self._invoke(ids.CUDA_FN_ROPE_FWD, None, [hRope, n, hX, hY, nFreqOffset])
+        self._call(ids.CUDA_FN_ROPE_FWD, [hRope, n, hX, hY, nFreqOffset])
 
     def RopeBackward(self, hRope, n, hX, hYdiff, hXdiff):
-        self._invoke(ids.CUDA_FN_ROPE_BWD, None, [hRope, n, hX, hYdiff, hXdiff])
+        self._call(ids.CUDA_FN_ROPE_BWD, [hRope, n, hX, hYdiff, hXdiff])
 
     # ------------------------------------------------------------------ extensions: decode, TFT
     def CreateDecode(self, nBatch, nHeads, nKvHeads, nHeadSize, nSeqLen, bCacheBf16=False, fTheta=10000.0) -> int:
@@ -295,31 +324,31 @@ class CudaDnn:
         self._invoke(ids.MCA_FN_DECODE_FREE, [float(h)])
 
     def DecodeStep(self, hDecode, hQ, hKnew, hVnew, hKcache, hVcache, hPos, nMaxLen, hOut):
-        self._invoke(ids.MCA_FN_DECODE_STEP, None, [hDecode, hQ, hKnew, hVnew, hKcache, hVcache, hPos, nMaxLen, hOut])
+        self._call(ids.MCA_FN_DECODE_STEP, [hDecode, hQ, hKnew, hVnew, hKcache, hVcache, hPos, nMaxLen, hOut])
 
     def DecodeQkv(self, hX, hRmsW, hWq, hWk, hWv, nBatch, nDim, nKvDim, hQ, hK, hV, fEps=1e-5):
         """RMSNorm + q,k,v projections of the new token (llama2_gpu.cpp:56-61)."""
-        self._invoke(ids.MCA_FN_DECODE_QKV, [float(fEps)], [hX, hRmsW, hWq, hWk, hWv, nBatch, nDim, nKvDim, hQ, hK, hV])
+        self._call(ids.MCA_FN_DECODE_QKV, [hX, hRmsW, hWq, hWk, hWv, nBatch, nDim, nKvDim, hQ, hK, hV], [float(fEps)])
 
     def DecodeOut(self, hAttn, hWo, nBatch, nDim, hX):
         """x += Wo . attn (llama2_gpu.cpp:78-81)."""
-        self._invoke(ids.MCA_FN_DECODE_OUT, None, [hAttn, hWo, nBatch, nDim, hX])
+        self._call(ids.MCA_FN_DECODE_OUT, [hAttn, hWo, nBatch, nDim, hX])
 
     def DecodeFfn(self, hX, hRmsW, hW1, hW2, hW3, nBatch, nDim, nHiddenDim, hHidden, fEps=1e-5):
         """x += W2 . (silu(W1 xn) * (W3 xn)), xn = rmsnorm(x) (llama2_gpu.cpp:84-97)."""
-        self._invoke(ids.MCA_FN_DECODE_FFN, [float(fEps)], [hX, hRmsW, hW1, hW2, hW3, nBatch, nDim, nHiddenDim, hHidden])
+        self._call(ids.MCA_FN_DECODE_FFN, [hX, hRmsW, hW1, hW2, hW3, nBatch, nDim, nHiddenDim, hHidden], [float(fEps)])
 
     def DecodeLogits(self, hX, hRmsW, hWcls, nBatch, nDim, nVocab, hLogits, fEps=1e-5):
         """logits = Wcls . rmsnorm(x) (llama2_gpu.cpp:101-105)."""
-        self._invoke(ids.MCA_FN_DECODE_LOGITS, [float(fEps)], [hX, hRmsW, hWcls, nBatch, nDim, nVocab, hLogits])
+        self._call(ids.MCA_FN_DECODE_LOGITS, [hX, hRmsW, hWcls, nBatch, nDim, nVocab, hLogits], [float(fEps)])
 
     def AttnScaledDotProductForwardPacked(self, hCuDnn, hAttn, nBlockSize, hQKV, hMask, hY, bBatchMask=False):
         """ATTN_FWD on the (B,T,3C) c_attn output: q, k, v are read in place, y is written as (B,T,C)."""
-        self._invoke(ids.MCA_FN_ATTN_FWD_PACKED, None,
+        self._call(ids.MCA_FN_ATTN_FWD_PACKED,
                      [hCuDnn, hAttn, nBlockSize, hQKV, hMask, hY, 1 if bBatchMask else 0])
 
     def AttnScaledDotProductBackwardPacked(self, hCuDnn, hAttn, hQKV, hdQKV, hMask, hY, hdY):
-        self._invoke(ids.MCA_FN_ATTN_BWD_PACKED, None, [hCuDnn, hAttn, hQKV, hdQKV, hMask, hY, hdY])
+        self._call(ids.MCA_FN_ATTN_BWD_PACKED, [hCuDnn, hAttn, hQKV, hdQKV, hMask, hY, hdY])
 
     def AttnForwardHost(self, q, k, v, y, bCausal, nHeadsPerChunk=0):
         """Forward for (B,H,T,D) numpy tensors in host memory (float32, or bf16 bit patterns as uint16),
@@ -334,8 +363,8 @@ class CudaDnn:
                       int(nHeadsPerChunk)])
 
     def TftAttnBackward(self, hQ, hK, hV, hMask, hdOut, hdAttn, nBatch, nHeads, nQ, nK, nDim, hdQ, hdK, hdV):
-        self._invoke(ids.MCA_FN_TFT_ATTN_BWD, None,
+        self._call(ids.MCA_FN_TFT_ATTN_BWD,
                      [hQ, hK, hV, hMask, hdOut, hdAttn, nBatch, nHeads, nQ, nK, nDim, hdQ, hdK, hdV])
 
     def TftAttnForward(self, hQ, hK, hV, hMask, nBatch, nHeads, nQ, nK, nDim, hOut, hAttn):
-        self._invoke(ids.MCA_FN_TFT_ATTN_FWD, None, [hQ, hK, hV, hMask, nBatch, nHeads, nQ, nK, nDim, hOut, hAttn])
+        self._call(ids.MCA_FN_TFT_ATTN_FWD, [hQ, hK, hV, hMask, nBatch, nHeads, nQ, nK, nDim, hOut, hAttn])
