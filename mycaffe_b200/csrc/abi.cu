@@ -16,6 +16,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "classify.cuh"
 #include "common.cuh"
 #include "kernels.h"
 
@@ -467,8 +468,8 @@ long attn_set(Kernel* k, long lInput, float* pf, long llInput, MCA_LONGLONG* pl)
 // freed it and been given the same address again, so nothing about it is remembered between calls.
 constexpr long kMaskClassMiss = -7001;   // internal: the class assumed for this call's kernels was wrong
 
-long resolve_mask(Kernel* k, AttnHandle& a, long hMask, bool batch_mask, int T, const float** mask, int* mode,
-                  bool need_host_answer, bool may_speculate = false) {
+// The mask and its mode before any classification: a (T,T) mask comes out as MCA_MASK_TT.
+long look_up_mask(Kernel* k, const AttnHandle& a, long hMask, bool batch_mask, int T, const float** mask, int* mode) {
   *mask = nullptr;
   if (a.flags & MCA_FLAG_CAUSAL_IMPLICIT) { *mode = MCA_MASK_CAUSAL; return 0; }
   if (hMask == 0) { *mode = MCA_MASK_NONE; return 0; }
@@ -476,35 +477,50 @@ long resolve_mask(Kernel* k, AttnHandle& a, long hMask, bool batch_mask, int T, 
   long e = check_f32(k, hMask, batch_mask ? (int64_t)a.B * T : (int64_t)T * T, &m);
   if (e) return e;
   *mask = m;
-  if (batch_mask) { *mode = MCA_MASK_BATCH; return 0; }
-  *mode = MCA_MASK_TT;
-  // The class goes to a pinned host word as well, tagged with this classification's number.
-  if (need_host_answer && k->answer_words() == nullptr) return ERROR_MEMORY_OUT;
+  *mode = batch_mask ? MCA_MASK_BATCH : MCA_MASK_TT;
+  return 0;
+}
+
+// A classification of `mask` whose answer goes to the handle's device flag and, tagged with this classification's number,
+// to the kernel index's pinned word.
+long new_class_job(Kernel* k, AttnHandle& a, const float* mask, int T, McaClassifyJob* job) {
+  if (k->answer_words() == nullptr) return ERROR_MEMORY_OUT;
   k->class_tag = (k->class_tag + 2) & 0x3ffffffe;
   k->synced = false;
-  if ((e = mca_classify_causal_mask_ws(m, T, a.causal_flag, need_host_answer ? k->h_answer : nullptr, k->class_tag, a.causal_flag + 6, 0)))
-    return e;
-  if (need_host_answer && may_speculate && !k->async && a.spec_allowed && a.spec_class >= 0) {
+  *job = McaClassifyJob{mask, T, a.causal_flag, k->h_answer, k->class_tag, a.causal_flag + 6};
+  return 0;
+}
+
+// After the job has been launched: the mode its kernels are chosen on.
+long settle_mask_mode(Kernel* k, AttnHandle& a, bool may_speculate, int* mode) {
+  if (may_speculate && !k->async && a.spec_allowed && a.spec_class >= 0) {
     a.spec_pending = true;
     a.spec_assumed = a.spec_class;
     if (a.spec_class == 1) *mode = MCA_MASK_CAUSAL;
     return 0;
   }
-  if (need_host_answer) {
-    // Poll the word: it arrives a microsecond after the kernel has written it, where a copy back and a stream
-    // synchronisation left the GPU idle for twenty.  The polling is bounded; a long queue ahead of the classification
-    // is waited for by a synchronisation.
-    const auto t0 = std::chrono::steady_clock::now();
-    while (k->answered_class() < 0 && std::chrono::steady_clock::now() - t0 < std::chrono::milliseconds(2)) {
-    }
-    if (k->answered_class() < 0) {
-      const cudaError_t ce = cudaStreamSynchronize(0);
-      if (ce != cudaSuccess) return ce;
-    }
-    a.spec_class = k->answered_class() == 1 ? 1 : 0;
-    if (a.spec_class == 1) *mode = MCA_MASK_CAUSAL;
+  // Poll the word: it arrives a microsecond after the kernel has written it, where a copy back and a stream
+  // synchronisation left the GPU idle for twenty.  The polling is bounded; a long queue ahead of the classification
+  // is waited for by a synchronisation.
+  const auto t0 = std::chrono::steady_clock::now();
+  while (k->answered_class() < 0 && std::chrono::steady_clock::now() - t0 < std::chrono::milliseconds(2)) {
   }
+  if (k->answered_class() < 0) {
+    const cudaError_t ce = cudaStreamSynchronize(0);
+    if (ce != cudaSuccess) return ce;
+  }
+  a.spec_class = k->answered_class() == 1 ? 1 : 0;
+  if (a.spec_class == 1) *mode = MCA_MASK_CAUSAL;
   return 0;
+}
+
+long resolve_mask(Kernel* k, AttnHandle& a, long hMask, bool batch_mask, int T, const float** mask, int* mode,
+                  bool need_host_answer, bool may_speculate = false) {
+  long e = look_up_mask(k, a, hMask, batch_mask, T, mask, mode);
+  if (e || *mode != MCA_MASK_TT) return e;
+  McaClassifyJob job;
+  if ((e = new_class_job(k, a, *mask, T, &job)) || (e = mca_classify_causal_mask_ws(&job, 0))) return e;
+  return need_host_answer ? settle_mask_mode(k, a, may_speculate, mode) : 0;
 }
 
 // Keep-bits of this call's (T,T) or batch mask, packed into buffers the handle owns (room for the configured block
@@ -639,25 +655,36 @@ long attn_fwd_once(Kernel* k, long llInput, MCA_LONGLONG* pl, int layout) {
         (e = check_f32(k, (long)pl[5], n_in, &v)) || (e = check_f32(k, (long)pl[7], n, &y)))
       return e;
     if (packed) { kk += C; v += 2 * C; }
-    const bool split_path = a.split_ws != nullptr && (mca_sdpa_backward_f32_tc_supported(a.D) != 0 || !a.training);
-    if ((e = resolve_mask(k, a, (long)pl[6], batch_mask, T, &mask, &mode, a.split_ws != nullptr, split_path))) return e;
     const bool save = a.training && T == a.block;
-    const bool bits = mode == MCA_MASK_TT || mode == MCA_MASK_BATCH;   // packed for the kernel; causal / none need nothing
     // Head sizes with a tensor-core forward but no tensor-core backward (128): the forward leaves the row statistics
     // the exact fp32 backward recomputes the probabilities from; a saved forward under a general or batch mask keeps
     // to the exact kernels, whose masked-row convention that backward shares.
     const bool tc_bwd = mca_sdpa_backward_f32_tc_supported(a.D) != 0;
-    if (a.split_ws != nullptr && (tc_bwd || !save || !bits)) {
-      if (bits && (e = pack_mask_bits(a, mask, mode, T))) return e;
-      const bool stats = save && !tc_bwd;
-      e = mca_sdpa_forward_f32_tc_masked(q, kk, v, mode == MCA_MASK_CAUSAL, a.B, a.H, T, a.D, y, stats ? a.row_max : nullptr,
-                                         stats ? a.row_sum : nullptr, save ? a.y_copy : nullptr, save && tc_bwd ? a.lse : nullptr,
-                                         a.split_ws, a.split_ws_bytes, a.causal_flag + 1, layout, bits ? a.mask_bits : nullptr,
-                                         bits ? mode : MCA_MASK_NONE, 0);
-      if (e) return e;
-      if (save) { remember_forward(a, T, mode, layout, 0, false); a.fwd_split = tc_bwd; }
-      return tc_status(k, a);
+    if ((e = look_up_mask(k, a, (long)pl[6], batch_mask, T, &mask, &mode))) return e;
+    const bool classify = mode == MCA_MASK_TT;
+    McaClassifyJob job;
+    if (classify && (e = new_class_job(k, a, mask, T, &job))) return e;
+    bool classified = !classify;
+    if (a.split_ws != nullptr && (tc_bwd || !save || mode != MCA_MASK_BATCH)) {
+      // the operands are split first, with the mask's classification in the same launch; where its answer has to be waited
+      // for, the GPU is busy meanwhile
+      if ((e = mca_split_forward_prepass(q, kk, v, a.B, a.H, T, a.D, a.split_ws, a.split_ws_bytes, layout, classify ? &job : nullptr, 0)))
+        return e;
+      if (classify && (e = settle_mask_mode(k, a, tc_bwd || !a.training, &mode))) return e;
+      classified = true;
+      const bool bits = mode == MCA_MASK_TT || mode == MCA_MASK_BATCH;   // packed for the kernel; causal / none need nothing
+      if (tc_bwd || !save || !bits) {
+        if (bits && (e = pack_mask_bits(a, mask, mode, T))) return e;
+        const bool stats = save && !tc_bwd;
+        e = mca_split_forward_main(mode == MCA_MASK_CAUSAL, a.B, a.H, T, a.D, y, stats ? a.row_max : nullptr,
+                                   stats ? a.row_sum : nullptr, save ? a.y_copy : nullptr, save && tc_bwd ? a.lse : nullptr, a.split_ws,
+                                   a.causal_flag + 1, layout, bits ? a.mask_bits : nullptr, bits ? mode : MCA_MASK_NONE, 0);
+        if (e) return e;
+        if (save) { remember_forward(a, T, mode, layout, 0, false); a.fwd_split = tc_bwd; }
+        return tc_status(k, a);
+      }
     }
+    if (!classified && (e = mca_classify_causal_mask_ws(&job, 0))) return e;
     e = mca_sdpa_forward_f32_layout(q, kk, v, mask, mode, a.causal_flag, a.B, a.H, T, a.D, y, save ? a.row_max : nullptr,
                                     save ? a.row_sum : nullptr, save ? a.y_copy : nullptr, layout, 0);
     if (!e && save) remember_forward(a, T, mode, layout, (long)pl[6], batch_mask);

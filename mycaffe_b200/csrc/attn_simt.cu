@@ -24,6 +24,7 @@
 // fp32 pipe: two warps per scheduler do not hide every load); B = 1, H = 12, T = 1516, D = 80 forward and backward: 1.75 -> 0.78 ms.
 #include <algorithm>
 
+#include "classify.cuh"
 #include "common.cuh"
 #include "kernels.h"
 
@@ -508,36 +509,9 @@ __global__ void classify_causal_kernel(const float* __restrict__ mask, int T, in
 }
 __global__ void set_int_kernel(int* p, int v) { *p = v; }
 
-// The same answer from one launch: a warp per row (16-byte loads when T allows), the blocks' mismatch counts and a
-// ticket in two scratch words that are zero before and after; the last block to finish writes the flag.
-__global__ void __launch_bounds__(256) classify_causal_rows_kernel(const float* __restrict__ mask, int T, int* __restrict__ flag,
-                                                                   int* __restrict__ host_flag, int host_base, int* __restrict__ scratch) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  bool bad = false;
-  for (int i = blockIdx.x * 8 + warp; i < T; i += gridDim.x * 8) {
-    const float* row = mask + (int64_t)i * T;
-    if ((T & 3) == 0) {
-      for (int j = lane * 4; j < T; j += 128) {
-        const float4 m = *reinterpret_cast<const float4*>(row + j);
-        bad |= m.x != (j <= i ? 1.f : 0.f) || m.y != (j + 1 <= i ? 1.f : 0.f) || m.z != (j + 2 <= i ? 1.f : 0.f) ||
-               m.w != (j + 3 <= i ? 1.f : 0.f);
-      }
-    } else {
-      for (int j = lane; j < T; j += 32) bad |= row[j] != (j <= i ? 1.f : 0.f);
-    }
-  }
-  const int any_bad = __syncthreads_or(bad ? 1 : 0);
-  if (threadIdx.x == 0) {
-    if (any_bad) atomicAdd(scratch, 1);
-    __threadfence();
-    if (atomicAdd(scratch + 1, 1) == (int)gridDim.x - 1) {
-      __threadfence();
-      const int causal = atomicExch(scratch, 0) == 0 ? 1 : 0;
-      *flag = causal;
-      if (host_flag != nullptr) *host_flag = host_base + causal;   // pinned host memory: read behind the next stream synchronisation
-      scratch[1] = 0;
-    }
-  }
+// The same answer from one launch (mca_classify_rows).
+__global__ void __launch_bounds__(256) classify_causal_rows_kernel(const McaClassifyJob job) {
+  mca_classify_rows(job, (int)blockIdx.x, (int)gridDim.x);
 }
 
 // The padded head size: what lies between two of these costs its zeros in every product (48 as 64 a third more work, 80 as
@@ -569,11 +543,10 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 
 }  // namespace
 
-int mca_classify_causal_mask_ws(const float* mask, int T, int* flag, int* host_flag, int host_base, int* scratch, void* stream) {
-  if (!mask || !flag || !scratch) return ERROR_PARAM_NULL;
-  if (T <= 0) return ERROR_PARAM_OUT_OF_RANGE;
-  const int blocks = std::min(1184, (T + 7) / 8);
-  classify_causal_rows_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(mask, T, flag, host_flag, host_base, scratch);
+int mca_classify_causal_mask_ws(const McaClassifyJob* job, void* stream) {
+  if (!job->mask || !job->flag || !job->scratch) return ERROR_PARAM_NULL;
+  if (job->T <= 0) return ERROR_PARAM_OUT_OF_RANGE;
+  classify_causal_rows_kernel<<<std::min(1184, (job->T + 7) / 8), 256, 0, (cudaStream_t)stream>>>(*job);
   return mca_launch_status();
 }
 

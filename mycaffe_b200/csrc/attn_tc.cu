@@ -149,9 +149,9 @@ struct TcParams {
   McaStrides ys;     // element strides of the output view
   void* y_more[7];   // further destinations of the same bf16 output tile (peer GPUs' buffers), same strides
   int n_more;
-  // MODE_SPLIT: the pre-pass's scale factors (split::SplitFac, device memory); exact softmax statistics for
+  // MODE_SPLIT: the pre-pass's scales of q, k, v of each (batch, head); exact softmax statistics for
   // the fp32 backward: row_max in natural-log units of the scaled logits and the matching row sum, (B*H, T) each
-  const float* split_fac;
+  const float4* split_scale;
   float* row_max;
   float* row_sum;
   float* y_copy;      // second copy of the fp32 output, (B*H, T, HD) contiguous, or null
@@ -448,7 +448,9 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     float m_used[2] = {-INFINITY, -INFINITY};
     float l[2] = {0.f, 0.f};                            // this thread's part of the row sums
     // split mode: the pre-pass scaled q and k by powers of two; dividing them out of the logit scale is exact
-    const float scale_log2 = SPLIT ? p.scale_log2 * __ldg(p.split_fac + split::FAC_INV_QK) : p.scale_log2;
+    float4 sc = make_float4(1.f, 1.f, 1.f, 1.f);
+    if constexpr (SPLIT) sc = __ldg(p.split_scale + bh);
+    const float scale_log2 = SPLIT ? p.scale_log2 * (1.0f / (sc.x * sc.y)) : p.scale_log2;
     for (int j = 0; j < n && ok; ++j) {
       TC_TRACE(x, j, 0);
       ok = __all_sync(0xffffffffu, mbar_wait_hot(bar(BAR_S_FULL + x), (uint32_t)(j & 1), p.status, 30 + x, j));
@@ -636,7 +638,7 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         const int qi = qrow0 + row;
         const float lsum = red_l[row];
         // split mode: the pre-pass scaled v by a power of two; dividing it out here is exact
-        const float inv = SPLIT ? __ldg(p.split_fac + split::FAC_INV_V) / lsum : 1.0f / lsum;
+        const float inv = SPLIT ? (1.0f / __ldg(p.split_scale + bh).z) / lsum : 1.0f / lsum;
         const uint32_t t_o32 = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(QT * BLK + x * BLK + half * OC);
         if constexpr (F32_OUT && QT == 2) {
           // fp32 output of the two-tile shape: each thread stores its own row's pieces.  (Staged like the other
@@ -749,7 +751,7 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 
 
 struct SplitExtras {
-  const float* fac = nullptr;   // split::SplitFac
+  const float4* scale = nullptr;   // of q, k, v of each (batch, head)
   float *row_max = nullptr, *row_sum = nullptr, *y_copy = nullptr;
 };
 
@@ -832,7 +834,7 @@ int launch_tc(const void* q, const void* k, const void* v, int causal, int B, in
   p.n_more = n_more;
   for (int i = 0; i < 7; ++i) p.y_more[i] = i < n_more ? y_more[i] : nullptr;
   p.scale_log2 = (1.0f / sqrtf((float)HD)) * 1.4426950408889634f;
-  p.split_fac = split ? split->fac : nullptr;
+  p.split_scale = split ? split->scale : nullptr;
   p.row_max = split ? split->row_max : nullptr;
   p.row_sum = split ? split->row_sum : nullptr;
   p.y_copy = split ? split->y_copy : nullptr;
@@ -845,19 +847,22 @@ int launch_tc(const void* q, const void* k, const void* v, int causal, int B, in
   return launch_shape<HD, MODE, false>(mq, mk, mv, p, B, H, T, mask != nullptr, st);
 }
 
+// The two halves of a split-operand forward: the pre-pass (which also classifies a (T,T) mask when asked to), and the kernel.
 template <int HD>
-int launch_split(const float* q, const float* k, const float* v, int causal, int B, int H, int T, float* y, float* row_max,
-                 float* row_sum, float* y_copy, float* lse, void* workspace, int* status, int layout, cudaStream_t st,
-                 const McaMaskBits* mask = nullptr) {
-  const int64_t rows = (int64_t)B * H * T;
-  const split::Workspace w = split::carve(workspace, rows, HD);
+int split_prepass(const float* q, const float* k, const float* v, int B, int H, int T, void* workspace, int layout, cudaStream_t st,
+                  const McaClassifyJob* cls) {
+  const split::Workspace w = split::carve(workspace, (int64_t)B * H, T, HD);
   split::Job job;
   job.src[0] = q; job.src[1] = k; job.src[2] = v;
   for (int i = 0; i < 3; ++i) { job.dst[i] = w.tensor[i]; job.slot[i] = i; }
-  int e = split::run<HD>(job, 3, mca_in_strides(layout, H, T, HD), H, T, rows, w, false, st);
-  if (e) return e;
+  return split::run<HD>(job, 3, mca_in_strides(layout, H, T, HD), B, H, T, w, st, nullptr, nullptr, cls);
+}
+template <int HD>
+int split_main(int causal, int B, int H, int T, float* y, float* row_max, float* row_sum, float* y_copy, float* lse, void* workspace,
+               int* status, int layout, cudaStream_t st, const McaMaskBits* mask) {
+  const split::Workspace w = split::carve(workspace, (int64_t)B * H, T, HD);
   SplitExtras ex;
-  ex.fac = w.fac; ex.row_max = row_max; ex.row_sum = row_sum; ex.y_copy = y_copy;
+  ex.scale = w.scale; ex.row_max = row_max; ex.row_sum = row_sum; ex.y_copy = y_copy;
   return launch_tc<HD, MODE_SPLIT>(w.tensor[0], w.tensor[1], w.tensor[2], causal, B, H, T, y, lse, status, layout, st, nullptr, 0,
                                    nullptr, &ex, mask);
 }
@@ -954,12 +959,12 @@ int mca_tc_narrow_len(int len) {
 
 int64_t mca_sdpa_forward_f32_tc_workspace_bytes(int B, int H, int T) {
   if (B <= 0 || H <= 0 || T <= 0) return -1;
-  return split::workspace_bytes((int64_t)B * H * T);
+  return split::workspace_bytes((int64_t)B * H, T);
 }
 
 int64_t mca_sdpa_forward_f32_tc_workspace_bytes_d(int B, int H, int T, int D) {
   if (B <= 0 || H <= 0 || T <= 0 || !mca_sdpa_forward_f32_tc_supported(D)) return -1;
-  return split::workspace_bytes((int64_t)B * H * T, D);
+  return split::workspace_bytes((int64_t)B * H, T, D);
 }
 
 int mca_sdpa_forward_f32_tc_supported(int D) { return D == 16 || D == 32 || D == 64 || D == 128; }
@@ -977,30 +982,56 @@ int mca_sdpa_forward_f32_tc_masked(const float* q, const float* k, const float* 
                                    float* y, float* row_max, float* row_sum, float* y_copy, float* lse, void* workspace,
                                    int64_t workspace_bytes, int* status, int layout, const uint32_t* mask_bits, int mask_mode,
                                    void* stream) {
+  // everything is checked before the pre-pass writes anything
+  if (!q || !k || !v || !y || !status || !workspace) return ERROR_PARAM_NULL;
   McaMaskBits mb;
   const McaMaskBits* mask = nullptr;
-  int me = mca_mask_bits_view(mask_bits, nullptr, mask_mode, T, false, &mb, &mask);
-  if (me) return me;
-  if (layout != MCA_LAYOUT_BHTD && layout != MCA_LAYOUT_PACKED) return ERROR_PARAM_OUT_OF_RANGE;
-  if (!q || !k || !v || !y || !status || !workspace) return ERROR_PARAM_NULL;
+  int e = mca_mask_bits_view(mask_bits, nullptr, mask_mode, T, false, &mb, &mask);
+  if (e) return e;
+  if (mask != nullptr && causal) return ERROR_ATTN_UNSUPPORTED_SHAPE;
   if ((row_max == nullptr) != (row_sum == nullptr)) return ERROR_PARAM_NULL;
+  if ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(y_copy)) & 15) return ERROR_PARAM_OUT_OF_RANGE;
+  if ((e = mca_split_forward_prepass(q, k, v, B, H, T, D, workspace, workspace_bytes, layout, nullptr, stream))) return e;
+  return mca_split_forward_main(causal, B, H, T, D, y, row_max, row_sum, y_copy, lse, workspace, status, layout, mask_bits, mask_mode,
+                                stream);
+}
+
+int mca_split_forward_prepass(const float* q, const float* k, const float* v, int B, int H, int T, int D, void* workspace,
+                              int64_t workspace_bytes, int layout, const McaClassifyJob* cls, void* stream) {
+  if (layout != MCA_LAYOUT_BHTD && layout != MCA_LAYOUT_PACKED) return ERROR_PARAM_OUT_OF_RANGE;
+  if (!q || !k || !v || !workspace) return ERROR_PARAM_NULL;
   if (B <= 0 || H <= 0 || T <= 0 || (int64_t)B * H > 65535) return ERROR_PARAM_OUT_OF_RANGE;
   if (!mca_sdpa_forward_f32_tc_supported(D)) return ERROR_ATTN_UNSUPPORTED_SHAPE;
   if (workspace_bytes < mca_sdpa_forward_f32_tc_workspace_bytes_d(B, H, T, D)) return ERROR_ATTN_SCRATCH_TOO_SMALL;
-  if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
-       reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(y_copy)) & 15)
-    return ERROR_PARAM_OUT_OF_RANGE;
+  if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) & 15) return ERROR_PARAM_OUT_OF_RANGE;
   if (reinterpret_cast<uintptr_t>(workspace) & 15) return ERROR_PARAM_OUT_OF_RANGE;
   cudaStream_t st = (cudaStream_t)stream;
   switch (D) {
-    case 16: return launch_split<16>(q, k, v, causal, B, H, T, y, row_max, row_sum, y_copy, lse, workspace, status, layout, st, mask);
-    case 32: return launch_split<32>(q, k, v, causal, B, H, T, y, row_max, row_sum, y_copy, lse, workspace, status, layout, st, mask);
-    case 64: return launch_split<64>(q, k, v, causal, B, H, T, y, row_max, row_sum, y_copy, lse, workspace, status, layout, st, mask);
-    case 128: return launch_split<128>(q, k, v, causal, B, H, T, y, row_max, row_sum, y_copy, lse, workspace, status, layout, st, mask);
+    case 16: return split_prepass<16>(q, k, v, B, H, T, workspace, layout, st, cls);
+    case 32: return split_prepass<32>(q, k, v, B, H, T, workspace, layout, st, cls);
+    case 64: return split_prepass<64>(q, k, v, B, H, T, workspace, layout, st, cls);
+    case 128: return split_prepass<128>(q, k, v, B, H, T, workspace, layout, st, cls);
   }
   return ERROR_ATTN_UNSUPPORTED_SHAPE;
 }
 
+int mca_split_forward_main(int causal, int B, int H, int T, int D, float* y, float* row_max, float* row_sum, float* y_copy, float* lse,
+                           void* workspace, int* status, int layout, const uint32_t* mask_bits, int mask_mode, void* stream) {
+  McaMaskBits mb;
+  const McaMaskBits* mask = nullptr;
+  int e = mca_mask_bits_view(mask_bits, nullptr, mask_mode, T, false, &mb, &mask);
+  if (e) return e;
+  if (!y || !status) return ERROR_PARAM_NULL;
+  if ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(y_copy)) & 15) return ERROR_PARAM_OUT_OF_RANGE;
+  cudaStream_t st = (cudaStream_t)stream;
+  switch (D) {
+    case 16: return split_main<16>(causal, B, H, T, y, row_max, row_sum, y_copy, lse, workspace, status, layout, st, mask);
+    case 32: return split_main<32>(causal, B, H, T, y, row_max, row_sum, y_copy, lse, workspace, status, layout, st, mask);
+    case 64: return split_main<64>(causal, B, H, T, y, row_max, row_sum, y_copy, lse, workspace, status, layout, st, mask);
+    case 128: return split_main<128>(causal, B, H, T, y, row_max, row_sum, y_copy, lse, workspace, status, layout, st, mask);
+  }
+  return ERROR_ATTN_UNSUPPORTED_SHAPE;
+}
 
 // ---------------------------------------------------------------------------------------------
 // Keep-bits of a float mask for the tensor-core kernels.  One warp per output word: bit i of word w of row r is

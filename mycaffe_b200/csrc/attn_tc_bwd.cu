@@ -75,7 +75,7 @@ __device__ __forceinline__ void split_pack(float v0, float v1, uint32_t& hi, uin
 constexpr float DS_SHIFT = 1.0f / 524288.0f, DS_UNSHIFT = 524288.0f, PT_SHIFT = 1024.0f, PT_UNSHIFT = 1.0f / 1024.0f;
 
 struct BwdParams {
-  const float* fac;    // split mode: the pre-pass's scale factors (split::SplitFac), device memory
+  const float4* scales;   // split mode: the pre-pass's scales (q, k, v, dY) of each (batch, head)
   const float* lse;    // (BH, T) log2-domain log-sum-exp of the scaled logits, from the forward kernel
   const float* delta;  // (BH, T) rowsum(dY o Y)
   void* out0;          // dq kernel: dQ;  dkdv kernel: dK
@@ -343,6 +343,11 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     const bool row_ok = qi < T;
     const float lse = row_ok ? p.lse[(int64_t)bh * T + qi] : 0.f;
     const float delta = row_ok ? p.delta[(int64_t)bh * T + qi] : 0.f;
+    float4 sc = make_float4(1.f, 1.f, 1.f, 1.f);   // powers of two: every product and quotient of them is exact
+    if constexpr (SPLIT) sc = __ldg(p.scales + bh);
+    const float sl2 = SPLIT ? p.scale_log2 * (1.0f / (sc.x * sc.y)) : p.scale_log2;
+    const float dmul = SPLIT ? DS_SHIFT : p.scale;
+    const float dsub = SPLIT ? delta * (sc.w * DS_SHIFT) * sc.z : delta * p.scale;
     for (int j = 0; j < n && ok; ++j) {
       ok = __all_sync(0xffffffffu, mbar_wait(bar(DQ_SDP_FULL), (uint32_t)(j & 1), p.status, 130, j));
       if (!ok) break;
@@ -365,9 +370,6 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       // dS = P o (dP - delta) scale with P = 2^(S scale_log2 - lse); adjacent keys go through as fp32 pairs.
       // Split mode: S and dP carry the pre-pass's scales; dS is kept in the units of dP' x 2^-19 and the factor
       // scale x 2^19 / (s_dy s_v s_k) is applied once to dQ.
-      const float sl2 = SPLIT ? p.scale_log2 * __ldg(p.fac + split::FAC_INV_QK) : p.scale_log2;
-      const float dmul = SPLIT ? DS_SHIFT : p.scale;
-      const float dsub = SPLIT ? delta * __ldg(p.fac + split::FAC_DYV) * DS_SHIFT : delta * p.scale;
       const float2 sc2 = make_float2(sl2, sl2), nl2 = make_float2(-lse, -lse);
       const float2 ps2 = make_float2(dmul, dmul), nd2 = make_float2(-dsub, -dsub);
       const float2 zero2 = make_float2(0.f, 0.f);
@@ -410,7 +412,7 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     const bool fin = ok && n > 0;
     if (fin) {
       tc_fence_after();
-      const float mul = SPLIT ? p.scale * DS_UNSHIFT * __ldg(p.fac + split::FAC_INV_DYVK) : 1.0f;
+      const float mul = SPLIT ? p.scale * DS_UNSHIFT * (1.0f / (sc.z * sc.y)) * (1.0f / sc.w) : 1.0f;
       stage_columns<PR, OC, SPLIT>(tile, row, qtr, t_row + C_DQ + qtr * OC, mul);
     }
     ew_bar_sync();
@@ -655,9 +657,11 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     float (*s_nlse)[BLK] = reinterpret_cast<float (*)[BLK]>(smem_gen + PL::OFF_STAGE_KV);
     float (*s_del)[BLK] = s_nlse + 2;
     // split mode: S^T and dP^T carry the pre-pass's scales; dS^T is kept in the units of dP' x 2^-19 and P^T 2^10 larger
-    const float sl2 = SPLIT ? p.scale_log2 * __ldg(p.fac + split::FAC_INV_QK) : p.scale_log2;
+    float4 sc = make_float4(1.f, 1.f, 1.f, 1.f);
+    if constexpr (SPLIT) sc = __ldg(p.scales + bh);
+    const float sl2 = SPLIT ? p.scale_log2 * (1.0f / (sc.x * sc.y)) : p.scale_log2;
     const float dmul = SPLIT ? DS_SHIFT : p.scale;
-    const float del_mul = SPLIT ? __ldg(p.fac + split::FAC_DYV) * DS_SHIFT : p.scale;
+    const float del_mul = SPLIT ? (sc.w * DS_SHIFT) * sc.z : p.scale;
     auto fetch = [&](int it) -> float {
       const int qi = (i_begin + it) * BLK + (tid & (BLK - 1));
       if (tid >= 2 * BLK || it >= n || qi >= T) return tid < BLK ? -INFINITY : 0.f;
@@ -766,8 +770,8 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     const bool fin = ok && n > 0;
     if (fin) {
       tc_fence_after();
-      const float mul_k = SPLIT ? p.scale * DS_UNSHIFT * __ldg(p.fac + split::FAC_INV_DYVQ) : 1.0f;
-      const float mul_v = SPLIT ? PT_UNSHIFT * __ldg(p.fac + split::FAC_INV_DY) : 1.0f;
+      const float mul_k = SPLIT ? p.scale * DS_UNSHIFT * (1.0f / (sc.z * sc.x)) * (1.0f / sc.w) : 1.0f;
+      const float mul_v = SPLIT ? PT_UNSHIFT * (1.0f / sc.w) : 1.0f;
       stage_columns<PR, OC, SPLIT>(tile_k, row, qtr, t_row + C_DK + qtr * OC, mul_k);
       stage_columns<PR, OC, SPLIT>(tile_v, row, qtr, t_row + C_DV + qtr * OC, mul_v);
     }
@@ -848,7 +852,7 @@ int launch_bwd(const void* q, const void* k, const void* v, const void* dy, cons
       (e = make_map_bf16(&mv, v, B, H, T, HD, sin)) || (e = make_map_bf16(&mdo, dy, B, H, T, HD, sout)))
     return e;
   BwdParams p;
-  p.fac = nullptr;
+  p.scales = nullptr;
   p.lse = lse; p.delta = delta; p.status = status; p.T = T; p.causal = causal; p.H = H;
   {
     // Q, K, V, dY of one (batch, head): keep a group's set under about 64 MB of the 126 MB L2
@@ -870,14 +874,13 @@ int launch_bwd_split(const float* dy, const float* y_copy, const float* lse, flo
                      float* dq, float* dk, float* dv, void* workspace, int* status, int layout, cudaStream_t st,
                      const McaMaskBits* mask = nullptr) {
   if (mask != nullptr && causal) return ERROR_ATTN_UNSUPPORTED_SHAPE;
-  const int64_t rows = (int64_t)B * H * T;
-  const split::Workspace w = split::carve(workspace, rows);
+  const split::Workspace w = split::carve(workspace, (int64_t)B * H, T);
   const McaStrides sin = mca_in_strides(layout, H, T, HD), sout = mca_out_strides(layout, H, T, HD);
   split::Job job;
   job.src[0] = dy; job.dst[0] = w.tensor[split::TENSOR_DY]; job.slot[0] = split::TENSOR_DY;
   job.src[1] = job.src[2] = nullptr; job.dst[1] = job.dst[2] = nullptr; job.slot[1] = job.slot[2] = 0;
   // the kernel that splits dY also forms delta = rowsum(dY o Y) from the elements it holds
-  int e = split::run<HD>(job, 1, sout, H, T, rows, w, true, st, y_copy, delta);
+  int e = split::run<HD>(job, 1, sout, B, H, T, w, st, y_copy, delta);
   if (e) return e;
   CUtensorMap mq, mk, mv, mdo;
   const McaStrides sp{(int64_t)H * T * 128, (int64_t)T * 128, 128};
@@ -887,7 +890,7 @@ int launch_bwd_split(const float* dy, const float* y_copy, const float* lse, flo
                          CU_TENSOR_MAP_SWIZZLE_128B)))
       return e;
   BwdParams p;
-  p.fac = w.fac;
+  p.scales = w.scale;
   p.lse = lse; p.delta = delta; p.status = status; p.T = T; p.causal = causal; p.H = H;
   {
     const int64_t g = (64ll << 20) / ((int64_t)4 * T * 256);

@@ -132,6 +132,10 @@ static inline int mca_smem_once(std::atomic<uint64_t>& done, F kern, size_t byte
 __device__ __forceinline__ void mca_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void mca_pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+inline bool mca_plain_launches() {   // MCA_NO_PDL: every launch the ordinary way (for comparisons)
+  static const bool plain = getenv("MCA_NO_PDL") != nullptr;
+  return plain;
+}
 template <typename... KArgs, typename... Args>
 static inline int mca_launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
   cudaLaunchConfig_t cfg = {};
@@ -139,8 +143,20 @@ static inline int mca_launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, 
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
-  static const bool plain = getenv("MCA_NO_PDL") != nullptr;   // every launch the ordinary way (for comparisons)
-  cfg.attrs = attr; cfg.numAttrs = plain ? 0 : 1;
+  cfg.attrs = attr; cfg.numAttrs = mca_plain_launches() ? 0 : 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+  if (e != cudaSuccess) { cudaGetLastError(); return (int)e; }
+  return mca_launch_status();
+}
+// The same with clusters of `ctas` CTAs along x.
+template <typename... KArgs, typename... Args>
+static inline int mca_launch_pdl_cluster(void (*kern)(KArgs...), cudaLaunchConfig_t cfg, int ctas, Args... args) {
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)ctas; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = mca_plain_launches() ? 1 : 2;
   cudaError_t e = cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
   if (e != cudaSuccess) { cudaGetLastError(); return (int)e; }
   return mca_launch_status();

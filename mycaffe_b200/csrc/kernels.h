@@ -7,10 +7,16 @@ struct McaMaskBits;
 int mca_mask_bits_view(const uint32_t* bits, const uint32_t* bits_t, int mask_mode, int T, int need_transpose, McaMaskBits* out,
                        const McaMaskBits** view);
 
-// Internal: mca_classify_causal_mask in one launch.  scratch: two device ints that are zero before the call and zero
-// again after it (a mismatch count and a ticket; the last block to finish writes *flag, and host_base + flag to
-// *host_flag in pinned host memory unless that is null).
-int mca_classify_causal_mask_ws(const float* mask, int T, int* flag, int* host_flag, int host_base, int* scratch, void* stream);
+// Internal: mca_classify_causal_mask in one launch.
+struct McaClassifyJob;
+int mca_classify_causal_mask_ws(const McaClassifyJob* job, void* stream);
+
+// Internal: the two halves of mca_sdpa_forward_f32_tc_masked -- the pre-pass that splits q, k, v (and classifies the caller's
+// (T,T) mask in the same launch when `cls` is given), and the kernel, which may then be chosen on the class.
+int mca_split_forward_prepass(const float* q, const float* k, const float* v, int B, int H, int T, int D, void* workspace,
+                              int64_t workspace_bytes, int layout, const McaClassifyJob* cls, void* stream);
+int mca_split_forward_main(int causal, int B, int H, int T, int D, float* y, float* row_max, float* row_sum, float* y_copy, float* lse,
+                           void* workspace, int* status, int layout, const uint32_t* mask_bits, int mask_mode, void* stream);
 
 // Internal: hand the current device's kernels the address of the process's failure words (McaFailWord).
 int mca_set_fail_words_fwd(int* words);

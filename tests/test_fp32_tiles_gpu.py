@@ -1,4 +1,4 @@
-"""The exact fp32 kernels at the edges of their tiles: both row-tile heights (64 for few or short heads, 128 otherwise), head
+"""The fp32 kernels at the edges of their tiles.  Exact ones: both row-tile heights (64 for few or short heads, 128 otherwise), head
 sizes either side of every padded size, the walked side's remainder, and head sizes whose
 rows are not 16-byte aligned (the copies that are not asynchronous).  Against the fp64 oracle."""
 import numpy as np
@@ -42,3 +42,25 @@ def test_tiles_forward_backward(cuda, B, H, T, D, kind):
     assert rel_err(y, oracle.sdpa_forward(q, k, v, mask, mode, f64=True)) < TOL
     for g, r in zip(got, oracle.sdpa_backward(q, k, v, dy, mask, mode, f64=True)):
         assert rel_err(g, r) < TOL
+
+
+@pytest.mark.parametrize("T,D", [(127, 64), (257, 32), (513, 64), (1025, 64), (2049, 16), (1100, 64)])
+def test_split_operand_scales_per_head(cuda, T, D):
+    """The operand split's scale belongs to a (batch, head): heads nine orders of magnitude apart keep their own precision, at every
+    number of CTAs a head is spread over and where a head outgrows the registers it is kept in."""
+    rng = np.random.default_rng(T + D)
+    B, H = 1, 3
+    mag = np.array([1e-5, 1.0, 3e3], np.float32).reshape(1, H, 1, 1)
+    q, k, v, dy = (rng.standard_normal((B, H, T, D)).astype(np.float32) for _ in range(4))
+    v, dy = v * mag, dy * mag[:, ::-1]
+    q, k = q * np.array([1e-4, 1.0, 1e3], np.float32).reshape(1, H, 1, 1), k * np.array([1e4, 1.0, 1e-3], np.float32).reshape(1, H, 1, 1)
+    mask = oracle.causal_mask(T)
+    a = Sdpa(cuda, B, T, H, D, training=True)
+    y = a.forward(q, k, v, mask)
+    got = a.backward(dy)
+    a.close()
+    ref_y, ref = oracle.sdpa_forward(q, k, v, mask, 1, f64=True), oracle.sdpa_backward(q, k, v, dy, mask, 1, f64=True)
+    for h in range(H):
+        assert rel_err(y[:, h], ref_y[:, h]) < TOL
+        for g, r in zip(got, ref):
+            assert rel_err(g[:, h], r[:, h]) < TOL
