@@ -384,7 +384,7 @@ int run_proj_tc(const GemvParams& p, cudaStream_t st) {
       return e;
   }
   if ((e = proj::make_map_2d(&mx, pieces, BF ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
-                             (int64_t)PL::PIECES * Bp, p.n, proj::KC, Bp, CU_TENSOR_MAP_SWIZZLE_128B)))
+                             (int64_t)proj::PIECES * Bp, p.n, proj::KC, proj::PIECES * Bp, CU_TENSOR_MAP_SWIZZLE_128B)))
     return e;
   auto pre = proj::x_pieces_kernel<BF>;
   static std::atomic<uint64_t> pre_done{0}, kern_done{0};

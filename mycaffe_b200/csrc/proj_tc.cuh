@@ -37,11 +37,13 @@ constexpr int MAX_B = 64;          // sequences (MMA N, rounded up to 16)
 constexpr int MAX_N = 16384;       // longest contraction
 constexpr int MAX_ITEMS = 296;     // (tile, slice) items when K is cut
 constexpr int MAX_TILES = 2048;
+constexpr int PIECES = 2;          // 16-bit pieces of an activation
+constexpr int MAX_SX = 16;         // stages of the activation ring, at most
 constexpr int CONV_WARPS = 8, EPI_WARPS = 4;
 constexpr int WARP_EPI0 = CONV_WARPS, WARP_TMA = CONV_WARPS + EPI_WARPS, WARP_MMA = WARP_TMA + 1, WARP_TMA_X = WARP_MMA + 1;
 constexpr int THREADS = (WARP_TMA_X + 1) * 32;
 constexpr float W_SCALE = 16.f;    // fp32 weights are split after this exact scaling (keeps the low halves normal)
-constexpr uint32_t TMEM_ALLOC = 256, ACC_COLS = 128;
+constexpr uint32_t TMEM_ALLOC = 512, ACC_COLS = 256;   // two accumulators of up to two results x two pieces x 64 sequences
 
 __device__ __align__(1024) uint16_t g_x_pieces[2 * MAX_B * MAX_N];
 __device__ float g_x_scale[MAX_B];
@@ -55,26 +57,23 @@ template <> struct Plan<float> {
 #ifndef MCA_PROJ_SW
 #define MCA_PROJ_SW 5
 #endif
-#ifndef MCA_PROJ_SX
-#define MCA_PROJ_SX 3
-#endif
-  static constexpr int SW = MCA_PROJ_SW, SX = MCA_PROJ_SX, PIECES = 2, FMT = 0;   // weight / activation ring depths; fp16 operands
+  static constexpr int SW = MCA_PROJ_SW, FMT = 0;                       // weight ring depth; fp16 operands
   static constexpr uint32_t W_BYTES = ROWS * KC * 4;                    // a slot: the fp32 tile, then hi | lo in its place
-  static constexpr uint32_t X_BYTES = PIECES * MAX_B * 128;
+  static constexpr uint32_t X_RING = 3 * PIECES * MAX_B * 128;          // the activation ring: as many stages as fit
   static constexpr uint32_t OP_BYTES = ROWS * KC * 2;                   // one fp16 operand tile (half a slot)
-  static constexpr uint32_t OFF_W = 0, OFF_X = OFF_W + SW * W_BYTES, OFF_OP = OFF_X + SX * X_BYTES;
+  static constexpr uint32_t OFF_W = 0, OFF_X = OFF_W + SW * W_BYTES, OFF_OP = OFF_X + X_RING;
   static constexpr uint32_t OFF_BAR = OFF_OP;
 };
 template <> struct Plan<__nv_bfloat16> {
   static constexpr bool CONVERT = false;
-  static constexpr int SW = 8, SX = 3, PIECES = 2, FMT = 1;            // bf16 operands
+  static constexpr int SW = 8, FMT = 1;                                // bf16 operands
   static constexpr uint32_t W_BYTES = ROWS * KC * 2;
-  static constexpr uint32_t X_BYTES = PIECES * MAX_B * 128;
+  static constexpr uint32_t X_RING = 6 * PIECES * MAX_B * 128;
   static constexpr uint32_t OP_BYTES = 0;
-  static constexpr uint32_t OFF_W = 0, OFF_X = OFF_W + SW * W_BYTES, OFF_OP = OFF_X + SX * X_BYTES;
+  static constexpr uint32_t OFF_W = 0, OFF_X = OFF_W + SW * W_BYTES, OFF_OP = OFF_X + X_RING;
   static constexpr uint32_t OFF_BAR = OFF_OP;
 };
-// barriers: wfull[SW] wempty[SW] xfull[SX] xempty[SX] convdone[SW] accfull[2] accfree[2], then the TMEM address
+// barriers: wfull[SW] wempty[SW] xfull[MAX_SX] xempty[MAX_SX] convdone[SW] accfull[2] accfree[2], then the TMEM address
 constexpr uint32_t BAR_BYTES = 512;
 template <typename WT> constexpr size_t smem_bytes() { return Plan<WT>::OFF_BAR + BAR_BYTES + EPI_WARPS * MAX_B * 4 + 1024; }
 
@@ -196,7 +195,12 @@ __global__ void __launch_bounds__(THREADS, 1) proj_tc_kernel(const __grid_consta
                                                              const __grid_constant__ CUtensorMap mw2,
                                                              const __grid_constant__ CUtensorMap mx, const Params p) {
   using PL = Plan<WT>;
-  constexpr int SW = PL::SW, SX = PL::SX;
+  constexpr int SW = PL::SW;
+  // The activation ring: a stage is the two pieces of every sequence for one k chunk, read from L2.  A chunk costs the
+  // tensor pipe a third of a microsecond and L2 answers after one, so with few sequences, whose stages are small, many are kept
+  // in flight (three of them, whatever their size, held 16 sequences to 40 % of the memory bandwidth).
+  const uint32_t x_piece_bytes = (uint32_t)p.Bp * 128u, x_stage_bytes = PIECES * x_piece_bytes;
+  const int SX = min((int)MAX_SX, (int)(PL::X_RING / x_stage_bytes));
   extern __shared__ unsigned char pj_smem_raw[];
   const uint32_t raw = smem_u32(pj_smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -205,8 +209,8 @@ __global__ void __launch_bounds__(THREADS, 1) proj_tc_kernel(const __grid_consta
   auto wfull = [&](int s) { return bar0 + 8u * s; };
   auto wempty = [&](int s) { return bar0 + 8u * (SW + s); };
   auto xfull = [&](int s) { return bar0 + 8u * (2 * SW + s); };
-  auto xempty = [&](int s) { return bar0 + 8u * (2 * SW + SX + s); };
-  constexpr int NB0 = 2 * SW + 2 * SX;
+  auto xempty = [&](int s) { return bar0 + 8u * (2 * SW + MAX_SX + s); };
+  constexpr int NB0 = 2 * SW + 2 * MAX_SX;
   auto convdone = [&](int c) { return bar0 + 8u * (NB0 + c); };        // [SW]: slot c holds the converted tiles
   auto accfull = [&](int a) { return bar0 + 8u * (NB0 + SW + a); };
   auto accfree = [&](int a) { return bar0 + 8u * (NB0 + SW + 2 + a); };
@@ -222,7 +226,7 @@ __global__ void __launch_bounds__(THREADS, 1) proj_tc_kernel(const __grid_consta
       mbar_init(wempty(s), 1);                              // the MMA has read the slot
       mbar_init(convdone(s), CONV_WARPS);
     }
-    for (int s = 0; s < SX; ++s) {
+    for (int s = 0; s < MAX_SX; ++s) {
       mbar_init(xfull(s), 1);
       mbar_init(xempty(s), 1);
     }
@@ -252,7 +256,6 @@ __global__ void __launch_bounds__(THREADS, 1) proj_tc_kernel(const __grid_consta
   const int nacc = p.swiglu ? 2 : 1;
   // k chunks of slice j: [j * kchunks / slices, (j + 1) * kchunks / slices)
   auto slice_lo = [&](int j) { return (int)(((int64_t)j * p.kchunks) / p.slices); };
-  const uint32_t x_piece_bytes = (uint32_t)p.Bp * 128u;
   bool ok = true;
 
   if (warp == WARP_TMA) {
@@ -288,19 +291,19 @@ __global__ void __launch_bounds__(THREADS, 1) proj_tc_kernel(const __grid_consta
     // ------------------------------------------------------------------ activation producer
     if (lane == 0) {
       mca_pdl_wait();                                     // the pieces are the pre-pass's output
-      int g = 0;
+      int g = 0, s = 0;
+      uint32_t ph = 0;
       for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
         const int u = item / p.slices, j = item - u * p.slices;
         const int k0 = slice_lo(j), k1 = slice_lo(j + 1);
         for (int mi = 0; mi < nacc && ok; ++mi) {
           for (int kc = k0; kc < k1; ++kc, ++g) {
-            const int s = g % SX;
-            ok = mbar_wait(xempty(s), (uint32_t)(((g / SX) & 1) ^ 1), status, 8, g);
+            ok = mbar_wait(xempty(s), ph ^ 1u, status, 8, g);
             if (!ok) break;
-            mbar_expect_tx(xfull(s), PL::PIECES * x_piece_bytes);
-#pragma unroll
-            for (int pc = 0; pc < PL::PIECES; ++pc)
-              tma_load_2d(base + PL::OFF_X + s * PL::X_BYTES + pc * x_piece_bytes, &mx, xfull(s), kc * KC, pc * p.Bp);
+            mbar_expect_tx(xfull(s), x_stage_bytes);
+            // both pieces are consecutive rows of the array: one box
+            tma_load_2d(base + PL::OFF_X + s * x_stage_bytes, &mx, xfull(s), kc * KC, 0);
+            if (++s == SX) { s = 0; ph ^= 1u; }
           }
         }
       }
@@ -308,8 +311,11 @@ __global__ void __launch_bounds__(THREADS, 1) proj_tc_kernel(const __grid_consta
   } else if (warp == WARP_MMA) {
     // ------------------------------------------------------------------ MMA issuer (one lane)
     if (lane == 0) {
-      const uint32_t idesc = make_idesc_fmt(ROWS, p.Bp, 0, 0, PL::FMT);
-      int g = 0, it = 0;
+      // hi and lo pieces of all sequences are one operand of 2 Bp columns: an instruction costs about the same up to 128
+      // columns, so W . [x_hi | x_lo] is one instruction per 16 k, and the epilogue adds the two halves of its result
+      const uint32_t idesc2 = make_idesc_fmt(ROWS, 2 * p.Bp, 0, 0, PL::FMT), idesc = make_idesc_fmt(ROWS, p.Bp, 0, 0, PL::FMT);
+      int g = 0, it = 0, sx = 0;
+      uint32_t xph = 0;
       for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++it) {
         const int u = item / p.slices, j = item - u * p.slices;
         const int k0 = slice_lo(j), k1 = slice_lo(j + 1);
@@ -318,35 +324,27 @@ __global__ void __launch_bounds__(THREADS, 1) proj_tc_kernel(const __grid_consta
         if (!ok) break;
         tc_fence_after();
         for (int mi = 0; mi < nacc && ok; ++mi) {
-          const uint32_t d_tmem = tmem_base + (uint32_t)a * ACC_COLS + (uint32_t)(mi * p.Bp);
+          const uint32_t d_tmem = tmem_base + (uint32_t)a * ACC_COLS + (uint32_t)(mi * 2 * p.Bp);
           for (int kc = k0; kc < k1; ++kc, ++g) {
-            const int sw = g % SW, sx = g % SX;
+            const int sw = g % SW;
             // fp32 weights: the slot holds the converted hi | lo tiles once all converter warps have arrived
             ok = mbar_wait(PL::CONVERT ? convdone(sw) : wfull(sw), (uint32_t)((g / SW) & 1), status, 3, g);
             if (!ok) break;
             const uint32_t a_hi = base + PL::OFF_W + sw * PL::W_BYTES, a_lo = a_hi + PL::OP_BYTES;
-            ok = mbar_wait(xfull(sx), (uint32_t)((g / SX) & 1), status, 9, g);
+            ok = mbar_wait(xfull(sx), xph, status, 9, g);
             if (!ok) break;
             tc_fence_after();
-            const uint32_t xs = base + PL::OFF_X + sx * PL::X_BYTES;
+            const uint32_t xs = base + PL::OFF_X + sx * x_stage_bytes;
 #pragma unroll
             for (int kk = 0; kk < KC / 16; ++kk) {
               const uint32_t first = (kc == k0 && kk == 0) ? 0u : 1u;
-              const uint64_t dx0 = make_desc(xs + kk * 32, 16, 1024);
-              const uint64_t dx1 = make_desc(xs + x_piece_bytes + kk * 32, 16, 1024);
-              const uint64_t da = make_desc(a_hi + kk * 32, 16, 1024);
-              if constexpr (PL::CONVERT) {
-                const uint64_t dl = make_desc(a_lo + kk * 32, 16, 1024);
-                umma_ss(d_tmem, da, dx0, idesc, first);     // hi . hi
-                umma_ss(d_tmem, da, dx1, idesc, 1u);        // hi . lo
-                umma_ss(d_tmem, dl, dx0, idesc, 1u);        // lo . hi
-              } else {
-                umma_ss(d_tmem, da, dx0, idesc, first);     // W . x_hi
-                umma_ss(d_tmem, da, dx1, idesc, 1u);        // W . x_lo
-              }
+              const uint64_t dx = make_desc(xs + kk * 32, 16, 1024);
+              umma_ss(d_tmem, make_desc(a_hi + kk * 32, 16, 1024), dx, idesc2, first);                             // W_hi . [x_hi | x_lo]
+              if constexpr (PL::CONVERT) umma_ss(d_tmem, make_desc(a_lo + kk * 32, 16, 1024), dx, idesc, 1u);      // W_lo . x_hi
             }
             umma_commit(wempty(sw));
             umma_commit(xempty(sx));
+            if (++sx == SX) { sx = 0; xph ^= 1u; }
           }
         }
         if (ok) umma_commit(accfull(a));
@@ -446,15 +444,24 @@ __global__ void __launch_bounds__(THREADS, 1) proj_tc_kernel(const __grid_consta
           }
         }
       };
+      // sixteen columns of a result: the x_hi half plus the x_lo half
+      auto load_acc = [&](uint32_t t, int col, float (&v)[16]) {
+        uint32_t h[16], l[16];
+        tmem_ld16(t + col, h);
+        tmem_ld16(t + col + p.Bp, l);
+        tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(h[i]) + __uint_as_float(l[i]);
+      };
       if (p.slices == 1) {
         for (int c0 = 0; c0 < p.Bp; c0 += 16) {
-          uint32_t va[16], vb[16];
           float fa[16], fb[16];
-          tmem_ld16(t_acc + c0, va);
-          if (p.swiglu) tmem_ld16(t_acc + p.Bp + c0, vb);
-          tmem_wait_ld();
+          load_acc(t_acc, c0, fa);
+          if (p.swiglu) load_acc(t_acc, 2 * p.Bp + c0, fb);
+          else {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) { fa[i] = __uint_as_float(va[i]); fb[i] = p.swiglu ? __uint_as_float(vb[i]) : 0.f; }
+            for (int i = 0; i < 16; ++i) fb[i] = 0.f;
+          }
           finish16(c0, fa, fb);
         }
         tc_fence_before();
@@ -463,11 +470,10 @@ __global__ void __launch_bounds__(THREADS, 1) proj_tc_kernel(const __grid_consta
       } else {
         float* part = g_partials + ((size_t)(u * p.slices + j) * ncols) * ROWS + r;
         for (int c0 = 0; c0 < ncols; c0 += 16) {
-          uint32_t v[16];
-          tmem_ld16(t_acc + c0, v);
-          tmem_wait_ld();
+          float v[16];
+          load_acc(t_acc, c0 < p.Bp ? c0 : p.Bp + c0, v);   // the second result starts behind both halves of the first
 #pragma unroll
-          for (int i = 0; i < 16; ++i) __stcg(part + (size_t)(c0 + i) * ROWS, __uint_as_float(v[i]));
+          for (int i = 0; i < 16; ++i) __stcg(part + (size_t)(c0 + i) * ROWS, v[i]);
         }
         tc_fence_before();
         __syncwarp();
