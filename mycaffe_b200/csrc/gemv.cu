@@ -373,7 +373,6 @@ int run_proj_tc(const GemvParams& p, cudaStream_t st) {
   }
   q.n_mats = p.n_mats; q.B = p.B; q.Bp = Bp; q.n = p.n; q.accumulate = p.accumulate; q.swiglu = p.swiglu;
   q.tiles = tiles; q.kchunks = mca_ceil_div(p.n, proj::KC);
-  q.slices = proj::pick_slices(tiles, q.kchunks, sms);
   CUtensorMap mw[3], mx;
   int e;
   for (int m = 0; m < 3; ++m) {
@@ -386,19 +385,17 @@ int run_proj_tc(const GemvParams& p, cudaStream_t st) {
   if ((e = proj::make_map_2d(&mx, pieces, BF ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
                              (int64_t)proj::PIECES * Bp, p.n, proj::KC, proj::PIECES * Bp, CU_TENSOR_MAP_SWIZZLE_128B)))
     return e;
-  auto pre = proj::x_pieces_kernel<BF>;
-  static std::atomic<uint64_t> pre_done{0}, kern_done{0};
-  if ((e = mca_smem_once(pre_done, pre, proj::MAX_N * 4))) return e;
   // both kernels are launched programmatically dependent: the pre-pass's launch overlaps the tail of whatever runs
   // before it (it waits for that before it reads or writes anything), the contraction's set-up overlaps the pre-pass
-  if ((e = mca_launch_pdl(pre, dim3(Bp), dim3(256), sizeof(float) * (size_t)p.n, st, p.x, p.norm_w, p.eps, p.n, p.B, Bp, pieces, xscale)))
-    return e;
+  const int nv = mca_ceil_div(p.n, 4 * proj::X_THREADS);
+  auto pre = nv <= 2 ? proj::x_pieces_kernel<BF, 2> : nv <= 4 ? proj::x_pieces_kernel<BF, 4> : proj::x_pieces_kernel<BF, 8>;
+  if ((e = mca_launch_pdl(pre, dim3(Bp), dim3(proj::X_THREADS), 0, st, p.x, p.norm_w, p.eps, p.n, p.B, Bp, pieces, xscale))) return e;
   const size_t smem = proj::smem_bytes<WT>();
   auto kern = proj::proj_tc_kernel<WT>;
+  static std::atomic<uint64_t> kern_done{0};
   if ((e = mca_smem_once(kern_done, kern, smem))) return e;
-  const int items = tiles * q.slices;
   // programmatic dependent launch: set-up and the first weight tiles overlap the pre-pass
-  return mca_launch_pdl(kern, dim3(std::min(items, sms)), dim3(proj::THREADS), smem, st, mw[0], mw[1], mw[2], mx, q);
+  return mca_launch_pdl(kern, dim3(proj::pick_ctas((int64_t)tiles * q.kchunks, sms)), dim3(proj::Roles<PL::CONVERT>::THREADS), smem, st, mw[0], mw[1], mw[2], mx, q);
 }
 
 template <typename WT>

@@ -14,18 +14,24 @@
 //     the three MMAs hi.hi + hi.lo + lo.hi into one fp32 accumulator in TMEM (the dropped lo.lo term is 2^-22);
 //   * bf16 weights: the TMA tile is the MMA operand itself, the activations are two bf16 pieces (16 mantissa bits; the
 //     weights themselves carry 8), two MMAs per k16.
-// Work items are (tile of 128 rows, slice of K): matrices with few rows (Wo, W2) are cut along K so that every SM
-// streams; a slice leaves its fp32 partial sums in a scratch array and the slice that arrives last (a ticket per
-// tile and quarter of its rows) adds all of them in slice order, so the result does not depend on timing.  The gated
-// pair W1/W3 of the feed-forward block is one item with two accumulators and silu(a) * b in the epilogue.
-// Roles of a CTA (480 threads, one CTA per SM, persistent over items): warps 0-7 convert, 8-11 epilogue (TMEM lanes
-// 32 (w - 8) ..), warp 12 TMA producer of the weights, warp 13 MMA issuer and TMEM owner, warp 14 TMA producer of the
+// The (tile of 128 rows) x (64-wide k chunk) units of all tiles, in that order, are dealt to the CTAs in equal contiguous
+// ranges: every SM streams the same number of bytes whatever the matrix (whole tiles, or tiles cut into a fixed number of
+// slices, left the last of two waves a seventh to a half empty: W1/W3 of 11008 rows, bf16, 16 sequences MEASURED_SK).
+// A CTA whose range covers part of a tile leaves fp32 partial sums in a scratch array, and the one that arrives last (a
+// ticket per tile and quarter of its rows) adds all of the tile's parts in their order, so the result does not depend on
+// timing.  The gated pair W1/W3 of the feed-forward block is one tile with two accumulators and silu(a) * b in the epilogue.
+// Roles of a CTA (one CTA per SM, persistent over its range): eight warps convert (fp32 weights only), eight are the epilogue
+// (two for each quarter of the TMEM lanes, alternating by eight columns: what is left to do when the last chunk has been
+// multiplied is a chain of memory round trips, so it is spread wide), one is the TMA producer of the weights, one the MMA
+// issuer and TMEM owner, one the TMA producer of the
 // activation pieces.  The weight ring (five 32 KB slots for fp32, eight 16 KB slots for bf16) and the activation ring
 // have their own barriers.  Every wait is bounded.
 // The activation pieces, per-sequence scales, partial sums and tickets live in arrays that are part of the library
 // image (about 24 MB per device): nothing is allocated, but two of these products must not overlap on one device.
 #pragma once
 #define MCA_TU_FAIL_FAMILY MCA_FAIL_PROJ
+#include <algorithm>
+
 #include "tc_common.cuh"
 
 namespace proj {
@@ -35,19 +41,22 @@ constexpr int ROWS = 128;          // weight rows per tile (MMA M)
 constexpr int KC = 64;             // k per stage: one 128-byte row of 16-bit operands
 constexpr int MAX_B = 64;          // sequences (MMA N, rounded up to 16)
 constexpr int MAX_N = 16384;       // longest contraction
-constexpr int MAX_ITEMS = 296;     // (tile, slice) items when K is cut
+constexpr int MAX_CTAS = 148;      // one per SM; each has room for two partial tiles, at either end of its range
 constexpr int MAX_TILES = 2048;
 constexpr int PIECES = 2;          // 16-bit pieces of an activation
 constexpr int MAX_SX = 16;         // stages of the activation ring, at most
-constexpr int CONV_WARPS = 8, EPI_WARPS = 4;
-constexpr int WARP_EPI0 = CONV_WARPS, WARP_TMA = CONV_WARPS + EPI_WARPS, WARP_MMA = WARP_TMA + 1, WARP_TMA_X = WARP_MMA + 1;
-constexpr int THREADS = (WARP_TMA_X + 1) * 32;
+constexpr int CONV_WARPS = 8, EPI_WARPS = 8;
+// warps of a CTA: converters (fp32 weights only), epilogue, weight TMA, MMA, activation TMA
+template <bool CONVERT> struct Roles {
+  static constexpr int EPI0 = CONVERT ? CONV_WARPS : 0, TMA = EPI0 + EPI_WARPS, MMA = TMA + 1, TMA_X = MMA + 1;
+  static constexpr int THREADS = (TMA_X + 1) * 32;
+};
 constexpr float W_SCALE = 16.f;    // fp32 weights are split after this exact scaling (keeps the low halves normal)
 constexpr uint32_t TMEM_ALLOC = 512, ACC_COLS = 256;   // two accumulators of up to two results x two pieces x 64 sequences
 
 __device__ __align__(1024) uint16_t g_x_pieces[2 * MAX_B * MAX_N];
 __device__ float g_x_scale[MAX_B];
-__device__ float g_partials[(size_t)MAX_ITEMS * ROWS * 2 * MAX_B];
+__device__ float g_partials[(size_t)MAX_CTAS * 2 * ROWS * 2 * MAX_B];
 __device__ unsigned int g_tickets[MAX_TILES * EPI_WARPS];
 __device__ int g_status[4];
 
@@ -75,13 +84,14 @@ template <> struct Plan<__nv_bfloat16> {
 };
 // barriers: wfull[SW] wempty[SW] xfull[MAX_SX] xempty[MAX_SX] convdone[SW] accfull[2] accfree[2], then the TMEM address
 constexpr uint32_t BAR_BYTES = 512;
-template <typename WT> constexpr size_t smem_bytes() { return Plan<WT>::OFF_BAR + BAR_BYTES + EPI_WARPS * MAX_B * 4 + 1024; }
+template <typename WT> constexpr size_t smem_bytes() { return Plan<WT>::OFF_BAR + BAR_BYTES + MAX_B * 4 + 1024; }
+static_assert(smem_bytes<float>() <= 227 * 1024 && smem_bytes<__nv_bfloat16>() <= 227 * 1024, "one CTA per SM");
 
 struct Params {
   float* out[3];
   int rows[3];
   int tile0[4];        // first tile of each matrix (not gated); tile0[n_mats] = tiles
-  int n_mats, B, Bp, n, accumulate, swiglu, slices, tiles, kchunks;
+  int n_mats, B, Bp, n, accumulate, swiglu, tiles, kchunks;
 };
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
@@ -103,26 +113,25 @@ __device__ __forceinline__ bool conv_bar_and(bool pred) {
   return r != 0;
 }
 
-__device__ __forceinline__ float block_sum(float v, float* red) {   // 256 threads
+constexpr int X_THREADS = 512;
+__device__ __forceinline__ float block_sum(float v, float* red) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  __syncthreads();
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
   float t = 0.f;
 #pragma unroll
-  for (int w = 0; w < 8; ++w) t += red[w];
+  for (int w = 0; w < X_THREADS / 32; ++w) t += red[w];
   return t;
 }
 __device__ __forceinline__ float block_max(float v, float* red) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  __syncthreads();
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
   float t = 0.f;
 #pragma unroll
-  for (int w = 0; w < 8; ++w) t = fmaxf(t, red[w]);
+  for (int w = 0; w < X_THREADS / 32; ++w) t = fmaxf(t, red[w]);
   return t;
 }
 
@@ -131,71 +140,93 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 //   BF16 = false: v / 2^e with 2^e chosen so that the row's largest magnitude lands in [2^13, 2^14), as fp16 hi + lo;
 //   BF16 = true:  v as two bf16 pieces, hi = bf16(v), lo = bf16(v - hi): 16 mantissa bits, two hundred times finer than
 //                 the bf16 weights they multiply.
-// Rows from B up to Bp are written as zeros.  One CTA of 256 threads per row.
-template <bool BF16>
-__global__ void __launch_bounds__(256) x_pieces_kernel(const float* __restrict__ x, const float* __restrict__ norm_w, float eps,
-                                                       int n, int B, int Bp, uint16_t* __restrict__ pieces,
-                                                       float* __restrict__ xscale) {
-  __shared__ float red[8];
-  extern __shared__ float xrow[];                       // the row, read from global memory once
+// Rows from B up to Bp are written as zeros.  One CTA per row, the row in its threads' registers (NV float4 each): this kernel
+// is a latency in front of every contraction (its x is the kernel before's last result), so the row is read once, with all
+// loads in flight and the norm's weights requested before that kernel has finished, and no shared memory is taken that an
+// SM still holding a contraction's CTA could not give (5.8 us of exposed time at n = 4096, 16 sequences -> MEASURED_XP).
+template <bool BF16, int NV>
+__global__ void __launch_bounds__(X_THREADS) x_pieces_kernel(const float* __restrict__ x, const float* __restrict__ norm_w, float eps,
+                                                             int n, int B, int Bp, uint16_t* __restrict__ pieces,
+                                                             float* __restrict__ xscale) {
+  __shared__ float red[2][X_THREADS / 32];
   const int b = blockIdx.x, tid = threadIdx.x;
   mca_pdl_launch_dependents();                          // the contraction kernel may start fetching weights
+  const bool live = b < B;
+  float4 g[NV], v[NV];
+  if (norm_w != nullptr && live) {
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int k = (tid + i * X_THREADS) * 4;
+      g[i] = k < n ? __ldg(reinterpret_cast<const float4*>(norm_w + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
   mca_pdl_wait();                                       // launched ahead of the kernels before it: their results (x, and the
                                                         // previous contraction's last reads of the pieces) come first
-  const size_t piece_stride = (size_t)Bp * n;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int k = (tid + i * X_THREADS) * 4;
+    v[i] = live && k < n ? *reinterpret_cast<const float4*>(x + (size_t)b * n + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  if (norm_w != nullptr && live) {
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      ss = fmaf(v[i].x, v[i].x, ss); ss = fmaf(v[i].y, v[i].y, ss); ss = fmaf(v[i].z, v[i].z, ss); ss = fmaf(v[i].w, v[i].w, ss);
+    }
+    ss = block_sum(ss, red[0]);
+    const float s = 1.0f / sqrtf(ss / (float)n + eps);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      v[i].x = g[i].x * (s * v[i].x); v[i].y = g[i].y * (s * v[i].y); v[i].z = g[i].z * (s * v[i].z); v[i].w = g[i].w * (s * v[i].w);
+    }
+  }
+  float down = 1.f;
+  if constexpr (!BF16) {
+    float amax = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
+    amax = block_max(amax, red[1]);
+    int e = 0;
+    if (amax > 0.f && amax < INFINITY) { frexpf(amax, &e); e -= 14; }
+    down = ldexpf(1.f, -e);
+    if (tid == 0 && live) xscale[b] = ldexpf(1.f, e) / W_SCALE;
+  } else {
+    if (tid == 0 && live) xscale[b] = 1.f;
+  }
   uint16_t* dst = pieces + (size_t)b * n;
-  if (b >= B) {
-    for (int k = tid; k < n; k += 256) {
-      dst[k] = 0; dst[piece_stride + k] = 0;
+  uint16_t* dst_lo = dst + (size_t)Bp * n;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int k = (tid + i * X_THREADS) * 4;
+    if (k >= n) continue;
+    const float e4[4] = {v[i].x * down, v[i].y * down, v[i].z * down, v[i].w * down};
+    uint32_t h[2], l[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      if constexpr (BF16) {
+        const __nv_bfloat16 h0 = __float2bfloat16_rn(e4[2 * j]), h1 = __float2bfloat16_rn(e4[2 * j + 1]);
+        h[j] = (uint32_t)__bfloat16_as_ushort(h0) | ((uint32_t)__bfloat16_as_ushort(h1) << 16);
+        l[j] = pack_bf16(e4[2 * j] - __bfloat162float(h0), e4[2 * j + 1] - __bfloat162float(h1));
+      } else {
+        const __half h0 = __float2half_rn(e4[2 * j]), h1 = __float2half_rn(e4[2 * j + 1]);
+        h[j] = (uint32_t)__half_as_ushort(h0) | ((uint32_t)__half_as_ushort(h1) << 16);
+        l[j] = pack_f16(e4[2 * j] - __half2float(h0), e4[2 * j + 1] - __half2float(h1));
+      }
     }
-    return;
+    *reinterpret_cast<uint2*>(dst + k) = make_uint2(h[0], h[1]);
+    *reinterpret_cast<uint2*>(dst_lo + k) = make_uint2(l[0], l[1]);
   }
-  const float* xr = x + (size_t)b * n;
-  float ss = 0.f;
-  for (int k = tid; k < n; k += 256) { const float v = xr[k]; xrow[k] = v; ss = fmaf(v, v, ss); }
-  float s = 1.f;
-  if (norm_w != nullptr) {
-    ss = block_sum(ss, red);
-    s = 1.0f / sqrtf(ss / (float)n + eps);
-  }
-  float amax = 0.f;
-  for (int k = tid; k < n; k += 256) {                  // a thread revisits only the elements it wrote itself
-    const float v = norm_w != nullptr ? __ldg(norm_w + k) * (s * xrow[k]) : xrow[k];
-    xrow[k] = v;
-    amax = fmaxf(amax, fabsf(v));
-  }
-  if (BF16) {
-    for (int k = tid; k < n; k += 256) {
-      const float v = xrow[k];
-      const __nv_bfloat16 h = __float2bfloat16_rn(v);
-      const __nv_bfloat16 l = __float2bfloat16_rn(v - __bfloat162float(h));
-      dst[k] = __bfloat16_as_ushort(h);
-      dst[piece_stride + k] = __bfloat16_as_ushort(l);
-    }
-    if (tid == 0) xscale[b] = 1.f;
-    return;
-  }
-  amax = block_max(amax, red);
-  int e = 0;
-  if (amax > 0.f && amax < INFINITY) { frexpf(amax, &e); e -= 14; }
-  const float down = ldexpf(1.f, -e);
-  for (int k = tid; k < n; k += 256) {
-    const float v = xrow[k] * down;
-    const __half h = __float2half_rn(v);
-    const __half l = __float2half_rn(v - __half2float(h));
-    dst[k] = __half_as_ushort(h);
-    dst[piece_stride + k] = __half_as_ushort(l);
-  }
-  if (tid == 0) xscale[b] = ldexpf(1.f, e) / W_SCALE;
 }
 
 template <typename WT>
-__global__ void __launch_bounds__(THREADS, 1) proj_tc_kernel(const __grid_constant__ CUtensorMap mw0,
+__global__ void __launch_bounds__(Roles<Plan<WT>::CONVERT>::THREADS, 1) proj_tc_kernel(const __grid_constant__ CUtensorMap mw0,
                                                              const __grid_constant__ CUtensorMap mw1,
                                                              const __grid_constant__ CUtensorMap mw2,
                                                              const __grid_constant__ CUtensorMap mx, const Params p) {
   using PL = Plan<WT>;
   constexpr int SW = PL::SW;
+  using RO = Roles<PL::CONVERT>;
+  constexpr int WARP_EPI0 = RO::EPI0, WARP_TMA = RO::TMA, WARP_MMA = RO::MMA, WARP_TMA_X = RO::TMA_X;
   // The activation ring: a stage is the two pieces of every sequence for one k chunk, read from L2.  A chunk costs the
   // tensor pipe a third of a microsecond and L2 answers after one, so with few sequences, whose stages are small, many are kept
   // in flight (three of them, whatever their size, held 16 sequences to 40 % of the memory bandwidth).
@@ -216,7 +247,7 @@ __global__ void __launch_bounds__(THREADS, 1) proj_tc_kernel(const __grid_consta
   auto accfree = [&](int a) { return bar0 + 8u * (NB0 + SW + 2 + a); };
   static_assert(8 * (NB0 + SW + 4) + 8 <= BAR_BYTES, "barriers fit their block");
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + PL::OFF_BAR + 8 * (NB0 + SW + 4));
-  float* cs = reinterpret_cast<float*>(gen + PL::OFF_BAR + BAR_BYTES);   // per-sequence output scales, one copy per epilogue warp
+  float* cs = reinterpret_cast<float*>(gen + PL::OFF_BAR + BAR_BYTES);   // per-sequence output scales
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int* status = g_status;
 
@@ -252,10 +283,20 @@ __global__ void __launch_bounds__(THREADS, 1) proj_tc_kernel(const __grid_consta
   const uint32_t tmem_base = *tmem_slot;
 
   mca_pdl_launch_dependents();   // a dependent launch may take the SMs as this kernel's CTAs leave them
-  const int items = p.tiles * p.slices;
   const int nacc = p.swiglu ? 2 : 1;
-  // k chunks of slice j: [j * kchunks / slices, (j + 1) * kchunks / slices)
-  auto slice_lo = [&](int j) { return (int)(((int64_t)j * p.kchunks) / p.slices); };
+  // this CTA's units [lo, hi) of the (tile, k chunk) order: segments (tile u, chunks [k0, k1))
+  const int64_t total = (int64_t)p.tiles * p.kchunks;
+  auto range_lo = [&](int c) { return (int)(((int64_t)c * total) / (int)gridDim.x); };
+  auto owner = [&](int64_t unit) { return (int)(((unit + 1) * (int)gridDim.x - 1) / total); };
+  const int lo = range_lo(blockIdx.x), hi = range_lo(blockIdx.x + 1);
+  struct Segment { int u, k0, k1; };
+  auto segment = [&](int pos) {
+    Segment g;
+    g.u = pos / p.kchunks;
+    g.k0 = pos - g.u * p.kchunks;
+    g.k1 = min(p.kchunks, g.k0 + hi - pos);
+    return g;
+  };
   bool ok = true;
 
   if (warp == WARP_TMA) {
@@ -265,19 +306,19 @@ __global__ void __launch_bounds__(THREADS, 1) proj_tc_kernel(const __grid_consta
     // converters have read it (fp32) or the MMA has (bf16).
     if (lane == 0) {
       int g = 0;
-      for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
-        const int u = item / p.slices, j = item - u * p.slices;
-        const int k0 = slice_lo(j), k1 = slice_lo(j + 1);
-        for (int mi = 0; mi < nacc && ok; ++mi) {
-          int m = mi, row0 = u * ROWS;
-          if (!p.swiglu) {
-            m = 0;
-            if (p.n_mats > 1 && u >= p.tile0[1]) m = 1;
-            if (p.n_mats > 2 && u >= p.tile0[2]) m = 2;
-            row0 = (u - p.tile0[m]) * ROWS;
-          }
-          const CUtensorMap* mw = m == 0 ? &mw0 : (m == 1 ? &mw1 : &mw2);
-          for (int kc = k0; kc < k1; ++kc, ++g) {
+      for (int pos = lo; pos < hi && ok;) {
+        const Segment sg = segment(pos);
+        pos += sg.k1 - sg.k0;
+        int m = 0, row0 = sg.u * ROWS;
+        if (!p.swiglu) {
+          if (p.n_mats > 1 && sg.u >= p.tile0[1]) m = 1;
+          if (p.n_mats > 2 && sg.u >= p.tile0[2]) m = 2;
+          row0 = (sg.u - p.tile0[m]) * ROWS;
+        }
+        for (int kc = sg.k0; kc < sg.k1 && ok; ++kc) {
+          for (int mi = 0; mi < nacc; ++mi, ++g) {
+            const int mm = p.swiglu ? mi : m;
+            const CUtensorMap* mw = mm == 0 ? &mw0 : (mm == 1 ? &mw1 : &mw2);
             const int s = g % SW;
             ok = mbar_wait(wempty(s), (uint32_t)(((g / SW) & 1) ^ 1), status, 1, g);
             if (!ok) break;
@@ -293,18 +334,16 @@ __global__ void __launch_bounds__(THREADS, 1) proj_tc_kernel(const __grid_consta
       mca_pdl_wait();                                     // the pieces are the pre-pass's output
       int g = 0, s = 0;
       uint32_t ph = 0;
-      for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
-        const int u = item / p.slices, j = item - u * p.slices;
-        const int k0 = slice_lo(j), k1 = slice_lo(j + 1);
-        for (int mi = 0; mi < nacc && ok; ++mi) {
-          for (int kc = k0; kc < k1; ++kc, ++g) {
-            ok = mbar_wait(xempty(s), ph ^ 1u, status, 8, g);
-            if (!ok) break;
-            mbar_expect_tx(xfull(s), x_stage_bytes);
-            // both pieces are consecutive rows of the array: one box
-            tma_load_2d(base + PL::OFF_X + s * x_stage_bytes, &mx, xfull(s), kc * KC, 0);
-            if (++s == SX) { s = 0; ph ^= 1u; }
-          }
+      for (int pos = lo; pos < hi && ok;) {
+        const Segment sg = segment(pos);
+        pos += sg.k1 - sg.k0;
+        for (int kc = sg.k0; kc < sg.k1; ++kc, ++g) {
+          ok = mbar_wait(xempty(s), ph ^ 1u, status, 8, g);
+          if (!ok) break;
+          mbar_expect_tx(xfull(s), x_stage_bytes);
+          // both pieces are consecutive rows of the array: one box
+          tma_load_2d(base + PL::OFF_X + s * x_stage_bytes, &mx, xfull(s), kc * KC, 0);
+          if (++s == SX) { s = 0; ph ^= 1u; }
         }
       }
     }
@@ -316,47 +355,47 @@ __global__ void __launch_bounds__(THREADS, 1) proj_tc_kernel(const __grid_consta
       const uint32_t idesc2 = make_idesc_fmt(ROWS, 2 * p.Bp, 0, 0, PL::FMT), idesc = make_idesc_fmt(ROWS, p.Bp, 0, 0, PL::FMT);
       int g = 0, it = 0, sx = 0;
       uint32_t xph = 0;
-      for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++it) {
-        const int u = item / p.slices, j = item - u * p.slices;
-        const int k0 = slice_lo(j), k1 = slice_lo(j + 1);
+      for (int pos = lo; pos < hi && ok; ++it) {
+        const Segment sg = segment(pos);
+        pos += sg.k1 - sg.k0;
         const int a = it & 1;
         ok = mbar_wait(accfree(a), (uint32_t)(((it >> 1) & 1) ^ 1), status, 2, it);
         if (!ok) break;
         tc_fence_after();
-        for (int mi = 0; mi < nacc && ok; ++mi) {
-          const uint32_t d_tmem = tmem_base + (uint32_t)a * ACC_COLS + (uint32_t)(mi * 2 * p.Bp);
-          for (int kc = k0; kc < k1; ++kc, ++g) {
+        for (int kc = sg.k0; kc < sg.k1 && ok; ++kc) {
+          ok = mbar_wait(xfull(sx), xph, status, 9, g);
+          if (!ok) break;
+          const uint32_t xs = base + PL::OFF_X + sx * x_stage_bytes;
+          for (int mi = 0; mi < nacc; ++mi, ++g) {       // the gated pair shares the chunk's activations
+            const uint32_t d_tmem = tmem_base + (uint32_t)a * ACC_COLS + (uint32_t)(mi * 2 * p.Bp);
             const int sw = g % SW;
             // fp32 weights: the slot holds the converted hi | lo tiles once all converter warps have arrived
             ok = mbar_wait(PL::CONVERT ? convdone(sw) : wfull(sw), (uint32_t)((g / SW) & 1), status, 3, g);
             if (!ok) break;
             const uint32_t a_hi = base + PL::OFF_W + sw * PL::W_BYTES, a_lo = a_hi + PL::OP_BYTES;
-            ok = mbar_wait(xfull(sx), xph, status, 9, g);
-            if (!ok) break;
             tc_fence_after();
-            const uint32_t xs = base + PL::OFF_X + sx * x_stage_bytes;
 #pragma unroll
             for (int kk = 0; kk < KC / 16; ++kk) {
-              const uint32_t first = (kc == k0 && kk == 0) ? 0u : 1u;
+              const uint32_t first = (kc == sg.k0 && kk == 0) ? 0u : 1u;
               const uint64_t dx = make_desc(xs + kk * 32, 16, 1024);
               umma_ss(d_tmem, make_desc(a_hi + kk * 32, 16, 1024), dx, idesc2, first);                             // W_hi . [x_hi | x_lo]
               if constexpr (PL::CONVERT) umma_ss(d_tmem, make_desc(a_lo + kk * 32, 16, 1024), dx, idesc, 1u);      // W_lo . x_hi
             }
             umma_commit(wempty(sw));
-            umma_commit(xempty(sx));
-            if (++sx == SX) { sx = 0; xph ^= 1u; }
           }
+          if (!ok) break;
+          umma_commit(xempty(sx));
+          if (++sx == SX) { sx = 0; xph ^= 1u; }
         }
         if (ok) umma_commit(accfull(a));
       }
     }
-  } else if (warp < CONV_WARPS) {
+  } else if (warp < WARP_EPI0) {
     // ------------------------------------------------------------------ converters (fp32 weights)
     if constexpr (PL::CONVERT) {
       int g = 0;
-      for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
-        const int u = item / p.slices, j = item - u * p.slices;
-        const int steps = nacc * (slice_lo(j + 1) - slice_lo(j));
+      {
+        const int steps = nacc * (hi - lo);
         for (int t = 0; t < steps; ++t, ++g) {
           const int s = g % SW;
           const bool mine = __all_sync(0xffffffffu, mbar_wait(wfull(s), (uint32_t)((g / SW) & 1), status, 5, g));
@@ -397,18 +436,19 @@ __global__ void __launch_bounds__(THREADS, 1) proj_tc_kernel(const __grid_consta
     }
   } else {
     // ------------------------------------------------------------------ epilogue warps
-    const int e = warp - WARP_EPI0;                       // TMEM lanes 32 e .. 32 e + 31
-    const int r = e * 32 + lane;                          // row of the tile
-    // per-sequence output scales, written by the pre-pass this launch may have overtaken: every warp keeps a copy
+    const int e = warp - WARP_EPI0, quarter = warp & 3;   // TMEM lanes 32 quarter .. 32 quarter + 31
+    const int r = quarter * 32 + lane;                    // row of the tile
+    const int col_first = (e >> 2) * 8;                   // this warp's columns: col_first + 16 i .. + 7
+    // per-sequence output scales, written by the pre-pass this launch may have overtaken: every warp writes the same copy
     mca_pdl_wait();
-    cs += e * MAX_B;
     cs[lane] = lane < p.B ? __ldcg(g_x_scale + lane) : 0.f;
     cs[lane + 32] = lane + 32 < p.B ? __ldcg(g_x_scale + lane + 32) : 0.f;
     __syncwarp();
-    const int ncols = nacc * p.Bp;
     int it = 0;
-    for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++it) {
-      const int u = item / p.slices, j = item - u * p.slices;
+    for (int pos = lo; pos < hi && ok; ++it) {
+      const Segment sg = segment(pos);
+      const int u = sg.u;
+      pos += sg.k1 - sg.k0;
       const int a = it & 1;
       int m = 0, row0 = u * ROWS;
       if (!p.swiglu) {
@@ -419,20 +459,28 @@ __global__ void __launch_bounds__(THREADS, 1) proj_tc_kernel(const __grid_consta
       float* outm = m == 0 ? p.out[0] : (m == 1 ? p.out[1] : p.out[2]);
       const int rows_m = m == 0 ? p.rows[0] : (m == 1 ? p.rows[1] : p.rows[2]);
       const int row = row0 + r;
+      const bool whole = sg.k0 == 0 && sg.k1 == p.kchunks;
+      // the parts of this tile: CTAs c_first .. c_last, all but the first of which begin inside it
+      const int c_first = owner((int64_t)u * p.kchunks), c_last = owner((int64_t)(u + 1) * p.kchunks - 1);
+      const int first_slot = 2 * c_first + (range_lo(c_first) / p.kchunks == u ? 0 : 1);
+      constexpr size_t SLOT = (size_t)2 * MAX_B * ROWS;   // floats of a part: (column, row)
+      auto slot_of = [&](int c) { return c == c_first ? first_slot : 2 * c; };
       ok = __all_sync(0xffffffffu, mbar_wait(accfull(a), (uint32_t)((it >> 1) & 1), status, 7, it));
       if (!ok) break;
       tc_fence_after();
-      const uint32_t t_acc = tmem_base + ((uint32_t)(e * 32) << 16) + (uint32_t)a * ACC_COLS;
-      // sixteen output elements of this thread's row: the products scaled back, gated if asked, added to the residual
-      // if asked (all sixteen residuals are requested before any is used)
-      auto finish16 = [&](int c0, const float (&va)[16], const float (&vb)[16]) {
+      const uint32_t t_acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)a * ACC_COLS;
+      // the residuals of eight output elements of this thread's row, requested before anything is waited for
+      auto residuals = [&](int c0, float (&res)[8]) {
+        const float* src = outm + (size_t)c0 * rows_m + row;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) res[i] = (p.accumulate && row < rows_m && c0 + i < p.B) ? __ldcg(src + (size_t)i * rows_m) : 0.f;
+      };
+      // eight output elements: the products scaled back, gated if asked, added to the residual
+      auto finish8 = [&](int c0, const float (&va)[8], const float (&vb)[8], const float (&res)[8]) {
         if (row >= rows_m) return;
-        float res[16];
         float* dst = outm + (size_t)c0 * rows_m + row;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) res[i] = (p.accumulate && c0 + i < p.B) ? __ldcg(dst + (size_t)i * rows_m) : 0.f;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
+        for (int i = 0; i < 8; ++i) {
           if (c0 + i < p.B) {
             const float sc = cs[c0 + i];
             float y = va[i] * sc;
@@ -444,82 +492,97 @@ __global__ void __launch_bounds__(THREADS, 1) proj_tc_kernel(const __grid_consta
           }
         }
       };
-      // sixteen columns of a result: the x_hi half plus the x_lo half
-      auto load_acc = [&](uint32_t t, int col, float (&v)[16]) {
-        uint32_t h[16], l[16];
-        tmem_ld16(t + col, h);
-        tmem_ld16(t + col + p.Bp, l);
+      // eight columns of a result: the x_hi half plus the x_lo half
+      auto load_acc = [&](uint32_t t, int col, float (&v)[8]) {
+        uint32_t h[8], l[8];
+        tmem_ld8(t + col, h);
+        tmem_ld8(t + col + p.Bp, l);
         tmem_wait_ld();
 #pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(h[i]) + __uint_as_float(l[i]);
+        for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(h[i]) + __uint_as_float(l[i]);
       };
-      if (p.slices == 1) {
-        for (int c0 = 0; c0 < p.Bp; c0 += 16) {
-          float fa[16], fb[16];
+      if (whole) {
+        for (int c0 = col_first; c0 < p.Bp; c0 += 16) {
+          float fa[8], fb[8], res[8];
+          residuals(c0, res);
           load_acc(t_acc, c0, fa);
           if (p.swiglu) load_acc(t_acc, 2 * p.Bp + c0, fb);
           else {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) fb[i] = 0.f;
+            for (int i = 0; i < 8; ++i) fb[i] = 0.f;
           }
-          finish16(c0, fa, fb);
+          finish8(c0, fa, fb, res);
         }
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(accfree(a));
-      } else {
-        float* part = g_partials + ((size_t)(u * p.slices + j) * ncols) * ROWS + r;
-        for (int c0 = 0; c0 < ncols; c0 += 16) {
-          float v[16];
-          load_acc(t_acc, c0 < p.Bp ? c0 : p.Bp + c0, v);   // the second result starts behind both halves of the first
+        continue;
+      }
+      float* part = g_partials + (size_t)slot_of(blockIdx.x) * SLOT + r;
+      for (int c0 = col_first; c0 < p.Bp; c0 += 16) {
+        for (int mi = 0; mi < nacc; ++mi) {
+          float v[8];
+          load_acc(t_acc, mi * 2 * p.Bp + c0, v);       // the second result starts behind both halves of the first
 #pragma unroll
-          for (int i = 0; i < 16; ++i) __stcg(part + (size_t)(c0 + i) * ROWS, v[i]);
+          for (int i = 0; i < 8; ++i) __stcg(part + (size_t)(mi * MAX_B + c0 + i) * ROWS, v[i]);
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(accfree(a));
-        // a ticket per (tile, quarter of its rows): the warp that arrives last for its quarter adds up all slices
-        __threadfence();
-        __syncwarp();
-        int last = 0;
-        if (lane == 0) {
-          const unsigned int old = atomicAdd(&g_tickets[u * EPI_WARPS + e], 1u);
-          last = old == (unsigned int)(p.slices - 1);
-          if (last) g_tickets[u * EPI_WARPS + e] = 0;    // ready for the next launch
-        }
-        last = __shfl_sync(0xffffffffu, last, 0);
-        if (last) {
-          __threadfence();
-          const float* p0 = g_partials + ((size_t)(u * p.slices) * ncols) * ROWS + r;
-          // Sixteen columns at a time, two slices per round: 32 loads are in flight together, and the sums are taken in
-          // slice order whoever arrived last.
-          auto gather = [&](int col0, float (&acc)[16]) {
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(accfree(a));
+      // a ticket per tile and epilogue warp: the one that arrives last adds up all parts
+      float res[8];
+      residuals(col_first, res);
+      __threadfence();
+      __syncwarp();
+      int last = 0;
+      if (lane == 0) {
+        const unsigned int old = atomicAdd(&g_tickets[u * EPI_WARPS + e], 1u);
+        last = old == (unsigned int)(c_last - c_first);
+        if (last) g_tickets[u * EPI_WARPS + e] = 0;    // ready for the next launch
+      }
+      last = __shfl_sync(0xffffffffu, last, 0);
+      if (!last) continue;
+      __threadfence();
+      // 64 loads in flight together; the sums are taken in the parts' order whoever arrived last
+      const float* p0 = g_partials + r;
+      for (int c0 = col_first; c0 < p.Bp; c0 += 16) {
+        float va[8], vb[8];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) acc[i] = 0.f;
-            for (int s0 = 0; s0 < p.slices; s0 += 2) {
-              float t[2][16];
+        for (int i = 0; i < 8; ++i) va[i] = vb[i] = 0.f;
+        if (c0 != col_first) residuals(c0, res);
+        if (p.swiglu) {
+          for (int s0 = c_first; s0 <= c_last; s0 += 4) {
+            float t[4][2][8];
 #pragma unroll
-              for (int q = 0; q < 2; ++q)
+            for (int q = 0; q < 4; ++q) {
+              const float* src = p0 + (size_t)slot_of(min(s0 + q, c_last)) * SLOT + (size_t)c0 * ROWS;
 #pragma unroll
-                for (int i = 0; i < 16; ++i)
-                  t[q][i] = s0 + q < p.slices ? __ldcg(p0 + ((size_t)(s0 + q) * ncols + col0 + i) * ROWS) : 0.f;
+              for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
-              for (int q = 0; q < 2; ++q)
-#pragma unroll
-                for (int i = 0; i < 16; ++i) acc[i] += t[q][i];
+                for (int i = 0; i < 8; ++i) t[q][mi][i] = s0 + q <= c_last ? __ldcg(src + (size_t)(mi * MAX_B + i) * ROWS) : 0.f;
             }
-          };
-          for (int c0 = 0; c0 < p.Bp; c0 += 16) {
-            float va[16], vb[16];
-            gather(c0, va);
-            if (p.swiglu) gather(p.Bp + c0, vb);
-            if (!p.swiglu) {
 #pragma unroll
-              for (int i = 0; i < 16; ++i) vb[i] = 0.f;
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+              for (int i = 0; i < 8; ++i) { va[i] += t[q][0][i]; vb[i] += t[q][1][i]; }
+          }
+        } else {
+          for (int s0 = c_first; s0 <= c_last; s0 += 8) {
+            float t[8][8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+              const float* src = p0 + (size_t)slot_of(min(s0 + q, c_last)) * SLOT + (size_t)c0 * ROWS;
+#pragma unroll
+              for (int i = 0; i < 8; ++i) t[q][i] = s0 + q <= c_last ? __ldcg(src + (size_t)i * ROWS) : 0.f;
             }
-            finish16(c0, va, vb);
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+#pragma unroll
+              for (int i = 0; i < 8; ++i) va[i] += t[q][i];
           }
         }
+        finish8(c0, va, vb, res);
       }
     }
   }
@@ -550,18 +613,7 @@ inline int make_map_2d(CUtensorMap* map, const void* basep, CUtensorMapDataType 
 
 inline bool& enabled() { static bool on = true; return on; }
 
-// K slices for `tiles` row tiles of `kchunks` stages each on `sms` SMs: the count that fills whole waves best, with at
-// least four stages per slice and at most MAX_ITEMS items.
-inline int pick_slices(int tiles, int kchunks, int sms) {
-  int best = 1;
-  double best_eff = (double)tiles / ((double)((tiles + sms - 1) / sms) * sms);
-  for (int s = 2; s <= 8; ++s) {
-    if (kchunks / s < 4 || tiles * s > MAX_ITEMS) break;
-    const int items = tiles * s;
-    const double eff = (double)items / ((double)((items + sms - 1) / sms) * sms);
-    if (eff > best_eff + 0.02) { best_eff = eff; best = s; }
-  }
-  return best;
-}
+// CTAs for `units` (row tile, k chunk) units on `sms` SMs: one per SM, with at least four units each.
+inline int pick_ctas(int64_t units, int sms) { return (int)std::max<int64_t>(1, std::min<int64_t>(std::min(sms, MAX_CTAS), units / 4)); }
 
 }  // namespace proj
