@@ -449,7 +449,7 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     float l[2] = {0.f, 0.f};                            // this thread's part of the row sums
     // split mode: the pre-pass scaled q and k by powers of two; dividing them out of the logit scale is exact
     float4 sc = make_float4(1.f, 1.f, 1.f, 1.f);
-    if constexpr (SPLIT) sc = __ldg(p.split_scale + bh);
+    if constexpr (SPLIT) sc = mca_ld_f4(reinterpret_cast<const float*>(p.split_scale + bh));
     const float scale_log2 = SPLIT ? p.scale_log2 * (1.0f / (sc.x * sc.y)) : p.scale_log2;
     for (int j = 0; j < n && ok; ++j) {
       TC_TRACE(x, j, 0);
@@ -638,7 +638,7 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         const int qi = qrow0 + row;
         const float lsum = red_l[row];
         // split mode: the pre-pass scaled v by a power of two; dividing it out here is exact
-        const float inv = SPLIT ? (1.0f / __ldg(p.split_scale + bh).z) / lsum : 1.0f / lsum;
+        const float inv = SPLIT ? (1.0f / mca_ld_f4(reinterpret_cast<const float*>(p.split_scale + bh)).z) / lsum : 1.0f / lsum;
         const uint32_t t_o32 = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(QT * BLK + x * BLK + half * OC);
         if constexpr (F32_OUT && QT == 2) {
           // fp32 output of the two-tile shape: each thread stores its own row's pieces.  (Staged like the other

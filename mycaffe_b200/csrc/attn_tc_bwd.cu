@@ -344,7 +344,7 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     const float lse = row_ok ? p.lse[(int64_t)bh * T + qi] : 0.f;
     const float delta = row_ok ? p.delta[(int64_t)bh * T + qi] : 0.f;
     float4 sc = make_float4(1.f, 1.f, 1.f, 1.f);   // powers of two: every product and quotient of them is exact
-    if constexpr (SPLIT) sc = __ldg(p.scales + bh);
+    if constexpr (SPLIT) sc = mca_ld_f4(reinterpret_cast<const float*>(p.scales + bh));
     const float sl2 = SPLIT ? p.scale_log2 * (1.0f / (sc.x * sc.y)) : p.scale_log2;
     const float dmul = SPLIT ? DS_SHIFT : p.scale;
     const float dsub = SPLIT ? delta * (sc.w * DS_SHIFT) * sc.z : delta * p.scale;
@@ -658,14 +658,14 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     float (*s_del)[BLK] = s_nlse + 2;
     // split mode: S^T and dP^T carry the pre-pass's scales; dS^T is kept in the units of dP' x 2^-19 and P^T 2^10 larger
     float4 sc = make_float4(1.f, 1.f, 1.f, 1.f);
-    if constexpr (SPLIT) sc = __ldg(p.scales + bh);
+    if constexpr (SPLIT) sc = mca_ld_f4(reinterpret_cast<const float*>(p.scales + bh));
     const float sl2 = SPLIT ? p.scale_log2 * (1.0f / (sc.x * sc.y)) : p.scale_log2;
     const float dmul = SPLIT ? DS_SHIFT : p.scale;
     const float del_mul = SPLIT ? (sc.w * DS_SHIFT) * sc.z : p.scale;
     auto fetch = [&](int it) -> float {
       const int qi = (i_begin + it) * BLK + (tid & (BLK - 1));
       if (tid >= 2 * BLK || it >= n || qi >= T) return tid < BLK ? -INFINITY : 0.f;
-      return tid < BLK ? -__ldg(p.lse + (int64_t)bh * T + qi) : -__ldg(p.delta + (int64_t)bh * T + qi) * del_mul;
+      return tid < BLK ? -mca_ld_f1(p.lse + (int64_t)bh * T + qi) : -mca_ld_f1(p.delta + (int64_t)bh * T + qi) * del_mul;
     };
     auto stage = [&](int it, float v) {
       if (tid < BLK) s_nlse[it & 1][tid] = v;
@@ -789,7 +789,7 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 
 // delta[row] = sum_c dY[row][c] * Y[row][c]  (bf16 inputs, fp32 result).  D / 8 lanes share a row (16-byte loads), so a
 // warp covers 256 / D rows.
-__global__ void bwd_delta_bf16_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ y,
+__global__ void bwd_delta_bf16_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* y,
                                       int64_t rows, int H, int T, int D, const McaStrides ys, float* __restrict__ delta) {
   mca_pdl_launch_dependents();
   mca_pdl_wait();   // dy and y are earlier kernels' output

@@ -131,6 +131,19 @@ static inline int mca_smem_once(std::atomic<uint64_t>& done, F kern, size_t byte
 
 __device__ __forceinline__ void mca_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void mca_pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Loads of what an earlier kernel wrote, in a kernel launched ahead of it: they stay behind mca_pdl_wait().  (A load through a
+// const __restrict__ pointer, or __ldg, promises that nobody writes the data while the kernel runs, and the compiler then
+// moves it up across the wait.)
+__device__ __forceinline__ float4 mca_ld_f4(const float* p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ float mca_ld_f1(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  return v;
+}
 
 inline bool mca_plain_launches() {   // MCA_NO_PDL: every launch the ordinary way (for comparisons)
   static const bool plain = getenv("MCA_NO_PDL") != nullptr;

@@ -401,9 +401,7 @@ __global__ void __launch_bounds__(DEC_THREADS, KVM == 1 ? 2 : 1) decode_split_ke
 
 // Combine pass: out[b,h,:] = sum_s exp(m_s - M) acc_s / sum_s exp(m_s - M) l_s.
 template <int HS>
-__global__ void __launch_bounds__(HS) decode_combine_kernel(const float* __restrict__ part_acc,
-                                                            const float* __restrict__ part_ml,
-                                                            const int* __restrict__ pos, int n_heads, int nsplit,
+__global__ void __launch_bounds__(HS) decode_combine_kernel(const float* part_acc, const float* part_ml, const int* pos, int n_heads, int nsplit,
                                                             int split_len, int pos_limit, float* __restrict__ out) {
   mca_pdl_launch_dependents();
   const int h = blockIdx.x, b = blockIdx.y, e = threadIdx.x;

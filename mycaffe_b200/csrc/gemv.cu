@@ -25,6 +25,7 @@
 // activation reads); larger batches take several passes.
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -388,7 +389,12 @@ int run_proj_tc(const GemvParams& p, cudaStream_t st) {
   // both kernels are launched programmatically dependent: the pre-pass's launch overlaps the tail of whatever runs
   // before it (it waits for that before it reads or writes anything), the contraction's set-up overlaps the pre-pass
   const int nv = mca_ceil_div(p.n, 4 * proj::X_THREADS);
-  auto pre = nv <= 2 ? proj::x_pieces_kernel<BF, 2> : nv <= 4 ? proj::x_pieces_kernel<BF, 4> : proj::x_pieces_kernel<BF, 8>;
+  const auto pick = [&](auto norm) {
+    constexpr bool N = decltype(norm)::value;
+    return nv <= 2 ? proj::x_pieces_kernel<BF, N, 2> : nv <= 4 ? proj::x_pieces_kernel<BF, N, 4> : nv <= 6 ? proj::x_pieces_kernel<BF, N, 6>
+                                                                                              : proj::x_pieces_kernel<BF, N, 8>;
+  };
+  auto pre = p.norm_w != nullptr ? pick(std::true_type{}) : pick(std::false_type{});
   if ((e = mca_launch_pdl(pre, dim3(Bp), dim3(proj::X_THREADS), 0, st, p.x, p.norm_w, p.eps, p.n, p.B, Bp, pieces, xscale))) return e;
   const size_t smem = proj::smem_bytes<WT>();
   auto kern = proj::proj_tc_kernel<WT>;

@@ -144,7 +144,7 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 // is a latency in front of every contraction (its x is the kernel before's last result), so the row is read once, with all
 // loads in flight and the norm's weights requested before that kernel has finished, and no shared memory is taken that an
 // SM still holding a contraction's CTA could not give (5.8 us of exposed time at n = 4096, 16 sequences -> MEASURED_XP).
-template <bool BF16, int NV>
+template <bool BF16, bool NORM, int NV>
 __global__ void __launch_bounds__(X_THREADS) x_pieces_kernel(const float* __restrict__ x, const float* __restrict__ norm_w, float eps,
                                                              int n, int B, int Bp, uint16_t* __restrict__ pieces,
                                                              float* __restrict__ xscale) {
@@ -152,8 +152,8 @@ __global__ void __launch_bounds__(X_THREADS) x_pieces_kernel(const float* __rest
   const int b = blockIdx.x, tid = threadIdx.x;
   mca_pdl_launch_dependents();                          // the contraction kernel may start fetching weights
   const bool live = b < B;
-  float4 g[NV], v[NV];
-  if (norm_w != nullptr && live) {
+  float4 g[NORM ? NV : 1], v[NV];
+  if (NORM && live) {
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int k = (tid + i * X_THREADS) * 4;
@@ -165,9 +165,9 @@ __global__ void __launch_bounds__(X_THREADS) x_pieces_kernel(const float* __rest
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int k = (tid + i * X_THREADS) * 4;
-    v[i] = live && k < n ? *reinterpret_cast<const float4*>(x + (size_t)b * n + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+    v[i] = live && k < n ? mca_ld_f4(x + (size_t)b * n + k) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  if (norm_w != nullptr && live) {
+  if (NORM && live) {
     float ss = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
@@ -177,7 +177,8 @@ __global__ void __launch_bounds__(X_THREADS) x_pieces_kernel(const float* __rest
     const float s = 1.0f / sqrtf(ss / (float)n + eps);
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      v[i].x = g[i].x * (s * v[i].x); v[i].y = g[i].y * (s * v[i].y); v[i].z = g[i].z * (s * v[i].z); v[i].w = g[i].w * (s * v[i].w);
+      const float4 gi = g[NORM ? i : 0];
+      v[i].x = gi.x * (s * v[i].x); v[i].y = gi.y * (s * v[i].y); v[i].z = gi.z * (s * v[i].z); v[i].w = gi.w * (s * v[i].w);
     }
   }
   float down = 1.f;
@@ -218,8 +219,10 @@ __global__ void __launch_bounds__(X_THREADS) x_pieces_kernel(const float* __rest
   }
 }
 
+// The register limit leaves room on the SM for a CTA of the pre-pass (512 threads of up to 32, or 40, registers): where it did
+// not, the SMs that held the pre-pass fetched no weights ahead and finished late.
 template <typename WT>
-__global__ void __launch_bounds__(Roles<Plan<WT>::CONVERT>::THREADS, 1) proj_tc_kernel(const __grid_constant__ CUtensorMap mw0,
+__global__ void __maxnreg__(Plan<WT>::CONVERT ? 72 : 112) proj_tc_kernel(const __grid_constant__ CUtensorMap mw0,
                                                              const __grid_constant__ CUtensorMap mw1,
                                                              const __grid_constant__ CUtensorMap mw2,
                                                              const __grid_constant__ CUtensorMap mx, const Params p) {
@@ -348,46 +351,54 @@ __global__ void __launch_bounds__(Roles<Plan<WT>::CONVERT>::THREADS, 1) proj_tc_
       }
     }
   } else if (warp == WARP_MMA) {
-    // ------------------------------------------------------------------ MMA issuer (one lane)
-    if (lane == 0) {
+    // ------------------------------------------------------------------ MMA issuer
+    // The warp runs this role in lock step and one elected lane issues: descriptors are warp-uniform values, made once and
+    // stepped by additions on their address field.  What a chunk costs the issuing thread is what bounds the kernel before
+    // the memory does.
+    {
+      const uint32_t leader = elect_one() ? 1u : 0u;
+      const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
       // hi and lo pieces of all sequences are one operand of 2 Bp columns: an instruction costs about the same up to 128
       // columns, so W . [x_hi | x_lo] is one instruction per 16 k, and the epilogue adds the two halves of its result
       const uint32_t idesc2 = make_idesc_fmt(ROWS, 2 * p.Bp, 0, 0, PL::FMT), idesc = make_idesc_fmt(ROWS, p.Bp, 0, 0, PL::FMT);
-      int g = 0, it = 0, sx = 0;
-      uint32_t xph = 0;
+      const uint64_t desc_w = make_desc(base + PL::OFF_W, 16, 1024), desc_x = make_desc(base + PL::OFF_X, 16, 1024);
+      const uint32_t x_step = x_stage_bytes >> 4;
+      int sw = 0, sx = 0, it = 0, g = 0;
+      uint32_t wph = 0, xph = 0;
       for (int pos = lo; pos < hi && ok; ++it) {
         const Segment sg = segment(pos);
-        pos += sg.k1 - sg.k0;
+        const int n = sg.k1 - sg.k0;
+        pos += n;
         const int a = it & 1;
-        ok = mbar_wait(accfree(a), (uint32_t)(((it >> 1) & 1) ^ 1), status, 2, it);
+        ok = __all_sync(0xffffffffu, mbar_wait(accfree(a), (uint32_t)(((it >> 1) & 1) ^ 1), status, 2, it));
         if (!ok) break;
         tc_fence_after();
-        for (int kc = sg.k0; kc < sg.k1 && ok; ++kc) {
-          ok = mbar_wait(xfull(sx), xph, status, 9, g);
+        const uint32_t d0 = tmem_u + (uint32_t)a * ACC_COLS;
+        for (int kc = 0; kc < n && ok; ++kc) {
+          ok = __all_sync(0xffffffffu, mbar_wait(xfull(sx), xph, status, 9, g));
           if (!ok) break;
-          const uint32_t xs = base + PL::OFF_X + sx * x_stage_bytes;
+          const uint64_t dx = desc_x + (uint64_t)((uint32_t)sx * x_step);
           for (int mi = 0; mi < nacc; ++mi, ++g) {       // the gated pair shares the chunk's activations
-            const uint32_t d_tmem = tmem_base + (uint32_t)a * ACC_COLS + (uint32_t)(mi * 2 * p.Bp);
-            const int sw = g % SW;
             // fp32 weights: the slot holds the converted hi | lo tiles once all converter warps have arrived
-            ok = mbar_wait(PL::CONVERT ? convdone(sw) : wfull(sw), (uint32_t)((g / SW) & 1), status, 3, g);
+            ok = __all_sync(0xffffffffu, mbar_wait(PL::CONVERT ? convdone(sw) : wfull(sw), wph, status, 3, g));
             if (!ok) break;
-            const uint32_t a_hi = base + PL::OFF_W + sw * PL::W_BYTES, a_lo = a_hi + PL::OP_BYTES;
             tc_fence_after();
+            const uint32_t d_tmem = d0 + (uint32_t)(mi * 2 * p.Bp);
+            const uint64_t dw = desc_w + (uint64_t)((uint32_t)sw * (PL::W_BYTES >> 4));
 #pragma unroll
             for (int kk = 0; kk < KC / 16; ++kk) {
-              const uint32_t first = (kc == sg.k0 && kk == 0) ? 0u : 1u;
-              const uint64_t dx = make_desc(xs + kk * 32, 16, 1024);
-              umma_ss(d_tmem, make_desc(a_hi + kk * 32, 16, 1024), dx, idesc2, first);                             // W_hi . [x_hi | x_lo]
-              if constexpr (PL::CONVERT) umma_ss(d_tmem, make_desc(a_lo + kk * 32, 16, 1024), dx, idesc, 1u);      // W_lo . x_hi
+              umma_ss_if<false>(leader, d_tmem, dw + 2 * kk, dx + 2 * kk, idesc2, (kc | kk) != 0 ? 1u : 0u);   // W_hi . [x_hi | x_lo]
+              if constexpr (PL::CONVERT)
+                umma_ss_if<false>(leader, d_tmem, dw + (PL::OP_BYTES >> 4) + 2 * kk, dx + 2 * kk, idesc, 1u);  // W_lo . x_hi
             }
-            umma_commit(wempty(sw));
+            umma_commit_if(leader, wempty(sw));
+            if (++sw == SW) { sw = 0; wph ^= 1u; }
           }
           if (!ok) break;
-          umma_commit(xempty(sx));
+          umma_commit_if(leader, xempty(sx));
           if (++sx == SX) { sx = 0; xph ^= 1u; }
         }
-        if (ok) umma_commit(accfull(a));
+        if (ok) umma_commit_if(leader, accfull(a));
       }
     }
   } else if (warp < WARP_EPI0) {
@@ -544,7 +555,7 @@ __global__ void __launch_bounds__(Roles<Plan<WT>::CONVERT>::THREADS, 1) proj_tc_
       last = __shfl_sync(0xffffffffu, last, 0);
       if (!last) continue;
       __threadfence();
-      // 64 loads in flight together; the sums are taken in the parts' order whoever arrived last
+      // all of a round's loads in flight together; the sums are taken in the parts' order whoever arrived last
       const float* p0 = g_partials + r;
       for (int c0 = col_first; c0 < p.Bp; c0 += 16) {
         float va[8], vb[8];
@@ -552,10 +563,11 @@ __global__ void __launch_bounds__(Roles<Plan<WT>::CONVERT>::THREADS, 1) proj_tc_
         for (int i = 0; i < 8; ++i) va[i] = vb[i] = 0.f;
         if (c0 != col_first) residuals(c0, res);
         if (p.swiglu) {
-          for (int s0 = c_first; s0 <= c_last; s0 += 4) {
-            float t[4][2][8];
+          constexpr int Q = PL::CONVERT ? 2 : 4;
+          for (int s0 = c_first; s0 <= c_last; s0 += Q) {
+            float t[Q][2][8];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
+            for (int q = 0; q < Q; ++q) {
               const float* src = p0 + (size_t)slot_of(min(s0 + q, c_last)) * SLOT + (size_t)c0 * ROWS;
 #pragma unroll
               for (int mi = 0; mi < 2; ++mi)
@@ -563,21 +575,22 @@ __global__ void __launch_bounds__(Roles<Plan<WT>::CONVERT>::THREADS, 1) proj_tc_
                 for (int i = 0; i < 8; ++i) t[q][mi][i] = s0 + q <= c_last ? __ldcg(src + (size_t)(mi * MAX_B + i) * ROWS) : 0.f;
             }
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
+            for (int q = 0; q < Q; ++q)
 #pragma unroll
               for (int i = 0; i < 8; ++i) { va[i] += t[q][0][i]; vb[i] += t[q][1][i]; }
           }
         } else {
-          for (int s0 = c_first; s0 <= c_last; s0 += 8) {
-            float t[8][8];
+          constexpr int Q = PL::CONVERT ? 4 : 8;
+          for (int s0 = c_first; s0 <= c_last; s0 += Q) {
+            float t[Q][8];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
+            for (int q = 0; q < Q; ++q) {
               const float* src = p0 + (size_t)slot_of(min(s0 + q, c_last)) * SLOT + (size_t)c0 * ROWS;
 #pragma unroll
               for (int i = 0; i < 8; ++i) t[q][i] = s0 + q <= c_last ? __ldcg(src + (size_t)i * ROWS) : 0.f;
             }
 #pragma unroll
-            for (int q = 0; q < 8; ++q)
+            for (int q = 0; q < Q; ++q)
 #pragma unroll
               for (int i = 0; i < 8; ++i) va[i] += t[q][i];
           }

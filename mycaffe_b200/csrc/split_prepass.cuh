@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(THREADS) split_kernel(const Job job, const Mca
       float acc = 0.f;
       if (in) {
         const float* yd = ydot + (out_row0 + row) * HD + c8;
-        const float4 y0 = *reinterpret_cast<const float4*>(yd), y1 = *reinterpret_cast<const float4*>(yd + 4);
+        const float4 y0 = mca_ld_f4(yd), y1 = mca_ld_f4(yd + 4);
         acc = fmaf(v0.x, y0.x, fmaf(v0.y, y0.y, fmaf(v0.z, y0.z, v0.w * y0.w)));
         acc += fmaf(v1.x, y1.x, fmaf(v1.y, y1.y, fmaf(v1.z, y1.z, v1.w * y1.w)));
       }
