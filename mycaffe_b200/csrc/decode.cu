@@ -61,6 +61,7 @@ struct DecodeParams {
   float* out;            // (B, n_heads*HS)
   int64_t cache_batch_stride;  // elements between sequences in the caches
   int n_heads, n_kv_heads, kv_mul, seq_len, split_len, nsplit;
+  int prefetch;          // launched ahead of the kernel before it: ask L2 for the split's rows meanwhile
   int pos_limit;         // positions must lie in [0, pos_limit): the planned splits and the cache cover no more
 };
 
@@ -161,6 +162,22 @@ __global__ void __launch_bounds__(DEC_THREADS, KVM == 1 ? 2 : 1) decode_split_ke
   __shared__ float s_ml[DEC_WARPS][KVM][2];
 
   mca_pdl_launch_dependents();   // a projection kernel that follows may start fetching its weights
+  if (p.prefetch) {
+    // The cache rows depend on nothing the kernels before this one compute (all but the new token's row), so they are asked
+    // for before the wait -- into L2, not registers: should the position or a row still be in the making, the wrong or
+    // stale lines of a prefetch harm nothing.
+    const int pb = *reinterpret_cast<const volatile int*>(p.pos + blockIdx.z);
+    if (pb >= 0 && pb < p.pos_limit) {
+      const int r0 = blockIdx.x * p.split_len, rows = min(pb, r0 + p.split_len) - r0;
+      constexpr int LINES = (HS * (int)sizeof(CT) + 127) / 128;
+      const int64_t off = (int64_t)blockIdx.z * p.cache_batch_stride + (int64_t)(blockIdx.y * KVM / p.kv_mul) * HS;
+      for (int i = threadIdx.x; i < rows * LINES; i += DEC_THREADS) {
+        const int64_t at = (off + (int64_t)(r0 + i / LINES) * p.n_kv_heads * HS) * (int)sizeof(CT) + (i % LINES) * 128;
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const char*>(p.k_cache) + at));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const char*>(p.v_cache) + at));
+      }
+    }
+  }
   mca_pdl_wait();                // launched ahead of the kernels before it: q is their output, and the scratch theirs to read
   const int b = blockIdx.z;
   const int h0 = blockIdx.y * KVM;          // first query head of this CTA
@@ -485,7 +502,7 @@ __global__ void __launch_bounds__(256) decode_exchange_kernel(const ExchangePara
 }
 
 template <typename CT, int HS>
-int launch_decode(const DecodeParams& p, int B, cudaStream_t st) {
+int launch_decode(const DecodeParams& p, int B, bool combine, cudaStream_t st) {
   const int kvmt = p.kv_mul >= 4 ? 4 : p.kv_mul;
   dim3 grid(p.nsplit, p.n_heads / kvmt, B);
   const size_t smem = sizeof(CT) == 2 ? DecRing<Epl<CT, HS>::value / 8>::BYTES : 0;   // the bf16 path's cp.async ring
@@ -518,7 +535,7 @@ int launch_decode(const DecodeParams& p, int B, cudaStream_t st) {
     e = mca_launch_status();
   }
   if (e) return e;
-  if (p.nsplit > 1) {
+  if (p.nsplit > 1 && combine) {
     // programmatic dependent launch: the combine pass is resident and waiting when the last split finishes
     e = mca_launch_pdl(decode_combine_kernel<HS>, dim3(p.n_heads, B), dim3(HS), 0, st, (const float*)p.part_acc,
                        (const float*)p.part_ml, p.pos, p.n_heads, p.nsplit, p.split_len, p.pos_limit, p.out);
@@ -603,10 +620,10 @@ int mca_decode_attention_static(const float* q, const float* k_new, const float*
                               MCA_STATIC_SCRATCH_FLOATS, out, stream);
 }
 
-int mca_decode_attention(const float* q, const float* k_new, const float* v_new, void* k_cache, void* v_cache,
-                         int cache_is_bf16, int64_t cache_batch_stride, const int* pos, int B, int n_heads,
-                         int n_kv_heads, int head_size, int seq_len, int max_len, const float* freq_real,
-                         const float* freq_imag, float* scratch, int64_t scratch_floats, float* out, void* stream) {
+static int decode_attention(const float* q, const float* k_new, const float* v_new, void* k_cache, void* v_cache,
+                            int cache_is_bf16, int64_t cache_batch_stride, const int* pos, int B, int n_heads, int n_kv_heads,
+                            int head_size, int seq_len, int max_len, const float* freq_real, const float* freq_imag, float* scratch,
+                            int64_t scratch_floats, float* out, McaDecodePartials* partials, void* stream) {
   if (!q || !k_cache || !v_cache || !pos || !out) return ERROR_PARAM_NULL;
   if ((k_new == nullptr) != (v_new == nullptr)) return ERROR_PARAM_NULL;
   if ((freq_real == nullptr) != (freq_imag == nullptr)) return ERROR_PARAM_NULL;
@@ -636,14 +653,34 @@ int mca_decode_attention(const float* q, const float* k_new, const float* v_new,
   p.pos_limit = max_len;   // <= seq_len, and the planned splits cover [0, max_len)
   if (p.kv_mul > 4 && p.kv_mul % 4 != 0) return ERROR_ATTN_UNSUPPORTED_SHAPE;
   if (p.kv_mul == 3) return ERROR_ATTN_UNSUPPORTED_SHAPE;
+  p.prefetch = B <= 8;     // exactly the launches made ahead (launch_decode)
+  if (partials != nullptr)
+    *partials = McaDecodePartials{p.part_acc, p.part_ml, pos, n_heads, head_size, p.nsplit, p.split_len, p.pos_limit};
+  const bool combine = partials == nullptr;
   cudaStream_t st = (cudaStream_t)stream;
   switch (head_size) {
 #define MCA_DECODE_CASE(HS_) \
-    case HS_: return cache_is_bf16 ? launch_decode<__nv_bfloat16, HS_>(p, B, st) : launch_decode<float, HS_>(p, B, st);
+    case HS_: return cache_is_bf16 ? launch_decode<__nv_bfloat16, HS_>(p, B, combine, st) : launch_decode<float, HS_>(p, B, combine, st);
     MCA_DECODE_CASE(32) MCA_DECODE_CASE(48) MCA_DECODE_CASE(64) MCA_DECODE_CASE(96) MCA_DECODE_CASE(128)
 #undef MCA_DECODE_CASE
   }
   return ERROR_ATTN_UNSUPPORTED_SHAPE;
+}
+
+int mca_decode_attention(const float* q, const float* k_new, const float* v_new, void* k_cache, void* v_cache,
+                         int cache_is_bf16, int64_t cache_batch_stride, const int* pos, int B, int n_heads, int n_kv_heads,
+                         int head_size, int seq_len, int max_len, const float* freq_real, const float* freq_imag, float* scratch,
+                         int64_t scratch_floats, float* out, void* stream) {
+  return decode_attention(q, k_new, v_new, k_cache, v_cache, cache_is_bf16, cache_batch_stride, pos, B, n_heads, n_kv_heads, head_size,
+                          seq_len, max_len, freq_real, freq_imag, scratch, scratch_floats, out, nullptr, stream);
+}
+
+int mca_decode_attention_partials(const float* q, const float* k_new, const float* v_new, void* k_cache, void* v_cache,
+                                  int cache_is_bf16, int64_t cache_batch_stride, const int* pos, int B, int n_heads, int n_kv_heads,
+                                  int head_size, int seq_len, int max_len, const float* freq_real, const float* freq_imag,
+                                  float* scratch, int64_t scratch_floats, float* out, McaDecodePartials* partials, void* stream) {
+  return decode_attention(q, k_new, v_new, k_cache, v_cache, cache_is_bf16, cache_batch_stride, pos, B, n_heads, n_kv_heads, head_size,
+                          seq_len, max_len, freq_real, freq_imag, scratch, scratch_floats, out, partials, stream);
 }
 
 int mca_decode_head_size_supported(int head_size) {

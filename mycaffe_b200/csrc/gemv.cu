@@ -62,7 +62,49 @@ struct GemvParams {
   int swiglu;                    // out[0][r] = silu(w[0] row r . x) * (w[1] row r . x); rows[1] == rows[0]
   int split;                     // S: warps of a CTA that share a row along K (1, 2, 4 or 8)
   float eps;
+  // x as the split-KV attention left it, one (maximum, sum) pair and hs weighted values per (sequence, head, split): the
+  // combine pass happens where the activations are staged (part_acc null: x is the input)
+  const float* part_acc = nullptr;
+  const float* part_ml = nullptr;
+  const int* pos = nullptr;
+  int n_heads = 0, hs = 0, nsplit = 0, split_len = 0, pos_limit = 0;
 };
+
+// Four values of the attention output of sequence b from its partials: sum_s exp(m_s - M) acc_s / sum_s exp(m_s - M) l_s.
+__device__ __forceinline__ float4 combine_partials(const GemvParams& p, int b, int k) {
+  const int h = k / p.hs, pb = p.pos[b];
+  float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (pb < 0 || pb >= p.pos_limit) return o;      // refused by the attention
+  const int n = min(p.nsplit, (pb + p.split_len) / p.split_len);
+  const int64_t slot0 = ((int64_t)b * p.n_heads + h) * p.nsplit;
+  const float* pa = p.part_acc + slot0 * p.hs + (k - h * p.hs);
+  const float* ml = p.part_ml + slot0 * 2;
+  float M = -INFINITY, ls = 0.f;
+  for (int s0 = 0; s0 < n; s0 += 8) {
+    float4 a[8];
+    float2 t[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int s = min(s0 + j, n - 1);
+      a[j] = mca_ld_f4(pa + (int64_t)s * p.hs);
+      t[j] = mca_ld_f2(ml + 2 * s);
+    }
+    float m8 = M;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) m8 = fmaxf(m8, t[j].x);
+    const float f0 = __expf(M - m8);              // 0 the first time
+    ls *= f0; o.x *= f0; o.y *= f0; o.z *= f0; o.w *= f0;
+    M = m8;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float f = s0 + j < n ? __expf(t[j].x - M) : 0.f;
+      ls = fmaf(t[j].y, f, ls);
+      o.x = fmaf(a[j].x, f, o.x); o.y = fmaf(a[j].y, f, o.y); o.z = fmaf(a[j].z, f, o.z); o.w = fmaf(a[j].w, f, o.w);
+    }
+  }
+  const float inv = 1.f / ls;
+  return make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
+}
 
 // NB sequences per pass, R weight rows per step per warp (they share the activation reads from
 // shared memory), THREADS per CTA, DEPTH ring steps per warp, each of U warp-wide vectors per row.  GLU: the two rows of a step are
@@ -144,7 +186,7 @@ __global__ void __launch_bounds__(THREADS) gemv_stream_kernel(const GemvParams p
   for (int k = tid * 4; k < n; k += THREADS * 4) {
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
-      const float4 v = *reinterpret_cast<const float4*>(p.x + (int64_t)(b0 + b) * n + k);
+      const float4 v = p.part_acc != nullptr ? combine_partials(p, b0 + b, k) : *reinterpret_cast<const float4*>(p.x + (int64_t)(b0 + b) * n + k);
       *reinterpret_cast<float4*>(xs + b * n + k) = v;
       ss[b] += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
     }
@@ -324,9 +366,17 @@ int launch_pass(GemvParams p, int b0, cudaStream_t st) {
     ctas_per_sm = c_ctas; sms = c_sms;
   }
   int grid = sms * std::max(1, ctas_per_sm);
-  int S = 1;
-  while (S < WARPS && total_steps / (grid * WARPS / S) < 8) S *= 2;
-  if (S > 1 && mca_ceil_div(total_steps, grid * WARPS / S) > GV_SPLIT_STEPS) S = 1;   // cannot happen by construction
+  // S warps share a row where that shortens the longest warp's walk: its ring steps are (row steps of a group) x (chunks of a
+  // row per warp), plus about one for the extra sum over the group.  (A rule on the row count alone gave short rows to
+  // eight warps of which only as many as it has chunks had work: a 110M model's feed-forward pair 5.7 -> MEASURED us.)
+  const int chunks = mca_ceil_div(p.n, 32 * WLoad<WT>::VEC * U);
+  int S = 1, best = INT32_MAX;
+  for (int c = 1; c <= WARPS; c *= 2) {
+    const int steps = mca_ceil_div(total_steps, grid * (WARPS / c));
+    if (c > 1 && (steps > GV_SPLIT_STEPS || c > chunks)) continue;
+    const int walk = steps * mca_ceil_div(chunks, c) + (c > 1 ? 1 : 0);
+    if (walk < best) { best = walk; S = c; }
+  }
   if (grid * (WARPS / S) > total_steps) grid = mca_ceil_div(total_steps, WARPS / S);
   p.split = S;
   return mca_launch_pdl(kern, dim3(grid), dim3(THREADS), smem, st, p, b0);
@@ -473,6 +523,20 @@ int mca_decode_out_proj(const float* attn, const void* wo, int weights_bf16, int
   p.w[0] = wo; p.w[1] = p.w[2] = nullptr;
   p.out[0] = x_inout; p.out[1] = p.out[2] = nullptr;
   p.rows[0] = dim; p.rows[1] = p.rows[2] = 0;
+  return weights_bf16 ? run_gemv<__nv_bfloat16>(p, (cudaStream_t)stream) : run_gemv<float>(p, (cudaStream_t)stream);
+}
+
+int mca_decode_out_proj_partials(const McaDecodePartials* a, const void* wo, int weights_bf16, int B, int dim, float* x_inout,
+                                 void* stream) {
+  if (B > 8 || dim % 8 != 0 || !al16(wo) || !al16(a->acc)) return ERROR_PARAM_OUT_OF_RANGE;
+  GemvParams p;
+  p.swiglu = 0;
+  p.x = nullptr; p.norm_w = nullptr; p.eps = 0.f; p.n = dim; p.B = B; p.accumulate = 1; p.n_mats = 1;
+  p.w[0] = wo; p.w[1] = p.w[2] = nullptr;
+  p.out[0] = x_inout; p.out[1] = p.out[2] = nullptr;
+  p.rows[0] = dim; p.rows[1] = p.rows[2] = 0;
+  p.part_acc = a->acc; p.part_ml = a->ml; p.pos = a->pos;
+  p.n_heads = a->n_heads; p.hs = a->hs; p.nsplit = a->nsplit; p.split_len = a->split_len; p.pos_limit = a->pos_limit;
   return weights_bf16 ? run_gemv<__nv_bfloat16>(p, (cudaStream_t)stream) : run_gemv<float>(p, (cudaStream_t)stream);
 }
 

@@ -24,3 +24,18 @@ int mca_set_fail_words_bwd(int* words);
 int mca_set_fail_words_probe(int* words);
 int mca_set_fail_words_decode(int* words);
 int mca_set_fail_words_proj(int* words);
+
+// Internal: the decode attention without its combine pass, for up to eight sequences whose partials mca_decode_out_proj_partials
+// combines while it stages its activations.  *partials is filled in when more than one split was planned; with one (nsplit 1)
+// the output is in `out` as mca_decode_attention leaves it.
+struct McaDecodePartials {
+  const float *acc, *ml;
+  const int* pos;
+  int n_heads, hs, nsplit, split_len, pos_limit;
+};
+int mca_decode_attention_partials(const float* q, const float* k_new, const float* v_new, void* k_cache, void* v_cache,
+                                  int cache_is_bf16, int64_t cache_batch_stride, const int* pos, int B, int n_heads, int n_kv_heads,
+                                  int head_size, int seq_len, int max_len, const float* freq_real, const float* freq_imag,
+                                  float* scratch, int64_t scratch_floats, float* out, McaDecodePartials* partials, void* stream);
+int mca_decode_out_proj_partials(const McaDecodePartials* partials, const void* wo, int weights_bf16, int B, int dim, float* x_inout,
+                                 void* stream);

@@ -138,8 +138,13 @@ class TransformerGpu:
             raise ValueError("configuration not supported (heads must divide dim, kv heads must divide heads)")
         self.workspace = torch.empty(need, device=self.device)
         self.logits = torch.empty(B, cfg["vocab_size"], device=self.device)
-        self._tokens = torch.zeros(B, dtype=torch.int32, device=self.device)
-        self._pos = torch.zeros(B, dtype=torch.int32, device=self.device)
+        # a step's inputs and its result cross the bus as one copy each, to and from pinned memory on the step's stream
+        self._inputs = torch.zeros(2, B, dtype=torch.int32, device=self.device)
+        self._tokens, self._pos = self._inputs[0], self._inputs[1]
+        self._inputs_host = torch.zeros(2, B, dtype=torch.int32, pin_memory=True)
+        self._inputs_np = self._inputs_host.numpy()
+        self._logits_host = torch.empty(B, cfg["vocab_size"], pin_memory=True)
+        self._logits_np = self._logits_host.numpy()
         self._w_c = McaLlamaWeights(*[t[n].data_ptr() for n in ("token_embedding_table", "rms_att_weight",
                                                                  "rms_ffn_weight", "rms_final_weight", "wq", "wk", "wv",
                                                                  "wo", "w1", "w2", "w3", "wcls")],
@@ -160,16 +165,18 @@ class TransformerGpu:
             raise RuntimeError(f"mca_llama_forward failed with {rc}")
 
     def _capture(self):
-        """One graph serves every token: tokens and positions are read from device memory, and the
-        split plan is the one for the longest sequence the cache holds (splits beyond a sequence's
-        length return at once)."""
+        """One graph serves every token: the copies either side of the step use fixed pinned buffers, tokens and positions
+        are read from device memory, and the split plan is the one for the longest sequence the cache holds (splits
+        beyond a sequence's length return at once)."""
         torch = self._torch
         side = torch.cuda.Stream(self.device)
         graph = torch.cuda.CUDAGraph()
         side.wait_stream(torch.cuda.current_stream(self.device))
         with torch.cuda.stream(side):
             graph.capture_begin()
+            self._inputs.copy_(self._inputs_host, non_blocking=True)
             self.enqueue(self.config["seq_len"], stream=side)
+            self._logits_host.copy_(self.logits, non_blocking=True)
             graph.capture_end()
         torch.cuda.current_stream(self.device).wait_stream(side)
         self._graph = graph
@@ -179,22 +186,24 @@ class TransformerGpu:
         torch = self._torch
         if self.config is None:
             raise RuntimeError("build() has not been called")
-        tokens = np.asarray(tokens, np.int32).reshape(self.batch)
-        pos = np.asarray(pos, np.int32).reshape(self.batch)
-        if pos.min() < 0 or pos.max() >= self.config["seq_len"]:
+        inputs = self._inputs_np          # the previous step has been waited for: nothing reads it any more
+        inputs[0] = np.asarray(tokens, np.int32).reshape(self.batch)
+        inputs[1] = np.asarray(pos, np.int32).reshape(self.batch)
+        lo, hi = min(inputs[1].tolist()), max(inputs[1].tolist())
+        if lo < 0 or hi >= self.config["seq_len"]:
             raise ValueError("position outside the cache")
         with torch.cuda.device(self.device):
-            self._tokens.copy_(torch.from_numpy(tokens))
-            self._pos.copy_(torch.from_numpy(pos))
+            stream = torch.cuda.current_stream(self.device)
             if self._graph is not None:
                 self._graph.replay()
             else:
-                self.enqueue(int(pos.max()) + 1)     # also the warm-up that precedes a capture
-                if self.use_graph:
-                    result = self.logits.cpu().numpy()
-                    self._capture()
-                    return result
-            result = self.logits.cpu().numpy()     # synchronises
+                self._inputs.copy_(self._inputs_host, non_blocking=True)
+                self.enqueue(hi + 1, stream)     # also the warm-up that precedes a capture
+                self._logits_host.copy_(self.logits, non_blocking=True)
+            stream.synchronize()
+            result = self._logits_np.copy()
+            if self._graph is None and self.use_graph:
+                self._capture()
             if self.batch > 8:
                 # above eight sequences the projections run on the tensor cores: a bounded wait that gave up there
                 # leaves stale logits and a status word
