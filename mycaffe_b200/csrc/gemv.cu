@@ -186,7 +186,8 @@ __global__ void __launch_bounds__(THREADS) gemv_stream_kernel(const GemvParams p
   for (int k = tid * 4; k < n; k += THREADS * 4) {
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
-      const float4 v = p.part_acc != nullptr ? combine_partials(p, b0 + b, k) : *reinterpret_cast<const float4*>(p.x + (int64_t)(b0 + b) * n + k);
+      const int bb = min(b0 + b, p.B - 1);   // a pass may be padded: the last sequence again, its sums not written
+      const float4 v = p.part_acc != nullptr ? combine_partials(p, bb, k) : *reinterpret_cast<const float4*>(p.x + (int64_t)bb * n + k);
       *reinterpret_cast<float4*>(xs + b * n + k) = v;
       ss[b] += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
     }
@@ -227,6 +228,7 @@ __global__ void __launch_bounds__(THREADS) gemv_stream_kernel(const GemvParams p
 #pragma unroll
       for (int b = 0; b < NB; ++b) {
         // val = hb * (1 / (1 + exp(-hb))) * hb2, llama2_cpu.cpp:359-367
+        if (b0 + b >= p.B) continue;
         float val = v[0][b];
         val *= (1.0f / (1.0f + expf(-val)));
         val *= v[R - 1][b];
@@ -242,6 +244,7 @@ __global__ void __launch_bounds__(THREADS) gemv_stream_kernel(const GemvParams p
         const int orows = m == 0 ? p.rows[0] : (m == 1 ? p.rows[1] : p.rows[2]);
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
+          if (b0 + b >= p.B) continue;
           float* dst = ob + (int64_t)(b0 + b) * orows + rr;
           *dst = p.accumulate ? (*dst + v[q][b]) : v[q][b];
         }
@@ -368,7 +371,7 @@ int launch_pass(GemvParams p, int b0, cudaStream_t st) {
   int grid = sms * std::max(1, ctas_per_sm);
   // S warps share a row where that shortens the longest warp's walk: its ring steps are (row steps of a group) x (chunks of a
   // row per warp), plus about one for the extra sum over the group.  (A rule on the row count alone gave short rows to
-  // eight warps of which only as many as it has chunks had work: a 110M model's feed-forward pair 5.7 -> MEASURED us.)
+  // eight warps of which only as many as it has chunks had work: a 110M model's feed-forward pair 9.8 -> 6.8 us.)
   const int chunks = mca_ceil_div(p.n, 32 * WLoad<WT>::VEC * U);
   int S = 1, best = INT32_MAX;
   for (int c = 1; c <= WARPS; c *= 2) {
@@ -465,21 +468,23 @@ int run_gemv(const GemvParams& p, cudaStream_t st) {
   constexpr size_t RING_1 = ring_bytes<1, 256, 4, 4>();   // = ring_bytes<2, 256, 4, 2>(), the one- and two-sequence kernels
   if (!fits(1, RING_1)) return ERROR_ATTN_UNSUPPORTED_SHAPE;
   const bool deep = xbytes + ring_bytes<1, 256, 6, 4>() <= 112 * 1024;   // half an SM's shared memory, less the per-CTA reserve
+  // Passes of 8, 4, 2 or 1 sequences; 5 to 7, and 3, are one padded pass (the weights are read once, and a pass over a small
+  // matrix is mostly launch and latency) where the padded activations fit.
   for (int b0 = 0; b0 < p.B && !e;) {
     const int left = p.B - b0;
     if (p.swiglu) {
-      if (left >= 8 && fits(8, RING_512)) { e = launch_pass<WT, 8, 2, 512, true, 6>(p, b0, st); b0 += 8; }
-      else if (left >= 4 && fits(4, RING_512)) { e = launch_pass<WT, 4, 2, 512, true, 6>(p, b0, st); b0 += 4; }
-      else if (left >= 4 && fits(4, RING_256)) { e = launch_pass<WT, 4, 2, 256, true, 6>(p, b0, st); b0 += 4; }
+      if (left >= 5 && fits(8, RING_512)) { e = launch_pass<WT, 8, 2, 512, true, 6>(p, b0, st); b0 += 8; }
+      else if (left >= 3 && fits(4, RING_512)) { e = launch_pass<WT, 4, 2, 512, true, 6>(p, b0, st); b0 += 4; }
+      else if (left >= 3 && fits(4, RING_256)) { e = launch_pass<WT, 4, 2, 256, true, 6>(p, b0, st); b0 += 4; }
       else if (left >= 2 && fits(2, RING_1)) { e = launch_pass<WT, 2, 2, 256, true, 4, 2>(p, b0, st); b0 += 2; }
       else {   // a deeper ring while two CTAs per SM still fit
         e = deep ? launch_pass<WT, 1, 2, 256, true, 6, 2>(p, b0, st) : launch_pass<WT, 1, 2, 256, true, 4, 2>(p, b0, st);
         b0 += 1;
       }
     } else {
-      if (left >= 8 && fits(8, RING_512)) { e = launch_pass<WT, 8, 2, 512, false, 6>(p, b0, st); b0 += 8; }
-      else if (left >= 4 && fits(4, RING_512)) { e = launch_pass<WT, 4, 2, 512, false, 6>(p, b0, st); b0 += 4; }
-      else if (left >= 4 && fits(4, RING_256)) { e = launch_pass<WT, 4, 2, 256, false, 6>(p, b0, st); b0 += 4; }
+      if (left >= 5 && fits(8, RING_512)) { e = launch_pass<WT, 8, 2, 512, false, 6>(p, b0, st); b0 += 8; }
+      else if (left >= 3 && fits(4, RING_512)) { e = launch_pass<WT, 4, 2, 512, false, 6>(p, b0, st); b0 += 4; }
+      else if (left >= 3 && fits(4, RING_256)) { e = launch_pass<WT, 4, 2, 256, false, 6>(p, b0, st); b0 += 4; }
       else if (left >= 2 && fits(2, RING_1)) { e = launch_pass<WT, 2, 1, 256, false, 4, 4>(p, b0, st); b0 += 2; }
       else {
         e = deep ? launch_pass<WT, 1, 1, 256, false, 6, 4>(p, b0, st) : launch_pass<WT, 1, 1, 256, false, 4, 4>(p, b0, st);

@@ -1,0 +1,35 @@
+"""Decode steps of one to nine sequences: the padded passes of the streaming projections (3, 5, 6 and 7 sequences), rows that are
+or are not shared by warps, splits with and without a combine pass, against the restated step over several tokens."""
+import numpy as np
+import pytest
+
+import oracle
+from helpers import rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("B", [1, 2, 3, 5, 6, 7, 8, 9])
+@pytest.mark.parametrize("dim,hidden,n_heads,n_kv,seq", [(288, 768, 6, 6, 64), (256, 1032, 4, 2, 700)])
+def test_steps_match_the_restated_model(B, dim, hidden, n_heads, n_kv, seq):
+    from mycaffe_b200.llama2 import TransformerGpu
+    rng = np.random.default_rng(B * 100 + dim)
+    cfg = dict(dim=dim, hidden_dim=hidden, n_layers=2, n_heads=n_heads, n_kv_heads=n_kv, vocab_size=77, seq_len=seq)
+    kv = dim // n_heads * n_kv
+    g = lambda *sh: (0.08 * rng.standard_normal(sh)).astype(np.float32)
+    w = {"rms_att_weight": 1 + g(2, dim), "rms_ffn_weight": 1 + g(2, dim), "rms_final_weight": 1 + g(dim),
+         "token_embedding_table": rng.standard_normal((77, dim)).astype(np.float32), "wq": g(2, dim, dim), "wk": g(2, kv, dim),
+         "wv": g(2, kv, dim), "wo": g(2, dim, dim), "w1": g(2, hidden, dim), "w2": g(2, dim, hidden), "w3": g(2, hidden, dim),
+         "wcls": g(77, dim)}
+    t = TransformerGpu(0, batch=B, use_graph=True)
+    t.load_weights(cfg, w)
+    kc, vc = (rng.standard_normal((2, B, seq, kv)).astype(np.float32) for _ in range(2))   # a context already in the caches
+    t.key_cache.copy_(t._torch.from_numpy(kc))
+    t.value_cache.copy_(t._torch.from_numpy(vc))
+    pos = rng.integers(0, seq - 3, B)
+    pos[0] = seq - 4
+    for step in range(3):                                  # eager, then from the graph
+        tok = rng.integers(0, 77, B)
+        ref = oracle.llama_forward(cfg, w, kc, vc, list(tok), list(pos + step))
+        assert rel_err(t.forward_batch(tok, pos + step), ref) < 1e-4
+    assert rel_err(t.key_cache.cpu().numpy(), kc) < 1e-5   # the appended rows, and nothing else
