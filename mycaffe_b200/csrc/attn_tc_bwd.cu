@@ -23,6 +23,8 @@
 // the pre-pass in split_prepass.cuh, each tensor scaled by a power of two), every product is the three kind::f16
 // products hi.hi + hi.lo + lo.hi into one fp32 TMEM tile, P^T / dS / dS^T are split the same way by the element-wise
 // warps, and the gradients are written in fp32.  Head sizes up to 64: a split tile is as large as a 128-wide bf16 one.
+#include <type_traits>
+
 #include "kernels.h"
 #include "tc_common.cuh"
 #include "split_prepass.cuh"
@@ -375,25 +377,33 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       const float2 zero2 = make_float2(0.f, 0.f);
       uint32_t pk[16];
       uint32_t pk_lo[SPLIT ? 16 : 1];
+      // keys of this thread's 32 that its row sees
+      const int visible = min(T, p.causal ? qi + 1 : T) - k0;
+      // Only the diagonal tile (causal) and the last one (keys beyond T) test their elements, in a loop of their own: tests in
+      // the other tiles' loop cost branches and selects per pair.  Rows beyond T need none: dY is zero there, and so is dS.
+      auto form_ds = [&](auto edge_tag) {
+        constexpr bool EDGE = decltype(edge_tag)::value;
 #pragma unroll
-      for (int i = 0; i < 32; i += 2) {
-        const float2 x = ffma2(make_float2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), sc2, nl2);
-        const float2 g = ffma2(make_float2(__uint_as_float(dp[i]), __uint_as_float(dp[i + 1])), ps2, nd2);
-        float e0 = fast_exp2(x.x), e1 = fast_exp2(x.y);
-        if constexpr (MASKED) {
-          if (((mw >> i) & 1u) == 0u) e0 = p_masked;
-          if (((mw >> (i + 1)) & 1u) == 0u) e1 = p_masked;
+        for (int i = 0; i < 32; i += 2) {
+          const float2 x = ffma2(make_float2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), sc2, nl2);
+          const float2 g = ffma2(make_float2(__uint_as_float(dp[i]), __uint_as_float(dp[i + 1])), ps2, nd2);
+          float e0 = fast_exp2(x.x), e1 = fast_exp2(x.y);
+          if constexpr (MASKED) {
+            if (((mw >> i) & 1u) == 0u) e0 = p_masked;
+            if (((mw >> (i + 1)) & 1u) == 0u) e1 = p_masked;
+          }
+          const float2 d = ffma2(make_float2(e0, e1), g, zero2);
+          float d0 = d.x, d1 = d.y;
+          if constexpr (EDGE) {
+            if (i >= visible) d0 = 0.f;
+            if (i + 1 >= visible) d1 = 0.f;
+          }
+          if constexpr (SPLIT) split_pack(d0, d1, pk[i / 2], pk_lo[i / 2]);
+          else pk[i / 2] = pack_bf16(d0, d1);
         }
-        const float2 d = ffma2(make_float2(e0, e1), g, zero2);
-        float d0 = d.x, d1 = d.y;
-        if (edge) {
-          const int kj = k0 + i;
-          if (!row_ok || kj >= T || (p.causal && kj > qi)) d0 = 0.f;
-          if (!row_ok || kj + 1 >= T || (p.causal && kj + 1 > qi)) d1 = 0.f;
-        } else if (!row_ok) { d0 = 0.f; d1 = 0.f; }
-        if constexpr (SPLIT) split_pack(d0, d1, pk[i / 2], pk_lo[i / 2]);
-        else pk[i / 2] = pack_bf16(d0, d1);
-      }
+      };
+      if (edge) form_ds(std::true_type{});
+      else form_ds(std::false_type{});
       if (j > 0) {  // the previous dQ product must have consumed the previous dS
         ok = __all_sync(0xffffffffu, mbar_wait(bar(DQ_DQ_DONE), (uint32_t)((j - 1) & 1), p.status, 131, j));
         if (!ok) break;
@@ -649,7 +659,6 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     const int kj = k0 + row;               // this thread's key
     constexpr int OC = HD / 4;
     const uint32_t t_row = tmem_base + ((uint32_t)lane_base << 16);
-    const bool key_ok = kj < T;
     // The query-dependent terms (minus log-sum-exp, minus delta x scale) are the same for every key row: the first 256
     // element-wise threads fetch one value each a step ahead and stage them in shared memory, so that the
     // inner loop reads them as broadcasts instead of 64 global loads per thread.  Rows beyond T get
@@ -700,34 +709,44 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       uint32_t pk_lo[SPLIT ? 16 : 1];
       tmem_ld32(t_row + C_ST + qtr * 32, s);
       tmem_wait_ld();
+      // The causal test is the diagonal tile's alone (a loop of its own, as in the dQ kernel).  A key beyond T needs none: its
+      // row of P^T and dS^T reaches only its own rows of dV and dK, which are not stored.
+      auto form_p = [&](auto diag_tag) {
+        constexpr bool DIAG = decltype(diag_tag)::value;
+        const int first = kj - q_base;      // queries before the key do not see it
 #pragma unroll
-      for (int i = 0; i < 32; i += 4) {
-        const float4 nl = *reinterpret_cast<const float4*>(nlse_s + i);
-        const float nls[4] = {nl.x, nl.y, nl.z, nl.w};
+        for (int i = 0; i < 32; i += 4) {
+          const float4 nl = *reinterpret_cast<const float4*>(nlse_s + i);
+          const float nls[4] = {nl.x, nl.y, nl.z, nl.w};
 #pragma unroll
-        for (int e = 0; e < 4; e += 2) {
-          const float2 x = ffma2(make_float2(__uint_as_float(s[i + e]), __uint_as_float(s[i + e + 1])), sc2,
-                                 make_float2(nls[e], nls[e + 1]));
-          float v0 = fast_exp2(x.x), v1 = fast_exp2(x.y);
-          if constexpr (MASKED) {
-            // a masked entry: 0, or 1 / T in a fully masked row (staged -lse = -inf; rows beyond T are staged the same
-            // way and stay 0)
-            if (((mw >> (i + e)) & 1u) == 0u) v0 = (nls[e] == -INFINITY && q_base + i + e < T) ? p.inv_T : 0.f;
-            if (((mw >> (i + e + 1)) & 1u) == 0u) v1 = (nls[e + 1] == -INFINITY && q_base + i + e + 1 < T) ? p.inv_T : 0.f;
+          for (int e = 0; e < 4; e += 2) {
+            const float2 x = ffma2(make_float2(__uint_as_float(s[i + e]), __uint_as_float(s[i + e + 1])), sc2,
+                                   make_float2(nls[e], nls[e + 1]));
+            float v0 = fast_exp2(x.x), v1 = fast_exp2(x.y);
+            if constexpr (MASKED) {
+              // a masked entry: 0, or 1 / T in a fully masked row (staged -lse = -inf; rows beyond T are staged the same
+              // way and stay 0)
+              if (((mw >> (i + e)) & 1u) == 0u) v0 = (nls[e] == -INFINITY && q_base + i + e < T) ? p.inv_T : 0.f;
+              if (((mw >> (i + e + 1)) & 1u) == 0u) v1 = (nls[e + 1] == -INFINITY && q_base + i + e + 1 < T) ? p.inv_T : 0.f;
+            }
+            if constexpr (DIAG) {
+              if (first > i + e) v0 = 0.f;
+              if (first > i + e + 1) v1 = 0.f;
+            }
+            s[i + e] = __float_as_uint(v0);
+            s[i + e + 1] = __float_as_uint(v1);
           }
-          if (!key_ok || (diag && kj > q_base + i + e)) v0 = 0.f;
-          if (!key_ok || (diag && kj > q_base + i + e + 1)) v1 = 0.f;
-          s[i + e] = __float_as_uint(v0);
-          s[i + e + 1] = __float_as_uint(v1);
+          if constexpr (SPLIT) {
+            split_pack(__uint_as_float(s[i]) * PT_SHIFT, __uint_as_float(s[i + 1]) * PT_SHIFT, pk[i / 2], pk_lo[i / 2]);
+            split_pack(__uint_as_float(s[i + 2]) * PT_SHIFT, __uint_as_float(s[i + 3]) * PT_SHIFT, pk[i / 2 + 1], pk_lo[i / 2 + 1]);
+          } else {
+            pk[i / 2] = pack_bf16(__uint_as_float(s[i]), __uint_as_float(s[i + 1]));
+            pk[i / 2 + 1] = pack_bf16(__uint_as_float(s[i + 2]), __uint_as_float(s[i + 3]));
+          }
         }
-        if constexpr (SPLIT) {
-          split_pack(__uint_as_float(s[i]) * PT_SHIFT, __uint_as_float(s[i + 1]) * PT_SHIFT, pk[i / 2], pk_lo[i / 2]);
-          split_pack(__uint_as_float(s[i + 2]) * PT_SHIFT, __uint_as_float(s[i + 3]) * PT_SHIFT, pk[i / 2 + 1], pk_lo[i / 2 + 1]);
-        } else {
-          pk[i / 2] = pack_bf16(__uint_as_float(s[i]), __uint_as_float(s[i + 1]));
-          pk[i / 2 + 1] = pack_bf16(__uint_as_float(s[i + 2]), __uint_as_float(s[i + 3]));
-        }
-      }
+      };
+      if (diag) form_p(std::true_type{});
+      else form_p(std::false_type{});
       tmem_st16(t_row + C_ST + qtr * 32, pk);
       if constexpr (SPLIT) tmem_st16(t_row + C_ST + qtr * 32 + 16, pk_lo);
       tmem_wait_st();
@@ -788,29 +807,45 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 }
 
 // delta[row] = sum_c dY[row][c] * Y[row][c]  (bf16 inputs, fp32 result).  D / 8 lanes share a row (16-byte loads), so a
-// warp covers 256 / D rows.
-__global__ void bwd_delta_bf16_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* y,
-                                      int64_t rows, int H, int T, int D, const McaStrides ys, float* __restrict__ delta) {
+// warp covers 256 / D rows; a CTA takes DELTA_STEPS of those per warp.  The kernel stands between the forward's tail and the
+// dK/dV kernel, so dY (which the forward does not write) is asked for into L2 before the wait, and all of a thread's loads
+// are in flight together behind it: T = 7001, 16 heads x 128: 18 us behind the forward -> 15.
+constexpr int DELTA_STEPS = 4;
+__global__ void __launch_bounds__(256) bwd_delta_bf16_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* y, int64_t rows, int H, int T,
+                                                             int D, const McaStrides ys, float* __restrict__ delta) {
   mca_pdl_launch_dependents();
-  mca_pdl_wait();   // dy and y are earlier kernels' output
   const int lane = threadIdx.x & 31, g = D / 8, rpw = 32 / g;        // g in {8, 16}
-  const int64_t row = ((int64_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5)) * rpw + lane / g;
-  float acc = 0.f;
-  if (row < rows) {
-    const unsigned bh = (unsigned)(row / T), bi = bh / (unsigned)H;
-    const int64_t off = (int64_t)bi * ys.b + (int64_t)(bh - bi * H) * ys.h + (row - (int64_t)bh * T) * ys.t + (lane % g) * 8;
-    const uint4 a = *reinterpret_cast<const uint4*>(dy + off);       // y and dy share the output layout
-    const uint4 b = *reinterpret_cast<const uint4*>(y + off);
-    const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
+  const int64_t row0 = ((int64_t)blockIdx.x * (256 / 32) + (threadIdx.x >> 5)) * rpw * DELTA_STEPS + lane / g;
+  int64_t off[DELTA_STEPS];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2 fa = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&aw[i]));
-      const float2 fb = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&bw[i]));
+  for (int i = 0; i < DELTA_STEPS; ++i) {
+    const int64_t row = min(row0 + i * rpw, rows - 1);
+    const unsigned bh = (unsigned)(row / T), bi = bh / (unsigned)H;
+    off[i] = (int64_t)bi * ys.b + (int64_t)(bh - bi * H) * ys.h + (row - (int64_t)bh * T) * ys.t + (lane % g) * 8;
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(dy + off[i]));
+  }
+  mca_pdl_wait();   // dy and y are earlier kernels' output
+  float4 a[DELTA_STEPS], b[DELTA_STEPS];
+#pragma unroll
+  for (int i = 0; i < DELTA_STEPS; ++i) {
+    a[i] = mca_ld_f4(reinterpret_cast<const float*>(dy + off[i]));   // y and dy share the output layout
+    b[i] = mca_ld_f4(reinterpret_cast<const float*>(y + off[i]));
+  }
+#pragma unroll
+  for (int i = 0; i < DELTA_STEPS; ++i) {
+    const uint32_t aw[4] = {__float_as_uint(a[i].x), __float_as_uint(a[i].y), __float_as_uint(a[i].z), __float_as_uint(a[i].w)};
+    const uint32_t bw[4] = {__float_as_uint(b[i].x), __float_as_uint(b[i].y), __float_as_uint(b[i].z), __float_as_uint(b[i].w)};
+    float acc = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 fa = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&aw[e]));
+      const float2 fb = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&bw[e]));
       acc = fmaf(fa.x, fb.x, fmaf(fa.y, fb.y, acc));
     }
+    for (int o = g / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    const int64_t row = row0 + i * rpw;
+    if (row < rows && lane % g == 0) delta[row] = acc;
   }
-  for (int o = g / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (row < rows && lane % g == 0) delta[row] = acc;
 }
 
 // Both kernels of one backward, with or without the caller's mask.
@@ -941,7 +976,7 @@ int mca_sdpa_backward_tc_masked(const void* q, const void* k, const void* v, con
   const int64_t rows = (int64_t)B * H * T;
   int e;
   {
-    const int64_t rows_per_block = 8 * (256 / D);   // eight warps, 256 / D rows each
+    const int64_t rows_per_block = 8 * (256 / D) * DELTA_STEPS;   // eight warps, 256 / D rows each a step
     e = mca_launch_pdl(bwd_delta_bf16_kernel, dim3((unsigned)((rows + rows_per_block - 1) / rows_per_block)), dim3(256), 0, st,
                        (const __nv_bfloat16*)dy, (const __nv_bfloat16*)y, rows, H, T, D, mca_out_strides(layout, H, T, D), delta_scratch);
   }
