@@ -11,9 +11,11 @@
 //
 // One CTA owns two 128-row query tiles of one (batch, head) and walks the keys 128 at a time:
 //   warps 0-7     softmax of query tile 0, warps 8-15 of query tile 1.  A warp reads 16 rows x
-//                 128 keys of S in the 16-lane quad layout (four threads per row), so the row
-//                 maximum and sum are two shuffles, no shared memory and no barrier; the two
-//                 groups run independently, one tile's exponentials over the other's loads.
+//                 128 keys of S in the 16-lane quad layout (four threads per row): one vote tells
+//                 whether any row's reference maximum has to be raised, and only then, and for the
+//                 final sums, do the four exchange anything; the two groups run independently.
+//                 P is handed to the MMA warp in three pieces (64, 32, 32 keys), so that a quarter
+//                 of P V is left to do when the last exponential is.
 //   warp 16       TMA producer (one lane)
 //   warp 17       MMA issuer: the warp runs in lock step and one elected lane issues, so that
 //                 descriptors are warp-uniform values (the issuing thread's instruction count per
@@ -97,6 +99,12 @@ template <int HD, int MODE, bool NARROW> struct Shape {
   static constexpr int THREADS = (QT * 8 + 2) * 32;
   static constexpr int CTAS_PER_SM = NARROW ? 2 : 1;
   static constexpr uint32_t TMEM_COLS = QT == 1 ? 256 : 512;   // S tiles in [0, QT x 128), O tiles behind them
+  // P apart from S, in columns [192, 256) that a narrow CTA of bf16 heads up to 64 wide has to spare: the next S is then
+  // formed as soon as the softmax warps hold this one in registers, and neither product stands in the way of the softmax
+  // from one tile to the next (elsewhere P overwrites S, and the next S waits for P V).  B=4 H=12 T=15832 D=64: 2.20 ->
+  // 2.11 ms, where the 1000 W power cap (1.56 GHz instead of 1.9) and the exponentials (1024 cycles a tile) are the bound.
+  static constexpr bool P_APART = NARROW && MODE == MODE_BF16 && HD <= 64;
+  static constexpr uint32_t P_COL = P_APART ? 192 : 0;
   static_assert(CTAS_PER_SM * (PL::BYTES + 1024) <= 227 * 1024, "shared memory of the CTAs of one SM");
 };
 
@@ -108,11 +116,13 @@ enum Bar : int {  // mbarrier indices
   BAR_V_EMPTY = 8,
   BAR_S_FULL = 10,   // [NQT]  S tile written by the MMA
   BAR_P_READY = 12,  // [NQT]  P written (and O rescaled) by the softmax warpgroup
-  BAR_O_DONE = 14,   // [NQT]  P V product of the step finished
+  BAR_O_DONE = 14,   // [NQT]  the last step's P V product finished (P_APART: every step's)
   BAR_DRAIN = 16,
   BAR_P_HALF = 17,   // [NQT]  first 64 key columns of P written
   BAR_RED = 19,      // [NQT]  the group's row sums are in shared memory (epilogue)
-  BAR_COUNT = 21
+  BAR_P_MOST = 21,   // [NQT]  first 96
+  BAR_S_FREE = 23,   // P_APART: S is in the softmax warps' registers
+  BAR_COUNT = 24
 };
 
 // Optional timeline capture for tuning (compiled out unless MCA_TC_TRACE is defined): one CTA
@@ -185,6 +195,7 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   constexpr int QT = SH::QT, STG = SH::STG;
   constexpr int WARP_TMA = SH::WARP_TMA, WARP_MMA = SH::WARP_MMA;
   constexpr uint32_t TMEM_COLS = SH::TMEM_COLS;
+  constexpr bool P_APART = SH::P_APART;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -339,15 +350,15 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           }
         }
       };
-      auto issue_pv = [&](int x, int st, bool first, int half) {
+      auto issue_pv = [&](int x, int st, bool first, int q_lo, int q_hi) {   // quarters of the keys
         // A: P rows in TMEM, 8 columns per step (16 bf16 or 8 tf32).  bf16 P is packed two keys per column
         // into the first 64 columns of the S tile; tf32 P overwrites S column for column.
         // B: V, one step = 16 or 8 key rows of 128 bytes per sub-tile.
         const uint64_t dv = desc_v0 + (uint64_t)((st * PL::TILE_BYTES) >> 4);
         const uint32_t d_tmem = tmem_base_u + QT * BLK + x * BLK;
-        const uint32_t a_tmem = tmem_base_u + x * BLK;
+        const uint32_t a_tmem = tmem_base_u + x * BLK + SH::P_COL;
 #pragma unroll
-        for (int kk = half * (KSTEPS_PV / 2); kk < (half + 1) * (KSTEPS_PV / 2); ++kk) {
+        for (int kk = q_lo * (KSTEPS_PV / 4); kk < q_hi * (KSTEPS_PV / 4); ++kk) {
           if constexpr (SPLIT) {
             // O += Phi Vhi + Phi Vlo + Plo Vhi: Phi in columns [0,64) of the S region, Plo in [64,128)
             const uint64_t dvk = dv + (uint64_t)((uint32_t)kk * V_STEP);
@@ -385,6 +396,17 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         if (!ok) break;
         TC_TRACE(3, j, 1);
         bool k_next_ready = false;
+        if constexpr (P_APART) {
+          if (j + 1 < n_max) {
+            ok = __all_sync(0xffffffffu, mbar_wait(bar(BAR_K_FULL + st_n), ph_n, p.status, 25, j));
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar(BAR_S_FREE), (uint32_t)(j & 1), p.status, 42, j));
+            if (!ok) break;
+            tc_fence_after();
+            issue_qk(0, st_n);
+            commit_by_leader(bar(BAR_S_FULL));
+            commit_by_leader(bar(BAR_K_EMPTY + st_n));
+          }
+        }
 #pragma unroll
         for (int x = 0; x < NQT; ++x) {
           if (j < n_tiles[x]) {
@@ -393,30 +415,32 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             if (!ok) break;
             TC_TRACE(2, j, x * 4 + 1);
             tc_fence_after();
-            issue_pv(x, st, j == 0, 0);
+            issue_pv(x, st, j == 0, 0, 2);
+            if (!P_APART && j + 1 < n_tiles[x] && !k_next_ready) {   // long there: waited for here, off the way from P to the next S
+              ok = __all_sync(0xffffffffu, mbar_wait(bar(BAR_K_FULL + st_n), ph_n, p.status, 25, j));
+              if (!ok) break;
+              k_next_ready = true;
+            }
+            ok = __all_sync(0xffffffffu, mbar_wait(bar(BAR_P_MOST + x), (uint32_t)(j & 1), p.status, 40 + x, j));
+            if (!ok) break;
+            tc_fence_after();
+            issue_pv(x, st, j == 0, 2, 3);
             ok = __all_sync(0xffffffffu, mbar_wait(bar(BAR_P_READY + x), (uint32_t)(j & 1), p.status, 23 + x, j));
             if (!ok) break;
             TC_TRACE(2, j, x * 4 + 3);
             tc_fence_after();
-            issue_pv(x, st, j == 0, 1);
+            issue_pv(x, st, j == 0, 3, 4);
             TC_TRACE(3, j, 4 + x);
-            commit_by_leader(bar(BAR_O_DONE + x));
+            if (!P_APART && j + 1 < n_tiles[x]) {
+              issue_qk(x, st_n);
+              commit_by_leader(bar(BAR_S_FULL + x));   // a commit covers every product before it: this one P V(j) too
+              TC_TRACE(2, j, x * 4 + 2);
+            } else {
+              commit_by_leader(bar(BAR_O_DONE + x));
+            }
           }
           if (x == NQT - 1) commit_by_leader(bar(BAR_V_EMPTY + st));
-          if (j + 1 < n_tiles[x]) {
-            if (!k_next_ready) {
-              TC_TRACE(3, j, 2);
-              ok = __all_sync(0xffffffffu, mbar_wait(bar(BAR_K_FULL + st_n), ph_n, p.status, 25, j));
-              if (!ok) break;
-              TC_TRACE(3, j, 3);
-              tc_fence_after();
-              k_next_ready = true;
-            }
-            issue_qk(x, st_n);
-            commit_by_leader(bar(BAR_S_FULL + x));
-            TC_TRACE(2, j, x * 4 + 2);
-          }
-          if (x == NQT - 1 && j + 1 < n_max) {
+          if (!P_APART && x == NQT - 1 && j + 1 < n_max) {
             if (!k_next_ready) {  // no query tile needs this K tile any more (cannot happen for n_max), keep the ring moving
               ok = __all_sync(0xffffffffu, mbar_wait(bar(BAR_K_FULL + st_n), ph_n, p.status, 26, j));
               if (!ok) break;
@@ -464,6 +488,11 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       tmem_ldq256_x8(t_s, s);
       tmem_ldq256_x8(t_s + 64, s + 32);
       tmem_wait_ld();
+      if constexpr (P_APART) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(BAR_S_FREE));
+      }
       TC_TRACE(x, j, 2);
       // Only the diagonal tile (causal) and the last tile (keys beyond T) need masking.
       if ((p.causal && j * BLK + BLK - 1 > qrow0) || (j * BLK + BLK > T)) {
@@ -490,6 +519,9 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           if (((w >> (8 * (g & 3) + e)) & 1u) == 0u && s[i] != 0xff800000u) s[i] = masked_s;
         }
       }
+      // Has a logit of this warp's rows outgrown its row's reference point?  That needs no row maximum: every thread looks
+      // at its own 32 logits of each row, and one vote tells the warp.  (The exchange between the four threads of a row
+      // is left to the rare step that raises a reference point.)
       float mx[2];
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -499,48 +531,40 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           ma = max3(ma, __uint_as_float(s[4 * g + 2 * h]), __uint_as_float(s[4 * g + 2 * h + 1]));
           mb = max3(mb, __uint_as_float(s[4 * g + 4 + 2 * h]), __uint_as_float(s[4 * g + 4 + 2 * h + 1]));
         }
-        float m = fmaxf(ma, mb);
-        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
-        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
-        mx[h] = m * scale_log2;
+        mx[h] = fmaxf(ma, mb) * scale_log2;
       }
+      const bool grown = mx[0] > m_used[0] + RESCALE_THRESHOLD || mx[1] > m_used[1] + RESCALE_THRESHOLD;
       TC_TRACE_W(j, 1);
-      float m_new[2];
-      bool raise = false;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        m_new[h] = m_used[h];
-        if (mx[h] > m_used[h] + RESCALE_THRESHOLD || j == 0) { m_new[h] = fmaxf(mx[h], m_used[h]); raise = raise || (j > 0); }
-        if (m_new[h] == -INFINITY) m_new[h] = 0.f;  // a row with no visible key yet (rows beyond T)
+      if constexpr (P_APART) {   // the previous P V product reads P, and O may be rescaled
+        if (j > 0) {
+          ok = __all_sync(0xffffffffu, mbar_wait(bar(BAR_O_DONE), (uint32_t)((j - 1) & 1), p.status, 32, j));
+          if (!ok) break;
+          tc_fence_after();
+        }
       }
-      if (__any_sync(0xffffffffu, raise)) {
-        // rescale this warp's 16 rows of O in TMEM: the previous P V product must have finished
-        ok = __all_sync(0xffffffffu, mbar_wait(bar(BAR_O_DONE + x), (uint32_t)((j - 1) & 1), p.status, 32 + x, j));
-        if (!ok) break;
-        tc_fence_after();
+      if (j == 0 || __any_sync(0xffffffffu, grown)) {
         float f[2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          f[h] = (m_new[h] != m_used[h]) ? fast_exp2(m_used[h] - m_new[h]) : 1.0f;
+          mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
+          mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
+          float m_new = mx[h] > m_used[h] + RESCALE_THRESHOLD ? mx[h] : m_used[h];
+          if (m_new == -INFINITY) m_new = 0.f;   // a row with no visible key yet (rows beyond T)
+          f[h] = m_new != m_used[h] ? fast_exp2(m_used[h] - m_new) : 1.0f;
           l[h] *= f[h];
+          m_used[h] = m_new;
         }
-        if constexpr (HD >= 32) {
+        if (j > 0) {
+          // rescale this warp's 16 rows of O in TMEM: the previous P V product has finished (P over S: before this S did)
 #pragma unroll
-          for (int c = 0; c < HD / 32; ++c) {
-            uint32_t o[16];
-            tmem_ldq256_x4(t_o + c * 32, o);
+          for (int c = 0; c < HD / 16; ++c) {   // 16 columns at a time: the logits are held in registers meanwhile
+            uint32_t o[8];
+            tmem_ldq256_x2(t_o + c * 16, o);
             tmem_wait_ld();
 #pragma unroll
-            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f[(i >> 1) & 1]);
-            tmem_stq256_x4(t_o + c * 32, o);
+            for (int i = 0; i < 8; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f[(i >> 1) & 1]);
+            tmem_stq256_x2(t_o + c * 16, o);
           }
-        } else {   // 16 columns
-          uint32_t o[8];
-          tmem_ldq256_x2(t_o, o);
-          tmem_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 8; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f[(i >> 1) & 1]);
-          tmem_stq256_x2(t_o, o);
         }
       }
       TC_TRACE_W(j, 2);
@@ -549,15 +573,15 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       // split mode: the probabilities are kept 2^6 larger (they stay below 2^14), so that their fp16 halves leave the
       // normal range only below 2^-20 of the row's largest; the row sum carries the same factor and it cancels
       constexpr float P_BIAS = SPLIT ? 6.0f : 0.0f;
-      const float2 nm2[2] = {make_float2(P_BIAS - m_new[0], P_BIAS - m_new[0]), make_float2(P_BIAS - m_new[1], P_BIAS - m_new[1])};
+      const float2 nm2[2] = {make_float2(P_BIAS - m_used[0], P_BIAS - m_used[0]), make_float2(P_BIAS - m_used[1], P_BIAS - m_used[1])};
       const float2 scale2 = make_float2(scale_log2, scale_log2);
       float2 rs2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-      uint32_t pk[16];
-      uint32_t pk_lo[SPLIT ? 16 : 1];
+      uint32_t pk[8];
+      uint32_t pk_lo[SPLIT ? 8 : 1];
       // exponentials of key groups [g_lo, g_hi) (8 keys each); bf16 results packed into pk[0..], tf32 in place;
       // split mode: hi = p with the mantissa cut to fp16 width (so the conversion is exact), lo = p - hi.
       // A thread's two adjacent keys of a row go through the scale-and-subtract and the row sum as one fp32 pair.
-      auto exp_groups = [&](const int g_lo, const int g_hi) {
+      auto exp_groups = [&](const int g_lo, const int g_hi) {   // pk holds the quarter's eight words
 #pragma unroll
         for (int g = g_lo; g < g_hi; ++g) {
 #pragma unroll
@@ -570,10 +594,10 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
               s[4 * g + 2 * h + 1] = __float_as_uint(p1);
             } else if constexpr (SPLIT) {
               const float h0 = __uint_as_float(__float_as_uint(p0) & 0xffffe000u), h1 = __uint_as_float(__float_as_uint(p1) & 0xffffe000u);
-              pk[2 * (g - g_lo) + h] = pack_f16(h0, h1);
-              pk_lo[2 * (g - g_lo) + h] = pack_f16(p0 - h0, p1 - h1);
+              pk[2 * (g & 3) + h] = pack_f16(h0, h1);
+              pk_lo[2 * (g & 3) + h] = pack_f16(p0 - h0, p1 - h1);
             } else {
-              pk[2 * (g - g_lo) + h] = pack_bf16(p0, p1);
+              pk[2 * (g & 3) + h] = pack_bf16(p0, p1);
             }
             rs2[h] = fadd2(rs2[h], make_float2(p0, p1));
           }
@@ -582,23 +606,30 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       // bf16 P: keys 2c, 2c+1 in column c of the S region (64 columns); tf32 P: in place of S.
       // The store of the first 64 keys completes behind the next exponentials, so its wait is short;
       // only the last quarter's store latency is exposed before the second product can finish.
-      exp_groups(0, 8);
-      if constexpr (TF32) tmem_stq256_x8(t_s, s);
-      else tmem_stq128_x8(t_s, pk);
-      if constexpr (SPLIT) tmem_stq128_x8(t_s + 64, pk_lo);
+      // a quarter: 32 keys of P
+      auto store_quarter = [&](const int i) {
+        if constexpr (TF32) tmem_stq256_x4(t_s + 32 * i, s + 16 * i);
+        else tmem_stq128_x4(t_s + SH::P_COL + 16 * i, pk);
+        if constexpr (SPLIT) tmem_stq128_x4(t_s + 64 + 16 * i, pk_lo);
+      };
+      exp_groups(0, 4);
+      store_quarter(0);
+      exp_groups(4, 8);
+      store_quarter(1);
       TC_TRACE(x, j, 3);
       exp_groups(8, 12);
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(BAR_P_HALF + x));
-      if constexpr (TF32) tmem_stq256_x4(t_s + 64, s + 32);
-      else tmem_stq128_x4(t_s + 32, pk);
-      if constexpr (SPLIT) tmem_stq128_x4(t_s + 96, pk_lo);
-      exp_groups(12, 16);
-      if constexpr (TF32) tmem_stq256_x4(t_s + 96, s + 48);
-      else tmem_stq128_x4(t_s + 48, pk);
-      if constexpr (SPLIT) tmem_stq128_x4(t_s + 112, pk_lo);
+      store_quarter(2);
+      exp_groups(12, 14);
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(BAR_P_MOST + x));
+      exp_groups(14, 16);
+      store_quarter(3);
       TC_TRACE(x, j, 4);
       tmem_wait_st();
       tc_fence_before();
@@ -606,8 +637,6 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       if (lane == 0) mbar_arrive(bar(BAR_P_READY + x));
       l[0] += rs2[0].x + rs2[0].y;
       l[1] += rs2[1].x + rs2[1].y;
-      m_used[0] = m_new[0];
-      m_used[1] = m_new[1];
       TC_TRACE(x, j, 5);
       TC_TRACE_W(j, 3);
     }
@@ -629,7 +658,7 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(BAR_RED + x));
       ok = __all_sync(0xffffffffu, mbar_wait(bar(BAR_RED + x), 0, p.status, 36 + x, n));
-      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar(BAR_O_DONE + x), (uint32_t)((n - 1) & 1), p.status, 34 + x, n));
+      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar(BAR_O_DONE + x), P_APART ? (uint32_t)((n - 1) & 1) : 0u, p.status, 34 + x, n));
       TC_PHASE(8, warp == 0 && lane == 0);
       if (ok) {
         tc_fence_after();
