@@ -306,10 +306,11 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       for (int j = 0; j < n && ok; ++j) {
         const int jn = j + 1;
         if (j + 1 < n) {
-          // next S / dP as soon as the element-wise warps hold the current ones in registers
-          ok = __all_sync(0xffffffffu, mbar_wait(bar(DQ_SDP_FREE), (uint32_t)(j & 1), p.status, 123, j));
-          if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar(DQ_K_FULL + jn % PL::K_STAGES), (uint32_t)((jn / PL::K_STAGES) & 1), p.status, 124, j));
+          // next S / dP as soon as the element-wise warps hold the current ones in registers (their tiles, long there,
+          // are waited for first)
+          ok = __all_sync(0xffffffffu, mbar_wait(bar(DQ_K_FULL + jn % PL::K_STAGES), (uint32_t)((jn / PL::K_STAGES) & 1), p.status, 124, j));
           if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar(DQ_V_FULL + jn % PL::V_STAGES), (uint32_t)((jn / PL::V_STAGES) & 1), p.status, 125, j));
+          if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar(DQ_SDP_FREE), (uint32_t)(j & 1), p.status, 123, j));
           if (!ok) break;
           tc_fence_after();
           issue_sdp(jn);
@@ -454,7 +455,9 @@ enum KvBar : int {
   KV_LD_READY = 15,  // the step's per-query log-sum-exp and delta are staged in shared memory
   KV_DPT_FULL = 16,  // dP^T written by the MMA
   KV_DST_READY = 17, // dS^T written to TMEM (over dP^T)
-  KV_BAR_COUNT = 18
+  KV_PT_HALF = 18,   // the first sixteen queries of every quarter of P^T, and
+  KV_DST_HALF = 19,  // of dS^T: their part of the product starts while the rest is formed
+  KV_BAR_COUNT = 20
 };
 
 template <int HD, bool SPLIT, bool MASKED>
@@ -498,7 +501,7 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     prefetch_tensormap(&map_q); prefetch_tensormap(&map_k); prefetch_tensormap(&map_v); prefetch_tensormap(&map_do);
   }
   if (tid == 0) {
-    for (int i = 0; i < KV_BAR_COUNT; ++i) mbar_init(bar(i), (i == KV_PT_READY || i == KV_LD_READY || i == KV_DST_READY) ? (uint32_t)EW_WARPS : 1u);
+    for (int i = 0; i < KV_BAR_COUNT; ++i) mbar_init(bar(i), (i == KV_PT_READY || i == KV_LD_READY || i == KV_DST_READY || i == KV_PT_HALF || i == KV_DST_HALF) ? (uint32_t)EW_WARPS : 1u);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == WARP_MMA) { tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), TMEM_COLS); tmem_relinquish(); }
@@ -579,9 +582,10 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         }
       };
       // acc += A^T-from-TMEM x B with B a 128 x HD tile read MN-major; split mode: hi.hi + hi.lo + lo.hi
-      auto issue_acc = [&](uint32_t d_col, uint32_t a_col, uint32_t b_addr, bool first_step) {
+      auto issue_acc = [&](uint32_t d_col, uint32_t a_col, uint32_t b_addr, bool first_step, int half) {   // half: the even or the odd sixteens
 #pragma unroll
-        for (int kk = 0; kk < BLK / 16; ++kk) {
+        for (int k2 = 0; k2 < BLK / 32; ++k2) {
+          const int kk = 2 * k2 + half;
           const uint32_t a_hi = tmem_u + a_col + (kk / 2) * 32 + (kk % 2) * 8;
           umma_ts_if<false>(leader, tmem_u + d_col, a_hi, make_desc(b_addr + kk * 2048, PL::SUB_BYTES, 1024), IDESC_ACC,
                             (!first_step || kk > 0) ? 1u : 0u);
@@ -625,30 +629,30 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       for (int it = 0; it < n && ok; ++it) {
         const uint32_t q_addr = q_stage(it), do_addr = do_stage(it);
         // dV += P^T dY: A from TMEM (16 queries = 8 packed columns per step), B MN-major
+        ok = __all_sync(0xffffffffu, mbar_wait(bar(KV_PT_HALF), (uint32_t)(it & 1), p.status, 225, it));
+        if (!ok) break;
+        tc_fence_after();
+        issue_acc(C_DV, C_ST, do_addr, it == 0, 0);
+        if (it + 1 < n && !(ok = wait_q(it + 1))) break;   // long there: waited for here, off the way from P^T to S^T
         ok = __all_sync(0xffffffffu, mbar_wait(bar(KV_PT_READY), (uint32_t)(it & 1), p.status, 222, it));
         if (!ok) break;
         tc_fence_after();
-        issue_acc(C_DV, C_ST, do_addr, it == 0);
-        umma_commit_if(leader, bar(KV_DO_EMPTY + it % PL::V_STAGES));   // dY(it) was last read by this product
-        if (it + 1 < n) {
-          ok = wait_q(it + 1);
-          if (!ok) break;
-          tc_fence_after();
-          issue_st(it + 1);
-        }
+        issue_acc(C_DV, C_ST, do_addr, it == 0, 1);
+        if (it + 1 < n) issue_st(it + 1);
+        umma_commit_if(leader, bar(KV_DO_EMPTY + it % PL::V_STAGES));   // dY(it) was last read by dV
         // dK += dS^T Q
+        ok = __all_sync(0xffffffffu, mbar_wait(bar(KV_DST_HALF), (uint32_t)(it & 1), p.status, 226, it));
+        if (!ok) break;
+        tc_fence_after();
+        issue_acc(C_DK, C_DPT, q_addr, it == 0, 0);
+        if (it + 1 < n && !(ok = wait_do(it + 1))) break;
         ok = __all_sync(0xffffffffu, mbar_wait(bar(KV_DST_READY), (uint32_t)(it & 1), p.status, 223, it));
         if (!ok) break;
         tc_fence_after();
-        issue_acc(C_DK, C_DPT, q_addr, it == 0);
+        issue_acc(C_DK, C_DPT, q_addr, it == 0, 1);
+        if (it + 1 < n) issue_dpt(it + 1);
+        else umma_commit_if(leader, bar(KV_ACC_DONE));
         umma_commit_if(leader, bar(KV_Q_EMPTY + it % PL::K_STAGES));
-        umma_commit_if(leader, bar(KV_ACC_DONE));
-        if (it + 1 < n) {
-          ok = wait_do(it + 1);
-          if (!ok) break;
-          tc_fence_after();
-          issue_dpt(it + 1);
-        }
       }
       umma_commit_if(leader, bar(KV_DRAIN));
       mbar_wait(bar(KV_DRAIN), 0, p.status, 227, 0);
@@ -711,11 +715,11 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       tmem_wait_ld();
       // The causal test is the diagonal tile's alone (a loop of its own, as in the dQ kernel).  A key beyond T needs none: its
       // row of P^T and dS^T reaches only its own rows of dV and dK, which are not stored.
-      auto form_p = [&](auto diag_tag) {
+      auto form_p = [&](auto diag_tag, const int lo, const int hi) {
         constexpr bool DIAG = decltype(diag_tag)::value;
         const int first = kj - q_base;      // queries before the key do not see it
 #pragma unroll
-        for (int i = 0; i < 32; i += 4) {
+        for (int i = lo; i < hi; i += 4) {
           const float4 nl = *reinterpret_cast<const float4*>(nlse_s + i);
           const float nls[4] = {nl.x, nl.y, nl.z, nl.w};
 #pragma unroll
@@ -745,14 +749,28 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
           }
         }
       };
-      if (diag) form_p(std::true_type{});
-      else form_p(std::false_type{});
-      tmem_st16(t_row + C_ST + qtr * 32, pk);
-      if constexpr (SPLIT) tmem_st16(t_row + C_ST + qtr * 32 + 16, pk_lo);
-      tmem_wait_st();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(KV_PT_READY));
+      // sixteen of the 32 queries are stored and handed over while the others are formed
+      auto store_half = [&](uint32_t col, int half) {
+        tmem_st8(t_row + col + qtr * 32 + half * 8, pk + half * 8);
+        if constexpr (SPLIT) tmem_st8(t_row + col + qtr * 32 + 16 + half * 8, pk_lo + half * 8);
+      };
+      auto hand_over = [&](int b) {
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(b));
+      };
+      auto pass1 = [&](auto diag_tag) {
+        form_p(diag_tag, 0, 16);
+        store_half(C_ST, 0);
+        form_p(diag_tag, 16, 24);
+        hand_over(KV_PT_HALF);
+        form_p(diag_tag, 24, 32);
+        store_half(C_ST, 1);
+        hand_over(KV_PT_READY);
+      };
+      if (diag) pass1(std::true_type{});
+      else pass1(std::false_type{});
       // pass 2: dS^T = P^T o (dP^T - delta) scale, packed to bf16 over dP^T
       ok = __all_sync(0xffffffffu, mbar_wait(bar(KV_DPT_FULL), (uint32_t)(it & 1), p.status, 233, it));
       if (!ok) break;
@@ -760,29 +778,32 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       uint32_t dp[32];
       tmem_ld32(t_row + C_DPT + qtr * 32, dp);
       tmem_wait_ld();
+      auto form_ds = [&](const int lo, const int hi) {
 #pragma unroll
-      for (int i = 0; i < 32; i += 4) {
-        const float4 de = *reinterpret_cast<const float4*>(del_s + i);
-        const float des[4] = {de.x, de.y, de.z, de.w};
+        for (int i = lo; i < hi; i += 4) {
+          const float4 de = *reinterpret_cast<const float4*>(del_s + i);
+          const float des[4] = {de.x, de.y, de.z, de.w};
 #pragma unroll
-        for (int e = 0; e < 4; e += 2) {
-          // (dP - delta) scale as one fused pair operation, then times P
-          const float2 g = ffma2(make_float2(__uint_as_float(dp[i + e]), __uint_as_float(dp[i + e + 1])), ps2,
-                                 make_float2(des[e], des[e + 1]));
-          const float2 d = ffma2(make_float2(__uint_as_float(s[i + e]), __uint_as_float(s[i + e + 1])), g, zero2);
-          if constexpr (SPLIT) split_pack(d.x, d.y, pk[(i + e) / 2], pk_lo[(i + e) / 2]);
-          else pk[(i + e) / 2] = pack_bf16(d.x, d.y);
+          for (int e = 0; e < 4; e += 2) {
+            // (dP - delta) scale as one fused pair operation, then times P
+            const float2 g = ffma2(make_float2(__uint_as_float(dp[i + e]), __uint_as_float(dp[i + e + 1])), ps2,
+                                   make_float2(des[e], des[e + 1]));
+            const float2 d = ffma2(make_float2(__uint_as_float(s[i + e]), __uint_as_float(s[i + e + 1])), g, zero2);
+            if constexpr (SPLIT) split_pack(d.x, d.y, pk[(i + e) / 2], pk_lo[(i + e) / 2]);
+            else pk[(i + e) / 2] = pack_bf16(d.x, d.y);
+          }
         }
-      }
+      };
+      form_ds(0, 16);
+      store_half(C_DPT, 0);
+      form_ds(16, 24);
+      hand_over(KV_DST_HALF);
+      form_ds(24, 32);
+      store_half(C_DPT, 1);
       if (it + 1 < n) stage(it + 1, next);
-      tmem_st16(t_row + C_DPT + qtr * 32, pk);
-      if constexpr (SPLIT) tmem_st16(t_row + C_DPT + qtr * 32 + 16, pk_lo);
-      tmem_wait_st();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(KV_DST_READY));
+      hand_over(KV_DST_READY);
     }
-    if (ok && n > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar(KV_ACC_DONE), (uint32_t)((n - 1) & 1), p.status, 232, n));
+    if (ok && n > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar(KV_ACC_DONE), 0, p.status, 232, n));
     constexpr int ESZ = SPLIT ? 4 : 2, PR = HD * ESZ / 16;
     uint8_t* tile_k = smem_gen + PL::OFF_RES0;         // the K and V tiles: every product has finished with them
     uint8_t* tile_v = smem_gen + PL::OFF_RES1;
