@@ -11,12 +11,12 @@
 //
 // Two kernels (no atomics, deterministic):
 //   * dq kernel: one CTA per 128-row query tile walks the key tiles:  S = Q K^T and dP = dY V^T
-//     (tcgen05.mma, both operands in shared memory), dS computed by sixteen warps straight from
+//     (tcgen05.mma, both operands in shared memory), dS computed by sixteen (or eight) warps straight from
 //     TMEM and written back as a bf16 A operand, dQ += dS K accumulated in TMEM.
 //   * dkdv kernel: one CTA per 128-row key tile walks the query tiles with the transposed
 //     products S^T = K Q^T and dP^T = V dY^T, so that P^T and dS^T come out in the layout the
 //     A operand of dV += P^T dY and dK += dS^T Q needs.
-// Q/K/V/dY tiles arrive by TMA (no multicast) through two-stage rings; every mbarrier wait is
+// Q/K/V/dY tiles arrive by TMA (no multicast) through rings; every mbarrier wait is
 // bounded as in the forward kernel.
 //
 // SPLIT = true is the variant for fp32 callers: every operand is carried as two fp16 halves (rows [hi | lo] written by
@@ -33,36 +33,42 @@ namespace {
 
 using namespace tc;
 
-constexpr int EW_WARPS = 16;                 // element-wise warps: four threads per row, 32 columns each
-constexpr int WARP_TMA = EW_WARPS;
-constexpr int WARP_MMA = EW_WARPS + 1;
-constexpr int BW_THREADS = (EW_WARPS + 2) * 32;
-
-template <int HD> struct BwdPlan {
-  static constexpr int SUB = HD / 64;
-  static constexpr uint32_t SUB_BYTES = BLK * 128;
-  static constexpr uint32_t TILE_BYTES = SUB * SUB_BYTES;  // 128 x HD bf16
-  // [0] and [1]: the two resident tiles (Q,dY or K,V); then two ring stages of two tiles each
-  static constexpr uint32_t OFF_RES0 = 0;
-  static constexpr uint32_t OFF_RES1 = TILE_BYTES;
-  static constexpr uint32_t OFF_RING = 2 * TILE_BYTES;     // stage s: tile a at +s*2*TILE, tile b at +TILE after it
-  static constexpr uint32_t OFF_BAR = 6 * TILE_BYTES;
-  static constexpr uint32_t BYTES = OFF_BAR + 256 + 1024;
+// What a CTA looks like.  It keeps two 128-row tiles (Q and dY, or K and V) and streams the other two tensors BN rows a step.
+//   WIDE    128 rows a step, sixteen element-wise warps (four threads per row, 32 columns each), all of TMEM, one CTA per SM.
+//   NARROW  64 rows a step, eight element-wise warps (two threads per row, 32 columns each), half of TMEM and under half of the
+//           shared memory: two CTAs share an SM, and one's set-up, first loads, pipeline fill and gradient stores run beside
+//           the other's steps.  At T = 1024 a causal CTA walks four and a half key tiles on average, and those fixed parts were
+//           half of its life: B=8 H=12 T=1024 D=64 bf16, dK/dV 59 -> 52 us, dQ 49 -> 40, the whole layer 142 -> 118; T = 9200 and
+//           more gain 4 % (two steps in flight).  For bf16 heads of 64; 128-wide heads and split operands have no room for two.
+// ROW: elements of 2 bytes per operand row (a split row is two 128-byte sub-tiles [hi | lo]).
+template <int ROW, bool NARROW> struct BwdPlan {
+  static constexpr int BN = NARROW ? 64 : 128;
+  static constexpr int EW_WARPS = NARROW ? 8 : 16;         // element-wise warps
+  static constexpr int WARP_TMA = EW_WARPS, WARP_MMA = EW_WARPS + 1, THREADS = (EW_WARPS + 2) * 32;
+  static constexpr int CTAS_PER_SM = NARROW ? 2 : 1;
+  static constexpr uint32_t TMEM_COLS = NARROW ? 256 : 512;
+  static constexpr int SUB = ROW / 64;
+  static constexpr uint32_t SUB_BYTES = BLK * 128;         // a resident tile's sub-tile; of a streamed one:
+  static constexpr uint32_t RING_SUB_BYTES = BN * 128;
+  static constexpr uint32_t TILE_BYTES = SUB * SUB_BYTES, RING_TILE_BYTES = SUB * RING_SUB_BYTES;
+  static constexpr uint32_t OFF_RES0 = 0, OFF_RES1 = TILE_BYTES;
   // dQ kernel: K lives until the step's dQ product, so its ring is one stage deeper than V's (K(j+2) could
   // otherwise only be requested when dQ(j) has finished, one step before it is needed, and every step
-  // would wait out the load latency): K stages at OFF_RING + {0,1,2} tiles, V stages behind them.
-  static constexpr int K_STAGES = 3, V_STAGES = 2;
-  static constexpr uint32_t OFF_KRING = OFF_RING;
-  static constexpr uint32_t OFF_VRING = OFF_RING + K_STAGES * TILE_BYTES;
-  static constexpr uint32_t OFF_BAR_DQ = OFF_VRING + V_STAGES * TILE_BYTES;
-  static constexpr uint32_t BYTES_DQ = OFF_BAR_DQ + 256 + 1024;
-  // dK/dV kernel: the same seven tiles, then barriers, the staged per-query terms ([2][128] floats twice) and the
+  // would wait out the load latency).  The dK/dV kernel has Q where the dQ kernel has K, and dY where it has V.
+  static constexpr int K_STAGES = NARROW ? 4 : 3, V_STAGES = NARROW ? 3 : 2;
+  static constexpr uint32_t OFF_KRING = 2 * TILE_BYTES;
+  static constexpr uint32_t OFF_VRING = OFF_KRING + K_STAGES * RING_TILE_BYTES;
+  static constexpr uint32_t OFF_BAR = OFF_VRING + V_STAGES * RING_TILE_BYTES;
+  static constexpr uint32_t BYTES_DQ = OFF_BAR + 256 + 1024;
+  // dK/dV kernel: behind the barriers the staged per-query terms ([2][BN] floats twice) and the
   // abort flag, all in dynamic shared memory (no static allocation, so the dynamic base keeps its alignment).
-  // At HD = 128 this leaves 752 bytes for aligning the base to 1024; the kernel checks that it fits.
-  static constexpr uint32_t OFF_STAGE_KV = OFF_BAR_DQ + 256;
-  static constexpr uint32_t OFF_FLAG_KV = OFF_STAGE_KV + 2 * 2 * BLK * 4;
+  // At 128-wide heads this leaves 752 bytes for aligning the base to 1024; the kernel checks that it fits.
+  static constexpr uint32_t OFF_STAGE_KV = OFF_BAR + 256;
+  static constexpr uint32_t OFF_FLAG_KV = OFF_STAGE_KV + 2 * 2 * BN * 4;
   static constexpr uint32_t NEED_KV = OFF_FLAG_KV + 16;
   static constexpr uint32_t BYTES_KV = (NEED_KV + 1024 <= 227u * 1024u) ? NEED_KV + 1024 : 227u * 1024u;
+  static_assert(CTAS_PER_SM == 1 || CTAS_PER_SM * ((BYTES_KV > BYTES_DQ ? BYTES_KV : BYTES_DQ) + 1024 + 128) <= 228 * 1024,
+                "shared memory of the CTAs of one SM");
 };
 
 // fp16 halves of a value the tensor core must see at fp32 accuracy: hi = v with the mantissa cut to fp16 width (the
@@ -102,10 +108,10 @@ struct BwdParams {
 
 // The gradient tiles leave through shared memory.  In the TMEM layout a thread owns a quarter of one row, so direct
 // stores are 32 sixteen-byte pieces from 32 rows per instruction (9-12 % of the backward at T = 1024 was these
-// stores).  Instead the sixteen element-wise warps write their pieces into a resident operand tile that every product
+// stores).  Instead the element-wise warps write their pieces into a resident operand tile that every product
 // has finished with (Q or K for the first result, dY or V for the second), meet at a named barrier, and each warp
-// stores eight whole rows.  Every element-wise warp reaches the barrier, also after a failed wait.
-__device__ __forceinline__ void ew_bar_sync() { asm volatile("bar.sync 1, %0;" ::"n"(EW_WARPS * 32) : "memory"); }
+// stores its share of whole rows.  Every element-wise warp reaches the barrier, also after a failed wait.
+template <int EW_WARPS> __device__ __forceinline__ void ew_bar_sync() { asm volatile("bar.sync 1, %0;" ::"n"(EW_WARPS * 32) : "memory"); }
 // 16-byte piece `piece` of row `row` of a staged 128-row tile with PR pieces per row (XOR-swizzled by row)
 template <int PR> __device__ __forceinline__ uint4* staged_piece(uint8_t* tile, int row, int piece) {
   return reinterpret_cast<uint4*>(tile) + row * PR + (piece ^ (row & (PR - 1)));
@@ -138,14 +144,14 @@ __device__ __forceinline__ void stage_columns(uint8_t* tile, int row, int qtr, u
     }
   }
 }
-// warp w of the sixteen stores rows 8 w .. 8 w + 7 of a staged tile; off0: element offset of the tile's row 0
-template <int PR, int ESZ>
+// warp w of the element-wise warps stores rows RPW w .. RPW (w + 1) - 1 of a staged tile; off0: element offset of the tile's row 0
+template <int PR, int ESZ, int RPW>
 __device__ __forceinline__ void store_staged_rows(uint8_t* tile, int w, int lane, void* out, int64_t off0, int64_t row_stride,
                                                   int rows_valid) {
   constexpr int RPI = 32 / PR;   // rows per store instruction
 #pragma unroll
-  for (int kk = 0; kk < 8 / RPI; ++kk) {
-    const int row = 8 * w + kk * RPI + lane / PR, piece = lane % PR;
+  for (int kk = 0; kk < RPW / RPI; ++kk) {
+    const int row = RPW * w + kk * RPI + lane / PR, piece = lane % PR;
     if (row < rows_valid)
       *reinterpret_cast<uint4*>(static_cast<char*>(out) + (off0 + (int64_t)row * row_stride) * ESZ + piece * 16) =
           *staged_piece<PR>(tile, row, piece);
@@ -153,35 +159,37 @@ __device__ __forceinline__ void store_staged_rows(uint8_t* tile, int w, int lane
 }
 
 // ---------------------------------------------------------------------------------------------
-// dQ kernel.  TMEM columns: S [0,128)  dP [128,256)  dS (bf16, packed) [256,320)  dQ [320,320+HD);
-// split mode: dS hi [256,320), dS lo [320,384), dQ [384,384+HD)
+// dQ kernel.  TMEM columns: S [0,BN)  dP [BN,2 BN)  dS (16-bit, packed) [2 BN, 5/2 BN) and, in split mode, its lo half
+// [5/2 BN, 3 BN)  dQ behind them
 // ---------------------------------------------------------------------------------------------
 enum DqBar : int {
   DQ_QDO_FULL = 0,
-  DQ_K_FULL = 1,    // [3]
-  DQ_K_EMPTY = 4,   // [3]
-  DQ_V_FULL = 7,    // [2]
-  DQ_V_EMPTY = 9,   // [2]
-  DQ_SDP_FULL = 11, // S and dP of the step written by the MMA
-  DQ_SDP_FREE = 12, // element-wise warps have S and dP in registers
-  DQ_DS_READY = 13, // dS written to TMEM
-  DQ_DQ_DONE = 14,  // dQ += dS K of the step finished (dS may be overwritten)
-  DQ_DRAIN = 15,
-  DQ_BAR_COUNT = 16
+  DQ_K_FULL = 1,    // [K_STAGES, at most 4]
+  DQ_K_EMPTY = 5,
+  DQ_V_FULL = 9,    // [V_STAGES, at most 3]
+  DQ_V_EMPTY = 12,
+  DQ_SDP_FULL = 15, // S and dP of the step written by the MMA
+  DQ_SDP_FREE = 16, // element-wise warps have S and dP in registers
+  DQ_DS_READY = 17, // dS written to TMEM
+  DQ_DQ_DONE = 18,  // dQ += dS K of the step finished (dS may be overwritten)
+  DQ_DRAIN = 19,
+  DQ_BAR_COUNT = 20
 };
 
-template <int HD, bool SPLIT, bool MASKED>
-__global__ void __launch_bounds__(BW_THREADS, 1)
+template <int HD, bool SPLIT, bool MASKED, bool NARROW>
+__global__ void __launch_bounds__((BwdPlan<SPLIT ? 128 : HD, NARROW>::THREADS), (BwdPlan<SPLIT ? 128 : HD, NARROW>::CTAS_PER_SM))
 sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                       const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
                       const BwdParams p) {
-  using PL = BwdPlan<SPLIT ? 128 : HD>;   // a split row is two 128-byte sub-tiles [hi | lo]
+  using PL = BwdPlan<SPLIT ? 128 : HD, NARROW>;
+  constexpr int BN = PL::BN, EW_WARPS = PL::EW_WARPS, WARP_TMA = PL::WARP_TMA, WARP_MMA = PL::WARP_MMA;
+  constexpr uint32_t TMEM_COLS = PL::TMEM_COLS;
   constexpr int FMT = SPLIT ? 0 : 1;       // operand format of the instruction descriptor: fp16 or bf16
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-  const uint32_t bar0 = smem_base + PL::OFF_BAR_DQ;
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + PL::OFF_BAR_DQ + DQ_BAR_COUNT * 8);
+  const uint32_t bar0 = smem_base + PL::OFF_BAR;
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + PL::OFF_BAR + DQ_BAR_COUNT * 8);
   auto bar = [&](int i) { return bar0 + 8u * (uint32_t)i; };
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // launch order -> work item: longest causal work first inside groups of p.group heads (see the forward kernel)
@@ -194,7 +202,7 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   const int bi = bh / p.H, hi = bh - bi * p.H;   // batch item and head
   const int qt = (int)gridDim.x - 1 - rank;
   const int q0 = qt * BLK;
-  const int n = p.causal ? (min(q0 + BLK, T) + BLK - 1) / BLK : (T + BLK - 1) / BLK;
+  const int n = ((p.causal ? min(q0 + BLK, T) : T) + BN - 1) / BN;   // key steps
 
   // set-up, each part by another warp so that their latencies overlap (status word, barriers, descriptors, TMEM)
   __shared__ int s_abort;
@@ -223,7 +231,8 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     mca_pdl_wait();
     return;
   }
-  constexpr uint32_t C_S = 0, C_DP = 128, C_DS = 256, C_DQ = SPLIT ? 384 : 320;
+  constexpr uint32_t C_S = 0, C_DP = BN, C_DS = 2 * BN, DS_LO = BN / 2, C_DQ = C_DS + (SPLIT ? BN : BN / 2);
+  static_assert(C_DQ + HD <= TMEM_COLS);
   bool ok = true;
 
   if (warp == WARP_TMA) {
@@ -231,25 +240,28 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       mbar_expect_tx(bar(DQ_QDO_FULL), 2 * PL::TILE_BYTES);
 #pragma unroll
       for (int s = 0; s < PL::SUB; ++s) {
-        tma_load_4d(smem_base + PL::OFF_RES0 + s * PL::SUB_BYTES, &map_q, bar(DQ_QDO_FULL), s * 64, q0, hi, bi);
-        tma_load_4d(smem_base + PL::OFF_RES1 + s * PL::SUB_BYTES, &map_do, bar(DQ_QDO_FULL), s * 64, q0, hi, bi);
+#pragma unroll
+        for (int r = 0; r < BLK; r += BN) {   // a copy's box is BN rows
+          tma_load_4d(smem_base + PL::OFF_RES0 + s * PL::SUB_BYTES + r * 128, &map_q, bar(DQ_QDO_FULL), s * 64, q0 + r, hi, bi);
+          tma_load_4d(smem_base + PL::OFF_RES1 + s * PL::SUB_BYTES + r * 128, &map_do, bar(DQ_QDO_FULL), s * 64, q0 + r, hi, bi);
+        }
       }
       int issued_k = 0, issued_v = 0;
       for (int j = 0; j < n && ok; ++j) {
         const int ks = j % PL::K_STAGES, vs = j % PL::V_STAGES;
         const uint32_t kph = (uint32_t)((j / PL::K_STAGES) & 1), vph = (uint32_t)((j / PL::V_STAGES) & 1);
-        const uint32_t k_dst = smem_base + PL::OFF_KRING + ks * PL::TILE_BYTES, v_dst = smem_base + PL::OFF_VRING + vs * PL::TILE_BYTES;
+        const uint32_t k_dst = smem_base + PL::OFF_KRING + ks * PL::RING_TILE_BYTES, v_dst = smem_base + PL::OFF_VRING + vs * PL::RING_TILE_BYTES;
         ok = mbar_wait(bar(DQ_K_EMPTY + ks), kph ^ 1u, p.status, 110, j);
         if (!ok) break;
-        mbar_expect_tx(bar(DQ_K_FULL + ks), PL::TILE_BYTES);
+        mbar_expect_tx(bar(DQ_K_FULL + ks), PL::RING_TILE_BYTES);
 #pragma unroll
-        for (int s = 0; s < PL::SUB; ++s) tma_load_4d(k_dst + s * PL::SUB_BYTES, &map_k, bar(DQ_K_FULL + ks), s * 64, j * BLK, hi, bi);
+        for (int s = 0; s < PL::SUB; ++s) tma_load_4d(k_dst + s * PL::RING_SUB_BYTES, &map_k, bar(DQ_K_FULL + ks), s * 64, j * BN, hi, bi);
         issued_k = j + 1;
         ok = mbar_wait(bar(DQ_V_EMPTY + vs), vph ^ 1u, p.status, 111, j);
         if (!ok) break;
-        mbar_expect_tx(bar(DQ_V_FULL + vs), PL::TILE_BYTES);
+        mbar_expect_tx(bar(DQ_V_FULL + vs), PL::RING_TILE_BYTES);
 #pragma unroll
-        for (int s = 0; s < PL::SUB; ++s) tma_load_4d(v_dst + s * PL::SUB_BYTES, &map_v, bar(DQ_V_FULL + vs), s * 64, j * BLK, hi, bi);
+        for (int s = 0; s < PL::SUB; ++s) tma_load_4d(v_dst + s * PL::RING_SUB_BYTES, &map_v, bar(DQ_V_FULL + vs), s * 64, j * BN, hi, bi);
         issued_v = j + 1;
       }
       if (!ok) {  // let copies in flight land (bounded) before the CTA's memory is released
@@ -266,7 +278,7 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     {
       const uint32_t leader = elect_one() ? 1u : 0u;
       const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
-      constexpr uint32_t IDESC_NT = make_idesc_fmt(BLK, BLK, 0, 0, FMT);  // both operands K-major
+      constexpr uint32_t IDESC_NT = make_idesc_fmt(BLK, BN, 0, 0, FMT);  // both operands K-major
       constexpr uint32_t IDESC_DQ = make_idesc_fmt(BLK, HD, 0, 1, FMT);   // A from TMEM, B = K tile MN-major
       const uint32_t q_addr = smem_base + PL::OFF_RES0, do_addr = smem_base + PL::OFF_RES1;
       // D = A B^T over the head dimension, both operands K-major in shared memory; split mode: hi.hi + hi.lo + lo.hi
@@ -274,7 +286,7 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         if constexpr (SPLIT) {
 #pragma unroll
           for (int term = 0; term < 3; ++term) {
-            const uint32_t oa = term == 2 ? PL::SUB_BYTES : 0u, ob = term == 1 ? PL::SUB_BYTES : 0u;
+            const uint32_t oa = term == 2 ? PL::SUB_BYTES : 0u, ob = term == 1 ? PL::RING_SUB_BYTES : 0u;
 #pragma unroll
             for (int kk = 0; kk < HD / 16; ++kk)
               umma_ss_if<false>(leader, tmem_u + d_col, make_desc(a_addr + oa + kk * 32, 16, 1024), make_desc(b_addr + ob + kk * 32, 16, 1024),
@@ -283,14 +295,14 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         } else {
 #pragma unroll
           for (int kk = 0; kk < HD / 16; ++kk) {
-            const uint32_t off = (kk / 4) * PL::SUB_BYTES + (kk % 4) * 32;
-            umma_ss_if<false>(leader, tmem_u + d_col, make_desc(a_addr + off, 16, 1024), make_desc(b_addr + off, 16, 1024), IDESC_NT, kk > 0);
+            umma_ss_if<false>(leader, tmem_u + d_col, make_desc(a_addr + (kk / 4) * PL::SUB_BYTES + (kk % 4) * 32, 16, 1024),
+                              make_desc(b_addr + (kk / 4) * PL::RING_SUB_BYTES + (kk % 4) * 32, 16, 1024), IDESC_NT, kk > 0);
           }
         }
       };
       auto issue_sdp = [&](int j) {
-        const uint32_t k_addr = smem_base + PL::OFF_KRING + (j % PL::K_STAGES) * PL::TILE_BYTES;
-        const uint32_t v_addr = smem_base + PL::OFF_VRING + (j % PL::V_STAGES) * PL::TILE_BYTES;
+        const uint32_t k_addr = smem_base + PL::OFF_KRING + (j % PL::K_STAGES) * PL::RING_TILE_BYTES;
+        const uint32_t v_addr = smem_base + PL::OFF_VRING + (j % PL::V_STAGES) * PL::RING_TILE_BYTES;
         issue_nt(C_S, q_addr, k_addr);
         issue_nt(C_DP, do_addr, v_addr);
       };
@@ -320,15 +332,15 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         ok = __all_sync(0xffffffffu, mbar_wait(bar(DQ_DS_READY), (uint32_t)(j & 1), p.status, 126, j));
         if (!ok) break;
         tc_fence_after();
-        const uint32_t k_addr = smem_base + PL::OFF_KRING + (j % PL::K_STAGES) * PL::TILE_BYTES;
+        const uint32_t k_addr = smem_base + PL::OFF_KRING + (j % PL::K_STAGES) * PL::RING_TILE_BYTES;
 #pragma unroll
-        for (int kk = 0; kk < BLK / 16; ++kk) {
-          umma_ts_if<false>(leader, tmem_u + C_DQ, tmem_u + C_DS + kk * 8, make_desc(k_addr + kk * 2048, PL::SUB_BYTES, 1024), IDESC_DQ,
+        for (int kk = 0; kk < BN / 16; ++kk) {
+          umma_ts_if<false>(leader, tmem_u + C_DQ, tmem_u + C_DS + kk * 8, make_desc(k_addr + kk * 2048, PL::RING_SUB_BYTES, 1024), IDESC_DQ,
                   (j > 0 || kk > 0) ? 1u : 0u);
           if constexpr (SPLIT) {   // + dS_hi K_lo + dS_lo K_hi
-            umma_ts_if<false>(leader, tmem_u + C_DQ, tmem_u + C_DS + kk * 8, make_desc(k_addr + PL::SUB_BYTES + kk * 2048, PL::SUB_BYTES, 1024),
+            umma_ts_if<false>(leader, tmem_u + C_DQ, tmem_u + C_DS + kk * 8, make_desc(k_addr + PL::RING_SUB_BYTES + kk * 2048, PL::RING_SUB_BYTES, 1024),
                               IDESC_DQ, 1u);
-            umma_ts_if<false>(leader, tmem_u + C_DQ, tmem_u + C_DS + 64 + kk * 8, make_desc(k_addr + kk * 2048, PL::SUB_BYTES, 1024), IDESC_DQ, 1u);
+            umma_ts_if<false>(leader, tmem_u + C_DQ, tmem_u + C_DS + DS_LO + kk * 8, make_desc(k_addr + kk * 2048, PL::RING_SUB_BYTES, 1024), IDESC_DQ, 1u);
           }
         }
         umma_commit_if(leader, bar(DQ_DQ_DONE));
@@ -341,7 +353,7 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     // ------------------------------------------------------------------ element-wise warps
     const int qtr = warp >> 2, lane_base = (warp & 3) * 32, row = lane_base + lane;
     const int qi = q0 + row;
-    constexpr int OC = HD / 4;
+    constexpr int OC = HD / (EW_WARPS / 4);
     const uint32_t t_row = tmem_base + ((uint32_t)lane_base << 16);
     const bool row_ok = qi < T;
     const float lse = row_ok ? p.lse[(int64_t)bh * T + qi] : 0.f;
@@ -362,12 +374,12 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(DQ_SDP_FREE));
-      const int k0 = j * BLK + qtr * 32;
-      const bool edge = (p.causal && j * BLK + BLK - 1 > q0) || (j * BLK + BLK > T);
+      const int k0 = j * BN + qtr * 32;
+      const bool edge = (p.causal && j * BN + BN - 1 > q0) || (j * BN + BN > T);
       uint32_t mw = 0xffffffffu;          // keep-bits of this thread's 32 keys
       float p_masked = 0.f;
       if constexpr (MASKED) {
-        mw = __ldg(p.mask_bits + (int64_t)bi * p.mask_batch_stride + (int64_t)min(qi, T - 1) * p.mask_row_stride + 4 * j + qtr);
+        mw = __ldg(p.mask_bits + (int64_t)bi * p.mask_batch_stride + (int64_t)min(qi, T - 1) * p.mask_row_stride + (BN / 32) * j + qtr);
         p_masked = (row_ok && lse == INFINITY) ? p.inv_T : 0.f;
       }
       // dS = P o (dP - delta) scale with P = 2^(S scale_log2 - lse); adjacent keys go through as fp32 pairs.
@@ -411,7 +423,7 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         tc_fence_after();
       }
       tmem_st16(t_row + C_DS + qtr * 16, pk);
-      if constexpr (SPLIT) tmem_st16(t_row + C_DS + 64 + qtr * 16, pk_lo);
+      if constexpr (SPLIT) tmem_st16(t_row + C_DS + DS_LO + qtr * 16, pk_lo);
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
@@ -426,9 +438,9 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       const float mul = SPLIT ? p.scale * DS_UNSHIFT * (1.0f / (sc.z * sc.y)) * (1.0f / sc.w) : 1.0f;
       stage_columns<PR, OC, SPLIT>(tile, row, qtr, t_row + C_DQ + qtr * OC, mul);
     }
-    ew_bar_sync();
+    ew_bar_sync<EW_WARPS>();
     if (fin)
-      store_staged_rows<PR, ESZ>(tile, warp, lane, p.out0, (int64_t)bi * p.os.b + (int64_t)hi * p.os.h + (int64_t)q0 * p.os.t, p.os.t,
+      store_staged_rows<PR, ESZ, BLK / EW_WARPS>(tile, warp, lane, p.out0, (int64_t)bi * p.os.b + (int64_t)hi * p.os.h + (int64_t)q0 * p.os.t, p.os.t,
                                  min(BLK, T - q0));
   }
   tc_fence_before();
@@ -438,40 +450,43 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
 }
 
 // ---------------------------------------------------------------------------------------------
-// dK/dV kernel.  TMEM columns: S^T [0,128)  dP^T [128,256)  dV [256,256+HD)  dK [384,384+HD);
+// dK/dV kernel.  TMEM columns: S^T [0,BN)  dP^T [BN,2 BN)  dV [2 BN,2 BN+HD)  dK [3 BN,3 BN+HD);
 // P^T and dS^T (bf16, packed) overwrite the first 16 columns of each 32-column quarter of S^T / dP^T; in split
 // mode their fp16 hi halves do, and the lo halves take the other 16 columns of the quarter.
 // ---------------------------------------------------------------------------------------------
 enum KvBar : int {
   KV_KV_FULL = 0,
-  KV_Q_FULL = 1,     // [3]  Q of a step (lives until the step's dK product: one stage deeper than dY)
-  KV_Q_EMPTY = 4,    // [3]
-  KV_DO_FULL = 7,    // [2]  dY of a step (last used by the step's dV product)
-  KV_DO_EMPTY = 9,   // [2]
-  KV_ST_FULL = 11,   // S^T written by the MMA
-  KV_PT_READY = 12,  // P^T written to TMEM (over S^T)
-  KV_ACC_DONE = 13,  // dV / dK products of the step finished
-  KV_DRAIN = 14,
-  KV_LD_READY = 15,  // the step's per-query log-sum-exp and delta are staged in shared memory
+  KV_Q_FULL = 1,     // [K_STAGES, at most 4]  Q of a step (lives until the step's dK product: one stage deeper than dY)
+  KV_Q_EMPTY = 5,
+  KV_DO_FULL = 9,    // [V_STAGES, at most 3]  dY of a step (last used by the step's dV product)
+  KV_DO_EMPTY = 12,
+  KV_ST_FULL = 15,   // S^T written by the MMA
   KV_DPT_FULL = 16,  // dP^T written by the MMA
-  KV_DST_READY = 17, // dS^T written to TMEM (over dP^T)
-  KV_PT_HALF = 18,   // the first sixteen queries of every quarter of P^T, and
-  KV_DST_HALF = 19,  // of dS^T: their part of the product starts while the rest is formed
-  KV_BAR_COUNT = 20
+  KV_ACC_DONE = 17,  // the last dV / dK products finished
+  KV_DRAIN = 18,
+  // the element-wise warps arrive on these:
+  KV_LD_READY = 19,  // the step's per-query log-sum-exp and delta are staged in shared memory
+  KV_PT_READY = 20,  // P^T written to TMEM (over S^T)
+  KV_DST_READY = 21, // dS^T written to TMEM (over dP^T)
+  KV_PT_HALF = 22,   // the first sixteen queries of every quarter of P^T, and
+  KV_DST_HALF = 23,  // of dS^T: their part of the product starts while the rest is formed
+  KV_BAR_COUNT = 24
 };
 
-template <int HD, bool SPLIT, bool MASKED>
-__global__ void __launch_bounds__(BW_THREADS, 1)
+template <int HD, bool SPLIT, bool MASKED, bool NARROW>
+__global__ void __launch_bounds__((BwdPlan<SPLIT ? 128 : HD, NARROW>::THREADS), (BwdPlan<SPLIT ? 128 : HD, NARROW>::CTAS_PER_SM))
 sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                         const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
                         const BwdParams p) {
-  using PL = BwdPlan<SPLIT ? 128 : HD>;
+  using PL = BwdPlan<SPLIT ? 128 : HD, NARROW>;
+  constexpr int BN = PL::BN, EW_WARPS = PL::EW_WARPS, WARP_TMA = PL::WARP_TMA, WARP_MMA = PL::WARP_MMA;
+  constexpr uint32_t TMEM_COLS = PL::TMEM_COLS;
   constexpr int FMT = SPLIT ? 0 : 1;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-  const uint32_t bar0 = smem_base + PL::OFF_BAR_DQ;   // same seven-tile plan as the dQ kernel: Q ring where it has K, dY ring where it has V
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + PL::OFF_BAR_DQ + KV_BAR_COUNT * 8);
+  const uint32_t bar0 = smem_base + PL::OFF_BAR;
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + PL::OFF_BAR + KV_BAR_COUNT * 8);
   auto bar = [&](int i) { return bar0 + 8u * (uint32_t)i; };
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // launch order -> work item: longest causal work first inside groups of p.group heads (see the forward kernel)
@@ -484,9 +499,8 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   const int bi = bh / p.H, hi = bh - bi * p.H;   // batch item and head
   const int kt = rank;                  // key tile; tile 0 has the most causal work and comes first
   const int k0 = kt * BLK;
-  const int n_q_tiles = (T + BLK - 1) / BLK;
-  const int i_begin = p.causal ? kt : 0;
-  const int n = n_q_tiles - i_begin;    // query tiles to walk
+  const int i_begin = p.causal ? k0 / BN : 0;
+  const int n = (T + BN - 1) / BN - i_begin;    // query steps to walk
 
   // the aligned plan must fit in what was requested (it does unless the dynamic base is unusually placed)
   uint32_t dyn_bytes;
@@ -501,7 +515,7 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     prefetch_tensormap(&map_q); prefetch_tensormap(&map_k); prefetch_tensormap(&map_v); prefetch_tensormap(&map_do);
   }
   if (tid == 0) {
-    for (int i = 0; i < KV_BAR_COUNT; ++i) mbar_init(bar(i), (i == KV_PT_READY || i == KV_LD_READY || i == KV_DST_READY || i == KV_PT_HALF || i == KV_DST_HALF) ? (uint32_t)EW_WARPS : 1u);
+    for (int i = 0; i < KV_BAR_COUNT; ++i) mbar_init(bar(i), i >= KV_LD_READY ? (uint32_t)EW_WARPS : 1u);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == WARP_MMA) { tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), TMEM_COLS); tmem_relinquish(); }
@@ -515,7 +529,8 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     if (warp == WARP_MMA) tmem_dealloc(tmem_base, TMEM_COLS);
     return;
   }
-  constexpr uint32_t C_ST = 0, C_DPT = 128, C_DV = 256, C_DK = 384;
+  constexpr uint32_t C_ST = 0, C_DPT = BN, C_DV = 2 * BN, C_DK = 3 * BN;
+  static_assert(HD <= BN);
   bool ok = true;
 
   if (warp == WARP_TMA) {
@@ -523,27 +538,30 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       mbar_expect_tx(bar(KV_KV_FULL), 2 * PL::TILE_BYTES);
 #pragma unroll
       for (int s = 0; s < PL::SUB; ++s) {
-        tma_load_4d(smem_base + PL::OFF_RES0 + s * PL::SUB_BYTES, &map_k, bar(KV_KV_FULL), s * 64, k0, hi, bi);
-        tma_load_4d(smem_base + PL::OFF_RES1 + s * PL::SUB_BYTES, &map_v, bar(KV_KV_FULL), s * 64, k0, hi, bi);
+#pragma unroll
+        for (int r = 0; r < BLK; r += BN) {
+          tma_load_4d(smem_base + PL::OFF_RES0 + s * PL::SUB_BYTES + r * 128, &map_k, bar(KV_KV_FULL), s * 64, k0 + r, hi, bi);
+          tma_load_4d(smem_base + PL::OFF_RES1 + s * PL::SUB_BYTES + r * 128, &map_v, bar(KV_KV_FULL), s * 64, k0 + r, hi, bi);
+        }
       }
       int issued = 0, issued_do = 0;
       for (int it = 0; it < n && ok; ++it) {
         const int qs = it % PL::K_STAGES, ds = it % PL::V_STAGES;
         const uint32_t qph = (uint32_t)((it / PL::K_STAGES) & 1), dph = (uint32_t)((it / PL::V_STAGES) & 1);
-        const uint32_t q_dst = smem_base + PL::OFF_KRING + qs * PL::TILE_BYTES, do_dst = smem_base + PL::OFF_VRING + ds * PL::TILE_BYTES;
+        const uint32_t q_dst = smem_base + PL::OFF_KRING + qs * PL::RING_TILE_BYTES, do_dst = smem_base + PL::OFF_VRING + ds * PL::RING_TILE_BYTES;
         ok = mbar_wait(bar(KV_Q_EMPTY + qs), qph ^ 1u, p.status, 210, it);
         if (!ok) break;
-        mbar_expect_tx(bar(KV_Q_FULL + qs), PL::TILE_BYTES);
+        mbar_expect_tx(bar(KV_Q_FULL + qs), PL::RING_TILE_BYTES);
 #pragma unroll
         for (int s = 0; s < PL::SUB; ++s)
-          tma_load_4d(q_dst + s * PL::SUB_BYTES, &map_q, bar(KV_Q_FULL + qs), s * 64, (i_begin + it) * BLK, hi, bi);
+          tma_load_4d(q_dst + s * PL::RING_SUB_BYTES, &map_q, bar(KV_Q_FULL + qs), s * 64, (i_begin + it) * BN, hi, bi);
         issued = it + 1;
         ok = mbar_wait(bar(KV_DO_EMPTY + ds), dph ^ 1u, p.status, 211, it);
         if (!ok) break;
-        mbar_expect_tx(bar(KV_DO_FULL + ds), PL::TILE_BYTES);
+        mbar_expect_tx(bar(KV_DO_FULL + ds), PL::RING_TILE_BYTES);
 #pragma unroll
         for (int s = 0; s < PL::SUB; ++s)
-          tma_load_4d(do_dst + s * PL::SUB_BYTES, &map_do, bar(KV_DO_FULL + ds), s * 64, (i_begin + it) * BLK, hi, bi);
+          tma_load_4d(do_dst + s * PL::RING_SUB_BYTES, &map_do, bar(KV_DO_FULL + ds), s * 64, (i_begin + it) * BN, hi, bi);
         issued_do = it + 1;
       }
       if (!ok) {
@@ -560,14 +578,14 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     {
       const uint32_t leader = elect_one() ? 1u : 0u;
       const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
-      constexpr uint32_t IDESC_NT = make_idesc_fmt(BLK, BLK, 0, 0, FMT);
+      constexpr uint32_t IDESC_NT = make_idesc_fmt(BLK, BN, 0, 0, FMT);
       constexpr uint32_t IDESC_ACC = make_idesc_fmt(BLK, HD, 0, 1, FMT);
       const uint32_t k_addr = smem_base + PL::OFF_RES0, v_addr = smem_base + PL::OFF_RES1;
       auto issue_nt = [&](uint32_t d_col, uint32_t a_addr, uint32_t b_addr) {
         if constexpr (SPLIT) {
 #pragma unroll
           for (int term = 0; term < 3; ++term) {
-            const uint32_t oa = term == 2 ? PL::SUB_BYTES : 0u, ob = term == 1 ? PL::SUB_BYTES : 0u;
+            const uint32_t oa = term == 2 ? PL::SUB_BYTES : 0u, ob = term == 1 ? PL::RING_SUB_BYTES : 0u;
 #pragma unroll
             for (int kk = 0; kk < HD / 16; ++kk)
               umma_ss_if<false>(leader, tmem_u + d_col, make_desc(a_addr + oa + kk * 32, 16, 1024), make_desc(b_addr + ob + kk * 32, 16, 1024),
@@ -576,22 +594,22 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         } else {
 #pragma unroll
           for (int kk = 0; kk < HD / 16; ++kk) {
-            const uint32_t off = (kk / 4) * PL::SUB_BYTES + (kk % 4) * 32;
-            umma_ss_if<false>(leader, tmem_u + d_col, make_desc(a_addr + off, 16, 1024), make_desc(b_addr + off, 16, 1024), IDESC_NT, kk > 0);
+            umma_ss_if<false>(leader, tmem_u + d_col, make_desc(a_addr + (kk / 4) * PL::SUB_BYTES + (kk % 4) * 32, 16, 1024),
+                              make_desc(b_addr + (kk / 4) * PL::RING_SUB_BYTES + (kk % 4) * 32, 16, 1024), IDESC_NT, kk > 0);
           }
         }
       };
-      // acc += A^T-from-TMEM x B with B a 128 x HD tile read MN-major; split mode: hi.hi + hi.lo + lo.hi
+      // acc += A^T-from-TMEM x B with B a BN x HD tile read MN-major; split mode: hi.hi + hi.lo + lo.hi
       auto issue_acc = [&](uint32_t d_col, uint32_t a_col, uint32_t b_addr, bool first_step, int half) {   // half: the even or the odd sixteens
 #pragma unroll
-        for (int k2 = 0; k2 < BLK / 32; ++k2) {
+        for (int k2 = 0; k2 < BN / 32; ++k2) {
           const int kk = 2 * k2 + half;
           const uint32_t a_hi = tmem_u + a_col + (kk / 2) * 32 + (kk % 2) * 8;
-          umma_ts_if<false>(leader, tmem_u + d_col, a_hi, make_desc(b_addr + kk * 2048, PL::SUB_BYTES, 1024), IDESC_ACC,
+          umma_ts_if<false>(leader, tmem_u + d_col, a_hi, make_desc(b_addr + kk * 2048, PL::RING_SUB_BYTES, 1024), IDESC_ACC,
                             (!first_step || kk > 0) ? 1u : 0u);
           if constexpr (SPLIT) {
-            umma_ts_if<false>(leader, tmem_u + d_col, a_hi, make_desc(b_addr + PL::SUB_BYTES + kk * 2048, PL::SUB_BYTES, 1024), IDESC_ACC, 1u);
-            umma_ts_if<false>(leader, tmem_u + d_col, a_hi + 16, make_desc(b_addr + kk * 2048, PL::SUB_BYTES, 1024), IDESC_ACC, 1u);
+            umma_ts_if<false>(leader, tmem_u + d_col, a_hi, make_desc(b_addr + PL::RING_SUB_BYTES + kk * 2048, PL::RING_SUB_BYTES, 1024), IDESC_ACC, 1u);
+            umma_ts_if<false>(leader, tmem_u + d_col, a_hi + 16, make_desc(b_addr + kk * 2048, PL::RING_SUB_BYTES, 1024), IDESC_ACC, 1u);
           }
         }
       };
@@ -600,8 +618,8 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       //   dV(it), S^T(it+1), dK(it), dP^T(it+1),
       // (the in-order pipe keeps every product behind the one that still reads the columns it overwrites),
       // so the element-wise warps work on P^T(it+1) while dK(it) and dP^T(it+1) run.
-      auto q_stage = [&](int it) { return smem_base + PL::OFF_KRING + (it % PL::K_STAGES) * PL::TILE_BYTES; };
-      auto do_stage = [&](int it) { return smem_base + PL::OFF_VRING + (it % PL::V_STAGES) * PL::TILE_BYTES; };
+      auto q_stage = [&](int it) { return smem_base + PL::OFF_KRING + (it % PL::K_STAGES) * PL::RING_TILE_BYTES; };
+      auto do_stage = [&](int it) { return smem_base + PL::OFF_VRING + (it % PL::V_STAGES) * PL::RING_TILE_BYTES; };
       auto wait_q = [&](int it) {
         return __all_sync(0xffffffffu, mbar_wait(bar(KV_Q_FULL + it % PL::K_STAGES), (uint32_t)((it / PL::K_STAGES) & 1), p.status, 221, it));
       };
@@ -661,14 +679,14 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     // ------------------------------------------------------------------ element-wise warps
     const int qtr = warp >> 2, lane_base = (warp & 3) * 32, row = lane_base + lane;
     const int kj = k0 + row;               // this thread's key
-    constexpr int OC = HD / 4;
+    constexpr int OC = HD / (EW_WARPS / 4);
     const uint32_t t_row = tmem_base + ((uint32_t)lane_base << 16);
-    // The query-dependent terms (minus log-sum-exp, minus delta x scale) are the same for every key row: the first 256
+    // The query-dependent terms (minus log-sum-exp, minus delta x scale) are the same for every key row: the first 2 BN
     // element-wise threads fetch one value each a step ahead and stage them in shared memory, so that the
     // inner loop reads them as broadcasts instead of 64 global loads per thread.  Rows beyond T get
     // lse = +inf, which makes their probabilities exactly zero.
-    float (*s_nlse)[BLK] = reinterpret_cast<float (*)[BLK]>(smem_gen + PL::OFF_STAGE_KV);
-    float (*s_del)[BLK] = s_nlse + 2;
+    float (*s_nlse)[BN] = reinterpret_cast<float (*)[BN]>(smem_gen + PL::OFF_STAGE_KV);
+    float (*s_del)[BN] = s_nlse + 2;
     // split mode: S^T and dP^T carry the pre-pass's scales; dS^T is kept in the units of dP' x 2^-19 and P^T 2^10 larger
     float4 sc = make_float4(1.f, 1.f, 1.f, 1.f);
     if constexpr (SPLIT) sc = mca_ld_f4(reinterpret_cast<const float*>(p.scales + bh));
@@ -676,20 +694,20 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     const float dmul = SPLIT ? DS_SHIFT : p.scale;
     const float del_mul = SPLIT ? (sc.w * DS_SHIFT) * sc.z : p.scale;
     auto fetch = [&](int it) -> float {
-      const int qi = (i_begin + it) * BLK + (tid & (BLK - 1));
-      if (tid >= 2 * BLK || it >= n || qi >= T) return tid < BLK ? -INFINITY : 0.f;
-      return tid < BLK ? -mca_ld_f1(p.lse + (int64_t)bh * T + qi) : -mca_ld_f1(p.delta + (int64_t)bh * T + qi) * del_mul;
+      const int qi = (i_begin + it) * BN + (tid & (BN - 1));
+      if (tid >= 2 * BN || it >= n || qi >= T) return tid < BN ? -INFINITY : 0.f;
+      return tid < BN ? -mca_ld_f1(p.lse + (int64_t)bh * T + qi) : -mca_ld_f1(p.delta + (int64_t)bh * T + qi) * del_mul;
     };
     auto stage = [&](int it, float v) {
-      if (tid < BLK) s_nlse[it & 1][tid] = v;
-      else if (tid < 2 * BLK) s_del[it & 1][tid - BLK] = v;
+      if (tid < BN) s_nlse[it & 1][tid] = v;
+      else if (tid < 2 * BN) s_del[it & 1][tid - BN] = v;
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(KV_LD_READY));
     };
     if (n > 0) stage(0, fetch(0));
     for (int it = 0; it < n && ok; ++it) {
       const int q_local = qtr * 32;                         // first of this thread's 32 queries within the tile
-      const int q_base = (i_begin + it) * BLK + q_local;
+      const int q_base = (i_begin + it) * BN + q_local;
       const float next = fetch(it + 1);                     // in flight while this step is processed
       ok = __all_sync(0xffffffffu, mbar_wait(bar(KV_LD_READY), (uint32_t)(it & 1), p.status, 231, it));
       if (!ok) break;
@@ -698,11 +716,11 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       tc_fence_after();
       const float* nlse_s = s_nlse[it & 1] + q_local;
       const float* del_s = s_del[it & 1] + q_local;
-      const bool diag = p.causal && (i_begin + it) * BLK < k0 + BLK;   // only the diagonal tile needs the causal test
+      const bool diag = p.causal && (i_begin + it) * BN < k0 + BLK;   // only the diagonal tile needs the causal test
       uint32_t mw = 0xffffffffu;          // keep-bits of this thread's key against its 32 queries of the step
       if constexpr (MASKED) {
         if (p.mask_bits_t != nullptr)
-          mw = __ldg(p.mask_bits_t + (int64_t)min(kj, T - 1) * p.mask_row_stride + 4 * (i_begin + it) + qtr);
+          mw = __ldg(p.mask_bits_t + (int64_t)min(kj, T - 1) * p.mask_row_stride + (BN / 32) * (i_begin + it) + qtr);
         else
           mw = ((__ldg(p.mask_bits + (int64_t)bi * p.mask_batch_stride + (min(kj, T - 1) >> 5)) >> (kj & 31)) & 1u) ? 0xffffffffu : 0u;
       }
@@ -815,11 +833,11 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       stage_columns<PR, OC, SPLIT>(tile_k, row, qtr, t_row + C_DK + qtr * OC, mul_k);
       stage_columns<PR, OC, SPLIT>(tile_v, row, qtr, t_row + C_DV + qtr * OC, mul_v);
     }
-    ew_bar_sync();
+    ew_bar_sync<EW_WARPS>();
     if (fin) {
       const int64_t off0 = (int64_t)bi * p.os.b + (int64_t)hi * p.os.h + (int64_t)k0 * p.os.t;
-      store_staged_rows<PR, ESZ>(tile_k, warp, lane, p.out0, off0, p.os.t, min(BLK, T - k0));
-      store_staged_rows<PR, ESZ>(tile_v, warp, lane, p.out1, off0, p.os.t, min(BLK, T - k0));
+      store_staged_rows<PR, ESZ, BLK / EW_WARPS>(tile_k, warp, lane, p.out0, off0, p.os.t, min(BLK, T - k0));
+      store_staged_rows<PR, ESZ, BLK / EW_WARPS>(tile_v, warp, lane, p.out1, off0, p.os.t, min(BLK, T - k0));
     }
   }
   tc_fence_before();
@@ -870,22 +888,22 @@ __global__ void __launch_bounds__(256) bwd_delta_bf16_kernel(const __nv_bfloat16
 }
 
 // Both kernels of one backward, with or without the caller's mask.
-template <int HD, bool SPLIT, bool MASKED>
+template <int HD, bool SPLIT, bool MASKED, bool NARROW>
 int launch_bwd_pair(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mdo, BwdParams p,
                     void* dq, void* dk, void* dv, int B, int H, int T, cudaStream_t st) {
-  using PL = BwdPlan<SPLIT ? 128 : HD>;
+  using PL = BwdPlan<SPLIT ? 128 : HD, NARROW>;
   const size_t smem_kv = PL::BYTES_KV, smem_dq = PL::BYTES_DQ;
   static std::atomic<uint64_t> done_kv{0}, done_dq{0};
   int e;
-  if ((e = mca_smem_once(done_kv, sdpa_bwd_dkdv_tc_kernel<HD, SPLIT, MASKED>, smem_kv)) ||
-      (e = mca_smem_once(done_dq, sdpa_bwd_dq_tc_kernel<HD, SPLIT, MASKED>, smem_dq)))
+  if ((e = mca_smem_once(done_kv, sdpa_bwd_dkdv_tc_kernel<HD, SPLIT, MASKED, NARROW>, smem_kv)) ||
+      (e = mca_smem_once(done_dq, sdpa_bwd_dq_tc_kernel<HD, SPLIT, MASKED, NARROW>, smem_dq)))
     return e;
   dim3 grid(mca_ceil_div(T, BLK), B * H);
   p.out0 = dk; p.out1 = dv;
-  e = mca_launch_pdl(sdpa_bwd_dkdv_tc_kernel<HD, SPLIT, MASKED>, grid, dim3(BW_THREADS), smem_kv, st, mq, mk, mv, mdo, p);
+  e = mca_launch_pdl(sdpa_bwd_dkdv_tc_kernel<HD, SPLIT, MASKED, NARROW>, grid, dim3(PL::THREADS), smem_kv, st, mq, mk, mv, mdo, p);
   if (e) return e;
   p.out0 = dq; p.out1 = nullptr;
-  return mca_launch_pdl(sdpa_bwd_dq_tc_kernel<HD, SPLIT, MASKED>, grid, dim3(BW_THREADS), smem_dq, st, mq, mk, mv, mdo, p);
+  return mca_launch_pdl(sdpa_bwd_dq_tc_kernel<HD, SPLIT, MASKED, NARROW>, grid, dim3(PL::THREADS), smem_dq, st, mq, mk, mv, mdo, p);
 }
 
 void set_mask(BwdParams& p, const McaMaskBits* mask, int T) {
@@ -901,11 +919,13 @@ int launch_bwd(const void* q, const void* k, const void* v, const void* dy, cons
                int causal, int B, int H, int T, void* dq, void* dk, void* dv, int* status, int layout, cudaStream_t st,
                const McaMaskBits* mask = nullptr) {
   if (mask != nullptr && causal) return ERROR_ATTN_UNSUPPORTED_SHAPE;
+  constexpr bool NARROW = HD <= 64;
+  constexpr int BN = BwdPlan<HD, NARROW>::BN;
   CUtensorMap mq, mk, mv, mdo;
   int e;
   const McaStrides sin = mca_in_strides(layout, H, T, HD), sout = mca_out_strides(layout, H, T, HD);
-  if ((e = make_map_bf16(&mq, q, B, H, T, HD, sin)) || (e = make_map_bf16(&mk, k, B, H, T, HD, sin)) ||
-      (e = make_map_bf16(&mv, v, B, H, T, HD, sin)) || (e = make_map_bf16(&mdo, dy, B, H, T, HD, sout)))
+  if ((e = make_map_bf16(&mq, q, B, H, T, HD, sin, BN)) || (e = make_map_bf16(&mk, k, B, H, T, HD, sin, BN)) ||
+      (e = make_map_bf16(&mv, v, B, H, T, HD, sin, BN)) || (e = make_map_bf16(&mdo, dy, B, H, T, HD, sout, BN)))
     return e;
   BwdParams p;
   p.scales = nullptr;
@@ -919,8 +939,8 @@ int launch_bwd(const void* q, const void* k, const void* v, const void* dy, cons
   p.scale = 1.0f / sqrtf((float)HD);
   p.scale_log2 = p.scale * 1.4426950408889634f;
   set_mask(p, mask, T);
-  if (mask != nullptr) return launch_bwd_pair<HD, false, true>(mq, mk, mv, mdo, p, dq, dk, dv, B, H, T, st);
-  return launch_bwd_pair<HD, false, false>(mq, mk, mv, mdo, p, dq, dk, dv, B, H, T, st);
+  if (mask != nullptr) return launch_bwd_pair<HD, false, true, NARROW>(mq, mk, mv, mdo, p, dq, dk, dv, B, H, T, st);
+  return launch_bwd_pair<HD, false, false, NARROW>(mq, mk, mv, mdo, p, dq, dk, dv, B, H, T, st);
 }
 
 // Split-operand backward for fp32 callers.  The workspace still holds the fp16 halves of q, k, v the forward's pre-pass
@@ -956,8 +976,8 @@ int launch_bwd_split(const float* dy, const float* y_copy, const float* lse, flo
   p.scale = 1.0f / sqrtf((float)HD);
   p.scale_log2 = p.scale * 1.4426950408889634f;
   set_mask(p, mask, T);
-  if (mask != nullptr) return launch_bwd_pair<HD, true, true>(mq, mk, mv, mdo, p, dq, dk, dv, B, H, T, st);
-  return launch_bwd_pair<HD, true, false>(mq, mk, mv, mdo, p, dq, dk, dv, B, H, T, st);
+  if (mask != nullptr) return launch_bwd_pair<HD, true, true, false>(mq, mk, mv, mdo, p, dq, dk, dv, B, H, T, st);
+  return launch_bwd_pair<HD, true, false, false>(mq, mk, mv, mdo, p, dq, dk, dv, B, H, T, st);
 }
 
 }  // namespace

@@ -475,21 +475,21 @@ inline EncodeTiledFn get_encode_fn() {
 
 // (BH, T, HD) bf16 tensor, box = 64 columns x 128 rows of one (b,h), 128-byte swizzle.
 inline int make_map_4d(CUtensorMap* map, const void* base, CUtensorMapDataType type, int elt, int B, int H, int T, int HD,
-                       const McaStrides& st, CUtensorMapSwizzle swizzle) {
+                       const McaStrides& st, CUtensorMapSwizzle swizzle, int box_rows = BLK) {
   EncodeTiledFn fn = get_encode_fn();
   if (!fn) return ERROR_NOT_IMPLEMENTED;
   cuuint64_t dims[4] = {(cuuint64_t)HD, (cuuint64_t)T, (cuuint64_t)H, (cuuint64_t)B};
   cuuint64_t strides[3] = {(cuuint64_t)st.t * elt, (cuuint64_t)st.h * elt, (cuuint64_t)st.b * elt};
-  cuuint32_t box[4] = {(cuuint32_t)(128 / elt), (cuuint32_t)BLK, 1, 1};
+  cuuint32_t box[4] = {(cuuint32_t)(128 / elt), (cuuint32_t)box_rows, 1, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = fn(map, type, 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : ERROR_PARAM_OUT_OF_RANGE;
 }
-// bf16 view (B, H, T, HD) with the given element strides, box = 64 columns (128 bytes) x 128 rows of one
+// bf16 view (B, H, T, HD) with the given element strides, box = 64 columns (128 bytes) x box_rows rows of one
 // (b,h), 128-byte swizzle.  Rows beyond T are zero-filled per head.
-inline int make_map_bf16(CUtensorMap* map, const void* base, int B, int H, int T, int HD, const McaStrides& st) {
-  return make_map_4d(map, base, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, B, H, T, HD, st, CU_TENSOR_MAP_SWIZZLE_128B);
+inline int make_map_bf16(CUtensorMap* map, const void* base, int B, int H, int T, int HD, const McaStrides& st, int box_rows = BLK) {
+  return make_map_4d(map, base, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, B, H, T, HD, st, CU_TENSOR_MAP_SWIZZLE_128B, box_rows);
 }
 // fp32 view, box = 32 columns (128 bytes) x 128 rows of one (b,h).  K-major operands
 // use the ordinary 128-byte swizzle; an MN-major tf32 operand (V) must use the 32-byte-atom variant
