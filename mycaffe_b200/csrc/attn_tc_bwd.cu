@@ -163,7 +163,7 @@ __device__ __forceinline__ void store_staged_rows(uint8_t* tile, int w, int lane
 // [5/2 BN, 3 BN)  dQ behind them
 // ---------------------------------------------------------------------------------------------
 enum DqBar : int {
-  DQ_QDO_FULL = 0,
+  DQ_Q_FULL = 0,
   DQ_K_FULL = 1,    // [K_STAGES, at most 4]
   DQ_K_EMPTY = 5,
   DQ_V_FULL = 9,    // [V_STAGES, at most 3]
@@ -173,7 +173,8 @@ enum DqBar : int {
   DQ_DS_READY = 17, // dS written to TMEM
   DQ_DQ_DONE = 18,  // dQ += dS K of the step finished (dS may be overwritten)
   DQ_DRAIN = 19,
-  DQ_BAR_COUNT = 20
+  DQ_DO_FULL = 20,
+  DQ_BAR_COUNT = 21
 };
 
 template <int HD, bool SPLIT, bool MASKED, bool NARROW>
@@ -237,15 +238,16 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
 
   if (warp == WARP_TMA) {
     if (lane == 0) {
-      mbar_expect_tx(bar(DQ_QDO_FULL), 2 * PL::TILE_BYTES);
+      // one resident tile; S(0) waits for Q and K(0) only, so those come first
+      auto load_resident = [&](uint32_t dst, const CUtensorMap* map, int full) {
+        mbar_expect_tx(bar(full), PL::TILE_BYTES);
 #pragma unroll
-      for (int s = 0; s < PL::SUB; ++s) {
+        for (int s = 0; s < PL::SUB; ++s)
 #pragma unroll
-        for (int r = 0; r < BLK; r += BN) {   // a copy's box is BN rows
-          tma_load_4d(smem_base + PL::OFF_RES0 + s * PL::SUB_BYTES + r * 128, &map_q, bar(DQ_QDO_FULL), s * 64, q0 + r, hi, bi);
-          tma_load_4d(smem_base + PL::OFF_RES1 + s * PL::SUB_BYTES + r * 128, &map_do, bar(DQ_QDO_FULL), s * 64, q0 + r, hi, bi);
-        }
-      }
+          for (int r = 0; r < BLK; r += BN)   // a copy's box is BN rows
+            tma_load_4d(smem_base + dst + s * PL::SUB_BYTES + r * 128, map, bar(full), s * 64, q0 + r, hi, bi);
+      };
+      load_resident(PL::OFF_RES0, &map_q, DQ_Q_FULL);
       int issued_k = 0, issued_v = 0;
       for (int j = 0; j < n && ok; ++j) {
         const int ks = j % PL::K_STAGES, vs = j % PL::V_STAGES;
@@ -257,6 +259,7 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
 #pragma unroll
         for (int s = 0; s < PL::SUB; ++s) tma_load_4d(k_dst + s * PL::RING_SUB_BYTES, &map_k, bar(DQ_K_FULL + ks), s * 64, j * BN, hi, bi);
         issued_k = j + 1;
+        if (j == 0) load_resident(PL::OFF_RES1, &map_do, DQ_DO_FULL);
         ok = mbar_wait(bar(DQ_V_EMPTY + vs), vph ^ 1u, p.status, 111, j);
         if (!ok) break;
         mbar_expect_tx(bar(DQ_V_FULL + vs), PL::RING_TILE_BYTES);
@@ -265,7 +268,8 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         issued_v = j + 1;
       }
       if (!ok) {  // let copies in flight land (bounded) before the CTA's memory is released
-        mbar_wait(bar(DQ_QDO_FULL), 0, p.status, 112, 0);
+        mbar_wait(bar(DQ_Q_FULL), 0, p.status, 112, 0);
+        if (issued_k > 0) mbar_wait(bar(DQ_DO_FULL), 0, p.status, 115, 0);
         for (int j = max(0, issued_k - PL::K_STAGES); j < issued_k; ++j)
           mbar_wait(bar(DQ_K_FULL + j % PL::K_STAGES), (uint32_t)((j / PL::K_STAGES) & 1), p.status, 113, j);
         for (int j = max(0, issued_v - PL::V_STAGES); j < issued_v; ++j)
@@ -306,12 +310,17 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         issue_nt(C_S, q_addr, k_addr);
         issue_nt(C_DP, do_addr, v_addr);
       };
-      ok = __all_sync(0xffffffffu, mbar_wait(bar(DQ_QDO_FULL), 0, p.status, 120, 0));
+      ok = __all_sync(0xffffffffu, mbar_wait(bar(DQ_Q_FULL), 0, p.status, 120, 0));
       if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar(DQ_K_FULL + 0), 0, p.status, 121, 0));
+      if (ok) {
+        tc_fence_after();
+        issue_nt(C_S, q_addr, smem_base + PL::OFF_KRING);
+        ok = __all_sync(0xffffffffu, mbar_wait(bar(DQ_DO_FULL), 0, p.status, 128, 0));
+      }
       if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar(DQ_V_FULL + 0), 0, p.status, 122, 0));
       if (ok) {
         tc_fence_after();
-        issue_sdp(0);
+        issue_nt(C_DP, do_addr, smem_base + PL::OFF_VRING);
         umma_commit_if(leader, bar(DQ_SDP_FULL));
         umma_commit_if(leader, bar(DQ_V_EMPTY + 0));
       }
@@ -455,7 +464,7 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
 // mode their fp16 hi halves do, and the lo halves take the other 16 columns of the quarter.
 // ---------------------------------------------------------------------------------------------
 enum KvBar : int {
-  KV_KV_FULL = 0,
+  KV_K_FULL = 0,
   KV_Q_FULL = 1,     // [K_STAGES, at most 4]  Q of a step (lives until the step's dK product: one stage deeper than dY)
   KV_Q_EMPTY = 5,
   KV_DO_FULL = 9,    // [V_STAGES, at most 3]  dY of a step (last used by the step's dV product)
@@ -464,13 +473,15 @@ enum KvBar : int {
   KV_DPT_FULL = 16,  // dP^T written by the MMA
   KV_ACC_DONE = 17,  // the last dV / dK products finished
   KV_DRAIN = 18,
+  KV_V_FULL = 19,
+  KV_DV_DONE = 20,   // the last dV product finished
   // the element-wise warps arrive on these:
-  KV_LD_READY = 19,  // the step's per-query log-sum-exp and delta are staged in shared memory
-  KV_PT_READY = 20,  // P^T written to TMEM (over S^T)
-  KV_DST_READY = 21, // dS^T written to TMEM (over dP^T)
-  KV_PT_HALF = 22,   // the first sixteen queries of every quarter of P^T, and
-  KV_DST_HALF = 23,  // of dS^T: their part of the product starts while the rest is formed
-  KV_BAR_COUNT = 24
+  KV_LD_READY = 21,  // the step's per-query log-sum-exp and delta are staged in shared memory
+  KV_PT_READY = 22,  // P^T written to TMEM (over S^T)
+  KV_DST_READY = 23, // dS^T written to TMEM (over dP^T)
+  KV_PT_HALF = 24,   // the first sixteen queries of every quarter of P^T, and
+  KV_DST_HALF = 25,  // of dS^T: their part of the product starts while the rest is formed
+  KV_BAR_COUNT = 26
 };
 
 template <int HD, bool SPLIT, bool MASKED, bool NARROW>
@@ -535,15 +546,16 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 
   if (warp == WARP_TMA) {
     if (lane == 0) {
-      mbar_expect_tx(bar(KV_KV_FULL), 2 * PL::TILE_BYTES);
+      // one resident tile; S^T(0) waits for K and Q(0) only, so those come first
+      auto load_resident = [&](uint32_t dst, const CUtensorMap* map, int full) {
+        mbar_expect_tx(bar(full), PL::TILE_BYTES);
 #pragma unroll
-      for (int s = 0; s < PL::SUB; ++s) {
+        for (int s = 0; s < PL::SUB; ++s)
 #pragma unroll
-        for (int r = 0; r < BLK; r += BN) {
-          tma_load_4d(smem_base + PL::OFF_RES0 + s * PL::SUB_BYTES + r * 128, &map_k, bar(KV_KV_FULL), s * 64, k0 + r, hi, bi);
-          tma_load_4d(smem_base + PL::OFF_RES1 + s * PL::SUB_BYTES + r * 128, &map_v, bar(KV_KV_FULL), s * 64, k0 + r, hi, bi);
-        }
-      }
+          for (int r = 0; r < BLK; r += BN)
+            tma_load_4d(smem_base + dst + s * PL::SUB_BYTES + r * 128, map, bar(full), s * 64, k0 + r, hi, bi);
+      };
+      load_resident(PL::OFF_RES0, &map_k, KV_K_FULL);
       int issued = 0, issued_do = 0;
       for (int it = 0; it < n && ok; ++it) {
         const int qs = it % PL::K_STAGES, ds = it % PL::V_STAGES;
@@ -556,6 +568,7 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         for (int s = 0; s < PL::SUB; ++s)
           tma_load_4d(q_dst + s * PL::RING_SUB_BYTES, &map_q, bar(KV_Q_FULL + qs), s * 64, (i_begin + it) * BN, hi, bi);
         issued = it + 1;
+        if (it == 0) load_resident(PL::OFF_RES1, &map_v, KV_V_FULL);
         ok = mbar_wait(bar(KV_DO_EMPTY + ds), dph ^ 1u, p.status, 211, it);
         if (!ok) break;
         mbar_expect_tx(bar(KV_DO_FULL + ds), PL::RING_TILE_BYTES);
@@ -565,7 +578,8 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         issued_do = it + 1;
       }
       if (!ok) {
-        mbar_wait(bar(KV_KV_FULL), 0, p.status, 212, 0);
+        mbar_wait(bar(KV_K_FULL), 0, p.status, 212, 0);
+        if (issued > 0) mbar_wait(bar(KV_V_FULL), 0, p.status, 215, 0);
         for (int it = max(0, issued - PL::K_STAGES); it < issued; ++it)
           mbar_wait(bar(KV_Q_FULL + it % PL::K_STAGES), (uint32_t)((it / PL::K_STAGES) & 1), p.status, 213, it);
         for (int it = max(0, issued_do - PL::V_STAGES); it < issued_do; ++it)
@@ -634,13 +648,17 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         issue_nt(C_DPT, v_addr, do_stage(it));
         umma_commit_if(leader, bar(KV_DPT_FULL));
       };
-      ok = __all_sync(0xffffffffu, mbar_wait(bar(KV_KV_FULL), 0, p.status, 220, 0));
+      ok = __all_sync(0xffffffffu, mbar_wait(bar(KV_K_FULL), 0, p.status, 220, 0));
       if (ok && n > 0) {
         ok = wait_q(0);
-        if (ok) ok = wait_do(0);
         if (ok) {
           tc_fence_after();
           issue_st(0);
+          ok = __all_sync(0xffffffffu, mbar_wait(bar(KV_V_FULL), 0, p.status, 228, 0));
+        }
+        if (ok) ok = wait_do(0);
+        if (ok) {
+          tc_fence_after();
           issue_dpt(0);
         }
       }
@@ -657,6 +675,7 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         tc_fence_after();
         issue_acc(C_DV, C_ST, do_addr, it == 0, 1);
         if (it + 1 < n) issue_st(it + 1);
+        else umma_commit_if(leader, bar(KV_DV_DONE));
         umma_commit_if(leader, bar(KV_DO_EMPTY + it % PL::V_STAGES));   // dY(it) was last read by dV
         // dK += dS^T Q
         ok = __all_sync(0xffffffffu, mbar_wait(bar(KV_DST_HALF), (uint32_t)(it & 1), p.status, 226, it));
@@ -821,17 +840,21 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       if (it + 1 < n) stage(it + 1, next);
       hand_over(KV_DST_READY);
     }
-    if (ok && n > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar(KV_ACC_DONE), 0, p.status, 232, n));
+    if (ok && n > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar(KV_DV_DONE), 0, p.status, 234, n));
     constexpr int ESZ = SPLIT ? 4 : 2, PR = HD * ESZ / 16;
     uint8_t* tile_k = smem_gen + PL::OFF_RES0;         // the K and V tiles: every product has finished with them
     uint8_t* tile_v = smem_gen + PL::OFF_RES1;
+    if (ok && n > 0) {   // dV beside the last dK product
+      tc_fence_after();
+      const float mul_v = SPLIT ? PT_UNSHIFT * (1.0f / sc.w) : 1.0f;
+      stage_columns<PR, OC, SPLIT>(tile_v, row, qtr, t_row + C_DV + qtr * OC, mul_v);
+      ok = __all_sync(0xffffffffu, mbar_wait(bar(KV_ACC_DONE), 0, p.status, 232, n));
+    }
     const bool fin = ok && n > 0;
     if (fin) {
       tc_fence_after();
       const float mul_k = SPLIT ? p.scale * DS_UNSHIFT * (1.0f / (sc.z * sc.x)) * (1.0f / sc.w) : 1.0f;
-      const float mul_v = SPLIT ? PT_UNSHIFT * (1.0f / sc.w) : 1.0f;
       stage_columns<PR, OC, SPLIT>(tile_k, row, qtr, t_row + C_DK + qtr * OC, mul_k);
-      stage_columns<PR, OC, SPLIT>(tile_v, row, qtr, t_row + C_DV + qtr * OC, mul_v);
     }
     ew_bar_sync<EW_WARPS>();
     if (fin) {
