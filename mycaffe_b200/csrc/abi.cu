@@ -40,6 +40,8 @@ struct AttnHandle {
   float *row_max = nullptr, *row_sum = nullptr, *y_copy = nullptr, *delta = nullptr, *lse = nullptr;
   void* split_ws = nullptr;    // fp16 halves of q, k, v for the split-operand tensor-core forward of fp32 handles
   int64_t split_ws_bytes = 0;
+  float* ds_ws = nullptr;      // dS between the two kernels of the exact fp32 backward (training handles that use it)
+  int64_t ds_floats = 0;
   float* mask_ws = nullptr;    // fp32 copies for a bf16 handle that is given a (T,T) or batch mask (allocated on first use)
   size_t mask_ws_floats = 0;
   uint32_t *mask_bits = nullptr, *mask_bits_t = nullptr;   // keep-bits of a (T,T) or batch mask for the tensor-core kernels
@@ -63,8 +65,9 @@ struct AttnHandle {
   bool status_pending = false;  // a tensor-core launch was made in asynchronous mode and its status words are unread
   void release() {
     cudaFree(row_max); cudaFree(row_sum); cudaFree(y_copy); cudaFree(delta); cudaFree(lse); cudaFree(causal_flag);
-    cudaFree(split_ws); cudaFree(mask_ws); cudaFree(mask_bits); cudaFree(mask_bits_t);
+    cudaFree(split_ws); cudaFree(ds_ws); cudaFree(mask_ws); cudaFree(mask_bits); cudaFree(mask_bits_t);
     split_ws = nullptr; split_ws_bytes = 0;
+    ds_ws = nullptr; ds_floats = 0;
     mask_ws = nullptr; mask_ws_floats = 0;
     mask_bits = mask_bits_t = nullptr; mask_bits_words = 0;
     row_max = row_sum = y_copy = delta = lse = nullptr;
@@ -420,6 +423,8 @@ long convert_mem(Kernel* k, long llInput, MCA_LONGLONG* pl) {
 
 // ---- attention ids ------------------------------------------------------------------------
 
+constexpr int64_t kMaxDsBytes = 1ll << 30;
+
 long attn_set(Kernel* k, long lInput, float* pf, long llInput, MCA_LONGLONG* pl) {
   long e;  // Device<T>::SetAttn, device.h:2463-2486 (exactly 9 longs there; 10th/11th are extensions)
   if ((e = verify_in(llInput, pl, 9, 11))) return e;
@@ -458,6 +463,15 @@ long attn_set(Kernel* k, long lInput, float* pf, long llInput, MCA_LONGLONG* pl)
     // simply keeps to the CUDA-core kernels.
     a.split_ws_bytes = mca_sdpa_forward_f32_tc_workspace_bytes_d(a.B, a.H, a.block, a.D);
     if (cudaMalloc(&a.split_ws, (size_t)a.split_ws_bytes) != cudaSuccess) { cudaGetLastError(); a.split_ws = nullptr; a.split_ws_bytes = 0; }
+  }
+  if (a.training && a.dtype != MCA_DTYPE_BF16 && ((a.flags & MCA_FLAG_EXACT_FP32) || !mca_sdpa_backward_f32_tc_supported(a.D))) {
+    // The exact fp32 backward passes dS from one kernel to the other: half of the (B,H,T,T) pair of tensors the reference keeps
+    // (attn.cu:436-452), up to a gigabyte.  Beyond that, or where it cannot be had, dS is formed twice.
+    const int64_t bytes = mca_sdpa_backward_f32_ws_bytes(a.B, a.H, a.block);
+    if (bytes <= kMaxDsBytes) {
+      if (cudaMalloc(&a.ds_ws, (size_t)bytes) == cudaSuccess) a.ds_floats = bytes / 4;
+      else { cudaGetLastError(); a.ds_ws = nullptr; }
+    }
   }
   a.configured = true;
   return 0;
@@ -834,8 +848,8 @@ long attn_bwd(Kernel* k, long llInput, MCA_LONGLONG* pl, int layout) {
   if (a.fwd_mask_handle != 0) {
     if ((e = resolve_mask(k, a, a.fwd_mask_handle, a.fwd_batch_mask, T, &mask, &mode, false))) return e;
   }
-  return mca_sdpa_backward_f32_layout(q, kk, v, dy, a.y_copy, mask, mode, a.causal_flag, a.row_max, a.row_sum, a.delta,
-                                      a.B, a.H, T, a.D, dq, dk, dv, layout, 0);
+  return mca_sdpa_backward_f32_ws(q, kk, v, dy, a.y_copy, mask, mode, a.causal_flag, a.row_max, a.row_sum, a.delta, a.B, a.H, T,
+                                  a.D, dq, dk, dv, a.ds_ws, a.ds_floats, layout, 0);
 }
 
 // ---- rope ids ------------------------------------------------------------------------------

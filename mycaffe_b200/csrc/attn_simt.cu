@@ -21,7 +21,7 @@
 // these reads and the transposed write free of bank conflicts and lets 128-wide heads fit (224 KB in the dK/dV kernel).
 // The tiles arrive by cp.async under the products that do not need them.
 // Backward of B = 2, H = 16, T = 1500, D = 128, causal: 2.71 ms with 64 x 64 tiles and 4 x 4 pieces, 1.92 ms with this (57 % of the
-// fp32 pipe: two warps per scheduler do not hide every load); B = 1, H = 12, T = 1516, D = 80 forward and backward: 1.75 -> 0.78 ms.
+// fp32 pipe: two warps per scheduler do not hide every load), 1.35 with dS formed once; B = 1, H = 12, T = 1516, D = 80 forward and backward: 1.75 -> 0.78 ms.
 #include <algorithm>
 
 #include "classify.cuh"
@@ -136,6 +136,20 @@ __device__ __forceinline__ void product_nt(const float* __restrict__ As, const f
     for (int b = 0; b < NB; ++b) s[a][b] = acc[a][b].x + acc[a][b].y;
 }
 
+// Row j of B, the columns of group cg.
+template <int DP, int R>
+__device__ __forceinline__ void load_columns(const float* __restrict__ Bs, int j, int cg, float2* bp, float& b1) {
+  using O = Out<DP, R>;
+  b1 = 0.f;
+#pragma unroll
+  for (int c = 0; c < O::N4; ++c) {
+    const float4 b = *reinterpret_cast<const float4*>(Bs + at<DP>(j, 16 * c + cg));
+    bp[2 * c] = make_float2(b.x, b.y); bp[2 * c + 1] = make_float2(b.z, b.w);
+  }
+  if constexpr (O::N2 > 0) bp[2 * O::N4] = *reinterpret_cast<const float2*>(Bs + at<DP>(j, (O::OFF2 + 2 * cg) >> 2) + ((2 * cg) & 3));
+  if constexpr (O::N1 > 0) b1 = Bs[at<DP>(j, (O::OFF1 + cg) >> 2) + (cg & 3)];
+}
+
 // acc[i] += sum_j X[j][r0 + i] * B[j][columns of group cg]
 template <int DP, int R>
 __device__ __forceinline__ void product_nn(const float* __restrict__ X, const float* __restrict__ Bs, int r0, int cg, Acc<DP, R>& acc) {
@@ -143,14 +157,8 @@ __device__ __forceinline__ void product_nn(const float* __restrict__ X, const fl
 #pragma unroll 2
   for (int j = 0; j < SX; ++j) {
     float2 bp[O::NP > 0 ? O::NP : 1];
-    float b1 = 0.f;
-#pragma unroll
-    for (int c = 0; c < O::N4; ++c) {
-      const float4 b = *reinterpret_cast<const float4*>(Bs + at<DP>(j, 16 * c + cg));
-      bp[2 * c] = make_float2(b.x, b.y); bp[2 * c + 1] = make_float2(b.z, b.w);
-    }
-    if constexpr (O::N2 > 0) bp[2 * O::N4] = *reinterpret_cast<const float2*>(Bs + at<DP>(j, (O::OFF2 + 2 * cg) >> 2) + ((2 * cg) & 3));
-    if constexpr (O::N1 > 0) b1 = Bs[at<DP>(j, (O::OFF1 + cg) >> 2) + (cg & 3)];
+    float b1;
+    load_columns<DP, R>(Bs, j, cg, bp, b1);
     float x[O::RPT];
 #pragma unroll
     for (int h = 0; h < O::RPT / 4; ++h) {
@@ -167,15 +175,15 @@ __device__ __forceinline__ void product_nn(const float* __restrict__ X, const fl
   }
 }
 
-// This thread's piece -> rows of a (T,D) view.
-template <int DP, int R>
+// This thread's piece -> rows row0, row0 + RS, ... of a (T,D) view.
+template <int DP, int R, int RS = 1>
 __device__ __forceinline__ void store_piece(float* __restrict__ g, int64_t ld, int row0, int cg, int T, int D, bool vec_ok,
                                             const Acc<DP, R>& acc) {
   using O = Out<DP, R>;
 #pragma unroll
   for (int i = 0; i < O::RPT; ++i) {
-    if (row0 + i >= T) continue;
-    float* dst = g + (int64_t)(row0 + i) * ld;
+    if (row0 + RS * i >= T) continue;
+    float* dst = g + (int64_t)(row0 + RS * i) * ld;
 #pragma unroll
     for (int c = 0; c < O::N4; ++c) {
       const int col = 64 * c + 4 * cg;
@@ -338,6 +346,13 @@ __global__ void sdpa_bwd_delta_kernel(const float* __restrict__ dY, const float*
 template <int DP, int R>
 constexpr size_t bwd_smem_bytes() { return sizeof(float) * (2 * (R + SX) * Row<DP>::LD + SX * R + 3 * SX); }
 
+// dS of (SX queries) x (R keys), as the dK/dV kernel leaves it for the dQ kernel: its tile X as it lies in shared memory, by head,
+// query block and key block.
+template <int R> __host__ __device__ __forceinline__ int64_t ds_tile(int bh, int qb, int kb, int T) {
+  const int nq = (T + SX - 1) / SX, nk = (T + R - 1) / R;
+  return (((int64_t)bh * nq + qb) * nk + kb) * (SX * R);
+}
+
 // dK, dV for one tile of R keys: walks the query tiles, recomputes P from the saved row
 // statistics, and accumulates dV += P^T dY, dK += dS^T Q (attn.cu:380-397, 637-657).
 template <int DP, int R>
@@ -345,8 +360,8 @@ __global__ void __launch_bounds__(NT) sdpa_bwd_dkdv_f32_kernel(
     const float* __restrict__ Q, const float* __restrict__ K, const float* __restrict__ V,
     const float* __restrict__ dY, const float* __restrict__ mask, int mask_mode, const int* __restrict__ causal_flag,
     const float* __restrict__ row_max, const float* __restrict__ row_sum, const float* __restrict__ delta, int H,
-    int T, int D, float scale, float* __restrict__ dK, float* __restrict__ dV, int vec_ok, int vec_out, const McaStrides sin,
-    const McaStrides sout) {
+    int T, int D, float scale, float* __restrict__ dK, float* __restrict__ dV, float* __restrict__ dS, int vec_ok, int vec_out,
+    const McaStrides sin, const McaStrides sout) {
   extern __shared__ __align__(16) float smem[];
   constexpr int LD = Row<DP>::LD, NA = R / 16, RPT = Out<DP, R>::RPT;
   float* Ks = smem;
@@ -415,18 +430,103 @@ __global__ void __launch_bounds__(NT) sdpa_bwd_dkdv_f32_kernel(
           *x = *x * (dp[a][bb] - de) * scale;
         }
       }
+      if (dS != nullptr) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncthreads();
+    if (dS != nullptr && tid == 0) {   // the whole tile as it lies, in one copy under the product
+      asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n\tcp.async.bulk.commit_group;" ::"l"(
+                       dS + ds_tile<R>(bh, q0 / SX, k0 / R, T)),
+                   "r"((uint32_t)__cvta_generic_to_shared(X)), "n"(SX * R * 4)
+                   : "memory");
+    }
     product_nn<DP, R>(X, Qs, r0, cg, dk);
+    if (dS != nullptr && tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // X may be overwritten
     __syncthreads();
     if (q0 + SX < T) load_rows<DP, SX>(Qs, Qg, sin.t, q0 + SX, T, D, vec_ok, tid);
     load_commit();
   }
   store_piece<DP, R>(dK + base, sin.t, k0 + r0, cg, T, D, vec_out != 0, dk);
   store_piece<DP, R>(dV + base, sin.t, k0 + r0, cg, T, D, vec_out != 0, dv);
+  if (dS != nullptr && tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
-// dQ for one tile of R queries: dQ = dS K with dS recomputed per key tile.
+// dQ for 64 queries from the dS the dK/dV kernel left: one product instead of three, so 5 of the backward's 7 are formed.  The FMA
+// pipe is the bound (67 % of it while a CTA is on the SM; the rest is the duplication of an operand for the pairs).  Steps of
+// 32 keys in a ring of three, so that two CTAs share an SM and four warps a scheduler; 64 queries a CTA whatever R is, so that
+// the last ones are short (128: 437 us, 64: 353); a thread's rows are 16 apart, so that the rows a warp reads at a time lie in
+// different banks.  dS (4 bytes per pair, written by one bulk copy a tile) costs the dK/dV kernel nothing that can be measured.
+// B = 2, H = 16, T = 1500, D = 128, causal: 911 -> 353 us, forward and backward 2048 -> 1480 us.
+constexpr int DS_KEYS = 32, DS_STAGES = 3;
+template <int DP> constexpr size_t dq_ds_smem_bytes() { return sizeof(float) * DS_STAGES * (SX * DS_KEYS + DS_KEYS * Row<DP>::LD); }
+template <int DP, int RK>
+__global__ void __launch_bounds__(NT, 2) sdpa_bwd_dq_ds_f32_kernel(const float* __restrict__ K, const float* dS, int mask_mode,
+                                                                   const int* __restrict__ causal_flag, int H, int T, int D,
+                                                                   float* __restrict__ dQ, int vec_ok, int vec_out, const McaStrides sin) {
+  extern __shared__ __align__(16) float smem[];
+  constexpr int R = SX;
+  using O = Out<DP, R>;
+  constexpr int A = R * DS_KEYS, STAGE = A + DS_KEYS * Row<DP>::LD;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int cg = (warp & 1) * 8 + lane_col(lane), rg = (warp >> 1) * 4 + lane_row(lane);   // rows rg + 16 i
+  const int bh = blockIdx.x, b = bh / H;
+  const int q0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * R;
+  const int mode = effective_mode(mask_mode, causal_flag);
+  const int64_t base = (int64_t)b * sin.b + (int64_t)(bh - b * H) * sin.h;
+  const int kv_end = (mode == MCA_MASK_CAUSAL) ? min(T, q0 + R) : T;
+  // This thread copies 16-byte vector lc of rows lr, lr + 32, ... of the step's dS (R rows of 32 keys).
+  constexpr int VPR = DS_KEYS / 4, RPP = NT / VPR;
+  const int lr = tid / VPR, lc = tid % VPR;
+  const float* src0 = dS + ds_tile<RK>(bh, q0 / SX, 0, T) + lr * RK;
+  auto load = [&](int k0, float* st) {
+    const float* src = src0 + (int64_t)(k0 / RK) * (SX * RK) + ((((k0 % RK) / 4 + lc) ^ (lr & 7)) << 2);
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(st + at<DS_KEYS>(lr, lc));
+#pragma unroll
+    for (int i = 0; i < R / RPP; ++i)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + i * RPP * DS_KEYS * 4), "l"(src + i * RPP * RK) : "memory");
+    load_rows<DP, DS_KEYS>(st + A, K + base, sin.t, k0, T, D, vec_ok, tid);
+  };
+  mca_pdl_wait();   // dS is the kernel before's
+#pragma unroll
+  for (int i = 0; i < DS_STAGES - 1; ++i) {
+    if (i * DS_KEYS < kv_end) load(i * DS_KEYS, smem + i * STAGE);
+    load_commit();
+  }
+  Acc<DP, R> dq;
+  dq.clear();
+  for (int k0 = 0, s = 0; k0 < kv_end; k0 += DS_KEYS, s = s + 1 == DS_STAGES ? 0 : s + 1) {
+    mca_cp_async_wait<DS_STAGES - 2>();
+    __syncthreads();                  // the step's tiles are in place, and the stage before them has been read
+    const int next = s == 0 ? DS_STAGES - 1 : s - 1;
+    if (k0 + (DS_STAGES - 1) * DS_KEYS < kv_end) load(k0 + (DS_STAGES - 1) * DS_KEYS, smem + next * STAGE);
+    load_commit();
+    const float *As = smem + s * STAGE, *Bs = As + A;
+#pragma unroll 2
+    for (int j4 = 0; j4 < DS_KEYS / 4; ++j4) {
+      float4 x[O::RPT];
+#pragma unroll
+      for (int i = 0; i < O::RPT; ++i) x[i] = *reinterpret_cast<const float4*>(As + at<DS_KEYS>(rg + 16 * i, j4));
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        const int j = 4 * j4 + jj;
+        float2 bp[O::NP > 0 ? O::NP : 1];
+        float b1;
+        load_columns<DP, R>(Bs, j, cg, bp, b1);
+#pragma unroll
+        for (int i = 0; i < O::RPT; ++i) {
+          const float xi = jj == 0 ? x[i].x : jj == 1 ? x[i].y : jj == 2 ? x[i].z : x[i].w;
+          const float2 xx = make_float2(xi, xi);
+#pragma unroll
+          for (int c = 0; c < O::NP; ++c) dq.p[i][c] = fma2(xx, bp[c], dq.p[i][c]);
+          if constexpr (O::N1 > 0) dq.s[i] = fmaf(xi, b1, dq.s[i]);
+        }
+      }
+    }
+  }
+  store_piece<DP, R, 16>(dQ + base, sin.t, q0 + rg, cg, T, D, vec_out != 0, dq);
+}
+
+// dQ for one tile of R queries: dQ = dS K with dS recomputed per key tile.  For when there is no room for dS, and for problems
+// small enough that this kernel runs beside the dK/dV kernel.
 template <int DP, int R>
 __global__ void __launch_bounds__(NT) sdpa_bwd_dq_f32_kernel(
     const float* __restrict__ Q, const float* __restrict__ K, const float* __restrict__ V,
@@ -614,7 +714,7 @@ int mca_sdpa_forward_f32_layout(const float* q, const float* k, const float* v, 
 template <int DP, int R>
 static int launch_bwd_tile(const float* q, const float* k, const float* v, const float* dy, const float* mask, int mode,
                            const int* flag, const float* rmax, const float* rsum, const float* delta, int B, int H, int T,
-                           int D, float* dq, float* dk, float* dv, int layout, cudaStream_t st) {
+                           int D, float* dq, float* dk, float* dv, float* ds, int64_t ds_floats, int layout, cudaStream_t st) {
   const McaStrides sin = mca_in_strides(layout, H, T, D), sout = mca_out_strides(layout, H, T, D);
   constexpr size_t smem = bwd_smem_bytes<DP, R>();
   static_assert(smem <= 227 * 1024, "one CTA per SM");
@@ -626,20 +726,34 @@ static int launch_bwd_tile(const float* q, const float* k, const float* v, const
   const int vec_out = (D % 4 == 0) && aligned16(dq) && aligned16(dk) && aligned16(dv);
   const float scale = 1.0f / sqrtf((float)D);
   dim3 grid(B * H, mca_ceil_div(T, R));
+  // dS passes through memory where there is room for it and the work, not the longest CTA, decides when the kernel ends: where
+  // SMs would be idle, the other dQ kernel runs on them beside the dK/dV kernel, and this one could not
+  // (the work per SM over the longest CTA's: 0.55, H = 9, T = 1088, D = 128: 406 -> 500 us; 0.8, B = 2, H = 7, T = 967,
+  // D = 96: 702 -> 547).
+  const bool causal = mode == MCA_MASK_CAUSAL || mode == MCA_MASK_TT;
+  const int64_t tiles = mca_ceil_div(T, R), steps = causal ? tiles * (tiles + 1) / 2 : tiles * tiles;
+  if (ds_floats < ds_tile<R>(B * H, 0, 0, T) || 3 * steps * B * H <= 2 * 148 * tiles) ds = nullptr;
   sdpa_bwd_dkdv_f32_kernel<DP, R><<<grid, NT, smem, st>>>(q, k, v, dy, mask, mode, flag, rmax, rsum, delta, H, T, D,
-                                                         scale, dk, dv, vec_ok, vec_out, sin, sout);
+                                                         scale, dk, dv, ds, vec_ok, vec_out, sin, sout);
   e = mca_launch_status();
   if (e) return e;
+  if (ds != nullptr) {
+    constexpr size_t smem_ds = dq_ds_smem_bytes<DP>();
+    static_assert(2 * (smem_ds + 1024) <= 228 * 1024, "two CTAs per SM");
+    static std::atomic<uint64_t> done_ds{0};
+    if ((e = mca_smem_once(done_ds, sdpa_bwd_dq_ds_f32_kernel<DP, R>, smem_ds))) return e;
+    return mca_launch_pdl(sdpa_bwd_dq_ds_f32_kernel<DP, R>, dim3(B * H, mca_ceil_div(T, SX)), dim3(NT), smem_ds, st, k, ds, mode, flag, H, T, D, dq, vec_ok, vec_out, sin);
+  }
   return mca_launch_pdl(sdpa_bwd_dq_f32_kernel<DP, R>, grid, dim3(NT), smem, st, q, k, v, dy, mask, mode, flag, rmax, rsum, delta, H,
                         T, D, scale, dq, vec_ok, vec_out, sin, sout);
 }
 template <int DP>
 static int launch_bwd(const float* q, const float* k, const float* v, const float* dy, const float* mask, int mode,
                       const int* flag, const float* rmax, const float* rsum, const float* delta, int B, int H, int T,
-                      int D, float* dq, float* dk, float* dv, int layout, cudaStream_t st) {
+                      int D, float* dq, float* dk, float* dv, float* ds, int64_t ds_floats, int layout, cudaStream_t st) {
   if (small_tiles(B, H, T, mode == MCA_MASK_CAUSAL || mode == MCA_MASK_TT))
-    return launch_bwd_tile<DP, 64>(q, k, v, dy, mask, mode, flag, rmax, rsum, delta, B, H, T, D, dq, dk, dv, layout, st);
-  return launch_bwd_tile<DP, 128>(q, k, v, dy, mask, mode, flag, rmax, rsum, delta, B, H, T, D, dq, dk, dv, layout, st);
+    return launch_bwd_tile<DP, 64>(q, k, v, dy, mask, mode, flag, rmax, rsum, delta, B, H, T, D, dq, dk, dv, ds, ds_floats, layout, st);
+  return launch_bwd_tile<DP, 128>(q, k, v, dy, mask, mode, flag, rmax, rsum, delta, B, H, T, D, dq, dk, dv, ds, ds_floats, layout, st);
 }
 
 int mca_sdpa_backward_f32(const float* q, const float* k, const float* v, const float* dy, const float* y_saved,
@@ -654,6 +768,20 @@ int mca_sdpa_backward_f32_layout(const float* q, const float* k, const float* v,
                                  const float* mask, int mask_mode, const int* causal_flag, const float* row_max,
                                  const float* row_sum, float* delta_scratch, int B, int H, int T, int D, float* dq,
                                  float* dk, float* dv, int layout, void* stream) {
+  return mca_sdpa_backward_f32_ws(q, k, v, dy, y_saved, mask, mask_mode, causal_flag, row_max, row_sum, delta_scratch, B, H, T, D, dq, dk,
+                                  dv, nullptr, 0, layout, stream);
+}
+
+int64_t mca_sdpa_backward_f32_ws_bytes(int B, int H, int T) {
+  // either tile size (small_tiles): whole blocks of 128 in both directions hold the one and the other
+  const int64_t blocks = mca_ceil_div(T, 128);
+  return (int64_t)B * H * blocks * blocks * (128 * 128 * 4);
+}
+
+int mca_sdpa_backward_f32_ws(const float* q, const float* k, const float* v, const float* dy, const float* y_saved, const float* mask,
+                             int mask_mode, const int* causal_flag, const float* row_max, const float* row_sum, float* delta_scratch,
+                             int B, int H, int T, int D, float* dq, float* dk, float* dv, float* ds, int64_t ds_floats, int layout,
+                             void* stream) {
   if (layout != MCA_LAYOUT_BHTD && layout != MCA_LAYOUT_PACKED) return ERROR_PARAM_OUT_OF_RANGE;
   if (!q || !k || !v || !dy || !y_saved || !row_max || !row_sum || !delta_scratch || !dq || !dk || !dv)
     return ERROR_PARAM_NULL;
@@ -666,13 +794,13 @@ int mca_sdpa_backward_f32_layout(const float* q, const float* k, const float* v,
   int e = mca_launch_status();
   if (e) return e;
   switch (pick_dp(D)) {
-    case 16: return launch_bwd<16>(q, k, v, dy, mask, mask_mode, causal_flag, row_max, row_sum, delta_scratch, B, H, T, D, dq, dk, dv, layout, st);
-    case 32: return launch_bwd<32>(q, k, v, dy, mask, mask_mode, causal_flag, row_max, row_sum, delta_scratch, B, H, T, D, dq, dk, dv, layout, st);
-    case 48: return launch_bwd<48>(q, k, v, dy, mask, mask_mode, causal_flag, row_max, row_sum, delta_scratch, B, H, T, D, dq, dk, dv, layout, st);
-    case 64: return launch_bwd<64>(q, k, v, dy, mask, mask_mode, causal_flag, row_max, row_sum, delta_scratch, B, H, T, D, dq, dk, dv, layout, st);
-    case 80: return launch_bwd<80>(q, k, v, dy, mask, mask_mode, causal_flag, row_max, row_sum, delta_scratch, B, H, T, D, dq, dk, dv, layout, st);
-    case 96: return launch_bwd<96>(q, k, v, dy, mask, mask_mode, causal_flag, row_max, row_sum, delta_scratch, B, H, T, D, dq, dk, dv, layout, st);
-    case 128: return launch_bwd<128>(q, k, v, dy, mask, mask_mode, causal_flag, row_max, row_sum, delta_scratch, B, H, T, D, dq, dk, dv, layout, st);
+    case 16: return launch_bwd<16>(q, k, v, dy, mask, mask_mode, causal_flag, row_max, row_sum, delta_scratch, B, H, T, D, dq, dk, dv, ds, ds_floats, layout, st);
+    case 32: return launch_bwd<32>(q, k, v, dy, mask, mask_mode, causal_flag, row_max, row_sum, delta_scratch, B, H, T, D, dq, dk, dv, ds, ds_floats, layout, st);
+    case 48: return launch_bwd<48>(q, k, v, dy, mask, mask_mode, causal_flag, row_max, row_sum, delta_scratch, B, H, T, D, dq, dk, dv, ds, ds_floats, layout, st);
+    case 64: return launch_bwd<64>(q, k, v, dy, mask, mask_mode, causal_flag, row_max, row_sum, delta_scratch, B, H, T, D, dq, dk, dv, ds, ds_floats, layout, st);
+    case 80: return launch_bwd<80>(q, k, v, dy, mask, mask_mode, causal_flag, row_max, row_sum, delta_scratch, B, H, T, D, dq, dk, dv, ds, ds_floats, layout, st);
+    case 96: return launch_bwd<96>(q, k, v, dy, mask, mask_mode, causal_flag, row_max, row_sum, delta_scratch, B, H, T, D, dq, dk, dv, ds, ds_floats, layout, st);
+    case 128: return launch_bwd<128>(q, k, v, dy, mask, mask_mode, causal_flag, row_max, row_sum, delta_scratch, B, H, T, D, dq, dk, dv, ds, ds_floats, layout, st);
   }
   return ERROR_ATTN_UNSUPPORTED_SHAPE;
 }

@@ -11,6 +11,14 @@ int mca_mask_bits_view(const uint32_t* bits, const uint32_t* bits_t, int mask_mo
 struct McaClassifyJob;
 int mca_classify_causal_mask_ws(const McaClassifyJob* job, void* stream);
 
+// Internal: mca_sdpa_backward_f32_layout with room for dS between its two kernels (ds_floats floats, 16-byte aligned; fewer than
+// mca_sdpa_backward_f32_ws_bytes asks for: dS is formed twice).
+int64_t mca_sdpa_backward_f32_ws_bytes(int B, int H, int T);
+int mca_sdpa_backward_f32_ws(const float* q, const float* k, const float* v, const float* dy, const float* y_saved, const float* mask,
+                             int mask_mode, const int* causal_flag, const float* row_max, const float* row_sum, float* delta_scratch,
+                             int B, int H, int T, int D, float* dq, float* dk, float* dv, float* ds, int64_t ds_floats, int layout,
+                             void* stream);
+
 // Internal: the two halves of mca_sdpa_forward_f32_tc_masked -- the pre-pass that splits q, k, v (and classifies the caller's
 // (T,T) mask in the same launch when `cls` is given), and the kernel, which may then be chosen on the class.
 int mca_split_forward_prepass(const float* q, const float* k, const float* v, int B, int H, int T, int D, void* workspace,
