@@ -272,7 +272,7 @@ MCA_API int mca_tc_narrow_len(int len);
 /* fp32 SDPA forward at fp32 accuracy on the tensor cores.  Same math as attn.cu:518-602 with a causal or absent mask.
  * q, k, v, y: fp32, (B,H,T,D) or the packed layout; D in {16, 32, 64, 128} (128: one query tile per CTA and
  * single-stage K and V, since a row's two halves are 512 bytes; forward only, the exact fp32 backward follows it from
- * row_max / row_sum).  A pre-pass scales each tensor by a power of two
+ * row_max / row_sum).  A pre-pass scales each (batch, head) of each tensor by a power of two
  * and writes every element as two fp16 halves hi = fp16(x), lo = fp16(x - hi) into `workspace`
  * (mca_sdpa_forward_f32_tc_workspace_bytes_d(B,H,T,D) bytes, 16-byte aligned); every contraction is then three
  * tcgen05 kind::f16 products hi.hi + hi.lo + lo.hi accumulated in fp32, P split the same way.  Within 1e-5 of the output

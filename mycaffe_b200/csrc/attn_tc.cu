@@ -35,7 +35,7 @@
 //   MODE_BF16   bf16 tensors, one kind::f16 product per contraction.
 //   MODE_TF32   fp32 tensors read as tf32 (kind::tf32), 64-wide heads.
 //   MODE_SPLIT  fp32 callers at fp32 accuracy: every operand x is carried as two fp16 values hi = fp16(x),
-//               lo = fp16(x - hi) (22 mantissa bits together; a pre-pass writes rows [hi | lo] after scaling each
+//               lo = fp16(x - hi) (22 mantissa bits together; a pre-pass writes rows [hi | lo] after scaling each head of each
 //               tensor by a power of two so that neither half leaves the fp16 range), and every contraction is three
 //               kind::f16 products hi.hi + hi.lo + lo.hi accumulated in the same fp32 TMEM tile.  P is split the
 //               same way by the softmax warps.  Measured against the fp64 oracle this is within 1e-5 of the output

@@ -20,7 +20,7 @@
 // bounded as in the forward kernel.
 //
 // SPLIT = true is the variant for fp32 callers: every operand is carried as two fp16 halves (rows [hi | lo] written by
-// the pre-pass in split_prepass.cuh, each tensor scaled by a power of two), every product is the three kind::f16
+// the pre-pass in split_prepass.cuh, each head of each tensor scaled by a power of two), every product is the three kind::f16
 // products hi.hi + hi.lo + lo.hi into one fp32 TMEM tile, P^T / dS / dS^T are split the same way by the element-wise
 // warps, and the gradients are written in fp32.  Head sizes up to 64: a split tile is as large as a 128-wide bf16 one.
 #include <type_traits>
