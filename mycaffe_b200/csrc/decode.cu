@@ -560,14 +560,18 @@ int mca_decode_plan(int B, int n_heads, int n_kv_heads, int head_size, int max_l
   if (groups * ((max_len + 127) / 128) <= 4 * 296) {
     // Few CTAs (one sequence, or a handful): a partly filled last wave costs as much as a full one, so the split
     // count is chosen by whole waves over the 296 resident CTAs -- time ~ waves x (set-up, about 64 keys' worth, + keys
-    // per split) -- instead of by a fixed length.  One sequence of 2339 keys and 32 heads: 9 splits of 260 keys in one
+    // per split) + combining -- instead of by a fixed length.  One sequence of 2339 keys and 32 heads: 9 splits of 260 keys in one
     // wave, where 128-key splits give 608 CTAs, i.e. two waves and sixteen stragglers.
+    // More than one split also costs the partial results' way through memory and the combine pass, some three microseconds: a
+    // fixed time, so as many keys as that reads of rows of this width (7 sequences of 382 keys, 16 heads of 48: 19.2 us with two
+    // splits, 17.6 with one; 15 of 293 keys, 8 heads of 128, the other way round: 19.6 and 19.9).
+    const int64_t combine_keys = 12288 / std::max(1, head_size);
     int64_t best_cost = INT64_MAX;
     int best_n = 1;
     for (int n = 1; n <= std::max(1, max_len / 128); ++n) {   // splits of at least 128 keys; up to 255 keys: one split, no scratch
       const int64_t len = ((max_len + n - 1) / n + 15) / 16 * 16;
       const int64_t waves = (groups * n + 295) / 296;
-      const int64_t cost = waves * (64 + len);
+      const int64_t cost = waves * (64 + len) + (n > 1 ? combine_keys : 0);
       if (cost < best_cost) { best_cost = cost; best_n = n; }
     }
     sl = (((int64_t)max_len + best_n - 1) / best_n + 15) / 16 * 16;
