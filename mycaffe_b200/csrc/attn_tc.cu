@@ -471,10 +471,10 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     const int qrow0 = q0 + x * BLK;
     float m_used[2] = {-INFINITY, -INFINITY};
     float l[2] = {0.f, 0.f};                            // this thread's part of the row sums
-    // split mode: the pre-pass scaled q and k by powers of two; dividing them out of the logit scale is exact
+    // split mode: the pre-pass scaled q and k by powers of two; the logit scale takes them out
     float4 sc = make_float4(1.f, 1.f, 1.f, 1.f);
     if constexpr (SPLIT) sc = mca_ld_f4(reinterpret_cast<const float*>(p.split_scale + bh));
-    const float scale_log2 = SPLIT ? p.scale_log2 * (1.0f / (sc.x * sc.y)) : p.scale_log2;
+    const float scale_log2 = SPLIT ? split::logit_scale(p.scale_log2, sc) : p.scale_log2;
     for (int j = 0; j < n && ok; ++j) {
       TC_TRACE(x, j, 0);
       ok = __all_sync(0xffffffffu, mbar_wait_hot(bar(BAR_S_FULL + x), (uint32_t)(j & 1), p.status, 30 + x, j));
@@ -666,8 +666,12 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         const int row = (warp & 3) * 32 + lane;
         const int qi = qrow0 + row;
         const float lsum = red_l[row];
-        // split mode: the pre-pass scaled v by a power of two; dividing it out here is exact
-        const float inv = SPLIT ? (1.0f / mca_ld_f4(reinterpret_cast<const float*>(p.split_scale + bh)).z) / lsum : 1.0f / lsum;
+        const float inv = 1.0f / lsum;
+        // split mode: the pre-pass scaled v by a power of two, taken out in a product of its own (next to lsum it could leave the
+        // normal numbers)
+        float inv_v = 1.0f;
+        if constexpr (SPLIT) inv_v = 1.0f / mca_ld_f4(reinterpret_cast<const float*>(p.split_scale + bh)).z;
+        auto f32_out = [&](uint32_t w) { return SPLIT ? __uint_as_float(w) * inv * inv_v : __uint_as_float(w) * inv; };
         const uint32_t t_o32 = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(QT * BLK + x * BLK + half * OC);
         if constexpr (F32_OUT && QT == 2) {
           // fp32 output of the two-tile shape: each thread stores its own row's pieces.  (Staged like the other
@@ -683,8 +687,7 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             if (qi < T) {
 #pragma unroll
               for (int i = 0; i < CHD; i += 4) {
-                const float4 w = make_float4(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv,
-                                             __uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
+                const float4 w = make_float4(f32_out(o[i]), f32_out(o[i + 1]), f32_out(o[i + 2]), f32_out(o[i + 3]));
                 *reinterpret_cast<float4*>(yrow_f + c * CHD + i) = w;
                 if constexpr (SPLIT) {
                   if (p.y_copy) *reinterpret_cast<float4*>(p.y_copy + ((int64_t)bh * T + qi) * HD + half * OC + c * CHD + i) = w;
@@ -715,10 +718,10 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           for (int i = 0; i < CH; i += EPP) {
             uint4 w;
             if constexpr (F32_OUT) {
-              w.x = __float_as_uint(__uint_as_float(o[i + 0]) * inv);
-              w.y = __float_as_uint(__uint_as_float(o[i + 1]) * inv);
-              w.z = __float_as_uint(__uint_as_float(o[i + 2]) * inv);
-              w.w = __float_as_uint(__uint_as_float(o[i + 3]) * inv);
+              w.x = __float_as_uint(f32_out(o[i + 0]));
+              w.y = __float_as_uint(f32_out(o[i + 1]));
+              w.z = __float_as_uint(f32_out(o[i + 2]));
+              w.w = __float_as_uint(f32_out(o[i + 3]));
             } else {
               w.x = pack_bf16(__uint_as_float(o[i + 0]) * inv, __uint_as_float(o[i + 1]) * inv);
               w.y = pack_bf16(__uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);

@@ -80,12 +80,14 @@ __device__ __forceinline__ void split_pack(float v0, float v1, uint32_t& hi, uin
 }
 // Split mode keeps dS 2^-19 smaller than dP' = dY' V'^T (both operands scaled to below 2^13, so |dP'| < 2^32 at 64-wide
 // heads) and P^T 2^10 larger than P <= 1: both then sit in the middle of the fp16 range.
-constexpr float DS_SHIFT = 1.0f / 524288.0f, DS_UNSHIFT = 524288.0f, PT_SHIFT = 1024.0f, PT_UNSHIFT = 1.0f / 1024.0f;
+using split::DS_SHIFT, split::DS_SHIFT_LOG2;
+constexpr float PT_SHIFT = 1024.0f;
+constexpr int PT_SHIFT_LOG2 = 10;
 
 struct BwdParams {
   const float4* scales;   // split mode: the pre-pass's scales (q, k, v, dY) of each (batch, head)
   const float* lse;    // (BH, T) log2-domain log-sum-exp of the scaled logits, from the forward kernel
-  const float* delta;  // (BH, T) rowsum(dY o Y)
+  const float* delta;  // (BH, T) rowsum(dY o Y); split mode: times the head's scale of dY and DS_SHIFT
   void* out0;          // dq kernel: dQ;  dkdv kernel: dK
   void* out1;          // dkdv kernel: dV
   int* status;
@@ -116,10 +118,11 @@ template <int EW_WARPS> __device__ __forceinline__ void ew_bar_sync() { asm vola
 template <int PR> __device__ __forceinline__ uint4* staged_piece(uint8_t* tile, int row, int piece) {
   return reinterpret_cast<uint4*>(tile) + row * PR + (piece ^ (row & (PR - 1)));
 }
-// this thread's OC columns of its row, scaled, as 16-byte pieces of bf16 or fp32
+// this thread's OC columns of its row, as 16-byte pieces of bf16, or of fp32 times scale x (the split operands' power of two)
 template <int PR, int OC, bool F32>
-__device__ __forceinline__ void stage_columns(uint8_t* tile, int row, int qtr, uint32_t t_addr, float mul) {
+__device__ __forceinline__ void stage_columns(uint8_t* tile, int row, int qtr, uint32_t t_addr, float scale, float2 pow2) {
   constexpr int CH = OC < 16 ? OC : 16;
+  const float first = scale * pow2.x;
 #pragma unroll
   for (int c = 0; c < OC / CH; ++c) {
     uint32_t o[CH];
@@ -128,19 +131,15 @@ __device__ __forceinline__ void stage_columns(uint8_t* tile, int row, int qtr, u
     else tmem_ld4(t_addr, o);
     tmem_wait_ld();
     if constexpr (F32) {
+      auto v = [&](int i) { return __float_as_uint(__uint_as_float(o[i]) * first * pow2.y); };
 #pragma unroll
       for (int i = 0; i < CH; i += 4)
-        *staged_piece<PR>(tile, row, (qtr * OC + c * CH + i) / 4) =
-            make_uint4(__float_as_uint(__uint_as_float(o[i]) * mul), __float_as_uint(__uint_as_float(o[i + 1]) * mul),
-                       __float_as_uint(__uint_as_float(o[i + 2]) * mul), __float_as_uint(__uint_as_float(o[i + 3]) * mul));
+        *staged_piece<PR>(tile, row, (qtr * OC + c * CH + i) / 4) = make_uint4(v(i), v(i + 1), v(i + 2), v(i + 3));
     } else {
+      auto v = [&](int i) { return pack_bf16(__uint_as_float(o[i]), __uint_as_float(o[i + 1])); };
 #pragma unroll
       for (int i = 0; i < CH; i += 8)
-        *staged_piece<PR>(tile, row, (qtr * OC + c * CH + i) / 8) =
-            make_uint4(pack_bf16(__uint_as_float(o[i + 0]) * mul, __uint_as_float(o[i + 1]) * mul),
-                       pack_bf16(__uint_as_float(o[i + 2]) * mul, __uint_as_float(o[i + 3]) * mul),
-                       pack_bf16(__uint_as_float(o[i + 4]) * mul, __uint_as_float(o[i + 5]) * mul),
-                       pack_bf16(__uint_as_float(o[i + 6]) * mul, __uint_as_float(o[i + 7]) * mul));
+        *staged_piece<PR>(tile, row, (qtr * OC + c * CH + i) / 8) = make_uint4(v(i), v(i + 2), v(i + 4), v(i + 6));
     }
   }
 }
@@ -369,9 +368,9 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     const float delta = row_ok ? p.delta[(int64_t)bh * T + qi] : 0.f;
     float4 sc = make_float4(1.f, 1.f, 1.f, 1.f);   // powers of two: every product and quotient of them is exact
     if constexpr (SPLIT) sc = mca_ld_f4(reinterpret_cast<const float*>(p.scales + bh));
-    const float sl2 = SPLIT ? p.scale_log2 * (1.0f / (sc.x * sc.y)) : p.scale_log2;
+    const float sl2 = SPLIT ? split::logit_scale(p.scale_log2, sc) : p.scale_log2;
     const float dmul = SPLIT ? DS_SHIFT : p.scale;
-    const float dsub = SPLIT ? delta * (sc.w * DS_SHIFT) * sc.z : delta * p.scale;
+    const float dsub = SPLIT ? delta * sc.z : delta * p.scale;
     for (int j = 0; j < n && ok; ++j) {
       ok = __all_sync(0xffffffffu, mbar_wait(bar(DQ_SDP_FULL), (uint32_t)(j & 1), p.status, 130, j));
       if (!ok) break;
@@ -444,8 +443,8 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     const bool fin = ok && n > 0;
     if (fin) {
       tc_fence_after();
-      const float mul = SPLIT ? p.scale * DS_UNSHIFT * (1.0f / (sc.z * sc.y)) * (1.0f / sc.w) : 1.0f;
-      stage_columns<PR, OC, SPLIT>(tile, row, qtr, t_row + C_DQ + qtr * OC, mul);
+      const float2 mul = split::pow2_factors(-DS_SHIFT_LOG2 - split::scale_exp(sc.y) - split::scale_exp(sc.z) - split::scale_exp(sc.w));
+      stage_columns<PR, OC, SPLIT>(tile, row, qtr, t_row + C_DQ + qtr * OC, p.scale, mul);
     }
     ew_bar_sync<EW_WARPS>();
     if (fin)
@@ -709,9 +708,9 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     // split mode: S^T and dP^T carry the pre-pass's scales; dS^T is kept in the units of dP' x 2^-19 and P^T 2^10 larger
     float4 sc = make_float4(1.f, 1.f, 1.f, 1.f);
     if constexpr (SPLIT) sc = mca_ld_f4(reinterpret_cast<const float*>(p.scales + bh));
-    const float sl2 = SPLIT ? p.scale_log2 * (1.0f / (sc.x * sc.y)) : p.scale_log2;
+    const float sl2 = SPLIT ? split::logit_scale(p.scale_log2, sc) : p.scale_log2;
     const float dmul = SPLIT ? DS_SHIFT : p.scale;
-    const float del_mul = SPLIT ? (sc.w * DS_SHIFT) * sc.z : p.scale;
+    const float del_mul = SPLIT ? sc.z : p.scale;
     auto fetch = [&](int it) -> float {
       const int qi = (i_begin + it) * BN + (tid & (BN - 1));
       if (tid >= 2 * BN || it >= n || qi >= T) return tid < BN ? -INFINITY : 0.f;
@@ -846,15 +845,15 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     uint8_t* tile_v = smem_gen + PL::OFF_RES1;
     if (ok && n > 0) {   // dV beside the last dK product
       tc_fence_after();
-      const float mul_v = SPLIT ? PT_UNSHIFT * (1.0f / sc.w) : 1.0f;
-      stage_columns<PR, OC, SPLIT>(tile_v, row, qtr, t_row + C_DV + qtr * OC, mul_v);
+      const float2 mul_v = split::pow2_factors(-PT_SHIFT_LOG2 - split::scale_exp(sc.w));
+      stage_columns<PR, OC, SPLIT>(tile_v, row, qtr, t_row + C_DV + qtr * OC, 1.0f, mul_v);
       ok = __all_sync(0xffffffffu, mbar_wait(bar(KV_ACC_DONE), 0, p.status, 232, n));
     }
     const bool fin = ok && n > 0;
     if (fin) {
       tc_fence_after();
-      const float mul_k = SPLIT ? p.scale * DS_UNSHIFT * (1.0f / (sc.z * sc.x)) * (1.0f / sc.w) : 1.0f;
-      stage_columns<PR, OC, SPLIT>(tile_k, row, qtr, t_row + C_DK + qtr * OC, mul_k);
+      const float2 mul_k = split::pow2_factors(-DS_SHIFT_LOG2 - split::scale_exp(sc.x) - split::scale_exp(sc.z) - split::scale_exp(sc.w));
+      stage_columns<PR, OC, SPLIT>(tile_k, row, qtr, t_row + C_DK + qtr * OC, p.scale, mul_k);
     }
     ew_bar_sync<EW_WARPS>();
     if (fin) {

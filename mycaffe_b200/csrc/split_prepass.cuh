@@ -73,20 +73,37 @@ __device__ __forceinline__ float4 ld_f4_hint(const float* ptr, uint64_t pol) {
 __device__ __forceinline__ float amax4(const float4& v) { return fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))); }
 
 // The power of two that brings max |x| into [2^12, 2^13): the largest fp16 is 65504 and the low half of an element
-// is about 2^-11 of it, so both halves of everything within 2^-14 of the maximum are normal fp16 numbers.  It is bounded so
-// that the products of three scales the kernels form stay finite (q, k, v: 2^40, dY: 2^100): heads whose largest
-// magnitude is below 2^-40 (2^-100) lose precision gradually, as they did next to any larger head.
-__device__ __forceinline__ float pow2_scale(float a, int slot) {
+// is about 2^-11 of it, so both halves of everything within 2^-14 of the maximum are normal fp16 numbers.  It lies in
+// [2^-115, 2^126], so that it and its reciprocal are normal (a subnormal maximum stays below 2^12; its halves carry every bit it
+// has, the split dS of such a V fewer).  Products of several scales are not: the kernels multiply by them through pow2_factors, or one
+// after the other where every partial product is bounded, as said there.
+__device__ __forceinline__ float pow2_scale(float a) {
   if (!(a > 0.f) || !(a < 3.0e38f)) return 1.0f;
   int e;
   frexpf(a, &e);                    // a = f * 2^e, f in [0.5, 1)
-  return ldexpf(1.0f, min(13 - e, slot == TENSOR_DY ? 100 : 40));
+  return ldexpf(1.0f, min(13 - e, 126));
 }
+__device__ __forceinline__ int scale_exp(float scale) { return (__float_as_int(scale) >> 23) - 127; }
+// 2^e as two factors, applied one after the other: exact wherever the result is a normal number, without an infinity or a
+// zero on the way (beyond 2^254 and 2^-252 the result is one anyway).
+__device__ __forceinline__ float2 pow2_factors(int e) {
+  const int h = e / 2;
+  return make_float2(ldexpf(1.0f, max(-126, min(127, h))), ldexpf(1.0f, max(-126, min(127, e - h))));
+}
+// Factor of the logits S' = Q'K'^T back to their own units (times `scale`).  |S'| < 2^33: below 2^-100 every logit is zero to
+// the exponential anyway, and the bound keeps the masked logit (a constant over this factor) finite.
+__device__ __forceinline__ float logit_scale(float scale, const float4& sc) {
+  return ldexpf(scale, max(-100, min(120, -(scale_exp(sc.x) + scale_exp(sc.y)))));
+}
+// dY' V'^T products (below 2^32) are taken down by this before dS is split, and delta is left by the pre-pass in the units of dY'
+// times this: delta x (the scale of v) is then below 2^13, whatever the magnitudes of dY and v.
+constexpr float DS_SHIFT = 1.0f / 524288.0f;
+constexpr int DS_SHIFT_LOG2 = -19;
 
 constexpr int THREADS = 256, KEEP = 4;   // eight-element pieces a thread keeps in registers
 
-// with ydot / delta given: also delta[row] = sum_c x[row][c] * ydot[row][c] (ydot contiguous rows), the softmax backward's
-// row term, from the elements this kernel holds anyway.
+// with ydot / delta given: also delta[row] = sum_c x[row][c] * ydot[row][c] (ydot contiguous rows) x scale x DS_SHIFT, the
+// softmax backward's row term in the units the backward kernels need, from the elements this kernel holds anyway.
 // grid: (CTAs of a cluster, BH, [the CTAs that classify the mask +] tensors); the classification comes first, so that its
 // answer is on the host before the tensors are done
 template <int HD>
@@ -150,7 +167,7 @@ __global__ void __launch_bounds__(THREADS) split_kernel(const Job job, const Mca
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // its peers may still be reading this CTA's word
   }
   const int slot = job.slot[which];
-  const float sc = pow2_scale(m, slot);
+  const float sc = pow2_scale(m), sc_delta = sc * DS_SHIFT;
   if (blockIdx.x == 0 && tid == 0) scale[bh * 4 + slot] = sc;
   constexpr int RH = row_halves(HD);
   const int64_t out_row0 = (int64_t)bh * T + row0;
@@ -162,8 +179,10 @@ __global__ void __launch_bounds__(THREADS) split_kernel(const Job job, const Mca
       if (in) {
         const float* yd = ydot + (out_row0 + row) * HD + c8;
         const float4 y0 = mca_ld_f4(yd), y1 = mca_ld_f4(yd + 4);
-        acc = fmaf(v0.x, y0.x, fmaf(v0.y, y0.y, fmaf(v0.z, y0.z, v0.w * y0.w)));
-        acc += fmaf(v1.x, y1.x, fmaf(v1.y, y1.y, fmaf(v1.z, y1.z, v1.w * y1.w)));
+        const float d[8] = {v0.x * sc_delta, v0.y * sc_delta, v0.z * sc_delta, v0.w * sc_delta,
+                            v1.x * sc_delta, v1.y * sc_delta, v1.z * sc_delta, v1.w * sc_delta};
+        acc = fmaf(d[0], y0.x, fmaf(d[1], y0.y, fmaf(d[2], y0.z, d[3] * y0.w)));
+        acc += fmaf(d[4], y1.x, fmaf(d[5], y1.y, fmaf(d[6], y1.z, d[7] * y1.w)));
       }
 #pragma unroll
       for (int o = V8 / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
