@@ -134,7 +134,7 @@ struct Kernel {
   float* stage = nullptr;  // grow-only fp32 staging buffer for float <-> bf16 transfers
   size_t stage_count = 0;
   bool synced = false;     // the call being dispatched has already synchronised the stream behind its last launch
-  bool fail_words = false; // this device's kernels raise the process's failure words (see g_fail_words)
+  bool fail_words = false; // this device's kernels raise its failure words (see g_fail)
   int* h_answer = nullptr; // pinned words for small device answers: a mask's class in [0], written by the kernel that finds it
   int* answer_words() {
     if (h_answer == nullptr) {
@@ -174,39 +174,37 @@ struct Kernel {
 Kernel* g_kernels[kMaxKernels];
 std::mutex g_table_lock;
 
-// McaFailWord array in pinned host memory, raised by the kernels of every device: behind a stream synchronisation one
-// host load says whether any device status word is worth reading.  A raised MCA_FAIL_TC word stays raised (it stands for
-// every attention handle's own status words, and a bounded wait giving up is no ordinary event); the other two families
-// have one status array per device and their word is lowered before that array is read.
-int* g_fail_words = nullptr;
-uint64_t g_fail_words_devices = 0;   // devices whose kernels know the address
+// The failure words (fail_words.h).  A raised MCA_FAIL_TC word stays raised (it stands for every attention handle's own status
+// words, and a bounded wait giving up is no ordinary event); the other two families have one status array per device and
+// their word is lowered before that array is read.
+McaFailTable g_fail;
+uint64_t g_fail_armed = 0;   // devices whose kernels know their row
 
 bool arm_fail_words(int dev) {   // under g_table_lock, with dev current
-  if (dev >= 64) return false;
-  if (g_fail_words == nullptr) {
-    if (cudaHostAlloc((void**)&g_fail_words, MCA_FAIL_WORDS * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+  if (dev >= MCA_FAIL_DEVICES) return false;
+  if (g_fail.words == nullptr) {
+    if (cudaHostAlloc((void**)&g_fail.words, McaFailTable::SIZE * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
       cudaGetLastError();
-      g_fail_words = nullptr;
+      g_fail.words = nullptr;
       return false;
     }
-    for (int i = 0; i < MCA_FAIL_WORDS; ++i) g_fail_words[i] = 0;
+    for (int i = 0; i < McaFailTable::SIZE; ++i) g_fail.words[i] = 0;
   }
-  if (!(g_fail_words_devices >> dev & 1)) {
-    if (mca_set_fail_words_fwd(g_fail_words) || mca_set_fail_words_bwd(g_fail_words) || mca_set_fail_words_probe(g_fail_words) ||
-        mca_set_fail_words_decode(g_fail_words) || mca_set_fail_words_proj(g_fail_words)) {
+  if (!(g_fail_armed >> dev & 1)) {
+    int* row = g_fail.row(dev);
+    if (mca_set_fail_words_fwd(row) || mca_set_fail_words_bwd(row) || mca_set_fail_words_probe(row) || mca_set_fail_words_decode(row) ||
+        mca_set_fail_words_proj(row)) {
       cudaGetLastError();
       return false;
     }
-    g_fail_words_devices |= 1ull << dev;
+    g_fail_armed |= 1ull << dev;
   }
   return true;
 }
 
-bool may_have_failed(const Kernel* k, McaFailWord family) {
-  return !k->fail_words || *reinterpret_cast<volatile int*>(g_fail_words + family) != 0;
-}
+bool may_have_failed(const Kernel* k, McaFailWord family) { return !k->fail_words || g_fail.raised(k->device, family); }
 void lower_fail_word(const Kernel* k, McaFailWord family) {
-  if (k->fail_words) *reinterpret_cast<volatile int*>(g_fail_words + family) = 0;
+  if (k->fail_words) g_fail.lower(k->device, family);
 }
 
 // The one synchronisation of a synchronous call.

@@ -6,6 +6,8 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include "fail_words.h"
+
 // Error codes of the reference's native layer that this path can return
 // (CudaDnnDLL/Cuda Files/util.h:128-146,198-211).  CUDA runtime codes pass through unchanged.
 constexpr int ERROR_BASE = 90000;
@@ -87,13 +89,6 @@ static inline int mca_launch_status() {
 }
 
 __host__ __device__ static inline int mca_ceil_div(int a, int b) { return (a + b - 1) / b; }
-
-// Failure words in pinned host memory (one array per process, visible to every device): a kernel that writes a failure
-// into its device status words also raises the word of its family here, so that a synchronous call learns from a plain
-// host load behind its one stream synchronisation that nothing failed.  (Copying the status words back after every call
-// cost a 3 us transfer and its launch on each.)  Each family's device code holds the array's address in a symbol of its
-// own translation unit, set when a kernel index is initialised; null (raw callers) means no word is raised.
-enum McaFailWord : int { MCA_FAIL_TC = 0, MCA_FAIL_DECODE = 1, MCA_FAIL_PROJ = 2, MCA_FAIL_WORDS = 4 };
 
 // Programmatic dependent launch.  A kernel launched with mca_launch_pdl may start while the
 // previous kernel of the stream is still running (once every CTA of that kernel has executed

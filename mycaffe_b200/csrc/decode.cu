@@ -45,7 +45,7 @@ template <typename CT, int HS> struct Epl {
 // Status words of the decode kernels: [0] number of sequences whose position was outside [0, max_len) since the
 // last read, [1] the first such sequence, [2] its position.  Such a sequence is not attended and its output is zero.
 __device__ int g_decode_status[4];
-__device__ int* g_fail_words;   // the process's failure words (McaFailWord), or null
+__device__ int* g_fail_words;   // this device's failure words (McaFailWord), or null
 
 struct DecodeParams {
   const float* q;        // (B, n_heads*HS): projection of the new token (before RoPE when fr != null)

@@ -26,7 +26,7 @@ int mca_split_forward_prepass(const float* q, const float* k, const float* v, in
 int mca_split_forward_main(int causal, int B, int H, int T, int D, float* y, float* row_max, float* row_sum, float* y_copy, float* lse,
                            void* workspace, int* status, int layout, const uint32_t* mask_bits, int mask_mode, void* stream);
 
-// Internal: hand the current device's kernels the address of the process's failure words (McaFailWord).
+// Internal: hand the current device's kernels the address of their row of failure words (McaFailWord).
 int mca_set_fail_words_fwd(int* words);
 int mca_set_fail_words_bwd(int* words);
 int mca_set_fail_words_probe(int* words);

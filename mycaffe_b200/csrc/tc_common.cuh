@@ -48,7 +48,7 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
   return t;
 }
 
-// Address of the process's failure words (see McaFailWord); one copy per translation unit that includes this header.
+// Address of this device's failure words (see McaFailWord); one copy per translation unit that includes this header.
 // MCA_TU_FAIL_FAMILY: which of the words this translation unit's kernels raise.
 #ifndef MCA_TU_FAIL_FAMILY
 #define MCA_TU_FAIL_FAMILY MCA_FAIL_TC
