@@ -40,8 +40,7 @@ struct AttnHandle {
   float *row_max = nullptr, *row_sum = nullptr, *y_copy = nullptr, *delta = nullptr, *lse = nullptr;
   void* split_ws = nullptr;    // fp16 halves of q, k, v for the split-operand tensor-core forward of fp32 handles
   int64_t split_ws_bytes = 0;
-  float* ds_ws = nullptr;      // dS between the two kernels of the exact fp32 backward (training handles that use it)
-  int64_t ds_floats = 0;
+  int64_t ds_floats = 0;       // room the exact fp32 backward of this handle asks of its kernel index (Kernel::ds_ws)
   float* mask_ws = nullptr;    // fp32 copies for a bf16 handle that is given a (T,T) or batch mask (allocated on first use)
   size_t mask_ws_floats = 0;
   uint32_t *mask_bits = nullptr, *mask_bits_t = nullptr;   // keep-bits of a (T,T) or batch mask for the tensor-core kernels
@@ -65,9 +64,9 @@ struct AttnHandle {
   bool status_pending = false;  // a tensor-core launch was made in asynchronous mode and its status words are unread
   void release() {
     cudaFree(row_max); cudaFree(row_sum); cudaFree(y_copy); cudaFree(delta); cudaFree(lse); cudaFree(causal_flag);
-    cudaFree(split_ws); cudaFree(ds_ws); cudaFree(mask_ws); cudaFree(mask_bits); cudaFree(mask_bits_t);
+    cudaFree(split_ws); cudaFree(mask_ws); cudaFree(mask_bits); cudaFree(mask_bits_t);
     split_ws = nullptr; split_ws_bytes = 0;
-    ds_ws = nullptr; ds_floats = 0;
+    ds_floats = 0;
     mask_ws = nullptr; mask_ws_floats = 0;
     mask_bits = mask_bits_t = nullptr; mask_bits_words = 0;
     row_max = row_sum = y_copy = delta = lse = nullptr;
@@ -133,6 +132,21 @@ struct Kernel {
   std::string last_detail;
   float* stage = nullptr;  // grow-only fp32 staging buffer for float <-> bf16 transfers
   size_t stage_count = 0;
+  float* ds_ws = nullptr;  // dS between the two kernels of an exact fp32 backward: one for all handles, whose backwards follow one
+  int64_t ds_ws_floats = 0;   // another on one stream; as large as the largest of them asks, and gone with the last of them
+  void fit_ds_ws() {       // after a handle has been set or released
+    int64_t need = 0;
+    for (const auto& kv : attn) need = std::max(need, kv.second.ds_floats);
+    if (need != 0 && need <= ds_ws_floats) return;
+    float* p = nullptr;
+    if (need != 0 && cudaMalloc(&p, (size_t)need * sizeof(float)) != cudaSuccess) {
+      cudaGetLastError();  // what there is stays; a backward it is too small for forms dS twice
+      return;
+    }
+    cudaFree(ds_ws);
+    ds_ws = p;
+    ds_ws_floats = need;
+  }
   bool synced = false;     // the call being dispatched has already synchronised the stream behind its last launch
   bool fail_words = false; // this device's kernels raise its failure words (see g_fail)
   int* h_answer = nullptr; // pinned words for small device answers: a mask's class in [0], written by the kernel that finds it
@@ -463,14 +477,12 @@ long attn_set(Kernel* k, long lInput, float* pf, long llInput, MCA_LONGLONG* pl)
     if (cudaMalloc(&a.split_ws, (size_t)a.split_ws_bytes) != cudaSuccess) { cudaGetLastError(); a.split_ws = nullptr; a.split_ws_bytes = 0; }
   }
   if (a.training && a.dtype != MCA_DTYPE_BF16 && ((a.flags & MCA_FLAG_EXACT_FP32) || !mca_sdpa_backward_f32_tc_supported(a.D))) {
-    // The exact fp32 backward passes dS from one kernel to the other: half of the (B,H,T,T) pair of tensors the reference keeps
-    // (attn.cu:436-452), up to a gigabyte.  Beyond that, or where it cannot be had, dS is formed twice.
+    // The exact fp32 backward passes dS from one kernel to the other, in at most a gigabyte.  Beyond that, or where it cannot be had,
+    // dS is formed twice.
     const int64_t bytes = mca_sdpa_backward_f32_ws_bytes(a.B, a.H, a.block);
-    if (bytes <= kMaxDsBytes) {
-      if (cudaMalloc(&a.ds_ws, (size_t)bytes) == cudaSuccess) a.ds_floats = bytes / 4;
-      else { cudaGetLastError(); a.ds_ws = nullptr; }
-    }
+    if (bytes <= kMaxDsBytes) a.ds_floats = bytes / 4;
   }
+  k->fit_ds_ws();
   a.configured = true;
   return 0;
 }
@@ -847,7 +859,7 @@ long attn_bwd(Kernel* k, long llInput, MCA_LONGLONG* pl, int layout) {
     if ((e = resolve_mask(k, a, a.fwd_mask_handle, a.fwd_batch_mask, T, &mask, &mode, false))) return e;
   }
   return mca_sdpa_backward_f32_ws(q, kk, v, dy, a.y_copy, mask, mode, a.causal_flag, a.row_max, a.row_sum, a.delta, a.B, a.H, T,
-                                  a.D, dq, dk, dv, a.ds_ws, a.ds_floats, layout, 0);
+                                  a.D, dq, dk, dv, k->ds_ws, k->ds_ws_floats, layout, 0);
 }
 
 // ---- rope ids ------------------------------------------------------------------------------
@@ -1298,6 +1310,7 @@ void kernel_cleanup(long idx) {
   cudaDeviceSynchronize();
   for (auto& kv : k->mem) cudaFree(kv.second.ptr);
   for (auto& kv : k->attn) kv.second.release();
+  cudaFree(k->ds_ws);
   for (auto& kv : k->rope) { cudaFree(kv.second.cos_t); cudaFree(kv.second.sin_t); }
   for (auto& kv : k->layernorm) cudaFree(kv.second.stdev);
   cudaFree(k->norm_scratch);
@@ -1351,6 +1364,7 @@ long run(Kernel* k, long fn, float* pf, long lInput, MCA_LONGLONG* pl, long llIn
       cudaStreamSynchronize(0);
       it->second.release();
       k->attn.erase(it);
+      k->fit_ds_ws();
       return 0;
     }
     case CUDNN_FN_ATTN_SET: return finish(k, attn_set(k, lInput, pf, llInput, pl));

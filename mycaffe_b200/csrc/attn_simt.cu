@@ -639,6 +639,14 @@ bool small_tiles(int B, int H, int T, bool causal) {
   return cost(64, 0.65) < cost(128, 1.0);
 }
 
+// dS passes through memory where the work, not the longest CTA, decides when the dK/dV kernel ends: where SMs would be idle,
+// the other dQ kernel runs on them beside the dK/dV kernel, and this one could not (the work per SM over the longest CTA's:
+// 0.55, H = 9, T = 1088, D = 128: 406 -> 500 us; 0.8, B = 2, H = 7, T = 967, D = 96: 702 -> 547).
+bool passes_ds(int R, int B, int H, int T, bool causal) {
+  const int64_t tiles = mca_ceil_div(T, R), steps = causal ? tiles * (tiles + 1) / 2 : tiles * tiles;
+  return 3 * steps * B * H > 2 * 148 * tiles;
+}
+
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 }  // namespace
@@ -726,13 +734,7 @@ static int launch_bwd_tile(const float* q, const float* k, const float* v, const
   const int vec_out = (D % 4 == 0) && aligned16(dq) && aligned16(dk) && aligned16(dv);
   const float scale = 1.0f / sqrtf((float)D);
   dim3 grid(B * H, mca_ceil_div(T, R));
-  // dS passes through memory where there is room for it and the work, not the longest CTA, decides when the kernel ends: where
-  // SMs would be idle, the other dQ kernel runs on them beside the dK/dV kernel, and this one could not
-  // (the work per SM over the longest CTA's: 0.55, H = 9, T = 1088, D = 128: 406 -> 500 us; 0.8, B = 2, H = 7, T = 967,
-  // D = 96: 702 -> 547).
-  const bool causal = mode == MCA_MASK_CAUSAL || mode == MCA_MASK_TT;
-  const int64_t tiles = mca_ceil_div(T, R), steps = causal ? tiles * (tiles + 1) / 2 : tiles * tiles;
-  if (ds_floats < ds_tile<R>(B * H, 0, 0, T) || 3 * steps * B * H <= 2 * 148 * tiles) ds = nullptr;
+  if (ds_floats < ds_tile<R>(B * H, 0, 0, T) || !passes_ds(R, B, H, T, mode == MCA_MASK_CAUSAL || mode == MCA_MASK_TT)) ds = nullptr;
   sdpa_bwd_dkdv_f32_kernel<DP, R><<<grid, NT, smem, st>>>(q, k, v, dy, mask, mode, flag, rmax, rsum, delta, H, T, D,
                                                          scale, dk, dv, ds, vec_ok, vec_out, sin, sout);
   e = mca_launch_status();
@@ -773,9 +775,12 @@ int mca_sdpa_backward_f32_layout(const float* q, const float* k, const float* v,
 }
 
 int64_t mca_sdpa_backward_f32_ws_bytes(int B, int H, int T) {
-  // either tile size (small_tiles): whole blocks of 128 in both directions hold the one and the other
-  const int64_t blocks = mca_ceil_div(T, 128);
-  return (int64_t)B * H * blocks * blocks * (128 * 128 * 4);
+  int64_t floats = 0;   // of the mask forms that have a use for it
+  for (const bool causal : {false, true}) {
+    const int R = small_tiles(B, H, T, causal) ? 64 : 128;
+    if (passes_ds(R, B, H, T, causal)) floats = std::max(floats, R == 64 ? ds_tile<64>(B * H, 0, 0, T) : ds_tile<128>(B * H, 0, 0, T));
+  }
+  return floats * 4;
 }
 
 int mca_sdpa_backward_f32_ws(const float* q, const float* k, const float* v, const float* dy, const float* y_saved, const float* mask,

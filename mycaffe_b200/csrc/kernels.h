@@ -12,7 +12,7 @@ struct McaClassifyJob;
 int mca_classify_causal_mask_ws(const McaClassifyJob* job, void* stream);
 
 // Internal: mca_sdpa_backward_f32_layout with room for dS between its two kernels (ds_floats floats, 16-byte aligned; fewer than
-// mca_sdpa_backward_f32_ws_bytes asks for: dS is formed twice).
+// mca_sdpa_backward_f32_ws_bytes asks for, which is 0 where it would not be used: dS is formed twice).
 int64_t mca_sdpa_backward_f32_ws_bytes(int B, int H, int T);
 int mca_sdpa_backward_f32_ws(const float* q, const float* k, const float* v, const float* dy, const float* y_saved, const float* mask,
                              int mask_mode, const int* causal_flag, const float* row_max, const float* row_sum, float* delta_scratch,

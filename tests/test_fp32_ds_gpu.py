@@ -27,3 +27,36 @@ def test_backward(B, H, T, D, kind):
         assert rel_err(g, r) < 2e-5
     a.close()
     cuda.Dispose()
+
+
+def test_handles_share_one_workspace():
+    """dS lives inside one backward: handles of one kernel index hold one workspace between them, none where dS is never passed on, and
+    it goes with the last of them.  Backwards in another order than the forwards use it in turn."""
+    import torch
+    cuda = CudaDnn(0)
+    used = lambda: -torch.cuda.mem_get_info()[0]
+    B, H, T, D = 2, 16, 1024, 96
+    ds, own = B * H * T * T * 4, B * H * T * (4 * 4 + D * 4)
+    new = lambda *s: Sdpa(cuda, *s, training=True, dtype=ids.MCA_DTYPE_F32, flags=ids.MCA_FLAG_EXACT_FP32)
+    new(B, T, H, D).close()                                   # the context's own allocations
+    start, slack = used(), 32 << 20
+    few = [new(1, 256, 2, D) for _ in range(32)]              # too little work for the two-kernel form
+    assert used() - start < slack
+    many = [new(B, T, H, D) for _ in range(4)]
+    assert used() - start < ds + 4 * own + slack
+    for a in few + many[1:]:
+        a.close()
+    small = new(8, 200, 16, D)
+    rng = np.random.default_rng(0)
+    cases = []
+    for a, shape in ((many[0], (B, H, T, D)), (small, (8, 16, 200, D))):
+        t = [rng.standard_normal(shape).astype(np.float32) for _ in range(4)]
+        a.forward(*t[:3], oracle.causal_mask(shape[2]))
+        cases.append((a, t))
+    for a, t in cases + cases[:1]:
+        for g, r in zip(a.backward(t[3]), oracle.sdpa_backward(*t, oracle.causal_mask(t[0].shape[2]), 1, f64=True)):
+            assert rel_err(g, r) < 2e-5
+    many[0].close()
+    small.close()
+    assert used() - start < slack
+    cuda.Dispose()
