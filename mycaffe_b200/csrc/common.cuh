@@ -111,17 +111,21 @@ __device__ __forceinline__ void mca_raise_fail_word(int* words, int family) {
   }
 }
 
-// Opt a kernel into `bytes` of dynamic shared memory, once per device (the attribute call costs more than the launch's
-// own host work when it is repeated).  done: a static of the instantiation that launches this kernel with this size.
+// Set a kernel's attribute once per device (the call costs more than the launch's own host work when it is repeated).
+// done: a static of the instantiation that launches this kernel with this value.
 template <typename F>
-static inline int mca_smem_once(std::atomic<uint64_t>& done, F kern, size_t bytes) {
+static inline int mca_attribute_once(std::atomic<uint64_t>& done, F kern, cudaFuncAttribute attribute, int value) {
   int dev = 0;
   MCA_CUDA_TRY(cudaGetDevice(&dev));
   const uint64_t bit = 1ull << (dev & 63);
   if (dev < 64 && (done.load(std::memory_order_acquire) & bit)) return 0;
-  MCA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  MCA_CUDA_TRY(cudaFuncSetAttribute(kern, attribute, value));
   if (dev < 64) done.fetch_or(bit, std::memory_order_release);
   return 0;
+}
+template <typename F>
+static inline int mca_smem_once(std::atomic<uint64_t>& done, F kern, size_t bytes) {
+  return mca_attribute_once(done, kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 __device__ __forceinline__ void mca_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

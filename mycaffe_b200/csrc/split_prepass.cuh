@@ -8,8 +8,8 @@
 //   float4 scale[BH]     the scales of q, k, v and dY of each (batch, head)
 //   from the next multiple of 1024 bytes: four tensors of rows x 128 fp16 (256 for 128-wide heads): q, k, v, dY
 //
-// It is bound by memory: 4 bytes read and 4 written per element.  A cluster of up to eight CTAs takes one (batch, head) of
-// one tensor: a CTA keeps its rows in registers (32 floats a thread; what a very long head has beyond that is read again,
+// It is bound by memory: 4 bytes read and 4 written per element.  A cluster of up to eight CTAs (sixteen for few heads) takes
+// one (batch, head) of one tensor: a CTA keeps its rows in registers (32 floats a thread; what a very long head has beyond that is read again,
 // from L2 if it fits), finds their largest magnitude, the CTAs exchange those through distributed shared memory, and the
 // rows are converted where they are.  One launch and one read from HBM, where a scale per tensor took a clear, a
 // grid-wide reduction and a second kernel that read everything again: B = 8, H = 12, T = 1024, D = 64,
@@ -74,9 +74,9 @@ __device__ __forceinline__ float amax4(const float4& v) { return fmaxf(fmaxf(fab
 
 // The power of two that brings max |x| into [2^12, 2^13): the largest fp16 is 65504 and the low half of an element
 // is about 2^-11 of it, so both halves of everything within 2^-14 of the maximum are normal fp16 numbers.  It lies in
-// [2^-115, 2^126], so that it and its reciprocal are normal (a subnormal maximum stays below 2^12; its halves carry every bit it
-// has, the split dS of such a V fewer).  Products of several scales are not: the kernels multiply by them through pow2_factors, or one
-// after the other where every partial product is bounded, as said there.
+// [2^-115, 2^126], so that it and its reciprocal are normal (a subnormal maximum stays below 2^12; its halves carry every
+// bit it has, the split dS of such a V fewer).  Products of several scales are not: the kernels multiply by them through
+// pow2_factors, or one after the other where every partial product is bounded, as said there.
 __device__ __forceinline__ float pow2_scale(float a) {
   if (!(a > 0.f) || !(a < 3.0e38f)) return 1.0f;
   int e;
@@ -104,17 +104,17 @@ constexpr int THREADS = 256, KEEP = 4;   // eight-element pieces a thread keeps 
 
 // with ydot / delta given: also delta[row] = sum_c x[row][c] * ydot[row][c] (ydot contiguous rows) x scale x DS_SHIFT, the
 // softmax backward's row term in the units the backward kernels need, from the elements this kernel holds anyway.
-// grid: (CTAs of a cluster, BH, [the CTAs that classify the mask +] tensors); the classification comes first, so that its
+// grid: (CTAs of a cluster, BH, cls_layers of CTAs that classify the mask + tensors); the classification comes first, so that its
 // answer is on the host before the tensors are done
 template <int HD>
 __global__ void __launch_bounds__(THREADS) split_kernel(const Job job, const McaStrides st, int H, int T,
                                                         float* __restrict__ scale, const float* __restrict__ ydot,
-                                                        float* __restrict__ delta, const McaClassifyJob cls) {
+                                                        float* __restrict__ delta, const McaClassifyJob cls, int cls_layers) {
   mca_pdl_launch_dependents();
   mca_pdl_wait();   // the tensors are earlier kernels' output
-  const int tid = threadIdx.x, which = (int)blockIdx.z - (cls.mask != nullptr ? 1 : 0);
+  const int tid = threadIdx.x, which = (int)blockIdx.z - cls_layers;
   if (which < 0) {
-    mca_classify_rows(cls, (int)(blockIdx.y * gridDim.x + blockIdx.x), (int)(gridDim.x * gridDim.y));
+    mca_classify_rows(cls, (int)((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x), cls_layers * (int)(gridDim.x * gridDim.y));
     return;
   }
   constexpr int V8 = HD / 8;
@@ -218,16 +218,27 @@ __global__ void __launch_bounds__(THREADS) split_kernel(const Job job, const Mca
 template <int HD>
 inline int run(const Job& job, int count, const McaStrides& st, int B, int H, int T, const Workspace& w, cudaStream_t stream,
                const float* ydot = nullptr, float* delta = nullptr, const McaClassifyJob* cls = nullptr) {
-  // CTAs of a cluster: as many as leave each at most what its threads keep in registers, up to the portable eight
+  // CTAs of a cluster: as many as leave each at most what its threads keep in registers, up to the portable eight -- or sixteen
+  // where a few long heads would not give every SM one (forward of
+  // four heads of 8192 rows 208 -> 198 us, of one of 16384 378 -> 360)
   const int64_t pieces = (int64_t)T * (HD / 8);
+  const int most = B * H * count * 8 < 148 ? 16 : 8;
   int ctas = 1;
-  while (ctas < 8 && pieces > (int64_t)ctas * KEEP * THREADS) ctas *= 2;
+  while (ctas < most && pieces > (int64_t)ctas * KEEP * THREADS) ctas *= 2;
+  if (ctas > 8) {
+    static std::atomic<uint64_t> done{0};
+    const int e = mca_attribute_once(done, split_kernel<HD>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e) return e;
+  }
+  // The mask is T x T whatever the heads are: as many layers as give every eight rows of it a CTA, up to 1184 CTAs (with
+  // one layer a single head of 16384 rows had eight CTAs read a gigabyte: 6.04 ms, 0.53 with this)
+  const int layers = cls != nullptr ? mca_ceil_div(std::min(1184, mca_ceil_div(T, 8)), ctas * B * H) : 0;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(ctas, B * H, count + (cls != nullptr ? 1 : 0));
+  cfg.gridDim = dim3(ctas, B * H, count + layers);
   cfg.blockDim = dim3(THREADS);
   cfg.stream = stream;
   return mca_launch_pdl_cluster(split_kernel<HD>, cfg, ctas, job, st, H, T, reinterpret_cast<float*>(w.scale), ydot, delta,
-                                cls != nullptr ? *cls : McaClassifyJob{});
+                                cls != nullptr ? *cls : McaClassifyJob{}, layers);
 }
 
 }  // namespace split
