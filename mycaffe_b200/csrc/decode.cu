@@ -21,6 +21,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "step_rules.h"
 
 // Scratch of the no-allocation entry point (mca_decode_attention_static): the split partials
 // live in this fixed array instead of caller-provided memory.  Every GPU that loads the library
@@ -657,7 +658,8 @@ static int decode_attention(const float* q, const float* k_new, const float* v_n
   p.pos_limit = max_len;   // <= seq_len, and the planned splits cover [0, max_len)
   if (p.kv_mul > 4 && p.kv_mul % 4 != 0) return ERROR_ATTN_UNSUPPORTED_SHAPE;
   if (p.kv_mul == 3) return ERROR_ATTN_UNSUPPORTED_SHAPE;
-  p.prefetch = B <= 8;     // exactly the launches made ahead (launch_decode)
+  p.prefetch = step_rules::prefetch_rows(partials != nullptr, B, cache_is_bf16 != 0,
+                                         2ll * B * max_len * n_kv_heads * head_size * (cache_is_bf16 ? 2 : 4));
   if (partials != nullptr)
     *partials = McaDecodePartials{p.part_acc, p.part_ml, pos, n_heads, head_size, p.nsplit, p.split_len, p.pos_limit};
   const bool combine = partials == nullptr;
