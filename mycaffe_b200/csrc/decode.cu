@@ -658,7 +658,7 @@ static int decode_attention(const float* q, const float* k_new, const float* v_n
   p.pos_limit = max_len;   // <= seq_len, and the planned splits cover [0, max_len)
   if (p.kv_mul > 4 && p.kv_mul % 4 != 0) return ERROR_ATTN_UNSUPPORTED_SHAPE;
   if (p.kv_mul == 3) return ERROR_ATTN_UNSUPPORTED_SHAPE;
-  p.prefetch = step_rules::prefetch_rows(partials != nullptr, B, cache_is_bf16 != 0,
+  p.prefetch = step_rules::prefetch_rows(partials != nullptr, B, cache_is_bf16 != 0, p.kv_mul,
                                          2ll * B * max_len * n_kv_heads * head_size * (cache_is_bf16 ? 2 : 4));
   if (partials != nullptr)
     *partials = McaDecodePartials{p.part_acc, p.part_ml, pos, n_heads, head_size, p.nsplit, p.split_len, p.pos_limit};

@@ -17,11 +17,13 @@ def holds(tmp_path, *claims):
 def test_rows_are_asked_for_ahead_only_where_that_gains(tmp_path):
     rows = "2ll * {} * {} * {} * {}".format      # sequences, keys, width, bytes
     holds(tmp_path,
-          f"!prefetch_rows(false, 7, false, {rows(7, 4096, 4096, 4)})",      # a call of its own: nothing to wait for
-          f"!prefetch_rows(false, 1, true, {rows(1, 256, 384, 2)})",
-          f"prefetch_rows(true, 1, false, {rows(1, 256, 768, 4)})",          # in a step
-          f"prefetch_rows(true, 8, false, {rows(8, 2048, 4096, 4)})",
-          f"prefetch_rows(true, 8, true, {rows(8, 1024, 768, 2)})",
-          f"!prefetch_rows(true, 1, true, {rows(1, 2048, 4096, 2)})",        # bf16 rows beside the weights in L2
-          f"!prefetch_rows(true, 1, true, {rows(1, 32768, 1024, 2)})",
-          f"!prefetch_rows(true, 9, false, {rows(9, 256, 768, 4)})")         # ordinary launches
+          f"!prefetch_rows(false, 7, false, 1, {rows(7, 4096, 4096, 4)})",   # a call of its own: nothing to wait for
+          f"!prefetch_rows(false, 1, true, 1, {rows(1, 256, 384, 2)})",
+          f"prefetch_rows(true, 1, false, 1, {rows(1, 256, 768, 4)})",       # in a step
+          f"prefetch_rows(true, 8, false, 1, {rows(8, 2048, 4096, 4)})",
+          f"prefetch_rows(true, 8, true, 1, {rows(8, 1024, 768, 2)})",
+          f"!prefetch_rows(true, 1, true, 1, {rows(1, 2048, 4096, 2)})",     # rows that are too many beside the weights in L2
+          f"!prefetch_rows(true, 1, true, 4, {rows(1, 32768, 1024, 2)})",
+          f"prefetch_rows(true, 8, false, 4, {rows(8, 2048, 1024, 4)})",
+          f"!prefetch_rows(true, 1, false, 4, {rows(1, 32768, 1024, 4)})",
+          f"!prefetch_rows(true, 9, false, 1, {rows(9, 256, 768, 4)})")         # ordinary launches
