@@ -660,9 +660,9 @@ static int decode_attention(const float* q, const float* k_new, const float* v_n
   if (p.kv_mul == 3) return ERROR_ATTN_UNSUPPORTED_SHAPE;
   p.prefetch = step_rules::prefetch_rows(partials != nullptr, B, cache_is_bf16 != 0, p.kv_mul,
                                          2ll * B * max_len * n_kv_heads * head_size * (cache_is_bf16 ? 2 : 4));
+  const bool combine = partials == nullptr || !step_rules::combine_in_projection(B, p.nsplit, n_heads * head_size);
   if (partials != nullptr)
-    *partials = McaDecodePartials{p.part_acc, p.part_ml, pos, n_heads, head_size, p.nsplit, p.split_len, p.pos_limit};
-  const bool combine = partials == nullptr;
+    *partials = McaDecodePartials{p.part_acc, p.part_ml, pos, n_heads, head_size, combine ? 1 : p.nsplit, p.split_len, p.pos_limit};
   cudaStream_t st = (cudaStream_t)stream;
   switch (head_size) {
 #define MCA_DECODE_CASE(HS_) \

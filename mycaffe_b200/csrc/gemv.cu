@@ -63,7 +63,7 @@ struct GemvParams {
   int split;                     // S: warps of a CTA that share a row along K (1, 2, 4 or 8)
   float eps;
   // x as the split-KV attention left it, one (maximum, sum) pair and hs weighted values per (sequence, head, split): the
-  // combine pass happens where the activations are staged (part_acc null: x is the input)
+  // combine pass happens where the activations are staged (kernels of PART; the others read x)
   const float* part_acc = nullptr;
   const float* part_ml = nullptr;
   const int* pos = nullptr;
@@ -110,8 +110,13 @@ __device__ __forceinline__ float4 combine_partials(const GemvParams& p, int b, i
 // shared memory), THREADS per CTA, DEPTH ring steps per warp, each of U warp-wide vectors per row.  GLU: the two rows of a step are
 // row r of w[0] and row r of w[1], combined by SwiGLU (R must be 2); otherwise they are
 // consecutive rows of the stacked matrix.
-template <typename WT, int NB, int R, int THREADS, bool GLU, int DEPTH, int U>
-__global__ void __launch_bounds__(THREADS) gemv_stream_kernel(const GemvParams p, int b0) {
+// PART: x is combined from the attention's partial results.  An instantiation of its own: as a branch of all of them it took
+// their registers and serialised the staging's loads (8 sequences of two 7B-shaped layers, bf16: 693 -> 774 us a step).
+// The kernels are compiled for the CTAs that shared memory lets an SM hold, two of 256 threads or one of 512: left to itself
+// the compiler kept the first to 40 registers and the 512-thread ones of four sequences to 64 (four layers 2048 wide, fp32, one
+// sequence: 209 -> 199 us a step; four sequences 307 -> 286).
+template <typename WT, int NB, int R, int THREADS, bool GLU, int DEPTH, int U, bool PART>
+__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) gemv_stream_kernel(const GemvParams p, int b0) {
   static_assert(!GLU || R == 2, "the gated form pairs one row of each matrix");
   constexpr int STEP = GLU ? 1 : R;   // output rows finished per step
   constexpr int WARPS = THREADS / 32;
@@ -187,7 +192,9 @@ __global__ void __launch_bounds__(THREADS) gemv_stream_kernel(const GemvParams p
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
       const int bb = min(b0 + b, p.B - 1);   // a pass may be padded: the last sequence again, its sums not written
-      const float4 v = p.part_acc != nullptr ? combine_partials(p, bb, k) : *reinterpret_cast<const float4*>(p.x + (int64_t)bb * n + k);
+      float4 v;
+      if constexpr (PART) v = combine_partials(p, bb, k);
+      else v = *reinterpret_cast<const float4*>(p.x + (int64_t)bb * n + k);
       *reinterpret_cast<float4*>(xs + b * n + k) = v;
       ss[b] += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
     }
@@ -341,14 +348,14 @@ __global__ void __launch_bounds__(THREADS) gemv_stream_kernel(const GemvParams p
 template <int R, int THREADS, int DEPTH, int U = 1>
 constexpr size_t ring_bytes() { return (size_t)(THREADS / 32) * DEPTH * R * U * 32 * sizeof(uint4); }
 
-template <typename WT, int NB, int R, int THREADS, bool GLU, int DEPTH, int U = 1>
+template <typename WT, int NB, int R, int THREADS, bool GLU, int DEPTH, int U = 1, bool PART = false>
 int launch_pass(GemvParams p, int b0, cudaStream_t st) {
   constexpr int STEP = GLU ? 1 : R;
   constexpr int WARPS = THREADS / 32;
   static_assert(ring_bytes<R, THREADS, DEPTH, U>() / WARPS >= sizeof(float) * GV_SPLIT_STEPS * R * NB, "partials fit the ring");
   const size_t smem = sizeof(float) * (size_t)NB * p.n + ring_bytes<R, THREADS, DEPTH, U>();
   if (smem > GV_SMEM_LIMIT) return ERROR_ATTN_UNSUPPORTED_SHAPE;
-  auto kern = gemv_stream_kernel<WT, NB, R, THREADS, GLU, DEPTH, U>;
+  auto kern = gemv_stream_kernel<WT, NB, R, THREADS, GLU, DEPTH, U, PART>;
   const int total_rows = GLU ? p.rows[0] : p.rows[0] + (p.n_mats > 1 ? p.rows[1] : 0) + (p.n_mats > 2 ? p.rows[2] : 0);
   const int total_steps = mca_ceil_div(total_rows, STEP);
   // every CTA resident at once; rows dealt evenly to groups of S warps.  The attribute and the
@@ -457,6 +464,9 @@ int run_proj_tc(const GemvParams& p, cudaStream_t st) {
   return mca_launch_pdl(kern, dim3(proj::pick_ctas((int64_t)tiles * q.kchunks, sms)), dim3(proj::Roles<PL::CONVERT>::THREADS), smem, st, mw[0], mw[1], mw[2], mx, q);
 }
 
+// one sequence: a deeper ring while two CTAs per SM still fit (half an SM's shared memory, less the per-CTA reserve)
+bool deep_ring(int n) { return sizeof(float) * (size_t)n + ring_bytes<1, 256, 6, 4>() <= 112 * 1024; }
+
 template <typename WT>
 int run_gemv(const GemvParams& p, cudaStream_t st) {
   int e = run_proj_tc<WT>(p, st);
@@ -467,7 +477,7 @@ int run_gemv(const GemvParams& p, cudaStream_t st) {
   constexpr size_t RING_512 = ring_bytes<2, 512, 6>(), RING_256 = ring_bytes<2, 256, 6>();
   constexpr size_t RING_1 = ring_bytes<1, 256, 4, 4>();   // = ring_bytes<2, 256, 4, 2>(), the one- and two-sequence kernels
   if (!fits(1, RING_1)) return ERROR_ATTN_UNSUPPORTED_SHAPE;
-  const bool deep = xbytes + ring_bytes<1, 256, 6, 4>() <= 112 * 1024;   // half an SM's shared memory, less the per-CTA reserve
+  const bool deep = deep_ring(p.n);
   // Passes of 8, 4, 2 or 1 sequences; 5 to 7, and 3, are one padded pass (the weights are read once, and a pass over a small
   // matrix is mostly launch and latency) where the padded activations fit.
   for (int b0 = 0; b0 < p.B && !e;) {
@@ -477,7 +487,7 @@ int run_gemv(const GemvParams& p, cudaStream_t st) {
       else if (left >= 3 && fits(4, RING_512)) { e = launch_pass<WT, 4, 2, 512, true, 6>(p, b0, st); b0 += 4; }
       else if (left >= 3 && fits(4, RING_256)) { e = launch_pass<WT, 4, 2, 256, true, 6>(p, b0, st); b0 += 4; }
       else if (left >= 2 && fits(2, RING_1)) { e = launch_pass<WT, 2, 2, 256, true, 4, 2>(p, b0, st); b0 += 2; }
-      else {   // a deeper ring while two CTAs per SM still fit
+      else {
         e = deep ? launch_pass<WT, 1, 2, 256, true, 6, 2>(p, b0, st) : launch_pass<WT, 1, 2, 256, true, 4, 2>(p, b0, st);
         b0 += 1;
       }
@@ -531,18 +541,21 @@ int mca_decode_out_proj(const float* attn, const void* wo, int weights_bf16, int
   return weights_bf16 ? run_gemv<__nv_bfloat16>(p, (cudaStream_t)stream) : run_gemv<float>(p, (cudaStream_t)stream);
 }
 
-int mca_decode_out_proj_partials(const McaDecodePartials* a, const void* wo, int weights_bf16, int B, int dim, float* x_inout,
-                                 void* stream) {
-  if (B > 8 || dim % 8 != 0 || !al16(wo) || !al16(a->acc)) return ERROR_PARAM_OUT_OF_RANGE;
+int mca_decode_out_proj_partials(const McaDecodePartials* a, const void* wo, int weights_bf16, int dim, float* x_inout, void* stream) {
+  if (dim % 8 != 0 || !al16(wo) || !al16(a->acc)) return ERROR_PARAM_OUT_OF_RANGE;
+  if (!gemv_supported(dim)) return ERROR_ATTN_UNSUPPORTED_SHAPE;
   GemvParams p;
   p.swiglu = 0;
-  p.x = nullptr; p.norm_w = nullptr; p.eps = 0.f; p.n = dim; p.B = B; p.accumulate = 1; p.n_mats = 1;
+  p.x = nullptr; p.norm_w = nullptr; p.eps = 0.f; p.n = dim; p.B = 1; p.accumulate = 1; p.n_mats = 1;
   p.w[0] = wo; p.w[1] = p.w[2] = nullptr;
   p.out[0] = x_inout; p.out[1] = p.out[2] = nullptr;
   p.rows[0] = dim; p.rows[1] = p.rows[2] = 0;
   p.part_acc = a->acc; p.part_ml = a->ml; p.pos = a->pos;
   p.n_heads = a->n_heads; p.hs = a->hs; p.nsplit = a->nsplit; p.split_len = a->split_len; p.pos_limit = a->pos_limit;
-  return weights_bf16 ? run_gemv<__nv_bfloat16>(p, (cudaStream_t)stream) : run_gemv<float>(p, (cudaStream_t)stream);
+  cudaStream_t st = (cudaStream_t)stream;
+  if (deep_ring(dim))
+    return weights_bf16 ? launch_pass<__nv_bfloat16, 1, 1, 256, false, 6, 4, true>(p, 0, st) : launch_pass<float, 1, 1, 256, false, 6, 4, true>(p, 0, st);
+  return weights_bf16 ? launch_pass<__nv_bfloat16, 1, 1, 256, false, 4, 4, true>(p, 0, st) : launch_pass<float, 1, 1, 256, false, 4, 4, true>(p, 0, st);
 }
 
 int mca_decode_ffn(const float* rms_weight, float eps, const void* w1, const void* w2, const void* w3, int weights_bf16,

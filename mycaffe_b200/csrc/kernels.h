@@ -33,9 +33,9 @@ int mca_set_fail_words_probe(int* words);
 int mca_set_fail_words_decode(int* words);
 int mca_set_fail_words_proj(int* words);
 
-// Internal: the decode attention without its combine pass, for up to eight sequences whose partials mca_decode_out_proj_partials
-// combines while it stages its activations.  *partials is filled in when more than one split was planned; with one (nsplit 1)
-// the output is in `out` as mca_decode_attention leaves it.
+// Internal: the decode attention inside a step of up to eight sequences.  Where step_rules says so its combine pass is left to
+// mca_decode_out_proj_partials (one sequence), which combines the partial results while it stages its activations: *partials
+// then says where they are; with nsplit 1 the output is in `out` as mca_decode_attention leaves it.
 struct McaDecodePartials {
   const float *acc, *ml;
   const int* pos;
@@ -45,5 +45,4 @@ int mca_decode_attention_partials(const float* q, const float* k_new, const floa
                                   int cache_is_bf16, int64_t cache_batch_stride, const int* pos, int B, int n_heads, int n_kv_heads,
                                   int head_size, int seq_len, int max_len, const float* freq_real, const float* freq_imag,
                                   float* scratch, int64_t scratch_floats, float* out, McaDecodePartials* partials, void* stream);
-int mca_decode_out_proj_partials(const McaDecodePartials* partials, const void* wo, int weights_bf16, int B, int dim, float* x_inout,
-                                 void* stream);
+int mca_decode_out_proj_partials(const McaDecodePartials* partials, const void* wo, int weights_bf16, int dim, float* x_inout, void* stream);

@@ -110,13 +110,13 @@ int mca_llama_forward(const McaLlamaConfig* cfg, const McaLlamaWeights* wt, cons
     void* vc = static_cast<char*>(st->value_cache) + (size_t)(l * layer_cache) * cb;
     const void* wo = mat(wt->wo, l, dim, dim);
     if (B <= 8) {
-      // the combine pass rides on the output projection's activation staging: one launch and one hop of the chain less
+      // a combine pass may ride on the output projection's activation staging: one launch and one hop of the chain less
       McaDecodePartials parts;
       e = mca_decode_attention_partials(q, k, v, kc, vc, st->cache_is_bf16, (int64_t)cfg->seq_len * kv_dim, pos, B, cfg->n_heads,
                                         cfg->n_kv_heads, hs, cfg->seq_len, max_len, st->freq_real, st->freq_imag, ws + w.scratch,
                                         w.scratch_floats, att, &parts, stream);
       if (e) return e;
-      e = parts.nsplit > 1 ? mca_decode_out_proj_partials(&parts, wo, wt->weights_bf16, B, dim, x, stream)
+      e = parts.nsplit > 1 ? mca_decode_out_proj_partials(&parts, wo, wt->weights_bf16, dim, x, stream)
                            : mca_decode_out_proj(att, wo, wt->weights_bf16, B, dim, x, stream);
     } else {
       e = mca_decode_attention(q, k, v, kc, vc, st->cache_is_bf16, (int64_t)cfg->seq_len * kv_dim, pos, B, cfg->n_heads,

@@ -16,4 +16,11 @@ inline bool prefetch_rows(bool in_step, int B, bool cache_bf16, int kv_mul, int6
   return in_step && B <= 8 && row_bytes <= most;
 }
 
+// Should the output projection combine the attention's splits while it stages its activations, instead of a kernel between the
+// two?  Every one of its CTAs then reads every partial result: worth the launch for one sequence and few of them (a
+// token of 6 layers, 8 splits: 6 heads of 48 118 us, 129 with the kernel; 12 of 64 156 and 165; 4 layers of 16 heads of 128 212 and
+// 216), not beyond (2 layers of 32 heads of 128, 9 splits: 237 us, 230 with the kernel; 37 splits of 8 kv heads 273 and 248),
+// nor for more sequences (8, with 8 splits, 4 layers of 16 heads of 128: 575 and 532 us).
+inline bool combine_in_projection(int B, int nsplit, int dim) { return B == 1 && nsplit > 1 && (int64_t)nsplit * dim <= 16384; }
+
 }  // namespace step_rules

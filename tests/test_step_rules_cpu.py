@@ -27,3 +27,11 @@ def test_rows_are_asked_for_ahead_only_where_that_gains(tmp_path):
           f"prefetch_rows(true, 8, false, 4, {rows(8, 2048, 1024, 4)})",
           f"!prefetch_rows(true, 1, false, 4, {rows(1, 32768, 1024, 4)})",
           f"!prefetch_rows(true, 9, false, 1, {rows(9, 256, 768, 4)})")         # ordinary launches
+
+
+def test_splits_are_combined_in_the_projection_for_one_sequence_and_few_of_them(tmp_path):
+    holds(tmp_path,
+          "combine_in_projection(1, 8, 768)", "combine_in_projection(1, 8, 2048)", "combine_in_projection(1, 2, 288)",
+          "!combine_in_projection(1, 1, 768)",                                    # nothing to combine
+          "!combine_in_projection(1, 9, 4096)", "!combine_in_projection(1, 37, 4096)",
+          "!combine_in_projection(2, 2, 288)", "!combine_in_projection(8, 8, 768)", "!combine_in_projection(5, 7, 4096)")
