@@ -9,12 +9,12 @@
 //   from the next multiple of 1024 bytes: four tensors of rows x 128 fp16 (256 for 128-wide heads): q, k, v, dY
 //
 // It is bound by memory: 4 bytes read and 4 written per element.  A cluster of up to eight CTAs (sixteen for few heads) takes
-// one (batch, head) of one tensor: a CTA keeps its rows in registers (32 floats a thread; what a very long head has beyond that is read again,
-// from L2 if it fits), finds their largest magnitude, the CTAs exchange those through distributed shared memory, and the
-// rows are converted where they are.  One launch and one read from HBM, where a scale per tensor took a clear, a
+// one (batch, head) of one tensor: a CTA keeps its rows in registers (32 floats a thread; what a very long head has beyond
+// that is read again, from L2 if it fits), finds their largest magnitude, the CTAs exchange those through distributed
+// shared memory, and the rows are converted where they are.  One launch and one read from HBM, where a scale per tensor took a clear, a
 // grid-wide reduction and a second kernel that read everything again: B = 8, H = 12, T = 1024, D = 64,
-// the pre-passes of forward and backward 71 -> 59 us together, and three launches fewer.
-// The same launch classifies the caller's (T,T) mask when it is given one (its CTAs follow those of the tensors).
+// the pre-passes of forward and backward 71 -> 54 us together (36 + 18 alone), and three launches fewer.
+// The same launch classifies the caller's (T,T) mask when it is given one (its CTAs come before those of the tensors).
 #pragma once
 #include <cuda_fp16.h>
 
@@ -84,16 +84,14 @@ __device__ __forceinline__ float pow2_scale(float a) {
   return ldexpf(1.0f, min(13 - e, 126));
 }
 __device__ __forceinline__ int scale_exp(float scale) { return (__float_as_int(scale) >> 23) - 127; }
+__device__ __forceinline__ float pow2(int e) { return __int_as_float((max(-126, min(127, e)) + 127) << 23); }
 // 2^e as two factors, applied one after the other: exact wherever the result is a normal number, without an infinity or a
 // zero on the way (beyond 2^254 and 2^-252 the result is one anyway).
-__device__ __forceinline__ float2 pow2_factors(int e) {
-  const int h = e / 2;
-  return make_float2(ldexpf(1.0f, max(-126, min(127, h))), ldexpf(1.0f, max(-126, min(127, e - h))));
-}
+__device__ __forceinline__ float2 pow2_factors(int e) { return make_float2(pow2(e / 2), pow2(e - e / 2)); }
 // Factor of the logits S' = Q'K'^T back to their own units (times `scale`).  |S'| < 2^33: below 2^-100 every logit is zero to
 // the exponential anyway, and the bound keeps the masked logit (a constant over this factor) finite.
 __device__ __forceinline__ float logit_scale(float scale, const float4& sc) {
-  return ldexpf(scale, max(-100, min(120, -(scale_exp(sc.x) + scale_exp(sc.y)))));
+  return scale * pow2(max(-100, min(120, -(scale_exp(sc.x) + scale_exp(sc.y)))));
 }
 // dY' V'^T products (below 2^32) are taken down by this before dS is split, and delta is left by the pre-pass in the units of dY'
 // times this: delta x (the scale of v) is then below 2^13, whatever the magnitudes of dY and v.
