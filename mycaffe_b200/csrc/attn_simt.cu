@@ -1,10 +1,11 @@
 // Exact-fp32 scaled-dot-product attention on CUDA cores: forward, and a recompute-based
-// backward.  This is the default fp32 path behind ATTN_FWD / ATTN_BWD: it reproduces the
+// backward.  Handles with MCA_FLAG_EXACT_FP32 run it, and fp32 handles where there is no split-operand tensor-core kernel
+// (attn_tc.cu, attn_tc_bwd.cu): other head sizes than 16, 32, 64 and 128, and the backward of 128.  It reproduces the
 // reference's arithmetic (attn.cu:518-661 of CudaDnnDLL) -- scale applied to the finished dot
 // product, masked logits overwritten with the finite value -1e29, max-subtracted softmax --
 // without ever materialising the (B,H,T,T) score tensors the reference allocates in
 // attnHandle::Set (attn.cu:436-452).  It accepts every mask form of the reference and any head
-// size up to 128.  The tensor-core kernels in attn_tc.cu cover the bf16 / tf32 variants.
+// size up to 128.
 //
 // Tiling.  What bounds these kernels is the fp32 FMA pipe, and what keeps a kernel from it is feeding the pipe: every
 // product reads both operands from shared memory, and a 16-byte load of a warp takes two cycles of the shared-memory pipe
@@ -451,11 +452,11 @@ __global__ void __launch_bounds__(NT) sdpa_bwd_dkdv_f32_kernel(
 }
 
 // dQ for 64 queries from the dS the dK/dV kernel left: one product instead of three, so 5 of the backward's 7 are formed.  The FMA
-// pipe is the bound (67 % of it while a CTA is on the SM; the rest is the duplication of an operand for the pairs).  Steps of
-// 32 keys in a ring of three, so that two CTAs share an SM and four warps a scheduler; 64 queries a CTA whatever R is, so that
-// the last ones are short (128: 437 us, 64: 353); a thread's rows are 16 apart, so that the rows a warp reads at a time lie in
-// different banks.  dS (4 bytes per pair, written by one bulk copy a tile) costs the dK/dV kernel nothing that can be measured.
-// B = 2, H = 16, T = 1500, D = 128, causal: 911 -> 353 us, forward and backward 2048 -> 1480 us.
+// pipe is the bound (70 % active; the dK/dV kernel, with two warps per scheduler, keeps it at 61 %).  Steps of 32 keys in a ring of
+// three, so that two CTAs share an SM and four warps a scheduler; 64 queries a CTA whatever R is, so that the last ones are
+// short; a thread's rows are 16 apart, so that the rows a warp reads at a time lie in different banks.
+// B = 2, H = 16, T = 1500, D = 128, causal, forward and backward: 2048 us with dS formed twice, 1486 with this (dK/dV 1146 and dQ
+// 238 us when each runs alone).
 constexpr int DS_KEYS = 32, DS_STAGES = 3;
 template <int DP> constexpr size_t dq_ds_smem_bytes() { return sizeof(float) * DS_STAGES * (SX * DS_KEYS + DS_KEYS * Row<DP>::LD); }
 template <int DP, int RK>
@@ -625,6 +626,9 @@ int pick_dp(int D) {
 // Rows per CTA: 128, or 64 where that is estimated to end sooner -- few or short heads, whose 128-row tiles would leave SMs
 // idle, or a last tile that is nearly empty.  A step of a 64-row tile is taken for 0.65 of a 128-row one (its products load
 // more per multiply-add); the kernel ends no sooner than its longest CTA nor than the work spread over 148 SMs.
+// Either tile throughout, forward and backward, us with 128 and with 64 rows: B=2 H=16 T=1536 D=128 key mask 4119 and 4727,
+// causal 1499 and 1570; B=1 H=16 T=1024 D=128 causal 570 and 478; B=1 H=8 T=700 D=128 403 and 258; B=2 H=16 T=1536 D=80 1533 and
+// 1414 (heads below 128 would bear a smaller factor).
 bool small_tiles(int B, int H, int T, bool causal) {
   auto cost = [&](int R, double step) {
     int64_t steps = 0;
