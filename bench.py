@@ -759,7 +759,7 @@ def run_fp32_prefill(cx, B=1, T=PF_T):
             "tensor_cores_ms": round(ms_tc, 3), "tflops": round(tf, 1), "cuda_cores_ms": round(ms_cc, 3),
             "cuda_cores_tflops": round(fl / (ms_cc * 1e-3) / 1e12, 1), "speedup": round(ms_cc / ms_tc, 2),
             "max_abs_diff_over_scale": diff / scale,
-            "roofline": tensor_roofline(cx, tf, "split::amax_kernel + split::rows_kernel + sdpa_fwd_tc_kernel<128,split>", ms_tc,
+            "roofline": tensor_roofline(cx, tf, "split::split_kernel<128> + sdpa_fwd_tc_kernel<128,split>", ms_tc,
                                         "useful flops of the fp32 problem over the whole call; the kernel executes three fp16 "
                                         "products per contraction, so 1/3 of the bf16 peak is its ceiling")}
 
