@@ -24,20 +24,40 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-// Sum over the G threads that share a row.  G == 32: the warp.  G > 32: the CTA (G == blockDim.x).
-template <int G>
-__device__ __forceinline__ float group_sum(float v, float* sred) {
-  v = warp_sum(v);
-  if (G == 32) return v;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0) sred[warp] = v;
-  __syncthreads();
-  float t = 0.f;
+// Sums of N values over the G threads that share a row.  G == 32: the warp.  G > 32: the CTA (G == blockDim.x), through one of two
+// buffers in turn, so that one barrier is enough.
+template <int G, int N>
+__device__ __forceinline__ void group_sum(float (&v)[N], float (*sred)[2][32], int& turn) {
 #pragma unroll
-  for (int w = 0; w < G / 32; ++w) t += sred[w];
+  for (int k = 0; k < N; ++k) v[k] = warp_sum(v[k]);
+  if (G == 32) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float (*buf)[32] = sred[turn];
+  turn ^= 1;
+  if (lane == 0) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) buf[k][warp] = v[k];
+  }
   __syncthreads();
-  return t;
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < G / 32; ++w) t += buf[k][w];
+    v[k] = t;
+  }
 }
+
+// a / b from r, the reciprocal of b as a division gives it: the quotient a r put right by its own remainder, which a fused
+// multiply-add forms exactly (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+// Dev. 34, 1990: correctly rounded but for a b whose significand is all ones).  A division per element was a third of these kernels'
+// instructions.  For b within 2^-60 .. 2^60 and |a| <= 2^60 (or sqrt(inner) b), so that nothing on the way overflows.
+constexpr float DIV_MAX = 1.152921504606847e18f;   // 2^60
+__device__ __forceinline__ float div_by(float a, float b, float r) {
+  const float q = a * r;
+  return fmaf(fmaf(-q, b, a), r, q);
+}
+__device__ __forceinline__ bool div_ok(float b) { return b >= 1.f / DIV_MAX && b <= DIV_MAX; }
 
 // The part of a row one thread holds: MAXV pieces of VEC floats, piece i at element (i*G + g)*VEC.
 template <int G, int MAXV, int VEC>
@@ -70,6 +90,20 @@ struct RowPart {
       }
     }
   }
+  template <typename F> __device__ __forceinline__ void each(F f) {
+#pragma unroll
+    for (int i = 0; i < MAXV; ++i)
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) f(v[i][j], i, j);
+  }
+  __device__ __forceinline__ void divide(float b) {
+    if (div_ok(b)) {
+      const float r = 1.f / b;
+      each([&](float& e, int, int) { e = div_by(e, b, r); });
+    } else {
+      each([&](float& e, int, int) { e = e / b; });
+    }
+  }
 };
 
 // which: 0 LayerNorm forward, 1 LayerNorm backward, 2 RMSNorm forward, 3 RMSNorm backward
@@ -87,49 +121,42 @@ struct NormParams {
 };
 
 template <int WHICH, int G, int MAXV, int VEC>
-__global__ void __launch_bounds__(G == 32 ? 256 : G) norm_rows_kernel(const NormParams p) {
-  __shared__ float sred[32];
+__global__ void __launch_bounds__(G == 32 ? 256 : G, G == 32 ? 2 : 1) norm_rows_kernel(const NormParams p) {
+  __shared__ float sred[2][2][32];
   extern __shared__ float dw_smem[];   // RMS bwd with G == 32: (inner) floats, the CTA's dW partial
   constexpr int GROUPS = G == 32 ? 8 : 1;   // rows in flight per CTA
+  using Part = RowPart<G, MAXV, VEC>;
   const int g = threadIdx.x % G, grp = threadIdx.x / G;
   const int inner = p.inner;
   const float inv_n = 1.0f / (float)inner;
-  RowPart<G, MAXV, VEC> dw;
-  if (WHICH == 3) {
-#pragma unroll
-    for (int i = 0; i < MAXV; ++i)
-#pragma unroll
-      for (int j = 0; j < VEC; ++j) dw.v[i][j] = 0.f;
-  }
+  int turn = 0;
+  Part dw;
+  if (WHICH == 3) dw.each([](float& e, int, int) { e = 0.f; });
   // every group walks the same number of rows so that the CTA-wide barriers of G > 32 stay uniform
   for (int64_t row0 = (int64_t)blockIdx.x * GROUPS; row0 < p.rows; row0 += (int64_t)gridDim.x * GROUPS) {
     const int64_t row = row0 + grp;
     const bool live = row < p.rows;
     const int64_t off = (live ? row : 0) * inner;
-    RowPart<G, MAXV, VEC> x;
+    Part x;
     x.load(p.a + off, inner, g);
     if (WHICH == 0) {
       // mean, centred squares, stdev = sqrt(var + eps), y = (x - mean) / stdev   (layernorm.cu:296-330)
-      float s = 0.f;
+      float s[1] = {0.f}, q[1] = {0.f};
+      x.each([&](float& e, int, int) { s[0] += e; });
+      group_sum<G>(s, sred, turn);
+      const float mean = s[0] * inv_n;
 #pragma unroll
-      for (int i = 0; i < MAXV; ++i)
-#pragma unroll
-        for (int j = 0; j < VEC; ++j) s += x.v[i][j];
-      const float mean = group_sum<G>(s, sred) * inv_n;
-      float q = 0.f;
-#pragma unroll
-      for (int i = 0; i < MAXV; ++i)
+      for (int i = 0; i < MAXV; ++i) {
+        const bool in = (i * G + g) * VEC < inner;
 #pragma unroll
         for (int j = 0; j < VEC; ++j) {
-          const bool in = (i * G + g) * VEC + j < inner;
           x.v[i][j] = in ? x.v[i][j] - mean : 0.f;
-          q += x.v[i][j] * x.v[i][j];
+          q[0] = fmaf(x.v[i][j], x.v[i][j], q[0]);
         }
-      const float sd = sqrtf(group_sum<G>(q, sred) * inv_n + p.eps);
-#pragma unroll
-      for (int i = 0; i < MAXV; ++i)
-#pragma unroll
-        for (int j = 0; j < VEC; ++j) x.v[i][j] = x.v[i][j] / sd;
+      }
+      group_sum<G>(q, sred, turn);
+      const float sd = sqrtf(q[0] * inv_n + p.eps);
+      x.divide(sd);                    // |x - mean| <= sqrt(inner) stdev
       if (live) {
         x.store(p.out + off, inner, g);
         if (g == 0) p.stat_out[row] = sd;
@@ -138,46 +165,43 @@ __global__ void __launch_bounds__(G == 32 ? 256 : G) norm_rows_kernel(const Norm
       // dx = (dy - (y * mean(y*dy) + mean(dy))) / stdev   (layernorm.cu:345-381).  The reference adds eps
       // to the first `rows` ELEMENTS of its row-broadcast stdev tensor before the division
       // (add_scalar over outer*channels items of a count-sized buffer, :377): reproduced here.
-      RowPart<G, MAXV, VEC> dy;
+      Part dy;
       dy.load(p.b + off, inner, g);
-      float s1 = 0.f, s2 = 0.f;
-#pragma unroll
-      for (int i = 0; i < MAXV; ++i)
-#pragma unroll
-        for (int j = 0; j < VEC; ++j) { s1 = fmaf(x.v[i][j], dy.v[i][j], s1); s2 += dy.v[i][j]; }
-      const float m1 = group_sum<G>(s1, sred) * inv_n;
-      const float m2 = group_sum<G>(s2, sred) * inv_n;
       const float sd = p.stat[live ? row : 0];
+      float s[2] = {0.f, 0.f};
 #pragma unroll
       for (int i = 0; i < MAXV; ++i)
 #pragma unroll
-        for (int j = 0; j < VEC; ++j) {
-          const int64_t flat = off + (i * G + g) * VEC + j;
-          const float denom = flat < p.rows ? sd + p.eps : sd;
-          x.v[i][j] = (dy.v[i][j] - (x.v[i][j] * m1 + m2)) / denom;
-        }
+        for (int j = 0; j < VEC; ++j) { s[0] = fmaf(x.v[i][j], dy.v[i][j], s[0]); s[1] += dy.v[i][j]; }
+      group_sum<G>(s, sred, turn);
+      const float m1 = s[0] * inv_n, m2 = s[1] * inv_n;
+      float most = 0.f;
+      x.each([&](float& e, int i, int j) {
+        e = dy.v[i][j] - (e * m1 + m2);
+        most = fmaxf(most, fabsf(e));
+      });
+      if (off < p.rows || !(most < DIV_MAX)) {
+        x.each([&](float& e, int i, int j) {
+          const float denom = off + (i * G + g) * VEC + j < p.rows ? sd + p.eps : sd;
+          e = e / denom;
+        });
+      } else {
+        x.divide(sd);
+      }
       if (live) x.store(p.out + off, inner, g);
     } else if (WHICH == 2) {
       // rms = sqrt(mean(x^2) + eps); y = w * (x * (1 / rms))   (RMSNormLayer.cs:158-173)
-      float q = 0.f;
-#pragma unroll
-      for (int i = 0; i < MAXV; ++i)
-#pragma unroll
-        for (int j = 0; j < VEC; ++j) q = fmaf(x.v[i][j], x.v[i][j], q);
-      const float rms = sqrtf(group_sum<G>(q, sred) * inv_n + p.eps);
+      float q[1] = {0.f};
+      x.each([&](float& e, int, int) { q[0] = fmaf(e, e, q[0]); });
+      group_sum<G>(q, sred, turn);
+      const float rms = sqrtf(q[0] * inv_n + p.eps);
       const float inv = rms == 0.f ? 0.f : 1.0f / rms;   // invert_kernel maps 0 to 0, math.cu:6018-6024
       if (p.w != nullptr) {
-        RowPart<G, MAXV, VEC> w;
+        Part w;
         w.load(p.w, inner, g);
-#pragma unroll
-        for (int i = 0; i < MAXV; ++i)
-#pragma unroll
-          for (int j = 0; j < VEC; ++j) x.v[i][j] = w.v[i][j] * (x.v[i][j] * inv);
+        x.each([&](float& e, int i, int j) { e = w.v[i][j] * (e * inv); });
       } else {
-#pragma unroll
-        for (int i = 0; i < MAXV; ++i)
-#pragma unroll
-          for (int j = 0; j < VEC; ++j) x.v[i][j] = x.v[i][j] * inv;
+        x.each([&](float& e, int, int) { e = e * inv; });
       }
       if (live) {
         x.store(p.out + off, inner, g);
@@ -186,33 +210,25 @@ __global__ void __launch_bounds__(G == 32 ? 256 : G) norm_rows_kernel(const Norm
     } else {
       // g = dy * w; dW += dy * (x * inv); dx = g * inv - x * sum(g * x) * inv^3 / n   (RMSNormLayer.cs:194-229:
       // dinv = sum(g x), drms = -dinv / rms^2, dmean = drms / (2 rms), dx += 2 x dmean / n)
-      RowPart<G, MAXV, VEC> dy;
+      Part dy;
       dy.load(p.b + off, inner, g);
       const float inv = live ? p.stat[row] : 0.f;
       if (p.w != nullptr) {
-        RowPart<G, MAXV, VEC> w;
+        Part w;
         w.load(p.w, inner, g);
-#pragma unroll
-        for (int i = 0; i < MAXV; ++i)
-#pragma unroll
-          for (int j = 0; j < VEC; ++j) {
-            dw.v[i][j] = fmaf(dy.v[i][j], x.v[i][j] * inv, dw.v[i][j]);
-            dy.v[i][j] *= w.v[i][j];
-          }
+        dy.each([&](float& e, int i, int j) {
+          dw.v[i][j] = fmaf(e, x.v[i][j] * inv, dw.v[i][j]);
+          e *= w.v[i][j];
+        });
       }
-      float s = 0.f;
-#pragma unroll
-      for (int i = 0; i < MAXV; ++i)
-#pragma unroll
-        for (int j = 0; j < VEC; ++j) s = fmaf(dy.v[i][j], x.v[i][j], s);
-      const float dinv = group_sum<G>(s, sred);
+      float s[1] = {0.f};
+      dy.each([&](float& e, int i, int j) { s[0] = fmaf(e, x.v[i][j], s[0]); });
+      group_sum<G>(s, sred, turn);
+      const float dinv = s[0];
       const float drms = -dinv * (inv * inv);
       const float dmean = drms * (0.5f * inv);
       const float c = 2.0f * dmean * inv_n;
-#pragma unroll
-      for (int i = 0; i < MAXV; ++i)
-#pragma unroll
-        for (int j = 0; j < VEC; ++j) x.v[i][j] = fmaf(x.v[i][j], c, dy.v[i][j] * inv);
+      x.each([&](float& e, int i, int j) { e = fmaf(e, c, dy.v[i][j] * inv); });
       if (live) x.store(p.out + off, inner, g);
     }
   }
@@ -240,26 +256,41 @@ __global__ void __launch_bounds__(G == 32 ? 256 : G) norm_rows_kernel(const Norm
   }
 }
 
-// dW[e] = sum over the CTAs' partials, in CTA order
-__global__ void norm_dw_reduce_kernel(const float* __restrict__ partial, int n_partials, int inner, float* __restrict__ dw) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= inner) return;
+// dW[e] = sum over the CTAs' partials: eight warps of a CTA take every eighth of them for 32 columns, and their sums are added in
+// order (one thread a column walked all 296 of them: rows of 768, 38 us).
+constexpr int DW_WARPS = 8;
+__global__ void __launch_bounds__(DW_WARPS * 32) norm_dw_reduce_kernel(const float* __restrict__ partial, int n_partials, int inner, float* __restrict__ dw) {
+  __shared__ float part[DW_WARPS][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, e = blockIdx.x * 32 + lane;
   float s = 0.f;
-  for (int c = 0; c < n_partials; ++c) s += partial[(int64_t)c * inner + e];
-  dw[e] = s;
+  if (e < inner) {
+#pragma unroll 8
+    for (int c = warp; c < n_partials; c += DW_WARPS) s += partial[(int64_t)c * inner + e];
+  }
+  part[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0 && e < inner) {
+#pragma unroll
+    for (int w = 1; w < DW_WARPS; ++w) s += part[w][lane];
+    dw[e] = s;
+  }
 }
 
 struct Shape { int G, MAXV, VEC; };
 
-// the narrowest group that holds a row; vector loads need inner % 4 == 0 and 16-byte aligned tensors
+// the narrowest group that holds a row, and no more pieces a thread than it takes (a row of 768 as eight pieces of a warp instead of
+// six: registers for three CTAs an SM instead of five, and a quarter of the arithmetic on zeros); vector loads need
+// inner % 4 == 0 and 16-byte aligned tensors
 bool pick(int inner, bool aligned, Shape* s) {
+  auto pieces = [&](int G, int VEC) { return (inner + G * VEC - 1) / (G * VEC); };
   if (aligned && inner % 4 == 0) {
-    if (inner <= 32 * 8 * 4) { *s = {32, 8, 4}; return true; }
-    if (inner <= 256 * 4 * 4) { *s = {256, 4, 4}; return true; }
+    if (inner <= 32 * 8 * 4) { *s = {32, (pieces(32, 4) + 1) / 2 * 2, 4}; return true; }
+    if (inner <= 256 * 4 * 4) { *s = {256, pieces(256, 4) <= 2 ? 2 : 4, 4}; return true; }
     if (inner <= 1024 * 4 * 4) { *s = {1024, 4, 4}; return true; }
     return false;
   }
-  if (inner <= 32 * 16) { *s = {32, 16, 1}; return true; }
+  if (inner <= 32 * 16) { *s = {32, pieces(32, 1) <= 8 ? 8 : 16, 1}; return true; }
+  if (inner <= 256 * 16) { *s = {256, pieces(256, 1) <= 4 ? 4 : 16, 1}; return true; }
   if (inner <= 1024 * 16) { *s = {1024, 16, 1}; return true; }
   return false;
 }
@@ -280,11 +311,19 @@ int dispatch_norm(const NormParams& p, bool aligned, int grid_cap, cudaStream_t 
   Shape s;
   if (!pick(p.inner, aligned, &s)) return ERROR_ATTN_UNSUPPORTED_SHAPE;
   if (s.VEC == 4) {
-    if (s.G == 32) return launch_norm<WHICH, 32, 8, 4>(p, grid_cap, st);
-    if (s.G == 256) return launch_norm<WHICH, 256, 4, 4>(p, grid_cap, st);
+    if (s.G == 32) {
+      switch (s.MAXV) {
+        case 2: return launch_norm<WHICH, 32, 2, 4>(p, grid_cap, st);
+        case 4: return launch_norm<WHICH, 32, 4, 4>(p, grid_cap, st);
+        case 6: return launch_norm<WHICH, 32, 6, 4>(p, grid_cap, st);
+        default: return launch_norm<WHICH, 32, 8, 4>(p, grid_cap, st);
+      }
+    }
+    if (s.G == 256) return s.MAXV == 2 ? launch_norm<WHICH, 256, 2, 4>(p, grid_cap, st) : launch_norm<WHICH, 256, 4, 4>(p, grid_cap, st);
     return launch_norm<WHICH, 1024, 4, 4>(p, grid_cap, st);
   }
-  if (s.G == 32) return launch_norm<WHICH, 32, 16, 1>(p, grid_cap, st);
+  if (s.G == 32) return s.MAXV == 8 ? launch_norm<WHICH, 32, 8, 1>(p, grid_cap, st) : launch_norm<WHICH, 32, 16, 1>(p, grid_cap, st);
+  if (s.G == 256) return s.MAXV == 4 ? launch_norm<WHICH, 256, 4, 1>(p, grid_cap, st) : launch_norm<WHICH, 256, 16, 1>(p, grid_cap, st);
   return launch_norm<WHICH, 1024, 16, 1>(p, grid_cap, st);
 }
 
@@ -337,6 +376,6 @@ int mca_rmsnorm_backward_f32(const float* x, const float* w, const float* dy, co
   const int grid = (int)std::min<int64_t>((rows + groups - 1) / groups, NORM_MAX_PARTIALS);
   int e = dispatch_norm<3>(p, aligned, NORM_MAX_PARTIALS, (cudaStream_t)stream);
   if (e || dw == nullptr) return e;
-  norm_dw_reduce_kernel<<<mca_ceil_div(inner, 256), 256, 0, (cudaStream_t)stream>>>(scratch, grid, inner, dw);
+  norm_dw_reduce_kernel<<<mca_ceil_div(inner, 32), DW_WARPS * 32, 0, (cudaStream_t)stream>>>(scratch, grid, inner, dw);
   return mca_launch_status();
 }

@@ -110,6 +110,89 @@ def test_rmsnorm_backward_is_deterministic_and_many_rows(cuda):
         cuda.FreeMemory(m)
 
 
+# either side of every change of the kernels' shape: pieces of 128 floats a warp, of 1024 a CTA, and the unaligned ones
+EDGES = [4, 252, 256, 260, 512, 516, 768, 772, 1024, 1028, 2048, 2052, 4096, 4100, 1, 255, 257, 511, 513, 1023, 1025, 4095, 4097]
+
+
+def layernorm(cuda, x, dy, eps):
+    """y and dx of (rows, inner) through the function ids."""
+    rows, inner = x.shape
+    h = cuda.CreateLayerNorm(0, x.size, 1, rows, inner, eps)
+    m = [cuda.AllocMemory(v) for v in (x, x.size, dy, x.size)]
+    cuda.LayerNormForward(h, m[0], m[1])
+    cuda.LayerNormBackward(h, m[1], m[2], m[3])
+    out = [cuda.GetMemory(m[i], x.size).reshape(x.shape) for i in (1, 3)]
+    for v in m:
+        cuda.FreeMemory(v)
+    cuda.FreeLayerNorm(h)
+    return out
+
+
+@pytest.mark.parametrize("inner", EDGES)
+def test_rows_at_the_edges_of_the_shapes(cuda, inner):
+    rng = np.random.default_rng(inner)
+    rows, eps = 37, 1e-5
+    x = rng.standard_normal((1, rows, inner)).astype(np.float32)
+    dy = rng.standard_normal(x.shape).astype(np.float32)
+    w = (1 + 0.2 * rng.standard_normal(inner)).astype(np.float32)
+    y, dx = layernorm(cuda, x[0], dy[0], eps)
+    y_ref, sd = oracle.layernorm_forward(x, eps)
+    if inner > 1:      # one element: zero, and the backward a difference of equal numbers
+        assert rel_err(y, y_ref[0]) < 1e-5
+        assert rel_err(dx, oracle.layernorm_backward(y_ref, dy, sd, eps)[0]) < 1e-5
+    m = [cuda.AllocMemory(v) for v in (x, w, dy, x.size, x.size, rows, inner)]
+    cuda.RmsNormForward(m[0], m[1], m[3], m[5], rows, inner, eps)
+    cuda.RmsNormBackward(m[0], m[1], m[2], m[5], m[4], m[6], rows, inner)
+    y, dx, dw = cuda.GetMemory(m[3], x.size), cuda.GetMemory(m[4], x.size), cuda.GetMemory(m[6], inner)
+    dx_ref, dw_ref = oracle.rmsnorm_layer_backward(x, w, dy, eps)
+    assert rel_err(y, oracle.rmsnorm_layer_forward(x, w, eps)[0].ravel()) < 1e-5
+    # at one element dx = dy w (1 / rms - x^2 / rms^3): a thousandth to a hundred-thousandth of its terms
+    scale = np.abs(dx_ref).max() if inner > 1 else np.abs(dy * w / x).max()
+    assert np.abs(dx - dx_ref.ravel()).max() / scale < 1e-5
+    assert rel_err(dw, dw_ref) < 1e-5
+    for v in m:
+        cuda.FreeMemory(v)
+
+
+@pytest.mark.parametrize("inner", [300, 768, 771, 2048])
+def test_layernorm_quotients_are_those_of_a_division(cuda, inner):
+    """Forward: rows of small multiples of 2^-10 that cancel in pairs have the mean 0 without a rounding, so y is x / stdev as a
+    division rounds it.  Backward: dy times 2^70 takes the plain division instead of the reciprocal's quotients and changes nothing
+    else (every operation before it is exact under a power of two): the same bits, 2^70 larger."""
+    import torch
+    from mycaffe_b200 import _lib
+    rng = np.random.default_rng(inner)
+    rows = 64
+    half = rng.integers(-4096, 4097, (rows, inner // 2)).astype(np.float32) / 1024
+    x = np.concatenate([half, -half, np.zeros((rows, inner % 2), np.float32)], 1)
+    x = np.take(x, rng.permutation(inner), 1)
+    t = torch.from_numpy(x).cuda()
+    y, sd = torch.empty_like(t), torch.empty(rows, device="cuda")
+    assert _lib.load().mca_layernorm_forward_f32(t.data_ptr(), y.data_ptr(), sd.data_ptr(), rows, inner, 1e-5, None) == 0
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(y.cpu().numpy(), x / sd.cpu().numpy()[:, None])
+    dy = rng.standard_normal(x.shape).astype(np.float32)
+    big = np.float32(2.0) ** 70
+    np.testing.assert_array_equal(layernorm(cuda, x, dy, 1e-5)[1] * big, layernorm(cuda, x, dy * big, 1e-5)[1])
+
+
+def test_layernorm_of_rows_that_are_not_finite(cuda):
+    """An infinity makes its own row nan and leaves the others as they are; a row whose squares overflow has an infinite
+    deviation and is zero, as the division by it is."""
+    rng = np.random.default_rng(5)
+    x = rng.standard_normal((16, 768)).astype(np.float32)
+    dy = rng.standard_normal(x.shape).astype(np.float32)
+    y0, dx0 = layernorm(cuda, x, dy, 1e-5)
+    bad, bad_dy = x.copy(), dy.copy()
+    bad[14, 5] = np.inf
+    bad[13] *= np.float32(1e25)
+    bad_dy[15, 7] = np.inf
+    y, dx = layernorm(cuda, bad, bad_dy, 1e-5)
+    assert np.isnan(y[14]).all() and (y[13] == 0).all() and not np.isfinite(dx[15]).any()
+    np.testing.assert_array_equal(y[:13], y0[:13])
+    np.testing.assert_array_equal(dx[:13], dx0[:13])
+
+
 def test_raw_entry_points_reject_bad_arguments():
     from mycaffe_b200 import _lib, function_ids as ids
     lib = _lib.load()
