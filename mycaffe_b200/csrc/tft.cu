@@ -10,6 +10,7 @@
 // (tens of MB): the kernel is launch/latency bound, not roofline bound.
 #include "common.cuh"
 #include "kernels.h"
+#include "tft_rules.h"
 
 namespace {
 
@@ -175,8 +176,8 @@ __device__ __forceinline__ void cp_async_wait_all_but(int n) {
   else asm volatile("cp.async.wait_group 1;" ::: "memory");
 }
 
-template <int D>
-__global__ void __launch_bounds__(TFT_THREADS, 2) tft_fwd_tiled_kernel(const float* __restrict__ Q, const float* __restrict__ K,
+template <int D, bool SPREAD>
+__global__ void __launch_bounds__(TFT_THREADS, 2) tft_fwd_tiled_kernel(const int ch_, const float* __restrict__ Q, const float* __restrict__ K,
                                                                        const float* __restrict__ V,
                                                                        const float* __restrict__ mask, int H, int Nq, int Nk,
                                                                        float scale, float* __restrict__ out,
@@ -187,16 +188,22 @@ __global__ void __launch_bounds__(TFT_THREADS, 2) tft_fwd_tiled_kernel(const flo
   float* Kt = smem;                                  // two tiles
   float* Qs = Kt + 2 * tile;                         // two (24, D) blocks
   float* ex = Qs + 2 * TQ * D;                       // [2 (max | sum)][2 key halves][24 rows]
-  const int b = blockIdx.y, q0 = blockIdx.x * TQ;
+  const int ch = SPREAD ? ch_ : 1;
+  const int b = blockIdx.y, q0 = (int)blockIdx.x / ch * TQ;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int rows = min(TQ, Nq - q0);
+  // SPREAD: a cluster of ch CTAs shares the heads (CTA hr has heads hr, hr + ch, ...); the first of them puts the head sums
+  // together, in the CTAs' order, and has V
+  const int hr = SPREAD ? (int)blockIdx.x % ch : 0, hn = SPREAD ? (H - hr + ch - 1) / ch : H;
 
-  // tile t: K of head t (with that head's 24 query rows) or, for t == H, V; one commit group per call.  Query rows
+  // tile t: K of this CTA's head t (with that head's 24 query rows) or, for t == hn, V; one commit group per call.  Query rows
   // beyond Nq are zero-filled (a copy with source size 0).
   auto load_tile = [&](int t) {
-    if (t > H) return;
-    if (t < H) {
-      const float* src = Q + (((int64_t)b * H + t) * Nq + q0) * D;
+    if (t > hn) return;
+    if (SPREAD && t == hn && hr != 0) { asm volatile("cp.async.commit_group;" ::: "memory"); return; }
+    const int head = hr + t * ch;
+    if (t < hn) {
+      const float* src = Q + (((int64_t)b * H + head) * Nq + q0) * D;
       float* dst = Qs + (t & 1) * TQ * D;
       for (int idx = tid; idx < TQ * (D / 4); idx += TFT_THREADS) {
         const int r = idx / (D / 4);
@@ -205,7 +212,7 @@ __global__ void __launch_bounds__(TFT_THREADS, 2) tft_fwd_tiled_kernel(const flo
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sa), "l"(src + (r < rows ? idx * 4 : 0)), "r"(nbytes) : "memory");
       }
     }
-    tile_to_smem_async_swz<D>(Kt + (t & 1) * tile, t < H ? K + ((int64_t)b * H + t) * Nk * D : V + (int64_t)b * Nk * D, Nk, tid);
+    tile_to_smem_async_swz<D>(Kt + (t & 1) * tile, t < hn ? K + ((int64_t)b * H + head) * Nk * D : V + (int64_t)b * Nk * D, Nk, tid);
   };
   load_tile(0);
   load_tile(1);
@@ -241,8 +248,8 @@ __global__ void __launch_bounds__(TFT_THREADS, 2) tft_fwd_tiled_kernel(const flo
 #pragma unroll
     for (int c = 0; c < TQ_C; ++c) pmr[r][c] = 0.f;
 
-  for (int h = 0; h < H; ++h) {
-    cp_async_wait_all_but(h + 1 <= H ? 1 : 0);   // tile h has landed (tile h+1 may still be in flight)
+  for (int h = 0; h < hn; ++h) {
+    cp_async_wait_all_but(1);           // tile h has landed (tile h+1 may still be in flight)
     __syncthreads();                    // K_h and Q_h visible to all; everyone is past the previous head
     const float* Kh = Kt + (h & 1) * tile;
     float acc[TQ_R][TQ_C];
@@ -305,7 +312,7 @@ __global__ void __launch_bounds__(TFT_THREADS, 2) tft_fwd_tiled_kernel(const flo
     }
     __syncthreads();                    // half-maxima exchanged; every reader of K_h is done
     load_tile(h + 2);                   // into the buffers K_h and Q_h occupied
-    if (h + 2 > H) asm volatile("cp.async.commit_group;" ::: "memory");   // keep one group per iteration
+    if (h + 2 > hn) asm volatile("cp.async.commit_group;" ::: "memory");   // keep one group per iteration
     float hs[TQ_R];
 #pragma unroll
     for (int r = 0; r < TQ_R; ++r) {
@@ -334,7 +341,40 @@ __global__ void __launch_bounds__(TFT_THREADS, 2) tft_fwd_tiled_kernel(const flo
   }
   // mean probabilities: to global memory from the registers, and into the free K buffer for the product with V
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-  float* pm = Kt + ((H + 1) & 1) * tile;                  // V is tile H, in buffer H & 1
+  float* pm = Kt + ((hn + 1) & 1) * tile;                 // V is tile hn, in buffer hn & 1
+  if constexpr (SPREAD) {
+    // the peers leave their sums at the start of their dynamic shared memory (24 x 192 floats, a place per thread; the tiles there
+    // have been read behind the barrier), the first CTA adds them to its own
+    float* share = smem;
+    const bool first = hr == 0;
+    if (!first) {
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < TQ_R; ++r)
+#pragma unroll
+        for (int c = 0; c < TQ_C; ++c) share[(r * TQ_C + c) * TFT_THREADS + tid] = pmr[r][c];
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (first) {
+      const uint32_t at = (uint32_t)__cvta_generic_to_shared(share + tid);
+      for (int p = 1; p < ch; ++p) {
+        uint32_t peer;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(at), "r"((int)(blockIdx.x % ch) + p));
+        float o[TQ_R][TQ_C];
+#pragma unroll
+        for (int r = 0; r < TQ_R; ++r)
+#pragma unroll
+          for (int c = 0; c < TQ_C; ++c)
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(o[r][c]) : "r"(peer + (r * TQ_C + c) * TFT_THREADS * 4) : "memory");
+#pragma unroll
+        for (int r = 0; r < TQ_R; ++r)
+#pragma unroll
+          for (int c = 0; c < TQ_C; ++c) pmr[r][c] += o[r][c];
+      }
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (!first) return;
+  }
 #pragma unroll
   for (int r = 0; r < TQ_R; ++r)
 #pragma unroll
@@ -346,7 +386,7 @@ __global__ void __launch_bounds__(TFT_THREADS, 2) tft_fwd_tiled_kernel(const flo
       }
     }
   __syncthreads();                      // V in place, pm complete
-  const float* Vt = Kt + (H & 1) * tile;
+  const float* Vt = Kt + (hn & 1) * tile;
   // out = pm V.  A thread owns four columns of six rows (rq, rq + 4, ...) over a slice of the keys: per key one
   // 16-byte read of V and six (broadcast) reads of pm feed 24 FMAs.  The slices' partial sums meet in shared memory
   // behind pm (the buffer holds Nk x D floats, pm takes 24 x Nk of them).
@@ -521,6 +561,12 @@ __global__ void __launch_bounds__(TFT_THREADS) tft_bwd_kernel(const float* __res
 //      of dS per row, four of K); the slices' partial sums meet in shared memory;
 //   after the tile's last head, dV (+)= (sum_h P_h)^T dO / H, one product for all heads.
 // The 1/H of the head mean is applied to dP once and to dV.
+//
+// With fewer batch items than would fill the chip an item has a cluster of CTAs, ch of them along the heads and ct along the row
+// tiles (tft_bwd_split).  A CTA's heads and tiles are every ch-th and ct-th.  dQ, and dK of one tile, belong to one CTA; what
+// several have a part of keeps its order, so that results do not depend on timing: the ct CTAs that hold a head add their
+// parts of dK (and of dV) one after the other, a cluster barrier between two; the head sum of P is put together by the first CTA
+// of a tile from its peers' shared memory, in the heads' order by CTA.
 // smem: Vt[nk4][d] | Kt[2][nk4][d] (16-byte pieces swizzled by row; nk4 = Nk rounded up to 4, rows beyond Nk zero) |
 //       Qs[2][24][d] | Gs[2][24][d] | Ps[24][192] | Ss[24][192] | ex[6][24]
 // ---------------------------------------------------------------------------------------------
@@ -642,9 +688,9 @@ __global__ void __launch_bounds__(TFT_THREADS, 1) tft_bwd_tiled_kernel(const flo
   for (int it = 0; it < iters; ++it) {
     const int t = it / H, h = it - t * H, q0 = t * TQ, rows = min(TQ, Nq - q0);
     const bool fresh = h == 0;                        // new rows: mask bits and dP have to be formed, the head sum starts
-    load_iter(it + 1);                                // into the buffers iteration it - 1 read (it ended with a barrier)
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();                                  // this iteration's tiles visible; everyone is past the previous one
+    load_iter(it + 1);                                // into the buffers that iteration read, its dO for dV last of all
     const float* Kh = Kt + (it & 1) * tile;
     const float* Qh = Qs + (it & 1) * TQ * D;
     const float* Gh = Gs + (it & 1) * TQ * D;
@@ -899,6 +945,382 @@ __global__ void __launch_bounds__(TFT_THREADS, 1) tft_bwd_tiled_kernel(const flo
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
+// The same for a batch item that has a cluster of CTAs (see above).  A kernel of its own: as an instantiation of one source the
+// compiler's schedule of the single-CTA form is 4-14 % slower (99 items, 8 heads, Nq 130, Nk 142, d 64: 500 -> 570 us).
+template <int D>
+__global__ void __launch_bounds__(TFT_THREADS, 1) tft_bwd_spread_kernel(const int ch, const int ct,
+                                                                       const float* __restrict__ Q, const float* __restrict__ K,
+                                                                       const float* __restrict__ V,
+                                                                       const float* __restrict__ mask,
+                                                                       const float* __restrict__ d_out,
+                                                                       const float* __restrict__ d_attn, int H, int Nq, int Nk,
+                                                                       float scale, float* __restrict__ dQ,
+                                                                       float* __restrict__ dK, float* __restrict__ dV) {
+  extern __shared__ __align__(16) float smem[];
+  constexpr int D4 = D / 4, SW = D4 >= 8 ? 7 : D4 - 1;
+  constexpr int NV = D / 16;                          // 16-byte column pieces of a thread's dK / dV tile
+  constexpr int RPT = D == 64 ? 6 : 3;                // phase D: rows per thread,
+  constexpr int RQ = TQ / RPT;                        //   row classes (a thread's rows are rq, rq + RQ, ...)
+  constexpr int SLOTS = TFT_THREADS / (D4 * RQ);      //   key slices
+  static_assert((SLOTS - 1) * TQ * D <= TQ * TQ_KEYS, "the partial sums of dQ must fit the buffer of P");
+  const int nk4 = (Nk + 3) & ~3;
+  const size_t tile = (size_t)nk4 * D;
+  float* Vt = smem;
+  float* Kt = Vt + tile;                              // two tiles
+  float* Qs = Kt + 2 * tile;                          // two (24, D) blocks
+  float* Gs = Qs + 2 * TQ * D;                        // two (24, D) blocks of the output gradient
+  float* Ps = Gs + 2 * TQ * D;                        // (24, 192) probabilities; later the partial sums of dQ
+  float* Ss = Ps + TQ * TQ_KEYS;                      // (24, 192) dS
+  float* ex = Ss + TQ * TQ_KEYS;                      // [max | sum | dot][2 key halves][24 rows]
+  const int b = blockIdx.y;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int tiles = (Nq + TQ - 1) / TQ;
+  // this CTA's place in the cluster, and its iterations: (row tile tr + ct i, head hr + ch k) for every i and k the cluster needs;
+  // what lies beyond the last tile or head is gone through without work (the barriers are everybody's)
+  const int hr = (int)blockIdx.x % ch, tr = (int)blockIdx.x / ch;
+  const int hn = (H + ch - 1) / ch, tn = (tiles + ct - 1) / ct, iters = hn * tn;
+  const float inv_h = 1.f / (float)H;
+  auto cluster_barrier = [] { asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory"); };
+
+  // what iteration `it` = (row tile, head) reads; one commit group per call, empty beyond the last iteration
+  auto load_iter = [&](int it) {
+    const int t = tr + ct * (it / hn), h = hr + ch * (it % hn);
+    if (it < iters && t < tiles && h < H) {
+      const int q0 = t * TQ, rows = min(TQ, Nq - q0);
+      rows24_async<D>(Qs + (it & 1) * TQ * D, Q + (((int64_t)b * H + h) * Nq + q0) * D, rows, tid);
+      rows24_async<D>(Gs + (it & 1) * TQ * D, d_out + ((int64_t)b * Nq + q0) * D, rows, tid);
+      tile_rows_async_swz<D>(Kt + (it & 1) * tile, K + ((int64_t)b * H + h) * Nk * D, Nk, tid);
+    }
+    if (it == 0) tile_rows_async_swz<D>(Vt, V + (int64_t)b * Nk * D, Nk, tid);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  load_iter(0);
+  // phase D reads K four rows at a time: the rows between Nk and nk4 are never copied, they must be zero
+  for (int idx = tid; idx < (nk4 - Nk) * D; idx += TFT_THREADS) {
+    Kt[(size_t)Nk * D + idx] = 0.f;
+    Kt[tile + (size_t)Nk * D + idx] = 0.f;
+  }
+
+  const int rg = w & 3, khalf = w >> 2;               // phases A, B: rows rg*6 .. +5, keys khalf*96 + lane + 32c
+  const int kg = tid >> 2, cg = tid & 3;              // phase C: keys kg + 64c, 16-byte column pieces cg, cg + 4, ...
+  const int c4 = tid % D4, rq = (tid / D4) % RQ, ks = tid / (D4 * RQ);   // phase D
+  const int n4 = nk4 / 4, per4 = (n4 + SLOTS - 1) / SLOTS;
+  const int jq0 = ks * per4, jq1 = min(n4, jq0 + per4);
+
+  float dk[TQ_C][NV * 4];
+#pragma unroll
+  for (int c = 0; c < TQ_C; ++c)
+#pragma unroll
+    for (int x = 0; x < NV * 4; ++x) dk[c][x] = 0.f;
+  float dp[TQ_R][TQ_C];
+  float pm[TQ_R][TQ_C];                               // the sum over the heads of this thread's probabilities (one row tile)
+  unsigned mbits = 0, dead = 0;
+
+  for (int it = 0; it < iters; ++it) {
+    const int ti = it / hn, hi = it - ti * hn, t = tr + ct * ti, h = hr + ch * hi, q0 = t * TQ, rows = min(TQ, Nq - q0);
+    const bool fresh = hi == 0;                       // new rows: mask bits and dP have to be formed, the head sum starts
+    const bool mine = t < tiles && h < H;                // (uniform over the CTA)
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                                  // this iteration's tiles visible; everyone is past the previous one
+    load_iter(it + 1);                                // into the buffers that iteration read
+    const float* Kh = Kt + (it & 1) * tile;
+    const float* Qh = Qs + (it & 1) * TQ * D;
+    const float* Gh = Gs + (it & 1) * TQ * D;
+    if (mine) {
+
+    // ---- A: scores and dP
+    float da[TQ_R][TQ_C];
+    if (fresh) {
+      float mv[TQ_R][TQ_C];
+#pragma unroll
+      for (int r = 0; r < TQ_R; ++r)
+#pragma unroll
+        for (int c = 0; c < TQ_C; ++c) {
+          const int i = min(rg * TQ_R + r, rows - 1), j = min(khalf * (32 * TQ_C) + lane + 32 * c, Nk - 1);
+          mv[r][c] = mask != nullptr ? __ldg(mask + (int64_t)(q0 + i) * Nk + j) : 0.f;
+          da[r][c] = d_attn != nullptr ? __ldg(d_attn + ((int64_t)b * Nq + q0 + i) * Nk + j) : 0.f;
+        }
+      mbits = dead = 0;
+#pragma unroll
+      for (int r = 0; r < TQ_R; ++r)
+#pragma unroll
+        for (int c = 0; c < TQ_C; ++c) {
+          const int i = rg * TQ_R + r, j = khalf * (32 * TQ_C) + lane + 32 * c;
+          if (j >= Nk) dead |= 1u << (r * TQ_C + c);
+          else if (i < rows && mv[r][c] == 1.0f) mbits |= 1u << (r * TQ_C + c);
+          if (i >= rows || j >= Nk) da[r][c] = 0.f;
+          dp[r][c] = 0.f;
+          pm[r][c] = 0.f;
+        }
+    }
+    float s[TQ_R][TQ_C];
+#pragma unroll
+    for (int r = 0; r < TQ_R; ++r)
+#pragma unroll
+      for (int c = 0; c < TQ_C; ++c) s[r][c] = 0.f;
+    {
+      const float* krow[TQ_C];
+      const float* vrow[TQ_C];
+      int ksw[TQ_C];
+#pragma unroll
+      for (int c = 0; c < TQ_C; ++c) {
+        const int j = min(khalf * (32 * TQ_C) + lane + 32 * c, Nk - 1);
+        krow[c] = Kh + (size_t)j * D;
+        vrow[c] = Vt + (size_t)j * D;
+        ksw[c] = j & SW;
+      }
+      if (fresh) {
+        tft_bwd_scores<D, true>(krow, vrow, ksw, Qh + rg * TQ_R * D, Gh + rg * TQ_R * D, s, dp);
+#pragma unroll
+        for (int r = 0; r < TQ_R; ++r)
+#pragma unroll
+          for (int c = 0; c < TQ_C; ++c) dp[r][c] = (dp[r][c] + da[r][c]) * inv_h;   // both head-mean terms (:797-812)
+      } else {
+        tft_bwd_scores<D, false>(krow, vrow, ksw, Qh + rg * TQ_R * D, Gh + rg * TQ_R * D, s, dp);
+      }
+    }
+
+    // ---- B: softmax and its backward
+    float hm[TQ_R];
+#pragma unroll
+    for (int r = 0; r < TQ_R; ++r) {
+      float m = -INFINITY;
+#pragma unroll
+      for (int c = 0; c < TQ_C; ++c) {
+        const unsigned bit = 1u << (r * TQ_C + c);
+        s[r][c] = (mbits & bit) ? MCA_MASKED_LOGIT : s[r][c] * scale;
+        if (!(dead & bit)) m = fmaxf(m, s[r][c]);
+      }
+      hm[r] = warp_max(m);
+    }
+    if (lane < TQ_R) {
+      float v = hm[0];
+#pragma unroll
+      for (int r = 1; r < TQ_R; ++r) v = lane == r ? hm[r] : v;
+      ex[khalf * TQ + rg * TQ_R + lane] = v;
+    }
+    __syncthreads();
+    float hs[TQ_R], hd[TQ_R];
+#pragma unroll
+    for (int r = 0; r < TQ_R; ++r) {
+      const float m = fmaxf(ex[rg * TQ_R + r], ex[TQ + rg * TQ_R + r]);
+      float sum = 0.f, dot = 0.f;
+#pragma unroll
+      for (int c = 0; c < TQ_C; ++c) {
+        s[r][c] = (dead & (1u << (r * TQ_C + c))) ? 0.f : tft_exp(s[r][c] - m);
+        sum += s[r][c];
+        dot = fmaf(s[r][c], dp[r][c], dot);
+      }
+      hs[r] = warp_sum(sum);
+      hd[r] = warp_sum(dot);
+    }
+    if (lane < TQ_R) {
+      float v = hs[0], u = hd[0];
+#pragma unroll
+      for (int r = 1; r < TQ_R; ++r) {
+        v = lane == r ? hs[r] : v;
+        u = lane == r ? hd[r] : u;
+      }
+      ex[2 * TQ + khalf * TQ + rg * TQ_R + lane] = v;
+      ex[4 * TQ + khalf * TQ + rg * TQ_R + lane] = u;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < TQ_R; ++r) {
+      const int i = rg * TQ_R + r;
+      const float inv = 1.f / (ex[2 * TQ + i] + ex[3 * TQ + i]);
+      const float dot = (ex[4 * TQ + i] + ex[5 * TQ + i]) * inv;      // sum_j P dP of the row
+#pragma unroll
+      for (int c = 0; c < TQ_C; ++c) {
+        const int j = khalf * (32 * TQ_C) + lane + 32 * c;
+        const float pj = s[r][c] * inv;
+        pm[r][c] += pj;
+        Ss[i * TQ_KEYS + j] = pj * (dp[r][c] - dot) * scale;          // softmax backward, then the 1/sqrt(d) (:822-831)
+      }
+    }
+    __syncthreads();                                  // P and dS complete
+
+    // ---- C: dK_h (this tile's part) = dS^T Q_h
+#pragma unroll 2
+    for (int r = 0; r < TQ; ++r) {
+      float sv[TQ_C];
+      float4 qv[NV];
+#pragma unroll
+      for (int c = 0; c < TQ_C; ++c) sv[c] = Ss[r * TQ_KEYS + kg + 64 * c];
+#pragma unroll
+      for (int x = 0; x < NV; ++x)
+        qv[x] = *reinterpret_cast<const float4*>(Qh + r * D + 4 * (cg + 4 * x));   // the four lanes of a key: distinct banks
+#pragma unroll
+      for (int c = 0; c < TQ_C; ++c)
+#pragma unroll
+        for (int x = 0; x < NV; ++x) {
+          dk[c][4 * x + 0] = fmaf(sv[c], qv[x].x, dk[c][4 * x + 0]);
+          dk[c][4 * x + 1] = fmaf(sv[c], qv[x].y, dk[c][4 * x + 1]);
+          dk[c][4 * x + 2] = fmaf(sv[c], qv[x].z, dk[c][4 * x + 2]);
+          dk[c][4 * x + 3] = fmaf(sv[c], qv[x].w, dk[c][4 * x + 3]);
+        }
+    }
+
+    // ---- D: dQ = dS K_h over this thread's slice of the keys
+    float o[RPT][4];
+#pragma unroll
+    for (int r = 0; r < RPT; ++r) o[r][0] = o[r][1] = o[r][2] = o[r][3] = 0.f;
+    for (int jq = jq0; jq < jq1; ++jq) {
+      const int j = 4 * jq;
+      float4 kv[4], sv[RPT];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) kv[u] = *reinterpret_cast<const float4*>(Kh + (size_t)(j + u) * D + ((c4 ^ ((j + u) & SW)) << 2));
+#pragma unroll
+      for (int r = 0; r < RPT; ++r) sv[r] = *reinterpret_cast<const float4*>(Ss + (rq + RQ * r) * TQ_KEYS + j);
+#pragma unroll
+      for (int r = 0; r < RPT; ++r) {
+        o[r][0] = fmaf(sv[r].x, kv[0].x, o[r][0]); o[r][1] = fmaf(sv[r].x, kv[0].y, o[r][1]);
+        o[r][2] = fmaf(sv[r].x, kv[0].z, o[r][2]); o[r][3] = fmaf(sv[r].x, kv[0].w, o[r][3]);
+      }
+#pragma unroll
+      for (int r = 0; r < RPT; ++r) {
+        o[r][0] = fmaf(sv[r].y, kv[1].x, o[r][0]); o[r][1] = fmaf(sv[r].y, kv[1].y, o[r][1]);
+        o[r][2] = fmaf(sv[r].y, kv[1].z, o[r][2]); o[r][3] = fmaf(sv[r].y, kv[1].w, o[r][3]);
+      }
+#pragma unroll
+      for (int r = 0; r < RPT; ++r) {
+        o[r][0] = fmaf(sv[r].z, kv[2].x, o[r][0]); o[r][1] = fmaf(sv[r].z, kv[2].y, o[r][1]);
+        o[r][2] = fmaf(sv[r].z, kv[2].z, o[r][2]); o[r][3] = fmaf(sv[r].z, kv[2].w, o[r][3]);
+      }
+#pragma unroll
+      for (int r = 0; r < RPT; ++r) {
+        o[r][0] = fmaf(sv[r].w, kv[3].x, o[r][0]); o[r][1] = fmaf(sv[r].w, kv[3].y, o[r][1]);
+        o[r][2] = fmaf(sv[r].w, kv[3].z, o[r][2]); o[r][3] = fmaf(sv[r].w, kv[3].w, o[r][3]);
+      }
+    }
+    __syncthreads();                                  // the buffer of the head sum now takes the partial sums of dQ
+    if (ks > 0) {
+#pragma unroll
+      for (int r = 0; r < RPT; ++r)
+        *reinterpret_cast<float4*>(Ps + (size_t)(ks - 1) * TQ * D + (rq + RQ * r) * D + c4 * 4) = make_float4(o[r][0], o[r][1], o[r][2], o[r][3]);
+    }
+    __syncthreads();
+    if (ks == 0) {
+#pragma unroll
+      for (int r = 0; r < RPT; ++r) {
+        const int i = rq + RQ * r;
+        float4 a = make_float4(o[r][0], o[r][1], o[r][2], o[r][3]);
+#pragma unroll
+        for (int s2 = 0; s2 < SLOTS - 1; ++s2) {
+          const float4 p4 = *reinterpret_cast<const float4*>(Ps + (size_t)s2 * TQ * D + i * D + c4 * 4);
+          a.x += p4.x; a.y += p4.y; a.z += p4.z; a.w += p4.w;
+        }
+        if (i < rows) *reinterpret_cast<float4*>(dQ + (((int64_t)b * H + h) * Nq + q0 + i) * D + c4 * 4) = a;
+      }
+    }
+    }
+    // Element (row kg + 64 c, column piece cg + 4 x) of dst: the first tile writes, later ones add (a fixed order).
+    auto add_piece = [&](float* dst, int c, int x, const float (&v)[NV * 4], float f) {
+      float4* g = reinterpret_cast<float4*>(dst + (int64_t)(kg + 64 * c) * D + 4 * (cg + 4 * x));
+      float4 acc4 = make_float4(v[4 * x] * f, v[4 * x + 1] * f, v[4 * x + 2] * f, v[4 * x + 3] * f);
+      if (t > 0) { const float4 old = __ldcg(g); acc4.x += old.x; acc4.y += old.y; acc4.z += old.z; acc4.w += old.w; }
+      *g = acc4;
+    };
+    // this tile's part of dK_h leaves the registers, the CTAs that hold this head one after the other
+    for (int turn = 0; turn < ct; ++turn) {
+      if (mine && turn == tr) {
+#pragma unroll
+        for (int c = 0; c < TQ_C; ++c) {
+          const int j = kg + 64 * c;
+#pragma unroll
+          for (int x = 0; x < NV; ++x) {
+            if (j < Nk) add_piece(dK + ((int64_t)b * H + h) * Nk * D, c, x, dk[c], 1.f);
+            dk[c][4 * x] = dk[c][4 * x + 1] = dk[c][4 * x + 2] = dk[c][4 * x + 3] = 0.f;
+          }
+        }
+      }
+      if (ct > 1) cluster_barrier();
+    }
+    if (hi == hn - 1) {
+      // the tile's last head: V's gradient is (sum_h P_h)^T dO / H, one product for all heads (the rows of dO are
+      // those of this iteration's buffer: a tile's first CTA has a head in the last round)
+      if (ch == 1) __syncthreads();                   // the partial sums of dQ have been read
+      else cluster_barrier();                         // (and so have the peers')
+      if (t < tiles) {
+#pragma unroll
+        for (int r = 0; r < TQ_R; ++r)
+#pragma unroll
+          for (int c = 0; c < TQ_C; ++c) Ps[(rg * TQ_R + r) * TQ_KEYS + khalf * (32 * TQ_C) + lane + 32 * c] = pm[r][c];
+      }
+      if (ch == 1) __syncthreads();
+      else cluster_barrier();
+      float dv[TQ_C][NV * 4];
+      const bool forms = t < tiles && hr == 0;   // the tile's first CTA
+      if (forms) {
+        if (ch > 1) {
+          // the peers' head sums onto this CTA's own; each thread its own elements
+          const uint32_t own = (uint32_t)__cvta_generic_to_shared(Ps);
+          for (int idx = tid * 4; idx < TQ * TQ_KEYS; idx += TFT_THREADS * 4) {
+            float4 a = *reinterpret_cast<const float4*>(Ps + idx);
+            for (int p = 1; p < min(ch, H); ++p) {
+              uint32_t at;
+              float4 o4;
+              asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(own + idx * 4), "r"(tr * ch + p));
+              asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(o4.x), "=f"(o4.y), "=f"(o4.z), "=f"(o4.w) : "r"(at) : "memory");
+              a.x += o4.x; a.y += o4.y; a.z += o4.z; a.w += o4.w;
+            }
+            *reinterpret_cast<float4*>(Ps + idx) = a;
+          }
+          __syncthreads();
+        }
+#pragma unroll
+        for (int c = 0; c < TQ_C; ++c)
+#pragma unroll
+          for (int x = 0; x < NV * 4; ++x) dv[c][x] = 0.f;
+#pragma unroll 2
+        for (int r = 0; r < TQ; ++r) {
+          float pv[TQ_C];
+          float4 gv[NV];
+#pragma unroll
+          for (int c = 0; c < TQ_C; ++c) pv[c] = Ps[r * TQ_KEYS + kg + 64 * c];
+#pragma unroll
+          for (int x = 0; x < NV; ++x) gv[x] = *reinterpret_cast<const float4*>(Gh + r * D + 4 * (cg + 4 * x));
+#pragma unroll
+          for (int c = 0; c < TQ_C; ++c)
+#pragma unroll
+            for (int x = 0; x < NV; ++x) {
+              dv[c][4 * x + 0] = fmaf(pv[c], gv[x].x, dv[c][4 * x + 0]);
+              dv[c][4 * x + 1] = fmaf(pv[c], gv[x].y, dv[c][4 * x + 1]);
+              dv[c][4 * x + 2] = fmaf(pv[c], gv[x].z, dv[c][4 * x + 2]);
+              dv[c][4 * x + 3] = fmaf(pv[c], gv[x].w, dv[c][4 * x + 3]);
+            }
+        }
+      }
+      for (int turn = 0; turn < ct; ++turn) {
+        if (forms && turn == tr) {
+#pragma unroll
+          for (int c = 0; c < TQ_C; ++c) {
+            if (kg + 64 * c < Nk) {
+#pragma unroll
+              for (int x = 0; x < NV; ++x) add_piece(dV + (int64_t)b * Nk * D, c, x, dv[c], inv_h);
+            }
+          }
+        }
+        if (ct > 1) cluster_barrier();
+      }
+      if (ch > 1 && ct == 1) cluster_barrier();   // the peers' Ps have been read
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+template <typename... KArgs, typename... Args>
+int launch_clusters(void (*kern)(KArgs...), int ctas, dim3 grid, size_t smem, cudaStream_t st, Args... args) {   // along x
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = dim3(TFT_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)ctas; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  MCA_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, KArgs(args)...));
+  return mca_launch_status();
+}
+
 }  // namespace
 
 int mca_tft_attention_backward_f32(const float* q, const float* k, const float* v, const float* mask,
@@ -911,13 +1333,20 @@ int mca_tft_attention_backward_f32(const float* q, const float* k, const float* 
   // the tiled kernel where the shape fits it, else the generic one
   const auto aligned = [](const void* p_) { return (reinterpret_cast<uintptr_t>(p_) & 15) == 0; };
   if ((d == 16 || d == 32 || d == 64) && Nk <= TQ_KEYS && aligned(q) && aligned(d_out) && aligned(dq) && aligned(dk) && aligned(dv)) {
+    const tft_rules::Split split = tft_rules::backward_split(B, H, mca_ceil_div(Nq, TQ));
     const size_t nk4 = ((size_t)Nk + 3) & ~(size_t)3;
     const size_t smem_t = sizeof(float) * (3 * nk4 * d + 4 * (size_t)TQ * d + 2 * (size_t)TQ * TQ_KEYS + 6 * TQ);
     const float sc = 1.0f / sqrtf((float)d);
     cudaStream_t st = (cudaStream_t)stream;
 #define MCA_TFT_BWD_TILED(D_)                                                                                                 \
-    MCA_CUDA_TRY(cudaFuncSetAttribute(tft_bwd_tiled_kernel<D_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t)); \
-    tft_bwd_tiled_kernel<D_><<<B, TFT_THREADS, smem_t, st>>>(q, k, v, mask, d_out, d_attn, H, Nq, Nk, sc, dq, dk, dv);
+    if (split.ch * split.ct == 1) {                                                                                          \
+      MCA_CUDA_TRY(cudaFuncSetAttribute(tft_bwd_tiled_kernel<D_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t)); \
+      tft_bwd_tiled_kernel<D_><<<B, TFT_THREADS, smem_t, st>>>(q, k, v, mask, d_out, d_attn, H, Nq, Nk, sc, dq, dk, dv); \
+    } else {                                                                                                                  \
+      MCA_CUDA_TRY(cudaFuncSetAttribute(tft_bwd_spread_kernel<D_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t)); \
+      return launch_clusters(tft_bwd_spread_kernel<D_>, split.ch * split.ct, dim3(split.ch * split.ct, B), smem_t, st, split.ch, split.ct, \
+                             q, k, v, mask, d_out, d_attn, H, Nq, Nk, sc, dq, dk, dv);                                        \
+    }
     if (d == 64) { MCA_TFT_BWD_TILED(64) } else if (d == 32) { MCA_TFT_BWD_TILED(32) } else { MCA_TFT_BWD_TILED(16) }
 #undef MCA_TFT_BWD_TILED
     return mca_launch_status();
@@ -946,9 +1375,15 @@ int mca_tft_attention_forward_f32(const float* q, const float* k, const float* v
     dim3 grid_t(mca_ceil_div(Nq, TQ), B);
     const float sc = 1.0f / sqrtf((float)d);
     cudaStream_t st = (cudaStream_t)stream;
+    const int ch = smem_t >= sizeof(float) * TQ * TQ_KEYS ? tft_rules::forward_split((int64_t)B * grid_t.x, H) : 1;
 #define MCA_TFT_TILED(D_)                                                                                                 \
-    MCA_CUDA_TRY(cudaFuncSetAttribute(tft_fwd_tiled_kernel<D_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t)); \
-    tft_fwd_tiled_kernel<D_><<<grid_t, TFT_THREADS, smem_t, st>>>(q, k, v, mask, H, Nq, Nk, sc, out, attn);
+    if (ch == 1) {                                                                                                        \
+      MCA_CUDA_TRY(cudaFuncSetAttribute(tft_fwd_tiled_kernel<D_, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t)); \
+      tft_fwd_tiled_kernel<D_, false><<<grid_t, TFT_THREADS, smem_t, st>>>(1, q, k, v, mask, H, Nq, Nk, sc, out, attn);   \
+    } else {                                                                                                              \
+      MCA_CUDA_TRY(cudaFuncSetAttribute(tft_fwd_tiled_kernel<D_, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t)); \
+      return launch_clusters(tft_fwd_tiled_kernel<D_, true>, ch, dim3(grid_t.x * ch, B), smem_t, st, ch, q, k, v, mask, H, Nq, Nk, sc, out, attn); \
+    }
     if (d == 64) { MCA_TFT_TILED(64) } else if (d == 32) { MCA_TFT_TILED(32) } else { MCA_TFT_TILED(16) }
 #undef MCA_TFT_TILED
     return mca_launch_status();

@@ -1,0 +1,39 @@
+// Choices of the TFT attention that depend on sizes alone (plain C++, so that they can be tested without a GPU).
+#pragma once
+#include <cstdint>
+
+namespace tft_rules {
+
+struct Split {
+  int ch, ct;      // CTAs of a batch item's cluster along the heads and along the row tiles
+};
+
+// Clusters of `ctas` CTAs that the chip holds at once, with one CTA per SM (cudaOccupancyMaxActiveClusters of the kernel).
+inline int resident_clusters(int ctas) { return ctas == 1 ? 148 : ctas == 2 ? 74 : ctas == 4 ? 33 : 15; }
+
+// How the backward of a batch item is spread.  In units of one product over a row tile and a head's keys: a CTA forms three for each
+// of its (tile, head) pairs, dP once a tile, and dV; a cluster barrier and what is added between two of them is about a
+// third of one; the weights are fitted to forward and backward of twelve shapes (us, all the splits measured, the best taken by
+// each): 24 items, 4 heads, 185 x 185, d 64 425 -> 226; 16, 8, 160 x 160, 32 481 -> 206; 48, 8, 27 x 132, 64 206 -> 143; 64, 4, 24 x 192, 64
+// 81 -> 64; 73, 1, 173 x 173, 32 144 -> 119; 256, 4, 24 x 192, 64 146 whole, 175 in two, 222 in four.
+inline Split backward_split(int B, int H, int tiles) {
+  Split best{1, 1};
+  double best_cost = 1e30;
+  for (int ch = 1; ch <= 8 && ch <= H; ch *= 2)
+    for (int ct = 1; ch * ct <= 8 && ct <= tiles; ct *= 2) {
+      const int hn = (H + ch - 1) / ch, tn = (tiles + ct - 1) / ct, c = ch * ct;
+      const int64_t rounds = (B + resident_clusters(c) - 1) / resident_clusters(c);
+      const double cost = rounds * (1.0 + tn * (3.0 * hn + 2.0 + (ct > 1 ? 0.6 * ct * (hn + 1) : 0.0) + (ch > 1 ? 0.7 + 0.1 * ch : 0.0)));
+      if (cost < best_cost * 0.97) { best_cost = cost; best = Split{ch, ct}; }
+    }
+  return best;
+}
+
+// Into how many CTAs the forward of a row tile's heads goes: while the tiles are fewer than the chip holds, two to an SM.
+inline int forward_split(int64_t tiles, int H) {
+  int ch = 1;
+  while (ch < 8 && 2 * ch <= H && 2 * ch * tiles <= 2 * 2 * resident_clusters(2)) ch *= 2;
+  return ch;
+}
+
+}  // namespace tft_rules

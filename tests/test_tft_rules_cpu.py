@@ -1,0 +1,36 @@
+"""How the TFT attention of few batch items is spread (csrc/tft_rules.h)."""
+import subprocess
+from pathlib import Path
+
+CSRC = Path(__file__).resolve().parent.parent / "mycaffe_b200" / "csrc"
+
+PROGRAM = r'''
+#include "tft_rules.h"
+#include <cstdio>
+using namespace tft_rules;
+static int bad = 0;
+static void claim(bool ok, const char* what, int B, int H, int tiles) { if (!ok) { std::printf("%s: B %d H %d tiles %d\n", what, B, H, tiles); bad = 1; } }
+static void is(int B, int H, int tiles, int ch, int ct) { const Split s = backward_split(B, H, tiles); claim(s.ch == ch && s.ct == ct, "choice", B, H, tiles); }
+int main() {
+  for (int B = 1; B <= 300; ++B)
+    for (int H = 1; H <= 20; ++H)
+      for (int tiles = 1; tiles <= 12; ++tiles) {
+        const Split s = backward_split(B, H, tiles);
+        claim(s.ch >= 1 && s.ct >= 1 && s.ch * s.ct <= 8 && s.ch <= H && s.ct <= tiles, "range", B, H, tiles);
+        const int f = forward_split((int64_t)B * tiles, H);
+        claim(f >= 1 && f <= 8 && f <= H && (f == 1 || (int64_t)f * B * tiles <= 296), "forward", B, H, tiles);
+      }
+  // as measured
+  is(256, 4, 1, 1, 1); is(128, 4, 1, 1, 1); is(99, 8, 6, 1, 1); is(78, 4, 8, 1, 1); is(64, 4, 1, 2, 1); is(24, 4, 8, 2, 2);
+  is(48, 8, 2, 2, 1); is(73, 1, 8, 1, 2); is(16, 8, 7, 4, 1); is(200, 8, 5, 2, 1); is(40, 1, 4, 1, 2); is(24, 2, 1, 2, 1);
+  return bad;
+}
+'''
+
+
+def test_the_spread_of_an_item_fits_a_cluster_and_is_the_measured_one(tmp_path):
+    (tmp_path / "main.cpp").write_text(PROGRAM)
+    exe = str(tmp_path / "main")
+    subprocess.run(["g++", "-std=c++17", "-Wall", "-Werror", "-I", str(CSRC), str(tmp_path / "main.cpp"), "-o", exe], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout

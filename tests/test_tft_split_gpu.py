@@ -1,0 +1,45 @@
+"""TFT attention with few batch items: the heads and row tiles of an item over a cluster of CTAs, against the fp64 oracle at the
+bound of the unsplit kernels (the same sums, the head sums and the tiles' parts in another fixed order)."""
+import numpy as np
+import pytest
+
+import oracle
+from helpers import rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def cuda():
+    from mycaffe_b200 import CudaDnn
+    c = CudaDnn(0)
+    yield c
+    c.Dispose()
+
+
+# heads that are no multiple of the CTAs along them, row tiles likewise, a last tile of one row, every head size, one head, one tile
+@pytest.mark.parametrize("with_attn_grad", [False, True])
+@pytest.mark.parametrize("B,H,Nq,Nk,d", [(2, 8, 24, 60, 32), (3, 4, 60, 60, 16), (2, 1, 100, 100, 64), (2, 5, 50, 70, 32), (1, 3, 49, 191, 64),
+                                         (16, 8, 160, 160, 32), (2, 7, 25, 33, 64), (40, 2, 73, 90, 16), (33, 6, 24, 192, 64)])
+def test_split_over_a_cluster(cuda, B, H, Nq, Nk, d, with_attn_grad):
+    rng = np.random.default_rng(B * 100 + H + Nq)
+    q = rng.standard_normal((B, H, Nq, d)).astype(np.float32)
+    k = rng.standard_normal((B, H, Nk, d)).astype(np.float32)
+    v = rng.standard_normal((B, Nk, d)).astype(np.float32)
+    mask = (np.arange(Nk)[None, :] > np.arange(Nq)[:, None] + Nk - Nq).astype(np.float32)
+    d_out = rng.standard_normal((B, Nq, d)).astype(np.float32)
+    d_attn = rng.standard_normal((B, Nq, Nk)).astype(np.float32) if with_attn_grad else None
+    h = [cuda.AllocMemory(a) for a in (q, k, v, mask, d_out)] + [cuda.AllocMemory(d_attn) if with_attn_grad else 0]
+    o = [cuda.AllocMemory(n) for n in (B * Nq * d, B * Nq * Nk, q.size, k.size, v.size)]
+    got = []
+    for _ in range(2):
+        cuda.TftAttnForward(h[0], h[1], h[2], h[3], B, H, Nq, Nk, d, o[0], o[1])
+        cuda.TftAttnBackward(h[0], h[1], h[2], h[3], h[4], h[5], B, H, Nq, Nk, d, o[2], o[3], o[4])
+        got.append([cuda.GetMemory(m, n) for m, n in zip(o, (B * Nq * d, B * Nq * Nk, q.size, k.size, v.size))])
+    ref = [*oracle.tft_forward(q, k, v, mask, f64=True), *oracle.tft_backward(q, k, v, mask, d_out, d_attn, f64=True)]
+    for a, b, r in zip(*got, ref):
+        assert rel_err(a, np.ravel(r)) < 2e-5
+        np.testing.assert_array_equal(a, b)          # whichever CTA came first
+    for m in h + o:
+        if m:
+            cuda.FreeMemory(m)
