@@ -51,13 +51,18 @@ __device__ __forceinline__ void group_sum(float (&v)[N], float (*sred)[2][32], i
 // a / b from r, the reciprocal of b as a division gives it: the quotient a r put right by its own remainder, which a fused
 // multiply-add forms exactly (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
 // Dev. 34, 1990: correctly rounded but for a b whose significand is all ones).  A division per element was a third of these kernels'
-// instructions.  For b within 2^-60 .. 2^60 and |a| <= 2^60 (or sqrt(inner) b), so that nothing on the way overflows.
-constexpr float DIV_MAX = 1.152921504606847e18f;   // 2^60
+// instructions.  The remainder is q b - a, not a - q b: a zero one then leaves the sign of a zero quotient as it is.
+// For b within 2^-60 .. 2^24 and a zero or |a| within 2^-100 .. 2^60 (or up to sqrt(inner) b): nothing overflows, the quotient is
+// normal (>= 2^-125) and the remainder, a multiple of the product of two last places (>= 2^-148), is held exactly.  Of smaller
+// numerators it is rounded, and at 2^-124 one quotient in twenty is not the division's.
+constexpr float DIV_A_MIN = 7.888609052210118e-31f, DIV_A_MAX = 1.152921504606847e18f;   // 2^-100, 2^60
+constexpr float DIV_B_MIN = 8.673617379884035e-19f, DIV_B_MAX = 16777216.f;              // 2^-60, 2^24
+// Orders magnitudes, zero above them all (two integer instructions an element for the smallest that is not zero).
+__device__ __forceinline__ unsigned above_zero(float a) { return 2u * __float_as_uint(a) - 1u; }
 __device__ __forceinline__ float div_by(float a, float b, float r) {
   const float q = a * r;
-  return fmaf(fmaf(-q, b, a), r, q);
+  return fmaf(fmaf(q, b, -a), -r, q);
 }
-__device__ __forceinline__ bool div_ok(float b) { return b >= 1.f / DIV_MAX && b <= DIV_MAX; }
 
 // The part of a row one thread holds: MAXV pieces of VEC floats, piece i at element (i*G + g)*VEC.
 template <int G, int MAXV, int VEC>
@@ -96,8 +101,9 @@ struct RowPart {
 #pragma unroll
       for (int j = 0; j < VEC; ++j) f(v[i][j], i, j);
   }
-  __device__ __forceinline__ void divide(float b) {
-    if (div_ok(b)) {
+  // least: the smallest above_zero of the elements
+  __device__ __forceinline__ void divide(float b, unsigned least) {
+    if (b >= DIV_B_MIN && b <= DIV_B_MAX && least >= above_zero(DIV_A_MIN)) {
       const float r = 1.f / b;
       each([&](float& e, int, int) { e = div_by(e, b, r); });
     } else {
@@ -145,18 +151,20 @@ __global__ void __launch_bounds__(G == 32 ? 256 : G, G == 32 ? 2 : 1) norm_rows_
       x.each([&](float& e, int, int) { s[0] += e; });
       group_sum<G>(s, sred, turn);
       const float mean = s[0] * inv_n;
+      unsigned least = ~0u;
 #pragma unroll
       for (int i = 0; i < MAXV; ++i) {
         const bool in = (i * G + g) * VEC < inner;
 #pragma unroll
         for (int j = 0; j < VEC; ++j) {
           x.v[i][j] = in ? x.v[i][j] - mean : 0.f;
+          least = min(least, above_zero(x.v[i][j]));
           q[0] = fmaf(x.v[i][j], x.v[i][j], q[0]);
         }
       }
       group_sum<G>(q, sred, turn);
       const float sd = sqrtf(q[0] * inv_n + p.eps);
-      x.divide(sd);                    // |x - mean| <= sqrt(inner) stdev
+      x.divide(sd, least);             // |x - mean| <= sqrt(inner) stdev
       if (live) {
         x.store(p.out + off, inner, g);
         if (g == 0) p.stat_out[row] = sd;
@@ -176,17 +184,19 @@ __global__ void __launch_bounds__(G == 32 ? 256 : G, G == 32 ? 2 : 1) norm_rows_
       group_sum<G>(s, sred, turn);
       const float m1 = s[0] * inv_n, m2 = s[1] * inv_n;
       float most = 0.f;
+      unsigned least = ~0u;
       x.each([&](float& e, int i, int j) {
         e = dy.v[i][j] - (e * m1 + m2);
         most = fmaxf(most, fabsf(e));
+        least = min(least, above_zero(e));
       });
-      if (off < p.rows || !(most < DIV_MAX)) {
+      if (off < p.rows || !(most < DIV_A_MAX)) {
         x.each([&](float& e, int i, int j) {
           const float denom = off + (i * G + g) * VEC + j < p.rows ? sd + p.eps : sd;
           e = e / denom;
         });
       } else {
-        x.divide(sd);
+        x.divide(sd, least);
       }
       if (live) x.store(p.out + off, inner, g);
     } else if (WHICH == 2) {

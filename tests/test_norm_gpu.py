@@ -176,6 +176,35 @@ def test_layernorm_quotients_are_those_of_a_division(cuda, inner):
     np.testing.assert_array_equal(layernorm(cuda, x, dy, 1e-5)[1] * big, layernorm(cuda, x, dy * big, 1e-5)[1])
 
 
+@pytest.mark.parametrize("inner", [300, 768, 771, 2048])
+def test_layernorm_quotients_of_vanishing_numbers(cuda, inner):
+    """Rows of small integers times 2^-80 .. 2^-143 and zeros of both signs: every sum is exact and the means are zero, so both
+    directions are the one division, also where the remainder of a quotient is too small for a subnormal number."""
+    import torch
+    from mycaffe_b200 import _lib
+    rng = np.random.default_rng(inner)
+    rows, eps = 64, 1e-5
+    unit = np.ldexp(np.float32(1), -80 - np.arange(rows))[:, None].astype(np.float32)
+    half = rng.integers(-64, 65, (rows, inner // 2)).astype(np.float32)
+    order, tail = rng.permutation(inner), np.zeros((rows, inner % 2), np.float32)
+    x = np.take(np.concatenate([half * unit, -half * unit, tail], 1), order, 1)
+    y = np.take(np.concatenate([rng.integers(-64, 65, half.shape).astype(np.float32)] * 2 + [tail], 1), order, 1)
+    assert np.signbit(x[x == 0]).any() and not np.signbit(x[x == 0]).all()
+    lib = _lib.load()
+    tx, ty = torch.from_numpy(x).cuda(), torch.from_numpy(y).cuda()
+    out, sd = torch.empty_like(tx), torch.empty(rows, device="cuda")
+    assert lib.mca_layernorm_forward_f32(tx.data_ptr(), out.data_ptr(), sd.data_ptr(), rows, inner, eps, None) == 0
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(out.cpu().numpy().view(np.int32), (x / sd.cpu().numpy()[:, None]).view(np.int32))
+    sd = rng.uniform(0.25, 4, rows).astype(np.float32)   # the halves of x cancel, those of y are equal: m1 = m2 = 0
+    tsd = torch.from_numpy(sd).cuda()
+    assert lib.mca_layernorm_backward_f32(ty.data_ptr(), tx.data_ptr(), tsd.data_ptr(), out.data_ptr(), rows, inner, eps, None) == 0
+    torch.cuda.synchronize()
+    denom = np.repeat(sd[:, None], inner, 1)
+    denom.ravel()[:rows] += np.float32(eps)              # the first `rows` elements, as the reference divides them
+    np.testing.assert_array_equal(out.cpu().numpy().view(np.int32), (x / denom).view(np.int32))
+
+
 def test_layernorm_of_rows_that_are_not_finite(cuda):
     """An infinity makes its own row nan and leaves the others as they are; a row whose squares overflow has an infinite
     deviation and is zero, as the division by it is."""
