@@ -15,8 +15,8 @@
 namespace {
 
 constexpr int TFT_ROWS = 8;        // query rows per CTA, one per warp
-constexpr int TFT_THREADS = 256;
-constexpr int TFT_TQ_ROWS = 24;   // query rows of a tile of the tiled kernels
+constexpr int TFT_THREADS = tft_rules::TILE_THREADS;
+constexpr int TFT_TQ_ROWS = tft_rules::TILE_ROWS;   // query rows of a tile of the tiled kernels
 
 // e^x for x <= 0 as one multiply and one ex2.approx (2 ulp): the softmax of the tiled kernels.  Arguments far below
 // the fp32 range (a masked logit against a real maximum) give exactly 0.
@@ -141,6 +141,7 @@ constexpr int TQ = TFT_TQ_ROWS;    // query rows per CTA
 constexpr int TQ_R = 6;            // rows of a register tile
 constexpr int TQ_C = 3;            // keys per lane of a register tile (32 lanes: 96 keys per warp)
 constexpr int TQ_KEYS = 2 * 32 * TQ_C;   // keys a CTA covers: 192
+static_assert(TQ_KEYS == tft_rules::TILE_KEYS);
 
 // (Nk, D) tile -> shared memory rows of exactly D floats; the 16-byte pieces of row j are stored at piece ^ (j & SW), so
 // that lanes reading the same piece of consecutive rows hit different banks without padding the rows.
@@ -1366,12 +1367,9 @@ int mca_tft_attention_forward_f32(const float* q, const float* k, const float* v
   if (B <= 0 || H <= 0 || Nq <= 0 || Nk <= 0 || d <= 0 || B > 65535) return ERROR_PARAM_OUT_OF_RANGE;
   if (d % 4 != 0 || (reinterpret_cast<uintptr_t>(k) & 15) || (reinterpret_cast<uintptr_t>(v) & 15))
     return ERROR_ATTN_UNSUPPORTED_SHAPE;
-  // the tiled kernel where the shape fits it (two K buffers and two CTAs per SM), else the generic one
-  const size_t smem_t = sizeof(float) * (2 * (size_t)Nk * d + 2 * (size_t)TQ * d + 4 * TQ);
-  const int slices = TFT_THREADS / d;   // key slices of the final product: TFT_THREADS / ((d / 4) * 4)
-  // a K buffer must also hold the mean probabilities (24 x Nk) and the partial outputs of the other slices
-  const bool room = (size_t)TQ * Nk + (size_t)(slices - 1) * TQ * d <= (size_t)Nk * d;
-  if ((d == 16 || d == 32 || d == 64) && Nk <= TQ_KEYS && smem_t <= 113 * 1024 && room && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+  // the tiled kernel where the call fits it, else the generic one
+  if (tft_rules::forward_tiled(Nk, d, q, out)) {
+    const size_t smem_t = tft_rules::forward_tiled_smem(Nk, d);
     dim3 grid_t(mca_ceil_div(Nq, TQ), B);
     const float sc = 1.0f / sqrtf((float)d);
     cudaStream_t st = (cudaStream_t)stream;

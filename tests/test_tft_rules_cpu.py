@@ -1,4 +1,4 @@
-"""How the TFT attention of few batch items is spread (csrc/tft_rules.h)."""
+"""Which kernel a TFT attention call takes and how few batch items are spread (csrc/tft_rules.h)."""
 import subprocess
 from pathlib import Path
 
@@ -23,6 +23,10 @@ int main() {
   // as measured
   is(256, 4, 1, 1, 1); is(128, 4, 1, 1, 1); is(99, 8, 6, 1, 1); is(78, 4, 8, 1, 1); is(64, 4, 1, 2, 1); is(24, 4, 8, 2, 2);
   is(48, 8, 2, 2, 1); is(73, 1, 8, 1, 2); is(16, 8, 7, 4, 1); is(200, 8, 5, 2, 1); is(40, 1, 4, 1, 2); is(24, 2, 1, 2, 1);
+  // the tiled forward copies Q and writes the output by 16 bytes: never from or to an address that is not a multiple of them
+  alignas(16) static float at[8];
+  claim(forward_tiled(192, 64, at, at + 4), "tiled", 0, 0, 192);
+  for (int o = 1; o < 4; ++o) claim(!forward_tiled(192, 64, at + o, at) && !forward_tiled(192, 64, at, at + o), "alignment", o, 0, 192);
   return bad;
 }
 '''
