@@ -1310,6 +1310,15 @@ __global__ void __launch_bounds__(TFT_THREADS, 1) tft_bwd_spread_kernel(const in
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
+// A kernel's shared-memory limit is set once, to what a CTA may have: one set to each call's own size could be lowered by another
+// thread's smaller call before this call's launch, which is then refused.
+constexpr size_t SMEM_MAX = 227 * 1024;
+template <auto KERN>
+int smem_limit() {
+  static std::atomic<uint64_t> done{0};
+  return mca_smem_once(done, KERN, SMEM_MAX);
+}
+
 template <typename... KArgs, typename... Args>
 int launch_clusters(void (*kern)(KArgs...), int ctas, dim3 grid, size_t smem, cudaStream_t st, Args... args) {   // along x
   cudaLaunchConfig_t cfg = {};
@@ -1341,10 +1350,10 @@ int mca_tft_attention_backward_f32(const float* q, const float* k, const float* 
     cudaStream_t st = (cudaStream_t)stream;
 #define MCA_TFT_BWD_TILED(D_)                                                                                                 \
     if (split.ch * split.ct == 1) {                                                                                          \
-      MCA_CUDA_TRY(cudaFuncSetAttribute(tft_bwd_tiled_kernel<D_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t)); \
+      if (const int e = smem_limit<tft_bwd_tiled_kernel<D_>>()) return e;                                                    \
       tft_bwd_tiled_kernel<D_><<<B, TFT_THREADS, smem_t, st>>>(q, k, v, mask, d_out, d_attn, H, Nq, Nk, sc, dq, dk, dv); \
     } else {                                                                                                                  \
-      MCA_CUDA_TRY(cudaFuncSetAttribute(tft_bwd_spread_kernel<D_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t)); \
+      if (const int e = smem_limit<tft_bwd_spread_kernel<D_>>()) return e;                                                   \
       return launch_clusters(tft_bwd_spread_kernel<D_>, split.ch * split.ct, dim3(split.ch * split.ct, B), smem_t, st, split.ch, split.ct, \
                              q, k, v, mask, d_out, d_attn, H, Nq, Nk, sc, dq, dk, dv);                                        \
     }
@@ -1354,8 +1363,8 @@ int mca_tft_attention_backward_f32(const float* q, const float* k, const float* 
   }
   const size_t smem = sizeof(float) * (2 * (size_t)Nk * (d + 4) + 2 * (size_t)Nk * d + 2 * (size_t)TFT_ROWS * Nk +
                                        2 * (size_t)TFT_ROWS * d);
-  if (smem > 227 * 1024) return ERROR_ATTN_UNSUPPORTED_SHAPE;
-  MCA_CUDA_TRY(cudaFuncSetAttribute(tft_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > SMEM_MAX) return ERROR_ATTN_UNSUPPORTED_SHAPE;
+  if (const int e = smem_limit<tft_bwd_kernel>()) return e;
   tft_bwd_kernel<<<B, TFT_THREADS, smem, (cudaStream_t)stream>>>(q, k, v, mask, d_out, d_attn, H, Nq, Nk, d,
                                                                   1.0f / sqrtf((float)d), dq, dk, dv);
   return mca_launch_status();
@@ -1376,10 +1385,10 @@ int mca_tft_attention_forward_f32(const float* q, const float* k, const float* v
     const int ch = smem_t >= sizeof(float) * TQ * TQ_KEYS ? tft_rules::forward_split((int64_t)B * grid_t.x, H) : 1;
 #define MCA_TFT_TILED(D_)                                                                                                 \
     if (ch == 1) {                                                                                                        \
-      MCA_CUDA_TRY(cudaFuncSetAttribute(tft_fwd_tiled_kernel<D_, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t)); \
+      if (const int e = smem_limit<tft_fwd_tiled_kernel<D_, false>>()) return e;                                         \
       tft_fwd_tiled_kernel<D_, false><<<grid_t, TFT_THREADS, smem_t, st>>>(1, q, k, v, mask, H, Nq, Nk, sc, out, attn);   \
     } else {                                                                                                              \
-      MCA_CUDA_TRY(cudaFuncSetAttribute(tft_fwd_tiled_kernel<D_, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t)); \
+      if (const int e = smem_limit<tft_fwd_tiled_kernel<D_, true>>()) return e;                                          \
       return launch_clusters(tft_fwd_tiled_kernel<D_, true>, ch, dim3(grid_t.x * ch, B), smem_t, st, ch, q, k, v, mask, H, Nq, Nk, sc, out, attn); \
     }
     if (d == 64) { MCA_TFT_TILED(64) } else if (d == 32) { MCA_TFT_TILED(32) } else { MCA_TFT_TILED(16) }
@@ -1387,8 +1396,8 @@ int mca_tft_attention_forward_f32(const float* q, const float* k, const float* v
     return mca_launch_status();
   }
   const size_t smem = sizeof(float) * ((size_t)Nk * (d + 4) + (size_t)H * TFT_ROWS * d + 2 * (size_t)TFT_ROWS * Nk);
-  if (smem > 227 * 1024) return ERROR_ATTN_UNSUPPORTED_SHAPE;
-  MCA_CUDA_TRY(cudaFuncSetAttribute(tft_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > SMEM_MAX) return ERROR_ATTN_UNSUPPORTED_SHAPE;
+  if (const int e = smem_limit<tft_fwd_kernel>()) return e;
   dim3 grid(mca_ceil_div(Nq, TFT_ROWS), B);
   tft_fwd_kernel<<<grid, TFT_THREADS, smem, (cudaStream_t)stream>>>(q, k, v, mask, H, Nq, Nk, d,
                                                                     1.0f / sqrtf((float)d), out, attn);

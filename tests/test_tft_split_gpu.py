@@ -1,5 +1,8 @@
 """TFT attention with few batch items: the heads and row tiles of an item over a cluster of CTAs, against the fp64 oracle at the
 bound of the unsplit kernels (the same sums, the head sums and the tiles' parts in another fixed order)."""
+import ctypes as C
+import subprocess
+
 import numpy as np
 import pytest
 
@@ -64,3 +67,65 @@ def test_queries_without_16_byte_alignment(cuda, B, H, Nq, Nk):
                                                          attn.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
         assert rel_err(out.cpu().numpy(), np.ravel(ref[0])) < 2e-5
         assert rel_err(attn.cpu().numpy(), np.ravel(ref[1])) < 2e-5
+
+
+HAMMER = r"""
+#include <thread>
+#include <vector>
+using Fwd = int (*)(void*, void*, void*, void*, int, int, int, int, int, void*, void*, void*);
+using Bwd = int (*)(void*, void*, void*, void*, void*, void*, int, int, int, int, int, void*, void*, void*, void*);
+struct Call { void* p[10]; int n[5]; int error; };   // q k v d_out | out attn dq dk dv | stream;  B H Nq Nk d
+extern "C" void hammer(Fwd fwd, Bwd bwd, Call* calls, int n_calls, int rounds) {
+  std::vector<std::thread> threads;
+  for (int i = 0; i < n_calls; ++i)
+    threads.emplace_back([=] {
+      Call& c = calls[i];
+      void* const* p = c.p;
+      const int* n = c.n;
+      for (int r = 0; r < rounds && c.error == 0; ++r) {
+        c.error = fwd(p[0], p[1], p[2], nullptr, n[0], n[1], n[2], n[3], n[4], p[4], p[5], p[9]);
+        if (c.error == 0) c.error = bwd(p[0], p[1], p[2], nullptr, p[3], nullptr, n[0], n[1], n[2], n[3], n[4], p[6], p[7], p[8], p[9]);
+      }
+    });
+  for (auto& t : threads) t.join();
+}
+"""
+
+
+class Call(C.Structure):
+    _fields_ = [("p", C.c_void_p * 10), ("n", C.c_int * 5), ("error", C.c_int)]
+
+
+def test_threads_with_different_sizes(cuda, tmp_path):
+    """Host threads that call the C entry points on streams of their own, some with long key rows and some with short ones: every launch
+    is accepted and every result is the one of the calls made alone."""
+    import torch
+    from mycaffe_b200 import _lib
+    (tmp_path / "hammer.cpp").write_text(HAMMER)
+    so = str(tmp_path / "hammer.so")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-pthread", str(tmp_path / "hammer.cpp"), "-o", so], check=True)
+    lib, hammer = _lib.load(), C.CDLL(so).hammer
+    hammer.restype = None
+    fwd, bwd = (C.cast(f, C.c_void_p) for f in (lib.mca_tft_attention_forward_f32, lib.mca_tft_attention_backward_f32))
+    B, H, Nq = 2, 2, 30
+    shapes = [(192, 64), (117, 64), (40, 32), (190, 32)]          # tiled and generic forwards, long and short rows of each
+    calls, outputs, keep = (Call * len(shapes))(), [], []
+    for call, (Nk, d) in zip(calls, shapes):
+        g = torch.Generator(device="cuda").manual_seed(Nk)
+        ins = [torch.randn(s, generator=g, device="cuda") for s in ((B, H, Nq, d), (B, H, Nk, d), (B, Nk, d), (B, Nq, d))]
+        outs = [torch.empty(s, device="cuda") for s in ((B, Nq, d), (B, Nq, Nk), (B, H, Nq, d), (B, H, Nk, d), (B, Nk, d))]
+        keep.append((ins, torch.cuda.Stream()))
+        outputs.append(outs)
+        call.p[:] = [t.data_ptr() for t in ins + outs] + [keep[-1][1].cuda_stream]
+        call.n[:] = [B, H, Nq, Nk, d]
+    torch.cuda.synchronize()
+    alone = []
+    for i, outs in enumerate(outputs):
+        hammer(fwd, bwd, C.byref(calls[i]), 1, 1)
+        torch.cuda.synchronize()
+        alone.append([t.clone() for t in outs])
+    hammer(fwd, bwd, calls, len(shapes), 3000)
+    torch.cuda.synchronize()
+    assert [c.error for c in calls] == [0] * len(shapes)
+    for outs, want in zip(outputs, alone):
+        assert all(torch.equal(a, b) for a, b in zip(outs, want))
