@@ -1,5 +1,8 @@
 """Decode steps of one to nine sequences: the padded passes of the streaming projections (3, 5, 6 and 7 sequences), rows that are
 or are not shared by warps, splits with and without a combine pass, against the restated step over several tokens."""
+import ctypes as C
+import subprocess
+
 import numpy as np
 import pytest
 
@@ -33,3 +36,50 @@ def test_steps_match_the_restated_model(B, dim, hidden, n_heads, n_kv, seq):
         ref = oracle.llama_forward(cfg, w, kc, vc, list(tok), list(pos + step))
         assert rel_err(t.forward_batch(tok, pos + step), ref) < 1e-4
     assert rel_err(t.key_cache.cpu().numpy(), kc) < 1e-5   # the appended rows, and nothing else
+
+
+HAMMER = r"""
+#include <thread>
+#include <vector>
+using Fn = int (*)(void*, void*, int, int, int, void*, void*);
+struct Call { void *x, *w, *out, *stream; int B, dim, error; };
+extern "C" void hammer(Fn fn, Call* calls, int n_calls, int rounds) {
+  std::vector<std::thread> threads;
+  for (int i = 0; i < n_calls; ++i)
+    threads.emplace_back([=] {
+      Call& c = calls[i];
+      for (int r = 0; r < rounds && c.error == 0; ++r) c.error = fn(c.x, c.w, 0, c.B, c.dim, c.out, c.stream);
+    });
+  for (auto& t : threads) t.join();
+}
+"""
+
+
+class Call(C.Structure):
+    _fields_ = [(n, C.c_void_p) for n in ("x", "w", "out", "stream")] + [(n, C.c_int) for n in ("B", "dim", "error")]
+
+
+@pytest.mark.parametrize("B", [1, 2, 4, 8])
+def test_threads_with_rows_of_different_lengths(B, tmp_path):
+    """Host threads whose projections read rows of different lengths through the same kernels, on streams of their own: every launch is
+    accepted."""
+    import torch
+    from mycaffe_b200 import _lib
+    (tmp_path / "hammer.cpp").write_text(HAMMER)
+    so = str(tmp_path / "hammer.so")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-pthread", str(tmp_path / "hammer.cpp"), "-o", so], check=True)
+    hammer = C.CDLL(so).hammer
+    hammer.restype = None
+    rounds, keep, calls = 3000, [], (Call * 4)()
+    for call, dim in zip(calls, (256, 1536, 512, 1024)):
+        w, x, out = torch.zeros(dim, dim, device="cuda"), torch.ones(B, dim, device="cuda"), torch.zeros(B, dim, device="cuda")
+        w[:, 3] = 1
+        stream = torch.cuda.Stream()
+        keep.append((w, x, out, stream))
+        call.x, call.w, call.out, call.stream, call.B, call.dim = x.data_ptr(), w.data_ptr(), out.data_ptr(), stream.cuda_stream, B, dim
+    torch.cuda.synchronize()
+    hammer(C.cast(_lib.load().mca_decode_out_proj, C.c_void_p), calls, len(calls), rounds)
+    torch.cuda.synchronize()
+    assert [c.error for c in calls] == [0] * len(calls)
+    for _, _, out, _ in keep:
+        assert bool((out == rounds).all())
