@@ -42,10 +42,12 @@ inline Split backward_split(int B, int H, int tiles) {
   return best;
 }
 
-// Into how many CTAs the forward of a row tile's heads goes: while the tiles are fewer than the chip holds, two to an SM.
+// Into how many CTAs the forward of a row tile's heads goes: as long as every tile's cluster is resident at once, with an SM to each
+// CTA.  Two CTAs on an SM take nearly twice as long, and their cluster's exchange comes on top (us, whole / over two: 128 tiles, 4 heads, 192 keys
+// 23.1 / 25.2; 3 heads 19.8 / 25.1; 74 tiles, 4 heads 23.0 / 16.9; over four 25.0).
 inline int forward_split(int64_t tiles, int H) {
   int ch = 1;
-  while (ch < 8 && 2 * ch <= H && 2 * ch * tiles <= 2 * 2 * resident_clusters(2)) ch *= 2;
+  while (ch < 8 && 2 * ch <= H && tiles <= resident_clusters(2 * ch)) ch *= 2;
   return ch;
 }
 

@@ -23,6 +23,11 @@ int main() {
   // as measured
   is(256, 4, 1, 1, 1); is(128, 4, 1, 1, 1); is(99, 8, 6, 1, 1); is(78, 4, 8, 1, 1); is(64, 4, 1, 2, 1); is(24, 4, 8, 2, 2);
   is(48, 8, 2, 2, 1); is(73, 1, 8, 1, 2); is(16, 8, 7, 4, 1); is(200, 8, 5, 2, 1); is(40, 1, 4, 1, 2); is(24, 2, 1, 2, 1);
+  // the forward: never two CTAs of clusters on an SM; as measured
+  for (int tiles = 1; tiles <= 400; ++tiles)
+    for (int H = 1; H <= 20; ++H) claim(forward_split(tiles, H) == 1 || forward_split(tiles, H) * tiles <= 148, "one CTA to an SM", 0, H, tiles);
+  claim(forward_split(128, 4) == 1 && forward_split(128, 3) == 1 && forward_split(80, 2) == 1 && forward_split(74, 4) == 2 && forward_split(50, 4) == 2 &&
+        forward_split(33, 6) == 4 && forward_split(16, 8) == 4 && forward_split(15, 8) == 8 && forward_split(8, 1) == 1, "forward choice", 0, 0, 0);
   // the tiled forward copies Q and writes the output by 16 bytes: never from or to an address that is not a multiple of them
   alignas(16) static float at[8];
   claim(forward_tiled(192, 64, at, at + 4), "tiled", 0, 0, 192);
