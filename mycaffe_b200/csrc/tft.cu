@@ -1343,7 +1343,7 @@ int mca_tft_attention_backward_f32(const float* q, const float* k, const float* 
   // the tiled kernel where the shape fits it, else the generic one
   const auto aligned = [](const void* p_) { return (reinterpret_cast<uintptr_t>(p_) & 15) == 0; };
   if ((d == 16 || d == 32 || d == 64) && Nk <= TQ_KEYS && aligned(q) && aligned(d_out) && aligned(dq) && aligned(dk) && aligned(dv)) {
-    const tft_rules::Split split = tft_rules::backward_split(B, H, mca_ceil_div(Nq, TQ));
+    const tft_rules::Split split = tft_rules::backward_split(B, H, mca_ceil_div(Nq, TQ), d);
     const size_t nk4 = ((size_t)Nk + 3) & ~(size_t)3;
     const size_t smem_t = sizeof(float) * (3 * nk4 * d + 4 * (size_t)TQ * d + 2 * (size_t)TQ * TQ_KEYS + 6 * TQ);
     const float sc = 1.0f / sqrtf((float)d);

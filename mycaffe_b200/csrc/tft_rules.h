@@ -28,15 +28,18 @@ inline int resident_clusters(int ctas) { return ctas == 1 ? 148 : ctas == 2 ? 74
 // of its (tile, head) pairs, dP once a tile, and dV; a cluster barrier and what is added between two of them is about a
 // third of one; the weights are fitted to forward and backward of twelve shapes (us, all the splits measured, the best taken by
 // each): 24 items, 4 heads, 185 x 185, d 64 425 -> 226; 16, 8, 160 x 160, 32 481 -> 206; 48, 8, 27 x 132, 64 206 -> 143; 64, 4, 24 x 192, 64
-// 81 -> 64; 73, 1, 173 x 173, 32 144 -> 119; 256, 4, 24 x 192, 64 146 whole, 175 in two, 222 in four.
-inline Split backward_split(int B, int H, int tiles) {
+// 81 -> 64; 73, 1, 173 x 173, 32 144 -> 119; 256, 4, 24 x 192, 64 146 whole, 175 in two, 222 in four.  Clusters that do not fit the chip at
+// once cost a twentieth more than their rounds say, with 16-wide heads, whose barriers weigh more, a tenth (the backward alone, us, 2 rounds
+// of whole items / 3 of two CTAs: 150 items, 4 heads, 160 x 160, d 16 298 / 328; 170, 6 429 / 439, 8 560 / 546; 150, 6, 100 x 100, d 32 403 / 370).
+inline Split backward_split(int B, int H, int tiles, int d = 64) {
   Split best{1, 1};
   double best_cost = 1e30;
   for (int ch = 1; ch <= 8 && ch <= H; ch *= 2)
     for (int ct = 1; ch * ct <= 8 && ct <= tiles; ct *= 2) {
       const int hn = (H + ch - 1) / ch, tn = (tiles + ct - 1) / ct, c = ch * ct;
       const int64_t rounds = (B + resident_clusters(c) - 1) / resident_clusters(c);
-      const double cost = rounds * (1.0 + tn * (3.0 * hn + 2.0 + (ct > 1 ? 0.6 * ct * (hn + 1) : 0.0) + (ch > 1 ? 0.7 + 0.1 * ch : 0.0)));
+      const double more = c > 1 && rounds > 1 ? (d <= 16 ? 1.1 : 1.05) : 1.0;
+      const double cost = more * rounds * (1.0 + tn * (3.0 * hn + 2.0 + (ct > 1 ? 0.6 * ct * (hn + 1) : 0.0) + (ch > 1 ? 0.7 + 0.1 * ch : 0.0)));
       if (cost < best_cost * 0.97) { best_cost = cost; best = Split{ch, ct}; }
     }
   return best;

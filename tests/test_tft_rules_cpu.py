@@ -23,6 +23,12 @@ int main() {
   // as measured
   is(256, 4, 1, 1, 1); is(128, 4, 1, 1, 1); is(99, 8, 6, 1, 1); is(78, 4, 8, 1, 1); is(64, 4, 1, 2, 1); is(24, 4, 8, 2, 2);
   is(48, 8, 2, 2, 1); is(73, 1, 8, 1, 2); is(16, 8, 7, 4, 1); is(200, 8, 5, 2, 1); is(40, 1, 4, 1, 2); is(24, 2, 1, 2, 1);
+  // the boundary between two rounds of whole items and three of clusters of two
+  auto whole = [](Split s) { return s.ch * s.ct == 1; };
+  auto in_two = [](Split s) { return s.ch == 2 && s.ct == 1; };
+  claim(whole(backward_split(150, 4, 7, 16)) && whole(backward_split(170, 6, 7, 16)) && in_two(backward_split(170, 8, 7, 16)) &&
+        whole(backward_split(200, 4, 8, 64)) && whole(backward_split(150, 4, 8, 64)) && in_two(backward_split(150, 6, 5, 32)) &&
+        in_two(backward_split(200, 8, 8, 64)) && in_two(backward_split(222, 6, 1, 64)), "rounds", 0, 0, 0);
   // the forward: never two CTAs of clusters on an SM; as measured
   for (int tiles = 1; tiles <= 400; ++tiles)
     for (int H = 1; H <= 20; ++H) claim(forward_split(tiles, H) == 1 || forward_split(tiles, H) * tiles <= 148, "one CTA to an SM", 0, H, tiles);
