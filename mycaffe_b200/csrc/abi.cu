@@ -230,6 +230,8 @@ void lower_fail_word(const Kernel* k, McaFailWord family) {
 // backward, 49.6 -> 47.6).  For the calls of one launch: behind the attention's chains of dependent launches the extra one is as
 // late as the record (3 x 8 heads of 200 x 64, forward and backward: 57.9 and 58.2 us).  Work that lasts longer than SPIN_US gains
 // nothing either and is waited for by the stream synchronisation, which also reports what went wrong where the word never comes.
+// The query refuses what the stream synchronisation refuses and the launch alone would not: a call while another stream captures in
+// the global or this thread's mode.
 constexpr int SPIN_US = 300;
 constexpr int DONE_STRIDE = 16;      // words: a line for each kernel index
 unsigned* g_done = nullptr;          // kMaxKernels lines of pinned memory
@@ -260,10 +262,15 @@ void arm_done_word(Kernel* k, int idx) {   // under g_table_lock, with the devic
 long sync_call(Kernel* k, bool by_word = false) {
   if (k->synced) return 0;
   if (by_word && k->done != nullptr && mca_launch_pdl(done_kernel, dim3(1), dim3(1), 0, 0, k->done, ++k->done_seq) == 0) {
-    const auto t0 = std::chrono::steady_clock::now();
-    for (int polls = 1; !k->synced; ++polls) {
-      k->synced = *const_cast<volatile unsigned*>(k->done) == k->done_seq;
-      if (polls % 64 == 0 && std::chrono::steady_clock::now() - t0 > std::chrono::microseconds(SPIN_US)) break;
+    const cudaError_t state = cudaStreamQuery(0);
+    k->synced = state == cudaSuccess;
+    if (state == cudaErrorNotReady) {
+      cudaGetLastError();
+      const auto t0 = std::chrono::steady_clock::now();
+      for (int polls = 1; !k->synced; ++polls) {
+        k->synced = *const_cast<volatile unsigned*>(k->done) == k->done_seq;
+        if (polls % 64 == 0 && std::chrono::steady_clock::now() - t0 > std::chrono::microseconds(SPIN_US)) break;
+      }
     }
     if (k->synced) {
       std::atomic_thread_fence(std::memory_order_acquire);
