@@ -148,6 +148,7 @@ struct Kernel {
     ds_ws_floats = need;
   }
   bool synced = false;     // the call being dispatched has already synchronised the stream behind its last launch
+  bool by_word = false;    // the call being dispatched is waited for by the done word (see sync_call)
   bool fail_words = false; // this device's kernels raise its failure words (see g_fail)
   unsigned* done = nullptr;   // pinned word that a synchronous call's last launch writes done_seq to, or null
   unsigned done_seq = 0;
@@ -225,13 +226,16 @@ void lower_fail_word(const Kernel* k, McaFailWord family) {
 
 // The one synchronisation of a synchronous call.  by_word: behind the call's launches one more thread is launched, dependent on
 // the last of them (it is resident when that ends), which writes the call's number to a pinned word, and the host watches the word: a
-// stream synchronisation waits for the launch's own completion record, 2 us later (a kernel of 10 us, launch to answer: 13.9 us
-// with it, 12.0 with the word; a stream memory operation that writes the word 15.3; LayerNorm of 8192 x 768, forward and
-// backward, 49.6 -> 47.6).  For the calls of one launch: behind the attention's chains of dependent launches the extra one is as
-// late as the record (3 x 8 heads of 200 x 64, forward and backward: 57.9 and 58.2 us).  Work that lasts longer than SPIN_US gains
-// nothing either and is waited for by the stream synchronisation, which also reports what went wrong where the word never comes.
+// stream synchronisation waits for the launch's own completion record, up to a microsecond later (us a call, with it / with the word:
+// LayerNorm backward 8192 x 768 18.9 / 18.2, 512 x 768 13.4 / 13.0, TFT forward 256 x 4 x 24 x 192 x 64 46.6 / 45.8; a stream memory
+// operation that writes the word costs more than it saves).  The calls that set it are those it was measured to help: TFT, and norm layers,
+// RoPE and conversions of WORD_MIN elements or more; a shorter kernel has ended before the second launch has left the host (LayerNorm
+// 64 x 64 12.0 / 12.4, conversion of 1024 11.5 / 12.2).  The projections gain nothing (768 wide 15.4 / 15.8) and the attention's
+// chains of dependent launches neither.
 // The query refuses what the stream synchronisation refuses and the launch alone would not: a call while another stream captures in
-// the global or this thread's mode.
+// the global or this thread's mode.  Work that lasts longer than SPIN_US gains nothing and is waited for by the stream synchronisation, which also
+// reports what went wrong where the word never comes.
+constexpr int64_t WORD_MIN = 1 << 18;
 constexpr int SPIN_US = 300;
 constexpr int DONE_STRIDE = 16;      // words: a line for each kernel index
 unsigned* g_done = nullptr;          // kMaxKernels lines of pinned memory
@@ -259,9 +263,9 @@ void arm_done_word(Kernel* k, int idx) {   // under g_table_lock, with the devic
   k->done_seq = *k->done;                  // the index's last owner has been waited for
 }
 
-long sync_call(Kernel* k, bool by_word = false) {
+long sync_call(Kernel* k) {
   if (k->synced) return 0;
-  if (by_word && k->done != nullptr && mca_launch_pdl(done_kernel, dim3(1), dim3(1), 0, 0, k->done, ++k->done_seq) == 0) {
+  if (k->by_word && k->done != nullptr && mca_launch_pdl(done_kernel, dim3(1), dim3(1), 0, 0, k->done, ++k->done_seq) == 0) {
     const cudaError_t state = cudaStreamQuery(0);
     k->synced = state == cudaSuccess;
     if (state == cudaErrorNotReady) {
@@ -341,9 +345,9 @@ long set_out(float v, MCA_LONG* plOutput, float** ppOutput) {
   return 0;
 }
 
-long finish(Kernel* k, long err, bool by_word = true) {
+long finish(Kernel* k, long err) {
   if (err) return err;
-  if (!k->async) return sync_call(k, by_word);  // the reference blocks after every op (attn.cu:601)
+  if (!k->async) return sync_call(k);  // the reference blocks after every op (attn.cu:601)
   return 0;
 }
 
@@ -482,6 +486,7 @@ long convert_mem(Kernel* k, long llInput, MCA_LONGLONG* pl) {
   const int64_t n = pl[2];
   if (n <= 0 || n > s->count || n > d->count) return ERROR_PARAM_OUT_OF_RANGE;
   if (s->bf16 == d->bf16) return (long)cudaMemcpyAsync(d->ptr, s->ptr, (size_t)n * (s->bf16 ? 2 : 4), cudaMemcpyDeviceToDevice, 0);
+  k->by_word = n >= WORD_MIN;
   if (d->bf16) return mca_convert_f32_to_bf16((const float*)s->ptr, d->ptr, n, 0);
   return mca_convert_bf16_to_f32(s->ptr, (float*)d->ptr, n, 0);
 }
@@ -976,6 +981,7 @@ long rope_run(Kernel* k, long llInput, MCA_LONGLONG* pl, bool backward) {
   const int64_t half = r.D / 2, full = half * r.H;
   const int64_t last_pos = std::min<int64_t>(n / 2 - 1, (int64_t)r.T * full - 1) / full;
   if ((off > 0 ? off : 0) + (last_pos + 1) * half > (int64_t)r.T * half) return ERROR_PARAM_OUT_OF_RANGE;
+  k->by_word = n >= WORD_MIN;
   return mca_rope_f32(x, y, n, r.T, r.H, r.D, r.cos_t, r.sin_t, off, backward ? 1 : 0, 0);
 }
 
@@ -1185,6 +1191,7 @@ long layernorm_run(Kernel* k, long llInput, MCA_LONGLONG* pl, bool backward) {
   if (it == k->layernorm.end()) return ERROR_LAYERNORM_NOT_INITIALIZED;
   LayerNormHandle& h = it->second;
   const int64_t n = h.rows * h.inner;
+  k->by_word = n >= WORD_MIN;
   if (!backward) {
     float *x, *y;
     if ((e = check_f32(k, (long)pl[1], n, &x)) || (e = check_f32(k, (long)pl[2], n, &y))) return e;
@@ -1203,6 +1210,7 @@ long rmsnorm_run(Kernel* k, long lInput, float* pf, long llInput, MCA_LONGLONG* 
   const int64_t rows = pl[backward ? 6 : 4], inner = pl[backward ? 7 : 5];
   if (rows <= 0 || inner <= 0 || inner > INT32_MAX) return ERROR_PARAM_OUT_OF_RANGE;
   const int64_t n = rows * inner;
+  k->by_word = n >= WORD_MIN;
   float *x, *w = nullptr;
   if ((e = check_f32(k, (long)pl[0], n, &x))) return e;
   if (pl[1] != 0 && (e = check_f32(k, (long)pl[1], inner, &w))) return e;
@@ -1240,6 +1248,7 @@ long tft_fwd(Kernel* k, long llInput, MCA_LONGLONG* pl) {
       (e = check_f32(k, (long)pl[10], (int64_t)B * Nq * Nk, &attn)))
     return e;
   if (pl[3] != 0 && (e = check_f32(k, (long)pl[3], (int64_t)Nq * Nk, &mask))) return e;
+  k->by_word = true;
   return mca_tft_attention_forward_f32(q, kk, v, mask, B, H, Nq, Nk, d, out, attn, 0);
 }
 
@@ -1256,6 +1265,7 @@ long tft_bwd(Kernel* k, long llInput, MCA_LONGLONG* pl) {
     return e;
   if (pl[3] != 0 && (e = check_f32(k, (long)pl[3], (int64_t)Nq * Nk, &mask))) return e;
   if (pl[5] != 0 && (e = check_f32(k, (long)pl[5], (int64_t)B * Nq * Nk, &ga))) return e;
+  k->by_word = true;
   return mca_tft_attention_backward_f32(q, kk, v, mask, go, ga, B, H, Nq, Nk, d, dq, dk, dv, 0);
 }
 
@@ -1384,7 +1394,7 @@ long run(Kernel* k, long fn, float* pf, long lInput, MCA_LONGLONG* pl, long llIn
   cudaError_t ce = cudaSetDevice(k->device);
   if (ce != cudaSuccess) return ce;
   k->last_detail.clear();
-  k->synced = false;
+  k->synced = k->by_word = false;
   long e;
   switch (fn) {
     case CUDA_FN_SETDEVICE: return 0;
@@ -1421,18 +1431,18 @@ long run(Kernel* k, long fn, float* pf, long lInput, MCA_LONGLONG* pl, long llIn
       k->fit_ds_ws();
       return 0;
     }
-    case CUDNN_FN_ATTN_SET: return finish(k, attn_set(k, lInput, pf, llInput, pl), false);
-    case CUDNN_FN_ATTN_FWD: return finish(k, attn_fwd(k, llInput, pl, MCA_LAYOUT_BHTD), false);
-    case CUDNN_FN_ATTN_BWD: return finish(k, attn_bwd(k, llInput, pl, MCA_LAYOUT_BHTD), false);
+    case CUDNN_FN_ATTN_SET: return finish(k, attn_set(k, lInput, pf, llInput, pl));
+    case CUDNN_FN_ATTN_FWD: return finish(k, attn_fwd(k, llInput, pl, MCA_LAYOUT_BHTD));
+    case CUDNN_FN_ATTN_BWD: return finish(k, attn_bwd(k, llInput, pl, MCA_LAYOUT_BHTD));
     case MCA_FN_ATTN_FWD_PACKED: {
       if ((e = verify_in(llInput, pl, 7, 7))) return e;
       MCA_LONGLONG a9[9] = {pl[0], pl[1], pl[2], pl[3], pl[3], pl[3], pl[4], pl[5], pl[6]};
-      return finish(k, attn_fwd(k, 9, a9, MCA_LAYOUT_PACKED), false);
+      return finish(k, attn_fwd(k, 9, a9, MCA_LAYOUT_PACKED));
     }
     case MCA_FN_ATTN_BWD_PACKED: {
       if ((e = verify_in(llInput, pl, 7, 7))) return e;
       MCA_LONGLONG a11[11] = {pl[0], pl[1], pl[2], pl[3], pl[2], pl[3], pl[2], pl[3], pl[4], pl[5], pl[6]};
-      return finish(k, attn_bwd(k, 11, a11, MCA_LAYOUT_PACKED), false);
+      return finish(k, attn_bwd(k, 11, a11, MCA_LAYOUT_PACKED));
     }
     case CUDA_FN_CREATE_LAYERNORM: return layernorm_create(k, lInput, pf, llInput, pl, plOutput, ppOutput);
     case CUDA_FN_FREE_LAYERNORM: return layernorm_free(k, lInput, pf);
