@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(TFT_THREADS) tft_fwd_kernel(const float* __res
 
 
 // ---------------------------------------------------------------------------------------------
-// Forward, tiled form (the shapes the TFT network runs: d in {16, 32, 64}, Nk <= 192).
+// Forward, tiled form (the shapes the TFT network runs: d = 64, Nk 116 .. 192; tft_rules::forward_tiled).
 //
 // One CTA = one batch item x 24 query rows, all heads.  The K tiles of the heads and then V (Nk x d each) stream through
 // two shared-memory buffers filled by asynchronous copies, two tiles ahead of the arithmetic.  The scores of the 24 rows
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(TFT_THREADS, 2) tft_fwd_tiled_kernel(const int
       o[r][2] = fmaf(pj, vv.z, o[r][2]); o[r][3] = fmaf(pj, vv.w, o[r][3]);
     }
   }
-  float* part = pm + (size_t)TQ * Nk;                     // (SLOTS - 1) x 24 x D floats (the launcher checks the room)
+  float* part = pm + (size_t)TQ * Nk;                     // (SLOTS - 1) x 24 x D floats (tft_rules::forward_tiled sees to the room)
   if (ks > 0) {
 #pragma unroll
     for (int r = 0; r < TQ / 4; ++r)
@@ -545,7 +545,7 @@ __global__ void __launch_bounds__(TFT_THREADS) tft_bwd_kernel(const float* __res
 }
 
 // ---------------------------------------------------------------------------------------------
-// Backward, tiled form (the shapes of the tiled forward: d in {16, 32, 64}, Nk <= 192).
+// Backward, tiled form (d in {16, 32, 64}, Nk <= 192).
 //
 // One CTA = one batch item; it walks the 24-row tiles of the queries and, inside a tile, the heads.  V stays in shared
 // memory; K_h, the 24 rows of Q_h and of the output gradient are double-buffered (the next iteration's arrive while
@@ -1378,21 +1378,18 @@ int mca_tft_attention_forward_f32(const float* q, const float* k, const float* v
     return ERROR_ATTN_UNSUPPORTED_SHAPE;
   // the tiled kernel where the call fits it, else the generic one
   if (tft_rules::forward_tiled(Nk, d, q, out)) {
-    const size_t smem_t = tft_rules::forward_tiled_smem(Nk, d);
-    dim3 grid_t(mca_ceil_div(Nq, TQ), B);
+    constexpr int D = 64;
+    const size_t smem_t = sizeof(float) * (2 * (size_t)Nk * D + 2 * (size_t)TQ * D + 4 * TQ);   // at most 109 KB: two CTAs per SM
+    const dim3 grid_t(mca_ceil_div(Nq, TQ), B);
     const float sc = 1.0f / sqrtf((float)d);
     cudaStream_t st = (cudaStream_t)stream;
-    const int ch = smem_t >= sizeof(float) * TQ * TQ_KEYS ? tft_rules::forward_split((int64_t)B * grid_t.x, H) : 1;
-#define MCA_TFT_TILED(D_)                                                                                                 \
-    if (ch == 1) {                                                                                                        \
-      if (const int e = smem_limit<tft_fwd_tiled_kernel<D_, false>>()) return e;                                         \
-      tft_fwd_tiled_kernel<D_, false><<<grid_t, TFT_THREADS, smem_t, st>>>(1, q, k, v, mask, H, Nq, Nk, sc, out, attn);   \
-    } else {                                                                                                              \
-      if (const int e = smem_limit<tft_fwd_tiled_kernel<D_, true>>()) return e;                                          \
-      return launch_clusters(tft_fwd_tiled_kernel<D_, true>, ch, dim3(grid_t.x * ch, B), smem_t, st, ch, q, k, v, mask, H, Nq, Nk, sc, out, attn); \
+    const int ch = tft_rules::forward_split((int64_t)B * grid_t.x, H);
+    if (ch > 1) {
+      if (const int e = smem_limit<tft_fwd_tiled_kernel<D, true>>()) return e;
+      return launch_clusters(tft_fwd_tiled_kernel<D, true>, ch, dim3(grid_t.x * ch, B), smem_t, st, ch, q, k, v, mask, H, Nq, Nk, sc, out, attn);
     }
-    if (d == 64) { MCA_TFT_TILED(64) } else if (d == 32) { MCA_TFT_TILED(32) } else { MCA_TFT_TILED(16) }
-#undef MCA_TFT_TILED
+    if (const int e = smem_limit<tft_fwd_tiled_kernel<D, false>>()) return e;
+    tft_fwd_tiled_kernel<D, false><<<grid_t, TFT_THREADS, smem_t, st>>>(1, q, k, v, mask, H, Nq, Nk, sc, out, attn);
     return mca_launch_status();
   }
   const size_t smem = sizeof(float) * ((size_t)Nk * (d + 4) + (size_t)H * TFT_ROWS * d + 2 * (size_t)TFT_ROWS * Nk);

@@ -1,20 +1,17 @@
 // Choices of the TFT attention that depend on sizes alone (plain C++, so that they can be tested without a GPU).
 #pragma once
-#include <cstddef>
 #include <cstdint>
 
 namespace tft_rules {
 
-// Whether the tiled forward takes a call: two K buffers and two CTAs per SM, a K buffer that also holds the mean probabilities
-// (24 x Nk) and the partial outputs of the other key slices, and 16-byte copies of Q and stores of the output (K and V are refused
-// unaligned by both kernels; the generic one reads Q and writes the output by the float).
+// Whether the tiled forward takes a call: 64-wide heads, no more keys than its register tiles cover, as many as a K buffer needs to
+// hold the mean probabilities and the other three key slices' partial outputs (24 Nk + 3 x 24 x 64 <= 64 Nk: 116), and 16-byte copies of
+// Q and stores of the output (K and V are refused unaligned by both kernels; the generic one reads Q and writes the output by the
+// float).
 constexpr int TILE_ROWS = 24, TILE_KEYS = 192, TILE_THREADS = 256;
-inline size_t forward_tiled_smem(int Nk, int d) { return sizeof(float) * (2 * (size_t)Nk * d + 2 * (size_t)TILE_ROWS * d + 4 * TILE_ROWS); }
 inline bool forward_tiled(int Nk, int d, const void* q, const void* out) {
-  if ((d != 16 && d != 32 && d != 64) || Nk > TILE_KEYS || forward_tiled_smem(Nk, d) > 113 * 1024) return false;
-  if (((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) & 15) != 0) return false;
-  const int slices = TILE_THREADS / d;   // of the final product: TILE_THREADS / ((d / 4) * 4)
-  return (size_t)TILE_ROWS * Nk + (size_t)(slices - 1) * TILE_ROWS * d <= (size_t)Nk * d;
+  const bool aligned = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+  return d == 64 && Nk <= TILE_KEYS && TILE_ROWS * (Nk + 3 * d) <= Nk * d && aligned;
 }
 
 struct Split {

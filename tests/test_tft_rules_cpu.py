@@ -36,8 +36,21 @@ int main() {
         forward_split(33, 6) == 4 && forward_split(16, 8) == 4 && forward_split(15, 8) == 8 && forward_split(8, 1) == 1, "forward choice", 0, 0, 0);
   // the tiled forward copies Q and writes the output by 16 bytes: never from or to an address that is not a multiple of them
   alignas(16) static float at[8];
-  claim(forward_tiled(192, 64, at, at + 4), "tiled", 0, 0, 192);
   for (int o = 1; o < 4; ++o) claim(!forward_tiled(192, 64, at + o, at) && !forward_tiled(192, 64, at, at + o), "alignment", o, 0, 192);
+  for (int Nk = 1; Nk <= 300; ++Nk)
+    for (int d = 4; d <= 128; d += 4) {
+      const int slices = 256 / d;
+      const bool room = 24 * Nk + (slices - 1) * 24 * d <= Nk * d, takes = forward_tiled(Nk, d, at, at + 4);
+      claim(takes == (d == 64 && Nk >= 116 && Nk <= 192), "tiled", d, 0, Nk);
+      claim(!takes || (room && 4 * (2 * Nk * d + 2 * 24 * d + 96) <= 113 * 1024 && 2 * Nk * d >= 24 * 192), "room", d, 0, Nk);
+    }
+  // what the shapes of test_tft_split_gpu.py take: 0 the generic forward, else the CTAs along the heads
+  auto forward = [&](int B, int H, int Nq, int Nk, int d) { return forward_tiled(Nk, d, at, at) ? forward_split((int64_t)B * ((Nq + 23) / 24), H) : 0; };
+  claim(forward(1, 3, 49, 191, 64) == 2 && forward(33, 6, 24, 192, 64) == 4 && forward(2, 8, 30, 116, 64) == 8 && forward(160, 4, 24, 120, 64) == 1 &&
+        forward(2, 7, 25, 33, 64) == 0 && forward(2, 8, 24, 115, 64) == 0 && forward(16, 8, 160, 160, 32) == 0, "forward", 0, 0, 0);
+  // and its backwards over many row tiles by one CTA
+  claim(whole(backward_split(140, 2, 5, 64)) && whole(backward_split(130, 1, 8, 32)) && whole(backward_split(150, 3, 4, 16)) &&
+        whole(backward_split(140, 1, 5, 64)), "whole items", 0, 0, 0);
   return bad;
 }
 '''

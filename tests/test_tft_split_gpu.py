@@ -20,19 +20,15 @@ def cuda():
     c.Dispose()
 
 
-# heads that are no multiple of the CTAs along them, row tiles likewise, a last tile of one row, every head size, one head, one tile
-@pytest.mark.parametrize("with_attn_grad", [False, True])
-@pytest.mark.parametrize("B,H,Nq,Nk,d", [(2, 8, 24, 60, 32), (3, 4, 60, 60, 16), (2, 1, 100, 100, 64), (2, 5, 50, 70, 32), (1, 3, 49, 191, 64),
-                                         (16, 8, 160, 160, 32), (2, 7, 25, 33, 64), (40, 2, 73, 90, 16), (33, 6, 24, 192, 64)])
-def test_split_over_a_cluster(cuda, B, H, Nq, Nk, d, with_attn_grad):
+def forward_and_backward(cuda, B, H, Nq, Nk, d, with_attn_grad, with_mask):
     rng = np.random.default_rng(B * 100 + H + Nq)
     q = rng.standard_normal((B, H, Nq, d)).astype(np.float32)
     k = rng.standard_normal((B, H, Nk, d)).astype(np.float32)
     v = rng.standard_normal((B, Nk, d)).astype(np.float32)
-    mask = (np.arange(Nk)[None, :] > np.arange(Nq)[:, None] + Nk - Nq).astype(np.float32)
+    mask = (np.arange(Nk)[None, :] > np.arange(Nq)[:, None] + Nk - Nq).astype(np.float32) if with_mask else None
     d_out = rng.standard_normal((B, Nq, d)).astype(np.float32)
     d_attn = rng.standard_normal((B, Nq, Nk)).astype(np.float32) if with_attn_grad else None
-    h = [cuda.AllocMemory(a) for a in (q, k, v, mask, d_out)] + [cuda.AllocMemory(d_attn) if with_attn_grad else 0]
+    h = [0 if a is None else cuda.AllocMemory(a) for a in (q, k, v, mask, d_out, d_attn)]
     o = [cuda.AllocMemory(n) for n in (B * Nq * d, B * Nq * Nk, q.size, k.size, v.size)]
     got = []
     for _ in range(2):
@@ -46,6 +42,46 @@ def test_split_over_a_cluster(cuda, B, H, Nq, Nk, d, with_attn_grad):
     for m in h + o:
         if m:
             cuda.FreeMemory(m)
+
+
+# heads that are no multiple of the CTAs along them, row tiles likewise, a last tile of one row, one head, one tile, every head size of
+# the backward; the forward (64-wide heads of 116 keys or more, else generic) over 1, 2, 4 and 8 CTAs: test_tft_rules_cpu.py
+FORWARDS = [(1, 3, 49, 191, 64), (33, 6, 24, 192, 64), (2, 8, 30, 116, 64), (160, 4, 24, 120, 64), (2, 8, 24, 115, 64)]
+
+
+@pytest.mark.parametrize("with_attn_grad", [False, True])
+@pytest.mark.parametrize("B,H,Nq,Nk,d", [(2, 8, 24, 60, 32), (3, 4, 60, 60, 16), (2, 1, 100, 100, 64), (2, 5, 50, 70, 32), (1, 3, 49, 191, 64),
+                                         (16, 8, 160, 160, 32), (2, 7, 25, 33, 64), (40, 2, 73, 90, 16), (33, 6, 24, 192, 64)] + FORWARDS[2:])
+def test_split_over_a_cluster(cuda, B, H, Nq, Nk, d, with_attn_grad):
+    forward_and_backward(cuda, B, H, Nq, Nk, d, with_attn_grad, with_mask=True)
+
+
+@pytest.mark.parametrize("B,H,Nq,Nk,d", FORWARDS)
+def test_split_without_a_mask(cuda, B, H, Nq, Nk, d):
+    forward_and_backward(cuda, B, H, Nq, Nk, d, with_attn_grad=False, with_mask=False)
+
+
+@pytest.mark.parametrize("B,H,Nq,Nk,d", [(140, 2, 100, 60, 64), (130, 1, 190, 33, 32), (150, 3, 90, 17, 16), (140, 1, 120, 192, 64)])
+def test_row_tiles_of_one_cta(cuda, B, H, Nq, Nk, d):
+    """Items that fill the chip: one CTA walks an item's row tiles and asks for the next tile's rows while it works on this one's.  They
+    must not land where a slower warp still reads: every one of many runs gives the bits of the first, and the first is the oracle's."""
+    import torch
+    from mycaffe_b200 import _lib
+    rng = np.random.default_rng(B + Nk)
+    q, k, v, go = (rng.standard_normal(s).astype(np.float32) for s in ((B, H, Nq, d), (B, H, Nk, d), (B, Nk, d), (B, Nq, d)))
+    t = [torch.from_numpy(a).cuda() for a in (q, k, v, go)]
+    o = [torch.empty_like(a) for a in t[:3]]
+    first = None
+    for _ in range(25):
+        for a in o:
+            a.fill_(float("nan"))
+        assert _lib.load().mca_tft_attention_backward_f32(*(a.data_ptr() for a in t[:3]), None, t[3].data_ptr(), None, B, H, Nq, Nk, d,
+                                                          *(a.data_ptr() for a in o), torch.cuda.current_stream().cuda_stream) == 0
+        if first is None:
+            first = [a.clone() for a in o]
+            for a, r in zip(first, oracle.tft_backward(q, k, v, None, go, None, f64=True)):
+                assert rel_err(a.cpu().numpy(), r) < 2e-5
+        assert all(torch.equal(a, b) for a, b in zip(o, first))
 
 
 @pytest.mark.parametrize("B,H,Nq,Nk", [(1, 3, 49, 191), (2, 2, 30, 120)])
