@@ -154,6 +154,21 @@ def test_rows_at_the_edges_of_the_shapes(cuda, inner):
         cuda.FreeMemory(v)
 
 
+@pytest.mark.parametrize("rows,inner", [(1184, 900), (1185, 900), (1184, 1024), (1185, 1024), (2500, 1024)])
+def test_rmsnorm_backward_of_eight_pieces_either_side_of_one_cta_per_sm(cuda, rows, inner):
+    rng = np.random.default_rng(rows)
+    x, dy = (rng.standard_normal((rows, inner)).astype(np.float32) for _ in range(2))
+    w = (1 + 0.2 * rng.standard_normal(inner)).astype(np.float32)
+    m = [cuda.AllocMemory(v) for v in (x, w, dy, x.size, x.size, rows, inner)]
+    cuda.RmsNormForward(m[0], m[1], m[3], m[5], rows, inner, 1e-5)
+    cuda.RmsNormBackward(m[0], m[1], m[2], m[5], m[4], m[6], rows, inner)
+    dx_ref, dw_ref = oracle.rmsnorm_layer_backward(x, w, dy, 1e-5)
+    assert rel_err(cuda.GetMemory(m[4], x.size), dx_ref.ravel()) < 1e-5
+    assert rel_err(cuda.GetMemory(m[6], inner), dw_ref) < 1e-5
+    for v in m:
+        cuda.FreeMemory(v)
+
+
 @pytest.mark.parametrize("inner", [300, 768, 771, 2048])
 def test_layernorm_quotients_are_those_of_a_division(cuda, inner):
     """Forward: rows of small multiples of 2^-10 that cancel in pairs have the mean 0 without a rounding, so y is x / stdev as a
