@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(G == 32 ? 256 : G, CTAS) norm_rows_kernel(cons
 }
 
 // dW[e] = sum over the CTAs' partials: eight warps of a CTA take every eighth of them for 32 columns, and their sums are added in
-// order (one thread a column walked all 296 of them: rows of 768, 38 us).
+// order (one thread a column walked all 296 of them, one behind the other).
 constexpr int DW_WARPS = 8;
 __global__ void __launch_bounds__(DW_WARPS * 32) norm_dw_reduce_kernel(const float* __restrict__ partial, int n_partials, int inner, float* __restrict__ dw) {
   __shared__ float part[DW_WARPS][32];
@@ -288,9 +288,10 @@ __global__ void __launch_bounds__(DW_WARPS * 32) norm_dw_reduce_kernel(const flo
 
 struct Shape { int G, MAXV, VEC; };
 
-// the narrowest group that holds a row, and no more pieces a thread than it takes (a row of 768 as eight pieces of a warp instead of
-// six: registers for three CTAs an SM instead of five, and a quarter of the arithmetic on zeros); vector loads need
-// inner % 4 == 0 and 16-byte aligned tensors
+// the narrowest group that holds a row, and as few pieces a thread as there is an instantiation for: every second number of 16-byte
+// pieces of a warp, two or four of 256 threads, four of 1024; of single floats 8 or 16, 4 or 16, and 16 (a LayerNorm of 768 as eight
+// pieces instead of six: a quarter of the arithmetic on zeros, and 96 registers in the backward, two CTAs an SM, instead of 79, three); vector
+// loads need inner % 4 == 0 and 16-byte aligned tensors
 bool pick(int inner, bool aligned, Shape* s) {
   auto pieces = [&](int G, int VEC) { return (inner + G * VEC - 1) / (G * VEC); };
   if (aligned && inner % 4 == 0) {

@@ -564,7 +564,7 @@ __global__ void __launch_bounds__(TFT_THREADS) tft_bwd_kernel(const float* __res
 // The 1/H of the head mean is applied to dP once and to dV.
 //
 // With fewer batch items than would fill the chip an item has a cluster of CTAs, ch of them along the heads and ct along the row
-// tiles (tft_bwd_split).  A CTA's heads and tiles are every ch-th and ct-th.  dQ, and dK of one tile, belong to one CTA; what
+// tiles (tft_rules::backward_split).  A CTA's heads and tiles are every ch-th and ct-th.  dQ, and dK of one tile, belong to one CTA; what
 // several have a part of keeps its order, so that results do not depend on timing: the ct CTAs that hold a head add their
 // parts of dK (and of dV) one after the other, a cluster barrier between two; the head sum of P is put together by the first CTA
 // of a tile from its peers' shared memory, in the heads' order by CTA.
