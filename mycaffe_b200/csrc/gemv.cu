@@ -369,12 +369,9 @@ int launch_pass(GemvParams p, int b0, cudaStream_t st) {
   auto kern = gemv_stream_kernel<WT, NB, R, THREADS, GLU, DEPTH, U, PART>;
   const int total_rows = GLU ? p.rows[0] : p.rows[0] + (p.n_mats > 1 ? p.rows[1] : 0) + (p.n_mats > 2 ? p.rows[2] : 0);
   const int total_steps = mca_ceil_div(total_rows, STEP);
-  // The limit is set once and to the largest size: one set to each call's own could be lowered by another thread's shorter rows before
-  // this call's launch, which is then refused.
-  static std::atomic<uint64_t> limit_set{0};
-  if (const int e = mca_smem_once(limit_set, kern, GV_SMEM_LIMIT)) return e;
   // every CTA resident at once; rows dealt evenly to groups of S warps.  The
-  // occupancy of this instantiation is looked up once per (device, shared-memory size).
+  // occupancy of this instantiation is looked up once per (device, shared-memory size).  The limit is the largest size: set to each
+  // call's own it could be lowered by another thread's shorter rows before this call's launch, which is then refused.
   int ctas_per_sm = 1, dev = 0, sms = 148;
   MCA_CUDA_TRY(cudaGetDevice(&dev));
   {
@@ -383,6 +380,7 @@ int launch_pass(GemvParams p, int b0, cudaStream_t st) {
     static size_t c_smem = 0;
     std::lock_guard<std::mutex> g(lock);
     if (c_dev != dev || c_smem != smem) {
+      MCA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GV_SMEM_LIMIT));
       MCA_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c_ctas, kern, THREADS, smem));
       MCA_CUDA_TRY(cudaDeviceGetAttribute(&c_sms, cudaDevAttrMultiProcessorCount, dev));
       c_dev = dev; c_smem = smem;
