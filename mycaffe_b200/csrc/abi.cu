@@ -228,9 +228,10 @@ void lower_fail_word(const Kernel* k, McaFailWord family) {
 // the last of them (it is resident when that ends), which writes the call's number to a pinned word, and the host watches the word: a
 // stream synchronisation waits for the launch's own completion record, up to a microsecond later (us a call, with it / with the word:
 // LayerNorm backward 8192 x 768 18.9 / 18.2, 512 x 768 13.4 / 13.0, TFT forward 256 x 4 x 24 x 192 x 64 46.6 / 45.8; a stream memory
-// operation that writes the word costs more than it saves).  The calls that set it are those it was measured to help: TFT, and norm layers,
-// RoPE and conversions of WORD_MIN elements or more; a shorter kernel has ended before the second launch has left the host (LayerNorm
-// 64 x 64 12.0 / 12.4, conversion of 1024 11.5 / 12.2).  The projections gain nothing (768 wide 15.4 / 15.8) and the attention's
+// operation that writes the word costs more than it saves).  The calls that set it are those it was measured to help: TFT, RoPE and
+// conversions of WORD_MIN elements or more, norm layers of a quarter of that, the RMSNorm backward (two launches) of twice that; a shorter
+// kernel has ended before the second launch has left the host (LayerNorm 64 x 64 12.0 / 12.4, 64 x 2048 12.4 / 12.4, 128 x 768 13.3 / 13.0;
+// RMSNorm backward 64 x 768 18.1 / 18.3, 768 x 768 19.4 / 19.3; conversion of 1024 11.5 / 12.2, of 2^18 12.2 / 12.2).  The projections gain nothing (768 wide 15.4 / 15.8) and the attention's
 // chains of dependent launches neither.
 // The query refuses what the stream synchronisation refuses and the launch alone would not: a call while another stream captures in
 // the global or this thread's mode.  Work that lasts longer than SPIN_US gains nothing and is waited for by the stream synchronisation, which also
@@ -1191,7 +1192,7 @@ long layernorm_run(Kernel* k, long llInput, MCA_LONGLONG* pl, bool backward) {
   if (it == k->layernorm.end()) return ERROR_LAYERNORM_NOT_INITIALIZED;
   LayerNormHandle& h = it->second;
   const int64_t n = h.rows * h.inner;
-  k->by_word = n >= WORD_MIN;
+  k->by_word = n >= WORD_MIN / 4;
   if (!backward) {
     float *x, *y;
     if ((e = check_f32(k, (long)pl[1], n, &x)) || (e = check_f32(k, (long)pl[2], n, &y))) return e;
@@ -1210,7 +1211,7 @@ long rmsnorm_run(Kernel* k, long lInput, float* pf, long llInput, MCA_LONGLONG* 
   const int64_t rows = pl[backward ? 6 : 4], inner = pl[backward ? 7 : 5];
   if (rows <= 0 || inner <= 0 || inner > INT32_MAX) return ERROR_PARAM_OUT_OF_RANGE;
   const int64_t n = rows * inner;
-  k->by_word = n >= WORD_MIN;
+  k->by_word = n >= (backward ? 2 * WORD_MIN : WORD_MIN / 4);
   float *x, *w = nullptr;
   if ((e = check_f32(k, (long)pl[0], n, &x))) return e;
   if (pl[1] != 0 && (e = check_f32(k, (long)pl[1], inner, &w))) return e;

@@ -1,5 +1,5 @@
 """A synchronous call returns when its results are there for everybody, whichever way the host waits for it: short calls, calls the host watches
-a word for (2^18 elements and more), calls that outlast the watching, and what a capture on another stream forbids."""
+a word for (norm layers of 2^16 elements and more), calls that outlast the watching, and what a capture on another stream forbids."""
 import subprocess
 import sys
 from pathlib import Path
