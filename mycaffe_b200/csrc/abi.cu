@@ -40,7 +40,7 @@ struct AttnHandle {
   float *row_max = nullptr, *row_sum = nullptr, *y_copy = nullptr, *delta = nullptr, *lse = nullptr;
   void* split_ws = nullptr;    // fp16 halves of q, k, v for the split-operand tensor-core forward of fp32 handles
   int64_t split_ws_bytes = 0;
-  int64_t ds_floats = 0;       // room the exact fp32 backward of this handle asks of its kernel index (Kernel::ds_ws)
+  int64_t ds_floats = 0;       // room for dS that the backward of this handle asks of its kernel index (Kernel::ds_ws)
   float* mask_ws = nullptr;    // fp32 copies for a bf16 handle that is given a (T,T) or batch mask (allocated on first use)
   size_t mask_ws_floats = 0;
   uint32_t *mask_bits = nullptr, *mask_bits_t = nullptr;   // keep-bits of a (T,T) or batch mask for the tensor-core kernels
@@ -132,7 +132,7 @@ struct Kernel {
   std::string last_detail;
   float* stage = nullptr;  // grow-only fp32 staging buffer for float <-> bf16 transfers
   size_t stage_count = 0;
-  float* ds_ws = nullptr;  // dS between the two kernels of an exact fp32 backward: one for all handles, whose backwards follow one
+  float* ds_ws = nullptr;  // dS between the two kernels of a backward: one for all handles, whose backwards follow one
   int64_t ds_ws_floats = 0;   // another on one stream; as large as the largest of them asks, and gone with the last of them
   void fit_ds_ws() {       // after a handle has been set or released
     int64_t need = 0;
@@ -540,6 +540,10 @@ long attn_set(Kernel* k, long lInput, float* pf, long llInput, MCA_LONGLONG* pl)
     // dS is formed twice.
     const int64_t bytes = mca_sdpa_backward_f32_ws_bytes(a.B, a.H, a.block);
     if (bytes <= kMaxDsBytes) a.ds_floats = bytes / 4;
+  } else if (a.training && (int64_t)a.B * a.H <= 65535) {
+    // The tensor-core backward does the same, as many heads at a time as fit.
+    const int64_t bytes = mca_sdpa_backward_tc_ws_bytes(a.B, a.H, a.block, a.D, a.dtype != MCA_DTYPE_BF16);
+    a.ds_floats = std::min<int64_t>(bytes, kMaxDsBytes) / 4;
   }
   k->fit_ds_ws();
   a.configured = true;
@@ -861,8 +865,8 @@ long attn_bwd(Kernel* k, long llInput, MCA_LONGLONG* pl, int layout) {
     const bool fwd_masked = a.fwd_mask_mode == MCA_MASK_TT || a.fwd_mask_mode == MCA_MASK_BATCH;
     if (fwd_masked && a.fwd_mask_handle == 0) {
       // the forward applied the mask on the tensor cores from the keep-bits it packed into the handle: so does this
-      e = mca_sdpa_backward_tc_masked(q, kk, v, a.y_copy, dy, a.lse, a.delta, MCA_DTYPE_BF16, 0, a.B, a.H, T, a.D, dq, dk, dv,
-                                      a.causal_flag + 1, layout, a.mask_bits, a.mask_bits_t, a.fwd_mask_mode, 0);
+      e = mca_sdpa_backward_tc_ws(q, kk, v, a.y_copy, dy, a.lse, a.delta, MCA_DTYPE_BF16, 0, a.B, a.H, T, a.D, dq, dk, dv,
+                                  a.causal_flag + 1, layout, a.mask_bits, a.mask_bits_t, a.fwd_mask_mode, k->ds_ws, k->ds_ws_floats * 4, 0);
       if (e) return e;
       return tc_status(k, a);
     }
@@ -887,9 +891,8 @@ long attn_bwd(Kernel* k, long llInput, MCA_LONGLONG* pl, int layout) {
       if ((e = mca_convert_f32_to_bf16(gq, dq, n, 0)) || (e = mca_convert_f32_to_bf16(gk, dk, n, 0))) return e;
       return mca_convert_f32_to_bf16(gv, dv, n, 0);
     }
-    e = mca_sdpa_backward_tc_layout(q, kk, v, a.y_copy, dy, a.lse, a.delta, MCA_DTYPE_BF16,
-                                    a.fwd_mask_mode == MCA_MASK_CAUSAL, a.B, a.H, T, a.D, dq, dk, dv, a.causal_flag + 1,
-                                    layout, 0);
+    e = mca_sdpa_backward_tc_ws(q, kk, v, a.y_copy, dy, a.lse, a.delta, MCA_DTYPE_BF16, a.fwd_mask_mode == MCA_MASK_CAUSAL, a.B, a.H, T,
+                                a.D, dq, dk, dv, a.causal_flag + 1, layout, nullptr, nullptr, MCA_MASK_NONE, k->ds_ws, k->ds_ws_floats * 4, 0);
     if (e) return e;
     return tc_status(k, a);
   }
@@ -904,9 +907,9 @@ long attn_bwd(Kernel* k, long llInput, MCA_LONGLONG* pl, int layout) {
     // the forward ran on the tensor cores with split operands; so does the backward, from the halves of q, k, v that
     // forward left in the handle's workspace (the reference's Backward likewise works on what its Forward saved)
     const bool bits = a.fwd_mask_mode == MCA_MASK_TT || a.fwd_mask_mode == MCA_MASK_BATCH;   // packed by the forward
-    e = mca_sdpa_backward_f32_tc_masked(dy, a.y_copy, a.lse, a.delta, a.fwd_mask_mode == MCA_MASK_CAUSAL, a.B, a.H, T, a.D, dq, dk,
-                                        dv, a.split_ws, a.split_ws_bytes, a.causal_flag + 1, layout, bits ? a.mask_bits : nullptr,
-                                        bits ? a.mask_bits_t : nullptr, bits ? a.fwd_mask_mode : MCA_MASK_NONE, 0);
+    e = mca_sdpa_backward_f32_tc_ws(dy, a.y_copy, a.lse, a.delta, a.fwd_mask_mode == MCA_MASK_CAUSAL, a.B, a.H, T, a.D, dq, dk, dv,
+                                    a.split_ws, a.split_ws_bytes, a.causal_flag + 1, layout, bits ? a.mask_bits : nullptr,
+                                    bits ? a.mask_bits_t : nullptr, bits ? a.fwd_mask_mode : MCA_MASK_NONE, k->ds_ws, k->ds_ws_floats * 4, 0);
     if (e) return e;
     return tc_status(k, a);
   }

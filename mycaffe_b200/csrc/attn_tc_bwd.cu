@@ -16,6 +16,7 @@
 //   * dkdv kernel: one CTA per 128-row key tile walks the query tiles with the transposed
 //     products S^T = K Q^T and dP^T = V dY^T, so that P^T and dS^T come out in the layout the
 //     A operand of dV += P^T dY and dK += dS^T Q needs.
+// Where it gains (passes_ds) the dkdv kernel leaves its dS tiles in a workspace and dQ = dS K is one product over them.
 // Q/K/V/dY tiles arrive by TMA (no multicast) through rings; every mbarrier wait is
 // bounded as in the forward kernel.
 //
@@ -32,6 +33,21 @@
 namespace {
 
 using namespace tc;
+
+// dS between the dK/dV kernel and the dQ kernel that is one product over it (DS): one 128 x 128 tile per (query tile, key tile)
+// of a head, the lower triangle alone under the causal mask.  A tile is the image of the tensor core's unswizzled MN-major A
+// operand: four blocks of 32 keys, each (hi, then in split mode lo) sixteen groups of 8 queries x 32 keys x 16 bytes.  A key's eight
+// queries are what a thread that reads dS^T from TMEM has in four registers, so a warp writes 512 consecutive bytes an instruction without
+// a shuffle, and the dQ kernel reads a tile by plain bulk copies.
+constexpr int DS_GROUP_BYTES = 32 * 16, DS_BLOCK_BYTES = 16 * DS_GROUP_BYTES;
+__host__ __device__ __forceinline__ int64_t ds_head_tiles(int T, int causal) {
+  const int64_t nt = (T + BLK - 1) / BLK;
+  return causal ? nt * (nt + 1) / 2 : nt * nt;
+}
+template <bool SPLIT> __host__ __device__ __forceinline__ int64_t ds_tile_offset(int64_t head, int qt, int kt, int T, int causal) {
+  const int nt = (T + BLK - 1) / BLK;
+  return (head * ds_head_tiles(T, causal) + (causal ? (int64_t)qt * (qt + 1) / 2 : (int64_t)qt * nt) + kt) * (SPLIT ? 8 : 4) * DS_BLOCK_BYTES;
+}
 
 // What a CTA looks like.  It keeps two 128-row tiles (Q and dY, or K and V) and streams the other two tensors BN rows a step.
 //   WIDE    128 rows a step, sixteen element-wise warps (four threads per row, 32 columns each), all of TMEM, one CTA per SM.
@@ -92,6 +108,8 @@ struct BwdParams {
   void* out1;          // dkdv kernel: dV
   int* status;
   int T, causal, H;
+  int bh0;             // first (batch, head) of this launch
+  uint8_t* ds;         // DS: the dS tiles of this launch's heads (see ds_tile_offset)
   int group;           // (batch, head) pairs whose CTAs are interleaved longest-first (their tensors fit in L2 together)
   float scale_log2;    // (1/sqrt(HD)) * log2(e)
   float scale;         // 1/sqrt(HD)
@@ -198,7 +216,7 @@ sdpa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   const int in_grp = lin - grp * p.group * (int)gridDim.x;
   const int grp_heads = min(p.group, (int)gridDim.y - grp * p.group);
   const int rank = in_grp / grp_heads;
-  const int bh = grp * p.group + (in_grp - rank * grp_heads), T = p.T;
+  const int bh = p.bh0 + grp * p.group + (in_grp - rank * grp_heads), T = p.T;
   const int bi = bh / p.H, hi = bh - bi * p.H;   // batch item and head
   const int qt = (int)gridDim.x - 1 - rank;
   const int q0 = qt * BLK;
@@ -483,7 +501,11 @@ enum KvBar : int {
   KV_BAR_COUNT = 26
 };
 
-template <int HD, bool SPLIT, bool MASKED, bool NARROW>
+// DS (WIDE CTAs): the dS tiles are also left in p.ds for sdpa_bwd_dq_ds_tc_kernel, half a step's at a time from the registers of the
+// element-wise warps.  They bound the kernel, so it costs 9 % (16 heads of 7001 x 128 333 -> 364 us).  Tried and slower: all of it behind
+// the step's last hand-over (366; split 64-wide heads 111 -> 117), a bulk copy from shared memory that a stage of Q gives up (400), four
+// warps of their own that read dS^T back from TMEM and keep the next dP^T waiting for it (418).
+template <int HD, bool SPLIT, bool MASKED, bool NARROW, bool DS>
 __global__ void __launch_bounds__((BwdPlan<SPLIT ? 128 : HD, NARROW>::THREADS), (BwdPlan<SPLIT ? 128 : HD, NARROW>::CTAS_PER_SM))
 sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                         const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
@@ -505,13 +527,14 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   const int in_grp = lin - grp * p.group * (int)gridDim.x;
   const int grp_heads = min(p.group, (int)gridDim.y - grp * p.group);
   const int rank = in_grp / grp_heads;
-  const int bh = grp * p.group + (in_grp - rank * grp_heads), T = p.T;
+  const int bh = p.bh0 + grp * p.group + (in_grp - rank * grp_heads), T = p.T;
   const int bi = bh / p.H, hi = bh - bi * p.H;   // batch item and head
   const int kt = rank;                  // key tile; tile 0 has the most causal work and comes first
   const int k0 = kt * BLK;
   const int i_begin = p.causal ? k0 / BN : 0;
   const int n = (T + BN - 1) / BN - i_begin;    // query steps to walk
 
+  static_assert(!DS || !NARROW);
   // the aligned plan must fit in what was requested (it does unless the dynamic base is unusually placed)
   uint32_t dyn_bytes;
   asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_bytes));
@@ -722,6 +745,11 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(KV_LD_READY));
     };
+    // DS: where this thread's key and its quarter's queries of the first query tile are
+    constexpr int SUBS = SPLIT ? 2 : 1;
+    uint8_t* d = nullptr;
+    if constexpr (DS)
+      d = p.ds + ds_tile_offset<SPLIT>(bh - p.bh0, i_begin, kt, T, p.causal) + (warp & 3) * SUBS * DS_BLOCK_BYTES + qtr * 4 * DS_GROUP_BYTES + lane * 16;
     if (n > 0) stage(0, fetch(0));
     for (int it = 0; it < n && ok; ++it) {
       const int q_local = qtr * 32;                         // first of this thread's 32 queries within the tile
@@ -830,14 +858,38 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
           }
         }
       };
+      // the same registers once more, to memory.  In the diagonal tile the pairs that the causal mask hides, and everywhere the keys beyond
+      // T, are zeros there whatever dP is: dQ is a sum over them, dK's rows are not.
+      auto pass_on = [&](int half) {
+        if constexpr (DS) {
+          if (diag || k0 + BLK > T) {
+            const int hidden = kj >= T ? 32 : diag ? kj - q_base : 0;   // of this thread's queries
+#pragma unroll
+            for (int i = 8 * half; i < 8 * half + 8; ++i) {
+              const uint32_t keep = (2 * i < hidden ? 0u : 0x0000ffffu) | (2 * i + 1 < hidden ? 0u : 0xffff0000u);
+              pk[i] &= keep;
+              if constexpr (SPLIT) pk_lo[i] &= keep;
+            }
+          }
+#pragma unroll
+          for (int g = 2 * half; g < 2 * half + 2; ++g) {
+            *reinterpret_cast<uint4*>(d + g * DS_GROUP_BYTES) = make_uint4(pk[4 * g], pk[4 * g + 1], pk[4 * g + 2], pk[4 * g + 3]);
+            if constexpr (SPLIT)
+              *reinterpret_cast<uint4*>(d + DS_BLOCK_BYTES + g * DS_GROUP_BYTES) = make_uint4(pk_lo[4 * g], pk_lo[4 * g + 1], pk_lo[4 * g + 2], pk_lo[4 * g + 3]);
+          }
+        }
+      };
       form_ds(0, 16);
       store_half(C_DPT, 0);
       form_ds(16, 24);
       hand_over(KV_DST_HALF);
+      pass_on(0);
       form_ds(24, 32);
       store_half(C_DPT, 1);
       if (it + 1 < n) stage(it + 1, next);
       hand_over(KV_DST_READY);
+      pass_on(1);
+      if constexpr (DS) d += (int64_t)(p.causal ? i_begin + it + 1 : (int)gridDim.x) * (4 * SUBS * DS_BLOCK_BYTES);   // the next query tile's
     }
     if (ok && n > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar(KV_DV_DONE), 0, p.status, 234, n));
     constexpr int ESZ = SPLIT ? 4 : 2, PR = HD * ESZ / 16;
@@ -865,6 +917,162 @@ sdpa_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   tc_fence_before();
   __syncthreads();
   if (warp == WARP_MMA) { tc_fence_after(); tmem_dealloc(tmem_base, TMEM_COLS); }
+}
+
+// ---------------------------------------------------------------------------------------------
+// dQ from the dS the dK/dV kernel left: dQ = dS K, one product instead of three.  A CTA accumulates QT query tiles of one head in
+// TMEM (columns [0, QT HD)) and streams steps of 64 keys: the halves of their dS tiles by bulk copies, the K rows by TMA.
+// Bound by the bytes of dS (HBM, or L2 where it is still there), so the ring is as deep as it fits: QT = 2 for 128-wide heads,
+// whose K rows are as many bytes as a dS half and are read once for both; QT = 1 and two CTAs per SM for the others, whose items are
+// short: one's first loads and last stores run beside the other's steps.
+// ---------------------------------------------------------------------------------------------
+template <int HD, bool SPLIT> struct DqDsPlan {
+  static constexpr int QT = HD == 128 ? 2 : 1, BN = 64, EW_WARPS = 8, WARP_TMA = 8, WARP_MMA = 9, THREADS = 320;
+  static constexpr int CTAS_PER_SM = QT == 2 ? 1 : 2;
+  static constexpr int SUB = SPLIT ? 2 : HD / 64;
+  static constexpr uint32_t SUB_BYTES = BN * 128, K_BYTES = SUB * SUB_BYTES;
+  static constexpr uint32_t HALF_BYTES = (SPLIT ? 4 : 2) * DS_BLOCK_BYTES;   // one query tile's dS of a step
+  static constexpr uint32_t STAGE_BYTES = QT * HALF_BYTES + K_BYTES;
+  static constexpr int STAGES = QT == 2 ? 4 : (SPLIT ? 2 : 4);
+  static constexpr uint32_t OFF_BAR = STAGES * STAGE_BYTES, BYTES = OFF_BAR + 128 + 1024;
+  static constexpr uint32_t TMEM_COLS = QT * HD < 32 ? 32 : QT * HD;
+  static_assert(STAGES * STAGE_BYTES >= (uint32_t)(QT * BLK * HD * (SPLIT ? 4 : 2)), "the finished tiles are staged in the ring");
+  static_assert(CTAS_PER_SM * (BYTES + 1024 + 64) <= 228 * 1024, "shared memory of the CTAs of one SM");
+};
+
+template <int HD, bool SPLIT>
+__global__ void __launch_bounds__((DqDsPlan<HD, SPLIT>::THREADS), (DqDsPlan<HD, SPLIT>::CTAS_PER_SM))
+sdpa_bwd_dq_ds_tc_kernel(const __grid_constant__ CUtensorMap map_k, const BwdParams p) {
+  using PL = DqDsPlan<HD, SPLIT>;
+  constexpr int QT = PL::QT, BN = PL::BN, EW_WARPS = PL::EW_WARPS, STAGES = PL::STAGES;
+  constexpr int FMT = SPLIT ? 0 : 1;
+  constexpr int FULL = 0, EMPTY = STAGES, DONE = 2 * STAGES, BAR_COUNT = 2 * STAGES + 1;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
+  auto bar = [&](int i) { return smem_base + PL::OFF_BAR + 8u * (uint32_t)i; };
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + PL::OFF_BAR + BAR_COUNT * 8);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, T = p.T;
+  // longest causal work first; the heads the dK/dV kernel wrote last, whose dS is still in L2, come first
+  const int heads = (int)gridDim.y, lin = (int)(blockIdx.y * gridDim.x + blockIdx.x);
+  const int n_groups = (heads + p.group - 1) / p.group, last = heads - (n_groups - 1) * p.group;   // heads of the last group
+  int grp, in_grp, grp_heads;
+  if (lin < last * (int)gridDim.x) { grp = n_groups - 1; in_grp = lin; grp_heads = last; }
+  else {
+    const int rest = lin - last * (int)gridDim.x, back = rest / (p.group * (int)gridDim.x);
+    grp = n_groups - 2 - back; in_grp = rest - back * p.group * (int)gridDim.x; grp_heads = p.group;
+  }
+  const int rank = in_grp / grp_heads;
+  const int head = grp * p.group + (in_grp - rank * grp_heads), bh = p.bh0 + head;
+  const int bi = bh / p.H, hi = bh - bi * p.H;
+  const int qt0 = ((int)gridDim.x - 1 - rank) * QT;
+  const int steps_T = (T + BN - 1) / BN, nt = (T + BLK - 1) / BLK;
+  // key steps that query tile qt0 + t sees
+  auto steps_of = [&](int t) { return qt0 + t >= nt ? 0 : p.causal ? min(2 * (qt0 + t + 1), steps_T) : steps_T; };
+  const int n0 = steps_of(0), n1 = QT == 2 ? steps_of(1) : 0, n = max(n0, n1);
+
+  __shared__ int s_abort;
+  mca_pdl_launch_dependents();
+  if (warp == PL::WARP_TMA && lane == 0) prefetch_tensormap(&map_k);
+  if (tid == 0) {
+    for (int i = 0; i < BAR_COUNT; ++i) mbar_init(bar(i), 1u);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == PL::WARP_MMA) { tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), PL::TMEM_COLS); tmem_relinquish(); }
+  mca_pdl_wait();   // dS is the kernel before's
+  if (tid == 32) s_abort = *reinterpret_cast<volatile int*>(p.status);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  if (s_abort != 0) {   // uniform, before any copy or product is issued
+    if (warp == PL::WARP_MMA) tmem_dealloc(tmem_base, PL::TMEM_COLS);
+    return;
+  }
+  bool ok = true;
+  if (warp == PL::WARP_TMA) {
+    if (lane == 0) {
+      int issued = 0;
+      for (int j = 0; j < n; ++j) {
+        const int s = j % STAGES;
+        ok = mbar_wait(bar(EMPTY + s), (uint32_t)((j / STAGES) & 1) ^ 1u, p.status, 310, j);
+        if (!ok) break;
+        const uint32_t dst = smem_base + s * PL::STAGE_BYTES, full = bar(FULL + s);
+        const int tiles = (j < n0 ? 1 : 0) + (j < n1 ? 1 : 0);
+        mbar_expect_tx(full, PL::K_BYTES + tiles * PL::HALF_BYTES);
+#pragma unroll
+        for (int t = 0; t < QT; ++t)
+          if (j < (t == 0 ? n0 : n1)) {
+            const uint8_t* src = p.ds + ds_tile_offset<SPLIT>(head, qt0 + t, j >> 1, T, p.causal) + (j & 1) * PL::HALF_BYTES;
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                             dst + t * PL::HALF_BYTES),
+                         "l"(src), "r"(PL::HALF_BYTES), "r"(full)
+                         : "memory");
+          }
+#pragma unroll
+        for (int b = 0; b < PL::SUB; ++b)
+          tma_load_4d(dst + QT * PL::HALF_BYTES + b * PL::SUB_BYTES, &map_k, full, b * 64, j * BN, hi, bi);
+        issued = j + 1;
+      }
+      if (!ok)  // let copies in flight land (bounded) before the CTA's memory is released
+        for (int j = max(0, issued - STAGES); j < issued; ++j)
+          mbar_wait(bar(FULL + j % STAGES), (uint32_t)((j / STAGES) & 1), p.status, 311, j);
+    }
+  } else if (warp == PL::WARP_MMA) {
+    const uint32_t leader = elect_one() ? 1u : 0u;
+    const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
+    constexpr uint32_t IDESC = make_idesc_fmt(BLK, HD, 1, 1, FMT);   // both operands MN-major
+    for (int j = 0; j < n && ok; ++j) {
+      const int s = j % STAGES;
+      ok = __all_sync(0xffffffffu, mbar_wait(bar(FULL + s), (uint32_t)((j / STAGES) & 1), p.status, 320, j));
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t a_addr = smem_base + s * PL::STAGE_BYTES, k_addr = a_addr + QT * PL::HALF_BYTES;
+#pragma unroll
+      for (int t = 0; t < QT; ++t)
+        if (j < (t == 0 ? n0 : n1)) {
+#pragma unroll
+          for (int kk = 0; kk < BN / 16; ++kk) {
+            const uint32_t a = a_addr + t * PL::HALF_BYTES + (kk / 2) * (PL::HALF_BYTES / 2) + (kk % 2) * 256;
+            const uint64_t a_hi = make_desc_plain(a, 128, DS_GROUP_BYTES);
+            const uint64_t b_hi = make_desc(k_addr + kk * 2048, PL::SUB_BYTES, 1024);
+            umma_ss_if<false>(leader, tmem_u + t * HD, a_hi, b_hi, IDESC, (j > 0 || kk > 0) ? 1u : 0u);
+            if constexpr (SPLIT) {   // + dS_hi K_lo + dS_lo K_hi
+              umma_ss_if<false>(leader, tmem_u + t * HD, a_hi, make_desc(k_addr + PL::SUB_BYTES + kk * 2048, PL::SUB_BYTES, 1024), IDESC, 1u);
+              umma_ss_if<false>(leader, tmem_u + t * HD, make_desc_plain(a + DS_BLOCK_BYTES, 128, DS_GROUP_BYTES), b_hi, IDESC, 1u);
+            }
+          }
+        }
+      umma_commit_if(leader, bar(EMPTY + s));
+    }
+    umma_commit_if(leader, bar(DONE));
+    mbar_wait(bar(DONE), 0, p.status, 321, 0);
+  } else {
+    // eight warps: with QT = 2 four a tile, a thread a whole row; with QT = 1 a thread half a row
+    const int t = QT == 2 ? warp >> 2 : 0, half = QT == 2 ? 0 : warp >> 2, lane_base = (warp & 3) * 32, row = lane_base + lane;
+    constexpr int OC = QT == 2 ? HD : HD / 2, ESZ = SPLIT ? 4 : 2, PR = HD * ESZ / 16;
+    const int q0 = (qt0 + t) * BLK;
+    uint8_t* tile = smem_gen + t * (BLK * HD * ESZ);
+    ok = __all_sync(0xffffffffu, mbar_wait(bar(DONE), 0, p.status, 330, n));
+    ok = ok && *reinterpret_cast<volatile int*>(p.status) == 0;
+    const bool fin = __all_sync(0xffffffffu, ok) && q0 < T;
+    if (fin) {
+      tc_fence_after();
+      float4 sc = make_float4(1.f, 1.f, 1.f, 1.f);
+      if constexpr (SPLIT) sc = mca_ld_f4(reinterpret_cast<const float*>(p.scales + bh));
+      const float2 mul = split::pow2_factors(-DS_SHIFT_LOG2 - split::scale_exp(sc.y) - split::scale_exp(sc.z) - split::scale_exp(sc.w));
+      stage_columns<PR, OC, SPLIT>(tile, row, half, tmem_base + ((uint32_t)lane_base << 16) + t * HD + half * OC, p.scale, mul);
+    }
+    ew_bar_sync<EW_WARPS>();
+    if (fin) {
+      constexpr int RPW = BLK * QT / EW_WARPS;
+      store_staged_rows<PR, ESZ, RPW>(tile, QT == 2 ? (warp & 3) : warp, lane, p.out0, (int64_t)bi * p.os.b + (int64_t)hi * p.os.h + (int64_t)q0 * p.os.t,
+                                      p.os.t, min(BLK, T - q0));
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == PL::WARP_MMA) { tc_fence_after(); tmem_dealloc(tmem_base, PL::TMEM_COLS); }
 }
 
 // delta[row] = sum_c dY[row][c] * Y[row][c]  (bf16 inputs, fp32 result).  D / 8 lanes share a row (16-byte loads), so a
@@ -909,20 +1117,71 @@ __global__ void __launch_bounds__(256) bwd_delta_bf16_kernel(const __nv_bfloat16
   }
 }
 
+// Is dS formed once and passed through memory?  Instead of S, dP and the exponentials a second time the dQ kernel then reads two (split:
+// four) bytes a pair from HBM, and the dK/dV kernel writes them from the warps that bound it (7001 x 128: 333 -> 364 us, dQ 253 -> 134); but
+// it waits for the whole dK/dV kernel, where the other one fills that kernel's last wave.  So there must be waves enough: 128-wide bf16
+// heads gain from about two times the longest CTA's work per SM (whole layer, us: 16 x 512 x 512 rows 96.7 -> 90.0, 16 heads of 4096 328 -> 312,
+// of 7001 878 -> 847, 192 of 1024 400 -> 367, 32 of 1024 68.3 -> 66.5; 16 heads of 2048 103.5 -> 103.6, 8 of 4096 180 -> 183).  64-wide split heads
+// have half the products to save and twice the bytes: short ones gain from their two CTAs per SM (256 of 128 59.8 -> 56.6, 192 of
+// 256 99.9 -> 93.9, 64 of 512 under a key mask 117.0 -> 110.9), long ones with many waves (96 of 1024 301 -> 295.5; 48 of
+// 1024 149.7 -> 151.4, 16 of 2048 159 -> 170).  Narrower split heads lose (96 of 1024 x 32 205 -> 218), and 64-wide bf16 ones, whose
+// narrow CTAs leave the element-wise warps no time for it, too (96 of 1024 120 -> 131).
+template <int HD, bool SPLIT> constexpr bool passes_ds(int64_t heads, int T, int causal) {
+  const int64_t nt = (T + BLK - 1) / BLK;
+  if (HD < 64 || (HD == 64 && !SPLIT)) return false;
+  if (!SPLIT) return heads * (causal ? nt + 1 : 2 * nt) >= 288;
+  return heads * nt >= (nt <= 4 ? 256 : 768);
+}
+// What the caller has for the dS tiles, and how many heads at a time go through it (0: none).
+struct DsRoom {
+  uint8_t* ptr;
+  int64_t bytes;
+};
+template <int HD, bool SPLIT> int ds_heads(const DsRoom& room, int64_t heads, int T, int causal) {
+  const int64_t fit = room.ptr == nullptr ? 0 : std::min<int64_t>(room.bytes / ds_tile_offset<SPLIT>(1, 0, 0, T, causal), heads);
+  if (fit == 0) return 0;
+  const int64_t launches = (heads + fit - 1) / fit, chunk = (heads + launches - 1) / launches;   // alike in size
+  return passes_ds<HD, SPLIT>(heads / launches, T, causal) ? (int)chunk : 0;
+}
+
 // Both kernels of one backward, with or without the caller's mask.
 template <int HD, bool SPLIT, bool MASKED, bool NARROW>
-int launch_bwd_pair(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mdo, BwdParams p,
-                    void* dq, void* dk, void* dv, int B, int H, int T, cudaStream_t st) {
+int launch_bwd_pair(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mdo, const CUtensorMap& mk64, BwdParams p,
+                    void* dq, void* dk, void* dv, int B, int H, int T, const DsRoom& room, cudaStream_t st) {
   using PL = BwdPlan<SPLIT ? 128 : HD, NARROW>;
-  const size_t smem_kv = PL::BYTES_KV, smem_dq = PL::BYTES_DQ;
-  static std::atomic<uint64_t> done_kv{0}, done_dq{0};
+  const size_t smem_kv = PL::BYTES_KV;
   int e;
-  if ((e = mca_smem_once(done_kv, sdpa_bwd_dkdv_tc_kernel<HD, SPLIT, MASKED, NARROW>, smem_kv)) ||
+  if constexpr (passes_ds<HD, SPLIT>(1 << 30, BLK, 0)) {
+    if (const int chunk = ds_heads<HD, SPLIT>(room, (int64_t)B * H, T, p.causal)) {
+      using PD = DqDsPlan<HD, SPLIT>;
+      static std::atomic<uint64_t> done_kv{0}, done_dq{0};
+      if ((e = mca_smem_once(done_kv, sdpa_bwd_dkdv_tc_kernel<HD, SPLIT, MASKED, NARROW, true>, smem_kv)) ||
+          (e = mca_smem_once(done_dq, sdpa_bwd_dq_ds_tc_kernel<HD, SPLIT>, (size_t)PD::BYTES)))
+        return e;
+      const int nt = mca_ceil_div(T, BLK), group = p.group;
+      p.ds = room.ptr;
+      for (p.bh0 = 0; p.bh0 < B * H; p.bh0 += chunk) {
+        const int heads = std::min(chunk, B * H - p.bh0);
+        p.group = std::min(group, heads);
+        p.out0 = dk; p.out1 = dv;
+        if ((e = mca_launch_pdl(sdpa_bwd_dkdv_tc_kernel<HD, SPLIT, MASKED, NARROW, true>, dim3(nt, heads), dim3(PL::THREADS), smem_kv, st, mq, mk, mv, mdo, p)))
+          return e;
+        p.out0 = dq; p.out1 = nullptr;
+        if ((e = mca_launch_pdl(sdpa_bwd_dq_ds_tc_kernel<HD, SPLIT>, dim3(mca_ceil_div(nt, PD::QT), heads), dim3(PD::THREADS), (size_t)PD::BYTES, st, mk64, p)))
+          return e;
+      }
+      return 0;
+    }
+  }
+  const size_t smem_dq = PL::BYTES_DQ;
+  static std::atomic<uint64_t> done_kv{0}, done_dq{0};
+  if ((e = mca_smem_once(done_kv, sdpa_bwd_dkdv_tc_kernel<HD, SPLIT, MASKED, NARROW, false>, smem_kv)) ||
       (e = mca_smem_once(done_dq, sdpa_bwd_dq_tc_kernel<HD, SPLIT, MASKED, NARROW>, smem_dq)))
     return e;
   dim3 grid(mca_ceil_div(T, BLK), B * H);
+  p.ds = nullptr; p.bh0 = 0;
   p.out0 = dk; p.out1 = dv;
-  e = mca_launch_pdl(sdpa_bwd_dkdv_tc_kernel<HD, SPLIT, MASKED, NARROW>, grid, dim3(PL::THREADS), smem_kv, st, mq, mk, mv, mdo, p);
+  e = mca_launch_pdl(sdpa_bwd_dkdv_tc_kernel<HD, SPLIT, MASKED, NARROW, false>, grid, dim3(PL::THREADS), smem_kv, st, mq, mk, mv, mdo, p);
   if (e) return e;
   p.out0 = dq; p.out1 = nullptr;
   return mca_launch_pdl(sdpa_bwd_dq_tc_kernel<HD, SPLIT, MASKED, NARROW>, grid, dim3(PL::THREADS), smem_dq, st, mq, mk, mv, mdo, p);
@@ -939,15 +1198,16 @@ void set_mask(BwdParams& p, const McaMaskBits* mask, int T) {
 template <int HD>
 int launch_bwd(const void* q, const void* k, const void* v, const void* dy, const float* lse, const float* delta,
                int causal, int B, int H, int T, void* dq, void* dk, void* dv, int* status, int layout, cudaStream_t st,
-               const McaMaskBits* mask = nullptr) {
+               const McaMaskBits* mask, const DsRoom& room) {
   if (mask != nullptr && causal) return ERROR_ATTN_UNSUPPORTED_SHAPE;
   constexpr bool NARROW = HD <= 64;
   constexpr int BN = BwdPlan<HD, NARROW>::BN;
-  CUtensorMap mq, mk, mv, mdo;
+  CUtensorMap mq, mk, mv, mdo, mk64;
   int e;
   const McaStrides sin = mca_in_strides(layout, H, T, HD), sout = mca_out_strides(layout, H, T, HD);
   if ((e = make_map_bf16(&mq, q, B, H, T, HD, sin, BN)) || (e = make_map_bf16(&mk, k, B, H, T, HD, sin, BN)) ||
-      (e = make_map_bf16(&mv, v, B, H, T, HD, sin, BN)) || (e = make_map_bf16(&mdo, dy, B, H, T, HD, sout, BN)))
+      (e = make_map_bf16(&mv, v, B, H, T, HD, sin, BN)) || (e = make_map_bf16(&mdo, dy, B, H, T, HD, sout, BN)) ||
+      (e = make_map_bf16(&mk64, k, B, H, T, HD, sin, 64)))
     return e;
   BwdParams p;
   p.scales = nullptr;
@@ -961,8 +1221,8 @@ int launch_bwd(const void* q, const void* k, const void* v, const void* dy, cons
   p.scale = 1.0f / sqrtf((float)HD);
   p.scale_log2 = p.scale * 1.4426950408889634f;
   set_mask(p, mask, T);
-  if (mask != nullptr) return launch_bwd_pair<HD, false, true, NARROW>(mq, mk, mv, mdo, p, dq, dk, dv, B, H, T, st);
-  return launch_bwd_pair<HD, false, false, NARROW>(mq, mk, mv, mdo, p, dq, dk, dv, B, H, T, st);
+  if (mask != nullptr) return launch_bwd_pair<HD, false, true, NARROW>(mq, mk, mv, mdo, mk64, p, dq, dk, dv, B, H, T, room, st);
+  return launch_bwd_pair<HD, false, false, NARROW>(mq, mk, mv, mdo, mk64, p, dq, dk, dv, B, H, T, room, st);
 }
 
 // Split-operand backward for fp32 callers.  The workspace still holds the fp16 halves of q, k, v the forward's pre-pass
@@ -970,7 +1230,7 @@ int launch_bwd(const void* q, const void* k, const void* v, const void* dy, cons
 template <int HD>
 int launch_bwd_split(const float* dy, const float* y_copy, const float* lse, float* delta, int causal, int B, int H, int T,
                      float* dq, float* dk, float* dv, void* workspace, int* status, int layout, cudaStream_t st,
-                     const McaMaskBits* mask = nullptr) {
+                     const McaMaskBits* mask, const DsRoom& room) {
   if (mask != nullptr && causal) return ERROR_ATTN_UNSUPPORTED_SHAPE;
   const split::Workspace w = split::carve(workspace, (int64_t)B * H, T);
   const McaStrides sin = mca_in_strides(layout, H, T, HD), sout = mca_out_strides(layout, H, T, HD);
@@ -980,13 +1240,15 @@ int launch_bwd_split(const float* dy, const float* y_copy, const float* lse, flo
   // the kernel that splits dY also forms delta = rowsum(dY o Y) from the elements it holds
   int e = split::run<HD>(job, 1, sout, B, H, T, w, st, y_copy, delta);
   if (e) return e;
-  CUtensorMap mq, mk, mv, mdo;
+  CUtensorMap mq, mk, mv, mdo, mk64;
   const McaStrides sp{(int64_t)H * T * 128, (int64_t)T * 128, 128};
   const CUtensorMap* maps[4] = {&mq, &mk, &mv, &mdo};
   for (int i = 0; i < 4; ++i)
     if ((e = make_map_4d(const_cast<CUtensorMap*>(maps[i]), w.tensor[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, B, H, T, 128, sp,
                          CU_TENSOR_MAP_SWIZZLE_128B)))
       return e;
+  if ((e = make_map_4d(&mk64, w.tensor[split::TENSOR_K], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, B, H, T, 128, sp, CU_TENSOR_MAP_SWIZZLE_128B, 64)))
+    return e;
   BwdParams p;
   p.scales = w.scale;
   p.lse = lse; p.delta = delta; p.status = status; p.T = T; p.causal = causal; p.H = H;
@@ -998,8 +1260,8 @@ int launch_bwd_split(const float* dy, const float* y_copy, const float* lse, flo
   p.scale = 1.0f / sqrtf((float)HD);
   p.scale_log2 = p.scale * 1.4426950408889634f;
   set_mask(p, mask, T);
-  if (mask != nullptr) return launch_bwd_pair<HD, true, true, false>(mq, mk, mv, mdo, p, dq, dk, dv, B, H, T, st);
-  return launch_bwd_pair<HD, true, false, false>(mq, mk, mv, mdo, p, dq, dk, dv, B, H, T, st);
+  if (mask != nullptr) return launch_bwd_pair<HD, true, true, false>(mq, mk, mv, mdo, mk64, p, dq, dk, dv, B, H, T, room, st);
+  return launch_bwd_pair<HD, true, false, false>(mq, mk, mv, mdo, mk64, p, dq, dk, dv, B, H, T, room, st);
 }
 
 }  // namespace
@@ -1022,6 +1284,20 @@ int mca_sdpa_backward_tc_masked(const void* q, const void* k, const void* v, con
                                 float* delta_scratch, int dtype, int causal, int B, int H, int T, int D, void* dq, void* dk,
                                 void* dv, int* status, int layout, const uint32_t* mask_bits, const uint32_t* mask_bits_t,
                                 int mask_mode, void* stream) {
+  return mca_sdpa_backward_tc_ws(q, k, v, y, dy, lse, delta_scratch, dtype, causal, B, H, T, D, dq, dk, dv, status, layout, mask_bits,
+                                 mask_bits_t, mask_mode, nullptr, 0, stream);
+}
+
+int64_t mca_sdpa_backward_tc_ws_bytes(int B, int H, int T, int D, int split) {
+  const int64_t heads = (int64_t)B * H;   // of the causal form: where the mask is another one they go through it in two parts
+  if (split ? D != 64 || !passes_ds<64, true>(heads, T, 1) : D != 128 || !passes_ds<128, false>(heads, T, 1)) return 0;
+  return split ? ds_tile_offset<true>(heads, 0, 0, T, 1) : ds_tile_offset<false>(heads, 0, 0, T, 1);
+}
+
+int mca_sdpa_backward_tc_ws(const void* q, const void* k, const void* v, const void* y, const void* dy, const float* lse,
+                            float* delta_scratch, int dtype, int causal, int B, int H, int T, int D, void* dq, void* dk, void* dv,
+                            int* status, int layout, const uint32_t* mask_bits, const uint32_t* mask_bits_t, int mask_mode, void* ds,
+                            int64_t ds_bytes, void* stream) {
   McaMaskBits mb;
   const McaMaskBits* mask = nullptr;
   int me = mca_mask_bits_view(mask_bits, mask_bits_t, mask_mode, T, true, &mb, &mask);
@@ -1044,8 +1320,9 @@ int mca_sdpa_backward_tc_masked(const void* q, const void* k, const void* v, con
                        (const __nv_bfloat16*)dy, (const __nv_bfloat16*)y, rows, H, T, D, mca_out_strides(layout, H, T, D), delta_scratch);
   }
   if (e) return e;
-  if (D == 128) return launch_bwd<128>(q, k, v, dy, lse, delta_scratch, causal, B, H, T, dq, dk, dv, status, layout, st, mask);
-  return launch_bwd<64>(q, k, v, dy, lse, delta_scratch, causal, B, H, T, dq, dk, dv, status, layout, st, mask);
+  const DsRoom room{static_cast<uint8_t*>(ds), ds_bytes};
+  if (D == 128) return launch_bwd<128>(q, k, v, dy, lse, delta_scratch, causal, B, H, T, dq, dk, dv, status, layout, st, mask, room);
+  return launch_bwd<64>(q, k, v, dy, lse, delta_scratch, causal, B, H, T, dq, dk, dv, status, layout, st, mask, room);
 }
 
 int mca_sdpa_backward_f32_tc(const float* dy, const float* y_copy, const float* lse, float* delta_scratch, int causal, int B,
@@ -1059,6 +1336,14 @@ int mca_sdpa_backward_f32_tc_masked(const float* dy, const float* y_copy, const 
                                     int B, int H, int T, int D, float* dq, float* dk, float* dv, void* workspace,
                                     int64_t workspace_bytes, int* status, int layout, const uint32_t* mask_bits,
                                     const uint32_t* mask_bits_t, int mask_mode, void* stream) {
+  return mca_sdpa_backward_f32_tc_ws(dy, y_copy, lse, delta_scratch, causal, B, H, T, D, dq, dk, dv, workspace, workspace_bytes, status,
+                                     layout, mask_bits, mask_bits_t, mask_mode, nullptr, 0, stream);
+}
+
+int mca_sdpa_backward_f32_tc_ws(const float* dy, const float* y_copy, const float* lse, float* delta_scratch, int causal, int B, int H,
+                                int T, int D, float* dq, float* dk, float* dv, void* workspace, int64_t workspace_bytes, int* status,
+                                int layout, const uint32_t* mask_bits, const uint32_t* mask_bits_t, int mask_mode, void* ds,
+                                int64_t ds_bytes, void* stream) {
   McaMaskBits mb;
   const McaMaskBits* mask = nullptr;
   int me = mca_mask_bits_view(mask_bits, mask_bits_t, mask_mode, T, true, &mb, &mask);
@@ -1072,10 +1357,11 @@ int mca_sdpa_backward_f32_tc_masked(const float* dy, const float* y_copy, const 
        reinterpret_cast<uintptr_t>(dv) | reinterpret_cast<uintptr_t>(workspace)) & 15)
     return ERROR_PARAM_OUT_OF_RANGE;
   cudaStream_t st = (cudaStream_t)stream;
+  const DsRoom room{static_cast<uint8_t*>(ds), ds_bytes};
   switch (D) {
-    case 16: return launch_bwd_split<16>(dy, y_copy, lse, delta_scratch, causal, B, H, T, dq, dk, dv, workspace, status, layout, st, mask);
-    case 32: return launch_bwd_split<32>(dy, y_copy, lse, delta_scratch, causal, B, H, T, dq, dk, dv, workspace, status, layout, st, mask);
-    case 64: return launch_bwd_split<64>(dy, y_copy, lse, delta_scratch, causal, B, H, T, dq, dk, dv, workspace, status, layout, st, mask);
+    case 16: return launch_bwd_split<16>(dy, y_copy, lse, delta_scratch, causal, B, H, T, dq, dk, dv, workspace, status, layout, st, mask, room);
+    case 32: return launch_bwd_split<32>(dy, y_copy, lse, delta_scratch, causal, B, H, T, dq, dk, dv, workspace, status, layout, st, mask, room);
+    case 64: return launch_bwd_split<64>(dy, y_copy, lse, delta_scratch, causal, B, H, T, dq, dk, dv, workspace, status, layout, st, mask, room);
   }
   return ERROR_ATTN_UNSUPPORTED_SHAPE;
 }

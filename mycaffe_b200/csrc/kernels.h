@@ -19,6 +19,18 @@ int mca_sdpa_backward_f32_ws(const float* q, const float* k, const float* v, con
                              int B, int H, int T, int D, float* dq, float* dk, float* dv, float* ds, int64_t ds_floats, int layout,
                              void* stream);
 
+// Internal: mca_sdpa_backward_tc_masked and mca_sdpa_backward_f32_tc_masked with room for dS between their two kernels (16-byte
+// aligned; null, or room for too few heads: dS is formed twice).  _ws_bytes: for all heads at once under the causal mask, 0 where it would not be used.
+int64_t mca_sdpa_backward_tc_ws_bytes(int B, int H, int T, int D, int split);
+int mca_sdpa_backward_tc_ws(const void* q, const void* k, const void* v, const void* y, const void* dy, const float* lse,
+                            float* delta_scratch, int dtype, int causal, int B, int H, int T, int D, void* dq, void* dk, void* dv,
+                            int* status, int layout, const uint32_t* mask_bits, const uint32_t* mask_bits_t, int mask_mode, void* ds,
+                            int64_t ds_bytes, void* stream);
+int mca_sdpa_backward_f32_tc_ws(const float* dy, const float* y_copy, const float* lse, float* delta_scratch, int causal, int B, int H,
+                                int T, int D, float* dq, float* dk, float* dv, void* workspace, int64_t workspace_bytes, int* status,
+                                int layout, const uint32_t* mask_bits, const uint32_t* mask_bits_t, int mask_mode, void* ds,
+                                int64_t ds_bytes, void* stream);
+
 // Internal: the two halves of mca_sdpa_forward_f32_tc_masked -- the pre-pass that splits q, k, v (and classifies the caller's
 // (T,T) mask in the same launch when `cls` is given), and the kernel, which may then be chosen on the class.
 int mca_split_forward_prepass(const float* q, const float* k, const float* v, int B, int H, int T, int D, void* workspace,

@@ -362,6 +362,11 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr, uint32_t lbo_b
   d |= (uint64_t)2 << 61;
   return d;
 }
+// MN-major operand without a swizzle: 8 MN x 8 K blocks of 128 bytes (a K index is 16 bytes), the next 8 K indices LBO bytes and the
+// next 8 MN indices SBO bytes later.
+__device__ __forceinline__ uint64_t make_desc_plain(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
+  return make_desc(smem_addr, lbo_bytes, sbo_bytes) & ~((uint64_t)7 << 61);
+}
 // Instruction descriptor, kind::f16, bf16 x bf16 -> fp32: c_format [4,6) = 1 (F32), a_format
 // [7,10) = 1 (BF16), b_format [10,13) = 1, a_major bit 15, b_major bit 16 (0 = K-major,
 // 1 = MN-major), N >> 3 at [17,23), M >> 4 at [24,29).

@@ -1,0 +1,68 @@
+"""The tensor-core backward where dS passes through memory: heads enough for that (128-wide bf16 and 64-wide split operands), lengths around
+its tiles and the pairs of them that share a CTA, every mask form, both layouts of a tile's last keys, against the fp64 oracle;
+and heads that go through the workspace in parts."""
+import numpy as np
+import pytest
+
+import oracle
+from gpu_util import Sdpa, bf16_round
+from helpers import rel_err
+from mycaffe_b200 import CudaDnn
+from mycaffe_b200 import function_ids as ids
+
+pytestmark = pytest.mark.gpu
+
+
+def handle(cuda, B, T, H, D, bf16, mode):
+    return Sdpa(cuda, B, T, H, D, training=True, dtype=ids.MCA_DTYPE_BF16 if bf16 else ids.MCA_DTYPE_F32,
+                flags=ids.MCA_FLAG_CAUSAL_IMPLICIT if mode == 3 else 0)
+
+
+@pytest.mark.parametrize("T", [65, 129, 193, 320])
+@pytest.mark.parametrize("bf16", [True, False])
+@pytest.mark.parametrize("kind", ["causal", "none", "keys", "pairs"])
+def test_backward(T, bf16, kind):
+    cuda = CudaDnn(0)
+    rng = np.random.default_rng(T)
+    B, H, D = 8, 18, 128 if bf16 else 64
+    cast = bf16_round if bf16 else (lambda a: a)
+    q, k, v, dy = (cast(rng.standard_normal((B, H, T, D)).astype(np.float32)) for _ in range(4))
+    mode = {"causal": 3, "none": 0, "keys": 2, "pairs": 1}[kind]
+    mask = {"keys": (rng.random((B, T)) > 0.3), "pairs": (rng.random((T, T)) > 0.3)}.get(kind)
+    mask = None if mask is None else mask.astype(np.float32)
+    a = handle(cuda, B, T, H, D, bf16, mode)
+    a.forward(q, k, v, mask, batch_mask=mode == 2)
+    # bf16: P, dS and the results are rounded to 2^-9; split: fp32 sums of products of 22-bit halves, as the path's other tests
+    for name, g, r in zip("qkv", a.backward(dy), oracle.sdpa_backward(q, k, v, dy, mask, mode, f64=True)):
+        assert rel_err(g, r) < (2e-2 if bf16 else 2e-5), name
+    a.close()
+    cuda.Dispose()
+
+
+def test_heads_in_parts():
+    """16 causal heads of 10000 x 128 ask for 1.7 GB and get 1: two launches of each kernel, against the kernels that form dS twice
+    (the raw entry point has no workspace).  Same products, same roundings: bf16's 2^-9 is far above any difference."""
+    import torch
+    from mycaffe_b200 import _lib
+    cuda, lib = CudaDnn(0), _lib.load()
+    H, T, D = 16, 10000, 128
+    gen = torch.Generator("cuda").manual_seed(3)
+    q, k, v, dy = (torch.randn(1, H, T, D, generator=gen, device="cuda").bfloat16() for _ in range(4))
+    a = handle(cuda, 1, T, H, D, True, 3)
+    host = lambda t: t.float().cpu().numpy()
+    y = a.forward(host(q), host(k), host(v), None)
+    got = a.backward(host(dy))
+    a.close()
+    y = torch.from_numpy(y).cuda().bfloat16()
+    lse, delta = torch.empty(H * T, device="cuda"), torch.empty(H * T, device="cuda")
+    status = torch.zeros(8, dtype=torch.int32, device="cuda")
+    grads = [torch.empty_like(q) for _ in range(3)]
+    y2 = torch.empty_like(q)
+    p = lambda t: t.data_ptr()
+    assert lib.mca_sdpa_forward_tc(p(q), p(k), p(v), ids.MCA_DTYPE_BF16, 1, 1, H, T, D, p(y2), p(lse), p(status), None) == 0
+    assert lib.mca_sdpa_backward_tc(p(q), p(k), p(v), p(y), p(dy), p(lse), p(delta), ids.MCA_DTYPE_BF16, 1, 1, H, T, D, *map(p, grads), p(status), None) == 0
+    torch.cuda.synchronize()
+    assert int(status[0]) == 0
+    for g, r in zip(got, grads):
+        assert rel_err(g, host(r)) < 2.0 ** -8
+    cuda.Dispose()
