@@ -612,7 +612,7 @@ long resolve_mask(Kernel* k, AttnHandle& a, long hMask, bool batch_mask, int T, 
 
 // Keep-bits of this call's (T,T) or batch mask, packed into buffers the handle owns (room for the configured block
 // size, allocated on first use).  The backward of the same handle reads what the forward packed.
-long pack_mask_bits(AttnHandle& a, const float* mask, int mode, int T) {
+long mask_bits_room(AttnHandle& a) {
   const size_t rows = (size_t)std::max(a.block, a.B);
   const size_t need = rows * (size_t)mca_mask_bits_row_words(a.block);
   if (a.mask_bits == nullptr || a.mask_bits_words < need) {
@@ -624,6 +624,11 @@ long pack_mask_bits(AttnHandle& a, const float* mask, int mode, int T) {
     }
     a.mask_bits_words = need;
   }
+  return 0;
+}
+long pack_mask_bits(AttnHandle& a, const float* mask, int mode, int T) {
+  const long e = mask_bits_room(a);
+  if (e) return e;
   return mca_mask_pack(mask, mode, a.B, T, a.mask_bits, a.mask_bits_t, 0);
 }
 
@@ -756,14 +761,21 @@ long attn_fwd_once(Kernel* k, long llInput, MCA_LONGLONG* pl, int layout) {
     bool classified = !classify;
     if (a.split_ws != nullptr && (tc_bwd || !save || mode != MCA_MASK_BATCH)) {
       // the operands are split first, with the mask's classification in the same launch; where its answer has to be waited
-      // for, the GPU is busy meanwhile
-      if ((e = mca_split_forward_prepass(q, kk, v, a.B, a.H, T, a.D, a.split_ws, a.split_ws_bytes, layout, classify ? &job : nullptr, 0)))
+      // for, the GPU is busy meanwhile.  A key mask is packed there too.
+      McaPackJob pack;
+      const bool key_bits = mode == MCA_MASK_BATCH;
+      if (key_bits) {
+        if ((e = mask_bits_room(a))) return e;
+        pack = McaPackJob{mask, a.mask_bits, a.B, T, mca_mask_bits_row_words(T)};
+      }
+      if ((e = mca_split_forward_prepass(q, kk, v, a.B, a.H, T, a.D, a.split_ws, a.split_ws_bytes, layout, classify ? &job : nullptr,
+                                         key_bits ? &pack : nullptr, 0)))
         return e;
       if (classify && (e = settle_mask_mode(k, a, tc_bwd || !a.training, &mode))) return e;
       classified = true;
       const bool bits = mode == MCA_MASK_TT || mode == MCA_MASK_BATCH;   // packed for the kernel; causal / none need nothing
       if (tc_bwd || !save || !bits) {
-        if (bits && (e = pack_mask_bits(a, mask, mode, T))) return e;
+        if (bits && !key_bits && (e = pack_mask_bits(a, mask, mode, T))) return e;
         const bool stats = save && !tc_bwd;
         e = mca_split_forward_main(mode == MCA_MASK_CAUSAL, a.B, a.H, T, a.D, y, stats ? a.row_max : nullptr,
                                    stats ? a.row_sum : nullptr, save ? a.y_copy : nullptr, save && tc_bwd ? a.lse : nullptr, a.split_ws,

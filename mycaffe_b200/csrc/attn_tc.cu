@@ -879,15 +879,15 @@ int launch_tc(const void* q, const void* k, const void* v, int causal, int B, in
   return launch_shape<HD, MODE, false>(mq, mk, mv, p, B, H, T, mask != nullptr, st);
 }
 
-// The two halves of a split-operand forward: the pre-pass (which also classifies a (T,T) mask when asked to), and the kernel.
+// The two halves of a split-operand forward: the pre-pass (which also classifies a (T,T) mask or packs a key mask when asked to), and the kernel.
 template <int HD>
 int split_prepass(const float* q, const float* k, const float* v, int B, int H, int T, void* workspace, int layout, cudaStream_t st,
-                  const McaClassifyJob* cls) {
+                  const McaClassifyJob* cls, const McaPackJob* pack) {
   const split::Workspace w = split::carve(workspace, (int64_t)B * H, T, HD);
   split::Job job;
   job.src[0] = q; job.src[1] = k; job.src[2] = v;
   for (int i = 0; i < 3; ++i) { job.dst[i] = w.tensor[i]; job.slot[i] = i; }
-  return split::run<HD>(job, 3, mca_in_strides(layout, H, T, HD), B, H, T, w, st, nullptr, nullptr, cls);
+  return split::run<HD>(job, 3, mca_in_strides(layout, H, T, HD), B, H, T, w, st, nullptr, nullptr, cls, pack);
 }
 template <int HD>
 int split_main(int causal, int B, int H, int T, float* y, float* row_max, float* row_sum, float* y_copy, float* lse, void* workspace,
@@ -1023,13 +1023,13 @@ int mca_sdpa_forward_f32_tc_masked(const float* q, const float* k, const float* 
   if (mask != nullptr && causal) return ERROR_ATTN_UNSUPPORTED_SHAPE;
   if ((row_max == nullptr) != (row_sum == nullptr)) return ERROR_PARAM_NULL;
   if ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(y_copy)) & 15) return ERROR_PARAM_OUT_OF_RANGE;
-  if ((e = mca_split_forward_prepass(q, k, v, B, H, T, D, workspace, workspace_bytes, layout, nullptr, stream))) return e;
+  if ((e = mca_split_forward_prepass(q, k, v, B, H, T, D, workspace, workspace_bytes, layout, nullptr, nullptr, stream))) return e;
   return mca_split_forward_main(causal, B, H, T, D, y, row_max, row_sum, y_copy, lse, workspace, status, layout, mask_bits, mask_mode,
                                 stream);
 }
 
 int mca_split_forward_prepass(const float* q, const float* k, const float* v, int B, int H, int T, int D, void* workspace,
-                              int64_t workspace_bytes, int layout, const McaClassifyJob* cls, void* stream) {
+                              int64_t workspace_bytes, int layout, const McaClassifyJob* cls, const McaPackJob* pack, void* stream) {
   if (layout != MCA_LAYOUT_BHTD && layout != MCA_LAYOUT_PACKED) return ERROR_PARAM_OUT_OF_RANGE;
   if (!q || !k || !v || !workspace) return ERROR_PARAM_NULL;
   if (B <= 0 || H <= 0 || T <= 0 || (int64_t)B * H > 65535) return ERROR_PARAM_OUT_OF_RANGE;
@@ -1039,10 +1039,10 @@ int mca_split_forward_prepass(const float* q, const float* k, const float* v, in
   if (reinterpret_cast<uintptr_t>(workspace) & 15) return ERROR_PARAM_OUT_OF_RANGE;
   cudaStream_t st = (cudaStream_t)stream;
   switch (D) {
-    case 16: return split_prepass<16>(q, k, v, B, H, T, workspace, layout, st, cls);
-    case 32: return split_prepass<32>(q, k, v, B, H, T, workspace, layout, st, cls);
-    case 64: return split_prepass<64>(q, k, v, B, H, T, workspace, layout, st, cls);
-    case 128: return split_prepass<128>(q, k, v, B, H, T, workspace, layout, st, cls);
+    case 16: return split_prepass<16>(q, k, v, B, H, T, workspace, layout, st, cls, pack);
+    case 32: return split_prepass<32>(q, k, v, B, H, T, workspace, layout, st, cls, pack);
+    case 64: return split_prepass<64>(q, k, v, B, H, T, workspace, layout, st, cls, pack);
+    case 128: return split_prepass<128>(q, k, v, B, H, T, workspace, layout, st, cls, pack);
   }
   return ERROR_ATTN_UNSUPPORTED_SHAPE;
 }
@@ -1071,15 +1071,14 @@ int mca_split_forward_main(int causal, int B, int H, int T, int D, float* y, flo
 // Rows are padded to whole 128-key tiles (mca_mask_bits_row_words(T) words).
 // ---------------------------------------------------------------------------------------------
 namespace {
-__global__ void __launch_bounds__(256) mask_pack_kernel(const float* __restrict__ mask, int rows, int T, int wpr,
-                                                        uint32_t* __restrict__ bits, uint32_t* __restrict__ bits_t) {
+__global__ void __launch_bounds__(256) mask_pack_kernel(const float* mask, int rows, int T, int wpr, uint32_t* bits, uint32_t* bits_t) {
+  mca_pdl_launch_dependents();
+  mca_pdl_wait();   // the mask may be the kernel before's, and the bits be read by it
   const int64_t word = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (word >= (int64_t)rows * wpr) return;
-  const int r = (int)(word / wpr), w = (int)(word - (int64_t)r * wpr);
-  const int c = 32 * w + lane;
-  const uint32_t keep = __ballot_sync(0xffffffffu, c < T && mask[(int64_t)r * T + c] != 0.f);
-  if (lane == 0) bits[word] = keep;
+  mca_pack_word(mask, bits, word, T, wpr, lane);
+  const int r = (int)(word / wpr), c = 32 * (int)(word - (int64_t)r * wpr) + lane;
   if (bits_t != nullptr) {   // square mask: the same word position of the transpose
     const uint32_t keep_t = __ballot_sync(0xffffffffu, c < T && mask[(int64_t)c * T + r] != 0.f);
     if (lane == 0) bits_t[word] = keep_t;
@@ -1111,9 +1110,8 @@ int mca_mask_pack(const float* mask, int mask_mode, int B, int T, uint32_t* bits
   if (mask_mode != MCA_MASK_TT && mask_mode != MCA_MASK_BATCH) return ERROR_PARAM_OUT_OF_RANGE;
   const int rows = mask_mode == MCA_MASK_TT ? T : B, wpr = mca_mask_bits_row_words(T);
   const int64_t words = (int64_t)rows * wpr;
-  mask_pack_kernel<<<(unsigned)((words + 7) / 8), 256, 0, (cudaStream_t)stream>>>(mask, rows, T, wpr, bits,
-                                                                               mask_mode == MCA_MASK_TT ? bits_t : nullptr);
-  return mca_launch_status();
+  return mca_launch_pdl(mask_pack_kernel, dim3((unsigned)((words + 7) / 8)), dim3(256), 0, (cudaStream_t)stream, mask, rows, T, wpr, bits,
+                        mask_mode == MCA_MASK_TT ? bits_t : nullptr);
 }
 
 int mca_set_fail_words_fwd(int* words) { return (int)cudaMemcpyToSymbol(tc::g_fail_words, &words, sizeof(words)); }

@@ -15,7 +15,25 @@ struct McaClassifyJob {
   int* scratch;
 };
 
+// Keep-bits of a (B,T) key mask, one warp ballot per word (see mca_mask_pack), by any number of CTAs of 256 threads of a kernel that has
+// something else to do.
+struct McaPackJob {
+  const float* mask;    // null: none
+  uint32_t* bits;
+  int rows, T, wpr;
+};
+
 #ifdef __CUDACC__
+__device__ __forceinline__ void mca_pack_word(const float* mask, uint32_t* bits, int64_t word, int T, int wpr, int lane) {
+  const int r = (int)(word / wpr), c = 32 * (int)(word - (int64_t)r * wpr) + lane;
+  const uint32_t keep = __ballot_sync(0xffffffffu, c < T && mask[(int64_t)r * T + c] != 0.f);
+  if (lane == 0) bits[word] = keep;
+}
+__device__ __forceinline__ void mca_pack_rows(const McaPackJob& j, int cta, int ctas) {
+  const int64_t words = (int64_t)j.rows * j.wpr;
+  for (int64_t word = (int64_t)cta * 8 + (threadIdx.x >> 5); word < words; word += (int64_t)ctas * 8)
+    mca_pack_word(j.mask, j.bits, word, j.T, j.wpr, threadIdx.x & 31);
+}
 __device__ __forceinline__ void mca_classify_rows(const McaClassifyJob& j, int cta, int ctas) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, T = j.T;
   bool bad = false;

@@ -9,6 +9,7 @@ int mca_mask_bits_view(const uint32_t* bits, const uint32_t* bits_t, int mask_mo
 
 // Internal: mca_classify_causal_mask in one launch.
 struct McaClassifyJob;
+struct McaPackJob;
 int mca_classify_causal_mask_ws(const McaClassifyJob* job, void* stream);
 
 // Internal: mca_sdpa_backward_f32_layout with room for dS between its two kernels (ds_floats floats, 16-byte aligned; fewer than
@@ -37,9 +38,9 @@ int mca_sdpa_forward_small(const float* q, const float* k, const float* v, const
                            int layout, void* stream);
 
 // Internal: the two halves of mca_sdpa_forward_f32_tc_masked -- the pre-pass that splits q, k, v (and classifies the caller's
-// (T,T) mask in the same launch when `cls` is given), and the kernel, which may then be chosen on the class.
+// (T,T) mask, or packs the key mask's bits, in the same launch when `cls` or `pack` is given), and the kernel, which may then be chosen on the class.
 int mca_split_forward_prepass(const float* q, const float* k, const float* v, int B, int H, int T, int D, void* workspace,
-                              int64_t workspace_bytes, int layout, const McaClassifyJob* cls, void* stream);
+                              int64_t workspace_bytes, int layout, const McaClassifyJob* cls, const McaPackJob* pack, void* stream);
 int mca_split_forward_main(int causal, int B, int H, int T, int D, float* y, float* row_max, float* row_sum, float* y_copy, float* lse,
                            void* workspace, int* status, int layout, const uint32_t* mask_bits, int mask_mode, void* stream);
 

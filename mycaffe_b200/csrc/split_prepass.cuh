@@ -102,17 +102,19 @@ constexpr int THREADS = 256, KEEP = 4;   // eight-element pieces a thread keeps 
 
 // with ydot / delta given: also delta[row] = sum_c x[row][c] * ydot[row][c] (ydot contiguous rows) x scale x DS_SHIFT, the
 // softmax backward's row term in the units the backward kernels need, from the elements this kernel holds anyway.
-// grid: (CTAs of a cluster, BH, cls_layers of CTAs that classify the mask + tensors); the classification comes first, so that its
-// answer is on the host before the tensors are done
+// grid: (CTAs of a cluster, BH, cls_layers of CTAs that classify a (T,T) mask or pack a key mask + tensors); the classification comes
+// first, so that its answer is on the host before the tensors are done
 template <int HD>
 __global__ void __launch_bounds__(THREADS) split_kernel(const Job job, const McaStrides st, int H, int T,
                                                         float* __restrict__ scale, const float* __restrict__ ydot,
-                                                        float* __restrict__ delta, const McaClassifyJob cls, int cls_layers) {
+                                                        float* __restrict__ delta, const McaClassifyJob cls, const McaPackJob pack, int cls_layers) {
   mca_pdl_launch_dependents();
   mca_pdl_wait();   // the tensors are earlier kernels' output
   const int tid = threadIdx.x, which = (int)blockIdx.z - cls_layers;
   if (which < 0) {
-    mca_classify_rows(cls, (int)((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x), cls_layers * (int)(gridDim.x * gridDim.y));
+    const int cta = (int)((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x), ctas = cls_layers * (int)(gridDim.x * gridDim.y);
+    if (pack.mask != nullptr) mca_pack_rows(pack, cta, ctas);
+    else mca_classify_rows(cls, cta, ctas);
     return;
   }
   constexpr int V8 = HD / 8;
@@ -215,7 +217,7 @@ __global__ void __launch_bounds__(THREADS) split_kernel(const Job job, const Mca
 // Split `count` tensors (q, k, v for the forward; dY for the backward) into the workspace.
 template <int HD>
 inline int run(const Job& job, int count, const McaStrides& st, int B, int H, int T, const Workspace& w, cudaStream_t stream,
-               const float* ydot = nullptr, float* delta = nullptr, const McaClassifyJob* cls = nullptr) {
+               const float* ydot = nullptr, float* delta = nullptr, const McaClassifyJob* cls = nullptr, const McaPackJob* pack = nullptr) {
   // CTAs of a cluster: as many as leave each at most what its threads keep in registers, up to the portable eight -- or sixteen
   // where a few long heads would not give every SM one (forward of
   // four heads of 8192 rows 208 -> 198 us, of one of 16384 378 -> 360)
@@ -230,13 +232,13 @@ inline int run(const Job& job, int count, const McaStrides& st, int B, int H, in
   }
   // The mask is T x T whatever the heads are: as many layers as give every eight rows of it a CTA, up to 1184 CTAs (with
   // one layer a single head of 16384 rows had eight CTAs read a gigabyte: 6.04 ms, 0.53 with this)
-  const int layers = cls != nullptr ? mca_ceil_div(std::min(1184, mca_ceil_div(T, 8)), ctas * B * H) : 0;
+  const int layers = cls != nullptr ? mca_ceil_div(std::min(1184, mca_ceil_div(T, 8)), ctas * B * H) : pack != nullptr ? 1 : 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ctas, B * H, count + layers);
   cfg.blockDim = dim3(THREADS);
   cfg.stream = stream;
   return mca_launch_pdl_cluster(split_kernel<HD>, cfg, ctas, job, st, H, T, reinterpret_cast<float*>(w.scale), ydot, delta,
-                                cls != nullptr ? *cls : McaClassifyJob{}, layers);
+                                cls != nullptr ? *cls : McaClassifyJob{}, pack != nullptr ? *pack : McaPackJob{}, layers);
 }
 
 }  // namespace split
