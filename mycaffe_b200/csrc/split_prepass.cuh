@@ -108,7 +108,6 @@ template <int HD>
 __global__ void __launch_bounds__(THREADS) split_kernel(const Job job, const McaStrides st, int H, int T,
                                                         float* __restrict__ scale, const float* __restrict__ ydot,
                                                         float* __restrict__ delta, const McaClassifyJob cls, const McaPackJob pack, int cls_layers) {
-  mca_pdl_launch_dependents();
   mca_pdl_wait();   // the tensors are earlier kernels' output
   const int tid = threadIdx.x, which = (int)blockIdx.z - cls_layers;
   if (which < 0) {
@@ -166,6 +165,10 @@ __global__ void __launch_bounds__(THREADS) split_kernel(const Job job, const Mca
     }
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // its peers may still be reading this CTA's word
   }
+  // Only now may the kernel behind this one be launched: its CTAs, launched at this kernel's top, took whatever SMs the kernel before had
+  // left, two to one of them where the grid has one for each (layers forward and backward, us: 12 heads of 1024 x 64 86 -> 82, 24 of 512
+  // 67.5 -> 64.0, 24 of 200 under a key mask 54.5 -> 52.9).
+  mca_pdl_launch_dependents();
   const int slot = job.slot[which];
   const float sc = pow2_scale(m), sc_delta = sc * DS_SHIFT;
   if (blockIdx.x == 0 && tid == 0) scale[bh * 4 + slot] = sc;
