@@ -184,7 +184,26 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) gemv_stream_k
   mca_pdl_launch_dependents();
 #pragma unroll
   for (int t = 0; t < DEPTH - 1; ++t) issue();
+  // so do the norm's weights, a thread's first GP pieces: asked for where they are needed, behind the sum of squares, they
+  // were a round trip to L2 in every kernel with a norm
+  constexpr int GP = 2;
+  float4 g_first[GP];
+#pragma unroll
+  for (int i = 0; i < GP; ++i) {
+    const int k = (tid + i * THREADS) * 4;
+    if (p.norm_w != nullptr && k < n) g_first[i] = __ldg(reinterpret_cast<const float4*>(p.norm_w + k));
+  }
   mca_pdl_wait();   // from here on the previous kernel's results are complete and visible
+
+  // The residual of a lane's first output (one matrix, then) is asked for here: at the end it is a round trip to L2 behind the last
+  // product.
+  constexpr int OUTS = GLU ? NB : R * NB;
+  const bool residual = !GLU && p.accumulate && p.n_mats == 1;
+  float first_res = 0.f;
+  if (residual) {
+    const int o = S == 1 ? lane : lane % OUTS, r = (step_lo + (S == 1 ? 0 : lane / OUTS)) * STEP + o / NB, b = b0 + o % NB;
+    if (seg == 0 && o < OUTS && r < total_rows && b < p.B) first_res = p.out[0][(int64_t)b * total_rows + r];
+  }
 
   // ---- phase 1: activations of this pass's sequences -> shared memory, RMS-normalised
   float ss[NB];
@@ -230,15 +249,18 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) gemv_stream_k
 #pragma unroll
       for (int b = 0; b < NB; ++b) scale[b] = s_scale[b];
     }
-    for (int k = tid * 4; k < n; k += THREADS * 4) {
-      const float4 g = *reinterpret_cast<const float4*>(p.norm_w + k);
+    auto normalise = [&](int k, const float4& g) {
 #pragma unroll
       for (int b = 0; b < NB; ++b) {
         float4 v = *reinterpret_cast<float4*>(xs + b * n + k);
         v.x = g.x * (scale[b] * v.x); v.y = g.y * (scale[b] * v.y); v.z = g.z * (scale[b] * v.z); v.w = g.w * (scale[b] * v.w);
         *reinterpret_cast<float4*>(xs + b * n + k) = v;
       }
-    }
+    };
+#pragma unroll
+    for (int i = 0; i < GP; ++i)
+      if ((tid + i * THREADS) * 4 < n) normalise((tid + i * THREADS) * 4, g_first[i]);
+    for (int k = (tid + GP * THREADS) * 4; k < n; k += THREADS * 4) normalise(k, *reinterpret_cast<const float4*>(p.norm_w + k));
   }
   __syncthreads();
 
@@ -246,8 +268,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) gemv_stream_k
   // Each is a lane's: one lane that wrote them all read every residual behind the store of the one before it (eight sequences,
   // sixteen round trips to L2; and eight exponentials and divisions for the gate): a token of 12 layers 768 wide, fp32, four
   // sequences 468 -> 420 us, eight 675 -> 581 (with the warp per sequence above).
-  constexpr int OUTS = GLU ? NB : R * NB;
-  auto emit = [&](int step, int q, int b, float v, float v2) {
+  auto emit = [&](int step, int q, int b, float v, float v2, bool first) {
     const int r = step * STEP;
     if (b0 + b >= p.B) return;
     if (GLU) {
@@ -261,7 +282,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) gemv_stream_k
       float* ob = m == 0 ? p.out[0] : (m == 1 ? p.out[1] : p.out[2]);
       const int orows = m == 0 ? p.rows[0] : (m == 1 ? p.rows[1] : p.rows[2]);
       float* dst = ob + (int64_t)(b0 + b) * orows + rr;
-      *dst = p.accumulate ? (*dst + v) : v;
+      *dst = p.accumulate ? ((first && residual ? first_res : *dst) + v) : v;
     }
   };
 
@@ -316,7 +337,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) gemv_stream_k
             if (GLU) { if (lane == b) (q == 0 ? v : v2) = acc[q][b]; }
             else if (lane == q * NB + b) v = acc[q][b];
           }
-        if (lane < OUTS) emit(step_lo + step, lane / NB, lane % NB, v, v2);
+        if (lane < OUTS) emit(step_lo + step, lane / NB, lane % NB, v, v2, step == 0);
       } else if (lane == step) {   // lane i keeps the sums of the group's step i until the group adds them
 #pragma unroll
         for (int q = 0; q < R; ++q)
@@ -351,7 +372,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) gemv_stream_k
         v += part[(st * R + q) * NB + b];
         if (GLU) v2 += part[(st * R + 1) * NB + b];
       }
-      emit(step_lo + st, q, b, v, v2);
+      emit(step_lo + st, q, b, v, v2, i == lane);
     }
   }
 }
