@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(THREADS) split_kernel(const Job job, const Mca
   mca_pdl_wait();   // the tensors are earlier kernels' output
   const int tid = threadIdx.x, which = (int)blockIdx.z - cls_layers;
   if (which < 0) {
+    mca_pdl_launch_dependents();   // what the others wait for below is no concern of these
     const int cta = (int)((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x), ctas = cls_layers * (int)(gridDim.x * gridDim.y);
     if (pack.mask != nullptr) mca_pack_rows(pack, cta, ctas);
     else mca_classify_rows(cls, cta, ctas);
