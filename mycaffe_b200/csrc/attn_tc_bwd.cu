@@ -1082,7 +1082,11 @@ sdpa_bwd_dq_ds_tc_kernel(const __grid_constant__ CUtensorMap map_k, const BwdPar
 constexpr int DELTA_STEPS = 4;
 __global__ void __launch_bounds__(256) bwd_delta_bf16_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* y, int64_t rows, int H, int T,
                                                              int D, const McaStrides ys, float* __restrict__ delta) {
-  mca_pdl_launch_dependents();
+  // Beyond three tiles a head the dK/dV kernel is let go only when the forward has left the SMs: launched before, its CTAs, of all
+  // lengths, took what was free, two to one SM where the grid has one for each (layers, us: 12 heads of 1024 x 64 40.6 -> 38.7, 8 of 2500 91.2 ->
+  // 88.2, 12 of 1024 x 128 41.6 -> 40.1; 48 of 300 x 64, short and alike, 24.1 -> 24.8, 24 of 200 20.6 -> 21.1).
+  const bool late = T > 3 * BLK;
+  if (!late) mca_pdl_launch_dependents();
   const int lane = threadIdx.x & 31, g = D / 8, rpw = 32 / g;        // g in {8, 16}
   const int64_t row0 = ((int64_t)blockIdx.x * (256 / 32) + (threadIdx.x >> 5)) * rpw * DELTA_STEPS + lane / g;
   int64_t off[DELTA_STEPS];
@@ -1094,6 +1098,7 @@ __global__ void __launch_bounds__(256) bwd_delta_bf16_kernel(const __nv_bfloat16
     asm volatile("prefetch.global.L2 [%0];" ::"l"(dy + off[i]));
   }
   mca_pdl_wait();   // dy and y are earlier kernels' output
+  if (late) mca_pdl_launch_dependents();
   float4 a[DELTA_STEPS], b[DELTA_STEPS];
 #pragma unroll
   for (int i = 0; i < DELTA_STEPS; ++i) {
