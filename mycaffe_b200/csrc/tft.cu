@@ -570,6 +570,8 @@ __global__ void __launch_bounds__(TFT_THREADS) tft_bwd_kernel(const float* __res
 // of a tile from its peers' shared memory, in the heads' order by CTA.
 // smem: Vt[nk4][d] | Kt[2][nk4][d] (16-byte pieces swizzled by row; nk4 = Nk rounded up to 4, rows beyond Nk zero) |
 //       Qs[2][24][d] | Gs[2][24][d] | Ps[24][192] | Ss[24][192] | ex[6][24]
+// PAIR (tft_rules::backward_pair): one tile in the place of Vt and both Kt.  A row tile's first iteration finds V in it, forms dP and then copies
+// its K; the next iteration's K (or V) is asked for behind the barrier after the last read of this one's.  Two CTAs share an SM.
 // ---------------------------------------------------------------------------------------------
 template <int D, bool WITH_DP>
 __device__ __forceinline__ void tft_bwd_scores(const float* const (&krow)[TQ_C], const float* const (&vrow)[TQ_C],
@@ -624,8 +626,8 @@ __device__ __forceinline__ void tft_bwd_scores(const float* const (&krow)[TQ_C],
   }
 }
 
-template <int D>
-__global__ void __launch_bounds__(TFT_THREADS, 1) tft_bwd_tiled_kernel(const float* __restrict__ Q, const float* __restrict__ K,
+template <int D, bool PAIR>
+__global__ void __launch_bounds__(TFT_THREADS, PAIR ? 2 : 1) tft_bwd_tiled_kernel(const float* __restrict__ Q, const float* __restrict__ K,
                                                                        const float* __restrict__ V,
                                                                        const float* __restrict__ mask,
                                                                        const float* __restrict__ d_out,
@@ -642,8 +644,8 @@ __global__ void __launch_bounds__(TFT_THREADS, 1) tft_bwd_tiled_kernel(const flo
   const int nk4 = (Nk + 3) & ~3;
   const size_t tile = (size_t)nk4 * D;
   float* Vt = smem;
-  float* Kt = Vt + tile;                              // two tiles
-  float* Qs = Kt + 2 * tile;                          // two (24, D) blocks
+  float* Kt = PAIR ? smem : Vt + tile;                // two tiles; PAIR: the one that V had
+  float* Qs = Kt + (PAIR ? 1 : 2) * tile;                          // two (24, D) blocks
   float* Gs = Qs + 2 * TQ * D;                        // two (24, D) blocks of the output gradient
   float* Ps = Gs + 2 * TQ * D;                        // (24, 192) probabilities; later the partial sums of dQ
   float* Ss = Ps + TQ * TQ_KEYS;                      // (24, 192) dS
@@ -655,7 +657,14 @@ __global__ void __launch_bounds__(TFT_THREADS, 1) tft_bwd_tiled_kernel(const flo
 
   // what iteration `it` = (row tile, head) reads; one commit group per call, empty beyond the last iteration
   auto load_iter = [&](int it) {
-    if (it < iters) {
+    if constexpr (PAIR) {
+      if (it < iters) {
+        const int t = it / H, h = it - t * H, q0 = t * TQ, rows = min(TQ, Nq - q0);
+        rows24_async<D>(Qs + (it & 1) * TQ * D, Q + (((int64_t)b * H + h) * Nq + q0) * D, rows, tid);
+        if (h == 0) rows24_async<D>(Gs + (t & 1) * TQ * D, d_out + ((int64_t)b * Nq + q0) * D, rows, tid);
+        tile_rows_async_swz<D>(Kt, h == 0 ? V + (int64_t)b * Nk * D : K + ((int64_t)b * H + h) * Nk * D, Nk, tid);
+      }
+    } else if (it < iters) {
       const int t = it / H, h = it - t * H, q0 = t * TQ, rows = min(TQ, Nq - q0);
       rows24_async<D>(Qs + (it & 1) * TQ * D, Q + (((int64_t)b * H + h) * Nq + q0) * D, rows, tid);
       rows24_async<D>(Gs + (it & 1) * TQ * D, d_out + ((int64_t)b * Nq + q0) * D, rows, tid);
@@ -668,7 +677,7 @@ __global__ void __launch_bounds__(TFT_THREADS, 1) tft_bwd_tiled_kernel(const flo
   // phase D reads K four rows at a time: the rows between Nk and nk4 are never copied, they must be zero
   for (int idx = tid; idx < (nk4 - Nk) * D; idx += TFT_THREADS) {
     Kt[(size_t)Nk * D + idx] = 0.f;
-    Kt[tile + (size_t)Nk * D + idx] = 0.f;
+    if constexpr (!PAIR) Kt[tile + (size_t)Nk * D + idx] = 0.f;
   }
 
   const int rg = w & 3, khalf = w >> 2;               // phases A, B: rows rg*6 .. +5, keys khalf*96 + lane + 32c
@@ -691,10 +700,10 @@ __global__ void __launch_bounds__(TFT_THREADS, 1) tft_bwd_tiled_kernel(const flo
     const bool fresh = h == 0;                        // new rows: mask bits and dP have to be formed, the head sum starts
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();                                  // this iteration's tiles visible; everyone is past the previous one
-    load_iter(it + 1);                                // into the buffers that iteration read, its dO for dV last of all
-    const float* Kh = Kt + (it & 1) * tile;
+    if constexpr (!PAIR) load_iter(it + 1);           // into the buffers that iteration read, its dO for dV last of all
+    const float* Kh = PAIR ? Kt : Kt + (it & 1) * tile;
     const float* Qh = Qs + (it & 1) * TQ * D;
-    const float* Gh = Gs + (it & 1) * TQ * D;
+    const float* Gh = Gs + ((PAIR ? t : it) & 1) * TQ * D;
 
     // ---- A: scores and dP
     float da[TQ_R][TQ_C];
@@ -737,7 +746,18 @@ __global__ void __launch_bounds__(TFT_THREADS, 1) tft_bwd_tiled_kernel(const flo
         vrow[c] = Vt + (size_t)j * D;
         ksw[c] = j & SW;
       }
-      if (fresh) {
+      if (PAIR && fresh) {
+        tft_bwd_scores<D, false>(krow, vrow, ksw, Gh + rg * TQ_R * D, Gh, dp, s);     // the tile is V's
+        __syncthreads();
+        tile_to_smem_async_swz<D>(Kt, K + ((int64_t)b * H + h) * Nk * D, Nk, tid);
+#pragma unroll
+        for (int r = 0; r < TQ_R; ++r)
+#pragma unroll
+          for (int c = 0; c < TQ_C; ++c) dp[r][c] = (dp[r][c] + da[r][c]) * inv_h;
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+      }
+      if (!PAIR && fresh) {
         tft_bwd_scores<D, true>(krow, vrow, ksw, Qh + rg * TQ_R * D, Gh + rg * TQ_R * D, s, dp);
 #pragma unroll
         for (int r = 0; r < TQ_R; ++r)
@@ -862,6 +882,7 @@ __global__ void __launch_bounds__(TFT_THREADS, 1) tft_bwd_tiled_kernel(const flo
       }
     }
     __syncthreads();                                  // the buffer of the head sum now takes the partial sums of dQ
+    if constexpr (PAIR) load_iter(it + 1);            // every warp is past its last read of K, V and Q
     if (ks > 0) {
 #pragma unroll
       for (int r = 0; r < RPT; ++r)
@@ -1344,14 +1365,20 @@ int mca_tft_attention_backward_f32(const float* q, const float* k, const float* 
   const auto aligned = [](const void* p_) { return (reinterpret_cast<uintptr_t>(p_) & 15) == 0; };
   if ((d == 16 || d == 32 || d == 64) && Nk <= TQ_KEYS && aligned(q) && aligned(d_out) && aligned(dq) && aligned(dk) && aligned(dv)) {
     const tft_rules::Split split = tft_rules::backward_split(B, H, mca_ceil_div(Nq, TQ), d);
+    const bool pair = tft_rules::backward_pair(B, d);
     const size_t nk4 = ((size_t)Nk + 3) & ~(size_t)3;
     const size_t smem_t = sizeof(float) * (3 * nk4 * d + 4 * (size_t)TQ * d + 2 * (size_t)TQ * TQ_KEYS + 6 * TQ);
     const float sc = 1.0f / sqrtf((float)d);
     cudaStream_t st = (cudaStream_t)stream;
 #define MCA_TFT_BWD_TILED(D_)                                                                                                 \
-    if (split.ch * split.ct == 1) {                                                                                          \
-      if (const int e = smem_limit<tft_bwd_tiled_kernel<D_>>()) return e;                                                    \
-      tft_bwd_tiled_kernel<D_><<<B, TFT_THREADS, smem_t, st>>>(q, k, v, mask, d_out, d_attn, H, Nq, Nk, sc, dq, dk, dv); \
+    if (pair || split.ch * split.ct == 1) {                                                                                  \
+      if (pair) {                                                                                                            \
+        if (const int e = smem_limit<tft_bwd_tiled_kernel<D_, (D_ <= 32)>>()) return e;                                            \
+        tft_bwd_tiled_kernel<D_, (D_ <= 32)><<<B, TFT_THREADS, smem_t - 2 * sizeof(float) * nk4 * D_, st>>>(q, k, v, mask, d_out, d_attn, H, Nq, Nk, sc, dq, dk, dv); \
+      } else {                                                                                                               \
+        if (const int e = smem_limit<tft_bwd_tiled_kernel<D_, false>>()) return e;                                           \
+        tft_bwd_tiled_kernel<D_, false><<<B, TFT_THREADS, smem_t, st>>>(q, k, v, mask, d_out, d_attn, H, Nq, Nk, sc, dq, dk, dv); \
+      }                                                                                                                      \
     } else {                                                                                                                  \
       if (const int e = smem_limit<tft_bwd_spread_kernel<D_>>()) return e;                                                   \
       return launch_clusters(tft_bwd_spread_kernel<D_>, split.ch * split.ct, dim3(split.ch * split.ct, B), smem_t, st, split.ch, split.ct, \

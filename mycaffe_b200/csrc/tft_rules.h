@@ -42,6 +42,13 @@ inline Split backward_split(int B, int H, int tiles, int d = 64) {
   return best;
 }
 
+// Whether the backward runs two items to an SM, with one buffer for V and then each head's K in turn: where there are more items than SMs.
+// One's copies and barriers then stand beside the other's products, which one item's own second buffer does less well (forward and backward,
+// us: 256 items, 8 heads, 40 x 192, d 16 291 -> 260; 300, 4, 24 x 150, 32 154 -> 142; 200, 8, 192 x 192, 32 1414 -> 1366; 170, 6, 160 x 160, 16
+// 614 -> 548; 155, 1, 5 x 40, 16 22.6 -> 20.5).  64-wide heads have not the registers (128 a thread, 100 spilled): 256, 4, 24 x 192
+// 137.3 -> 136.6, 192 x 192 988 -> 1088.
+inline bool backward_pair(int B, int d) { return d <= 32 && B > 148; }
+
 // Into how many CTAs the forward of a row tile's heads goes: as long as every tile's cluster is resident at once, with an SM to each
 // CTA.  Two CTAs on an SM take nearly twice as long, and their cluster's exchange comes on top (us, whole / over two: 128 tiles, 4 heads, 192 keys
 // 23.1 / 25.2; 3 heads 19.8 / 25.1; 74 tiles, 4 heads 23.0 / 16.9; over four 25.0).
