@@ -133,7 +133,7 @@ struct Kernel {
   float* stage = nullptr;  // grow-only fp32 staging buffer for float <-> bf16 transfers
   size_t stage_count = 0;
   float* ds_ws = nullptr;  // dS between the two kernels of a backward: one for all handles, whose backwards follow one
-  int64_t ds_ws_floats = 0;   // another on one stream; as large as the largest of them asks, and gone with the last of them
+  int64_t ds_ws_floats = 0;   // another on one stream; as large as the largest of them has asked, and gone with the last of them
   void fit_ds_ws() {       // after a handle has been set or released
     int64_t need = 0;
     for (const auto& kv : attn) need = std::max(need, kv.second.ds_floats);
@@ -147,6 +147,9 @@ struct Kernel {
     ds_ws = p;
     ds_ws_floats = need;
   }
+  // What a handle sees of it: no more than it asked for, so that its kernels, and its gradients' last bits, do not depend on which other
+  // handles there are.
+  int64_t ds_room(const AttnHandle& a) const { return std::min(a.ds_floats, ds_ws_floats); }
   bool synced = false;     // the call being dispatched has already synchronised the stream behind its last launch
   bool by_word = false;    // the call being dispatched is waited for by the done word (see sync_call)
   bool fail_words = false; // this device's kernels raise its failure words (see g_fail)
@@ -880,7 +883,7 @@ long attn_bwd(Kernel* k, long llInput, MCA_LONGLONG* pl, int layout) {
     if (fwd_masked && a.fwd_mask_handle == 0) {
       // the forward applied the mask on the tensor cores from the keep-bits it packed into the handle: so does this
       e = mca_sdpa_backward_tc_ws(q, kk, v, a.y_copy, dy, a.lse, a.delta, MCA_DTYPE_BF16, 0, a.B, a.H, T, a.D, dq, dk, dv,
-                                  a.causal_flag + 1, layout, a.mask_bits, a.mask_bits_t, a.fwd_mask_mode, k->ds_ws, k->ds_ws_floats * 4, 0);
+                                  a.causal_flag + 1, layout, a.mask_bits, a.mask_bits_t, a.fwd_mask_mode, k->ds_ws, k->ds_room(a) * 4, 0);
       if (e) return e;
       return tc_status(k, a);
     }
@@ -906,7 +909,7 @@ long attn_bwd(Kernel* k, long llInput, MCA_LONGLONG* pl, int layout) {
       return mca_convert_f32_to_bf16(gv, dv, n, 0);
     }
     e = mca_sdpa_backward_tc_ws(q, kk, v, a.y_copy, dy, a.lse, a.delta, MCA_DTYPE_BF16, a.fwd_mask_mode == MCA_MASK_CAUSAL, a.B, a.H, T,
-                                a.D, dq, dk, dv, a.causal_flag + 1, layout, nullptr, nullptr, MCA_MASK_NONE, k->ds_ws, k->ds_ws_floats * 4, 0);
+                                a.D, dq, dk, dv, a.causal_flag + 1, layout, nullptr, nullptr, MCA_MASK_NONE, k->ds_ws, k->ds_room(a) * 4, 0);
     if (e) return e;
     return tc_status(k, a);
   }
@@ -923,7 +926,7 @@ long attn_bwd(Kernel* k, long llInput, MCA_LONGLONG* pl, int layout) {
     const bool bits = a.fwd_mask_mode == MCA_MASK_TT || a.fwd_mask_mode == MCA_MASK_BATCH;   // packed by the forward
     e = mca_sdpa_backward_f32_tc_ws(dy, a.y_copy, a.lse, a.delta, a.fwd_mask_mode == MCA_MASK_CAUSAL, a.B, a.H, T, a.D, dq, dk, dv,
                                     a.split_ws, a.split_ws_bytes, a.causal_flag + 1, layout, bits ? a.mask_bits : nullptr,
-                                    bits ? a.mask_bits_t : nullptr, bits ? a.fwd_mask_mode : MCA_MASK_NONE, k->ds_ws, k->ds_ws_floats * 4, 0);
+                                    bits ? a.mask_bits_t : nullptr, bits ? a.fwd_mask_mode : MCA_MASK_NONE, k->ds_ws, k->ds_room(a) * 4, 0);
     if (e) return e;
     return tc_status(k, a);
   }
@@ -935,7 +938,7 @@ long attn_bwd(Kernel* k, long llInput, MCA_LONGLONG* pl, int layout) {
     if ((e = resolve_mask(k, a, a.fwd_mask_handle, a.fwd_batch_mask, T, &mask, &mode, false))) return e;
   }
   return mca_sdpa_backward_f32_ws(q, kk, v, dy, a.y_copy, mask, mode, a.causal_flag, a.row_max, a.row_sum, a.delta, a.B, a.H, T,
-                                  a.D, dq, dk, dv, k->ds_ws, k->ds_ws_floats, layout, 0);
+                                  a.D, dq, dk, dv, k->ds_ws, k->ds_room(a), layout, 0);
 }
 
 // ---- rope ids ------------------------------------------------------------------------------

@@ -66,3 +66,24 @@ def test_heads_in_parts():
     for g, r in zip(got, grads):
         assert rel_err(g, host(r)) < 2.0 ** -8
     cuda.Dispose()
+
+
+@pytest.mark.parametrize("bf16,B,H,T", [(False, 8, 8, 512), (True, 1, 16, 2048)])
+def test_a_handle_does_not_see_the_room_of_others(bf16, B, H, T):
+    """The gradients' bits are the same whether or not a handle that asked for more room exists."""
+    cuda = CudaDnn(0)
+    rng = np.random.default_rng(1)
+    D = 128 if bf16 else 64
+    t = [rng.standard_normal((B, H, T, D)).astype(np.float32) for _ in range(4)]
+    got = []
+    for alone in (True, False):
+        other = None if alone else handle(cuda, 1, 4096, 32, D, bf16, 3)
+        a = handle(cuda, B, T, H, D, bf16, 0)
+        a.forward(*t[:3], None)
+        got.append(a.backward(t[3]))
+        a.close()
+        if other:
+            other.close()
+    for g, r in zip(*got):
+        assert np.array_equal(g, r)
+    cuda.Dispose()
