@@ -18,6 +18,7 @@
 
 #include "classify.cuh"
 #include "common.cuh"
+#include "ds_rules.h"
 #include "kernels.h"
 
 namespace {
@@ -497,7 +498,6 @@ long convert_mem(Kernel* k, long llInput, MCA_LONGLONG* pl) {
 
 // ---- attention ids ------------------------------------------------------------------------
 
-constexpr int64_t kMaxDsBytes = 1ll << 30;
 
 long attn_set(Kernel* k, long lInput, float* pf, long llInput, MCA_LONGLONG* pl) {
   long e;  // Device<T>::SetAttn, device.h:2463-2486 (exactly 9 longs there; 10th/11th are extensions)
@@ -542,11 +542,10 @@ long attn_set(Kernel* k, long lInput, float* pf, long llInput, MCA_LONGLONG* pl)
     // The exact fp32 backward passes dS from one kernel to the other, in at most a gigabyte.  Beyond that, or where it cannot be had,
     // dS is formed twice.
     const int64_t bytes = mca_sdpa_backward_f32_ws_bytes(a.B, a.H, a.block);
-    if (bytes <= kMaxDsBytes) a.ds_floats = bytes / 4;
-  } else if (a.training && (int64_t)a.B * a.H <= 65535) {
+    if (bytes <= ds_rules::MAX_BYTES) a.ds_floats = bytes / 4;
+  } else if (a.training && (a.dtype == MCA_DTYPE_BF16 ? (int64_t)a.B * a.H <= 65535 : a.split_ws != nullptr)) {
     // The tensor-core backward does the same, as many heads at a time as fit.
-    const int64_t bytes = mca_sdpa_backward_tc_ws_bytes(a.B, a.H, a.block, a.D, a.dtype != MCA_DTYPE_BF16);
-    a.ds_floats = std::min<int64_t>(bytes, kMaxDsBytes) / 4;
+    a.ds_floats = ds_rules::room((int64_t)a.B * a.H, a.block, a.D, a.dtype != MCA_DTYPE_BF16, (a.flags & MCA_FLAG_CAUSAL_IMPLICIT) != 0) / 4;
   }
   k->fit_ds_ws();
   a.configured = true;

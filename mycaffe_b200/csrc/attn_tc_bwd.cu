@@ -16,7 +16,7 @@
 //   * dkdv kernel: one CTA per 128-row key tile walks the query tiles with the transposed
 //     products S^T = K Q^T and dP^T = V dY^T, so that P^T and dS^T come out in the layout the
 //     A operand of dV += P^T dY and dK += dS^T Q needs.
-// Where it gains (passes_ds) the dkdv kernel leaves its dS tiles in a workspace and dQ = dS K is one product over them.
+// Where it gains (ds_rules) the dkdv kernel leaves its dS tiles in a workspace and dQ = dS K is one product over them.
 // Q/K/V/dY tiles arrive by TMA (no multicast) through rings; every mbarrier wait is
 // bounded as in the forward kernel.
 //
@@ -26,6 +26,7 @@
 // warps, and the gradients are written in fp32.  Head sizes up to 64: a split tile is as large as a 128-wide bf16 one.
 #include <type_traits>
 
+#include "ds_rules.h"
 #include "kernels.h"
 #include "tc_common.cuh"
 #include "split_prepass.cuh"
@@ -40,13 +41,10 @@ using namespace tc;
 // queries are what a thread that reads dS^T from TMEM has in four registers, so a warp writes 512 consecutive bytes an instruction without
 // a shuffle, and the dQ kernel reads a tile by plain bulk copies.
 constexpr int DS_GROUP_BYTES = 32 * 16, DS_BLOCK_BYTES = 16 * DS_GROUP_BYTES;
-__host__ __device__ __forceinline__ int64_t ds_head_tiles(int T, int causal) {
-  const int64_t nt = (T + BLK - 1) / BLK;
-  return causal ? nt * (nt + 1) / 2 : nt * nt;
-}
-template <bool SPLIT> __host__ __device__ __forceinline__ int64_t ds_tile_offset(int64_t head, int qt, int kt, int T, int causal) {
+static_assert(ds_rules::TILE == BLK && ds_rules::tile_bytes(false) == 4 * DS_BLOCK_BYTES && ds_rules::tile_bytes(true) == 8 * DS_BLOCK_BYTES);
+template <bool SPLIT> __device__ __forceinline__ int64_t ds_tile_offset(int64_t head, int qt, int kt, int T, int causal) {
   const int nt = (T + BLK - 1) / BLK;
-  return (head * ds_head_tiles(T, causal) + (causal ? (int64_t)qt * (qt + 1) / 2 : (int64_t)qt * nt) + kt) * (SPLIT ? 8 : 4) * DS_BLOCK_BYTES;
+  return (head * ds_rules::head_tiles(T, causal) + (causal ? (int64_t)qt * (qt + 1) / 2 : (int64_t)qt * nt) + kt) * ds_rules::tile_bytes(SPLIT);
 }
 
 // What a CTA looks like.  It keeps two 128-row tiles (Q and dY, or K and V) and streams the other two tensors BN rows a step.
@@ -1122,32 +1120,11 @@ __global__ void __launch_bounds__(256) bwd_delta_bf16_kernel(const __nv_bfloat16
   }
 }
 
-// Is dS formed once and passed through memory?  Instead of S, dP and the exponentials a second time the dQ kernel then reads two (split:
-// four) bytes a pair from HBM, and the dK/dV kernel writes them from the warps that bound it (7001 x 128: 333 -> 364 us, dQ 253 -> 134); but
-// it waits for the whole dK/dV kernel, where the other one fills that kernel's last wave.  So there must be waves enough: 128-wide bf16
-// heads gain from about two times the longest CTA's work per SM (whole layer, us: 16 x 512 x 512 rows 96.7 -> 90.0, 16 heads of 4096 328 -> 312,
-// of 7001 878 -> 847, 192 of 1024 400 -> 367, 32 of 1024 68.3 -> 66.5; 16 heads of 2048 103.5 -> 103.6, 8 of 4096 180 -> 183).  64-wide split heads
-// have half the products to save and twice the bytes: short ones gain from their two CTAs per SM (256 of 128 59.8 -> 56.6, 192 of
-// 256 99.9 -> 93.9, 64 of 512 under a key mask 117.0 -> 110.9), long ones with many waves (96 of 1024 301 -> 295.5; 48 of
-// 1024 149.7 -> 151.4, 16 of 2048 159 -> 170).  Narrower split heads lose (96 of 1024 x 32 205 -> 218), and 64-wide bf16 ones, whose
-// narrow CTAs leave the element-wise warps no time for it, too (96 of 1024 120 -> 131).
-template <int HD, bool SPLIT> constexpr bool passes_ds(int64_t heads, int T, int causal) {
-  const int64_t nt = (T + BLK - 1) / BLK;
-  if (HD < 64 || (HD == 64 && !SPLIT)) return false;
-  if (!SPLIT) return heads * (causal ? nt + 1 : 2 * nt) >= 288;
-  return heads * nt >= (nt <= 4 ? 256 : 768);
-}
-// What the caller has for the dS tiles, and how many heads at a time go through it (0: none).
+// What the caller has for the dS tiles (see ds_rules); with less than the plan asks dS is formed twice.
 struct DsRoom {
   uint8_t* ptr;
   int64_t bytes;
 };
-template <int HD, bool SPLIT> int ds_heads(const DsRoom& room, int64_t heads, int T, int causal) {
-  const int64_t fit = room.ptr == nullptr ? 0 : std::min<int64_t>(room.bytes / ds_tile_offset<SPLIT>(1, 0, 0, T, causal), heads);
-  if (fit == 0) return 0;
-  const int64_t launches = (heads + fit - 1) / fit, chunk = (heads + launches - 1) / launches;   // alike in size
-  return passes_ds<HD, SPLIT>(heads / launches, T, causal) ? (int)chunk : 0;
-}
 
 // Both kernels of one backward, with or without the caller's mask.
 template <int HD, bool SPLIT, bool MASKED, bool NARROW>
@@ -1156,8 +1133,9 @@ int launch_bwd_pair(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensor
   using PL = BwdPlan<SPLIT ? 128 : HD, NARROW>;
   const size_t smem_kv = PL::BYTES_KV;
   int e;
-  if constexpr (passes_ds<HD, SPLIT>(1 << 30, BLK, 0)) {
-    if (const int chunk = ds_heads<HD, SPLIT>(room, (int64_t)B * H, T, p.causal)) {
+  if constexpr (ds_rules::possible(HD, SPLIT)) {
+    const ds_rules::Plan plan = ds_rules::plan((int64_t)B * H, T, HD, SPLIT, p.causal);
+    if (plan.parts != 0 && room.ptr != nullptr && plan.bytes <= room.bytes) {
       using PD = DqDsPlan<HD, SPLIT>;
       static std::atomic<uint64_t> done_kv{0}, done_dq{0};
       if ((e = mca_smem_once(done_kv, sdpa_bwd_dkdv_tc_kernel<HD, SPLIT, MASKED, NARROW, true>, smem_kv)) ||
@@ -1165,8 +1143,9 @@ int launch_bwd_pair(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensor
         return e;
       const int nt = mca_ceil_div(T, BLK), group = p.group;
       p.ds = room.ptr;
-      for (p.bh0 = 0; p.bh0 < B * H; p.bh0 += chunk) {
-        const int heads = std::min(chunk, B * H - p.bh0);
+      for (int i = 0; i < plan.parts; ++i) {
+        p.bh0 = ds_rules::part_begin((int64_t)B * H, plan.parts, i);
+        const int heads = ds_rules::part_begin((int64_t)B * H, plan.parts, i + 1) - p.bh0;
         p.group = std::min(group, heads);
         p.out0 = dk; p.out1 = dv;
         if ((e = mca_launch_pdl(sdpa_bwd_dkdv_tc_kernel<HD, SPLIT, MASKED, NARROW, true>, dim3(nt, heads), dim3(PL::THREADS), smem_kv, st, mq, mk, mv, mdo, p)))
@@ -1291,12 +1270,6 @@ int mca_sdpa_backward_tc_masked(const void* q, const void* k, const void* v, con
                                 int mask_mode, void* stream) {
   return mca_sdpa_backward_tc_ws(q, k, v, y, dy, lse, delta_scratch, dtype, causal, B, H, T, D, dq, dk, dv, status, layout, mask_bits,
                                  mask_bits_t, mask_mode, nullptr, 0, stream);
-}
-
-int64_t mca_sdpa_backward_tc_ws_bytes(int B, int H, int T, int D, int split) {
-  const int64_t heads = (int64_t)B * H;   // of the causal form: where the mask is another one they go through it in two parts
-  if (split ? D != 64 || !passes_ds<64, true>(heads, T, 1) : D != 128 || !passes_ds<128, false>(heads, T, 1)) return 0;
-  return split ? ds_tile_offset<true>(heads, 0, 0, T, 1) : ds_tile_offset<false>(heads, 0, 0, T, 1);
 }
 
 int mca_sdpa_backward_tc_ws(const void* q, const void* k, const void* v, const void* y, const void* dy, const float* lse,

@@ -21,8 +21,7 @@ int mca_sdpa_backward_f32_ws(const float* q, const float* k, const float* v, con
                              void* stream);
 
 // Internal: mca_sdpa_backward_tc_masked and mca_sdpa_backward_f32_tc_masked with room for dS between their two kernels (16-byte
-// aligned; null, or room for too few heads: dS is formed twice).  _ws_bytes: for all heads at once under the causal mask, 0 where it would not be used.
-int64_t mca_sdpa_backward_tc_ws_bytes(int B, int H, int T, int D, int split);
+// aligned; null, or less than ds_rules::plan asks for: dS is formed twice).
 int mca_sdpa_backward_tc_ws(const void* q, const void* k, const void* v, const void* y, const void* dy, const float* lse,
                             float* delta_scratch, int dtype, int causal, int B, int H, int T, int D, void* dq, void* dk, void* dv,
                             int* status, int layout, const uint32_t* mask_bits, const uint32_t* mask_bits_t, int mask_mode, void* ds,
