@@ -1126,9 +1126,10 @@ struct DsRoom {
   int64_t bytes;
 };
 
-// Both kernels of one backward, with or without the caller's mask.
-template <int HD, bool SPLIT, bool MASKED, bool NARROW>
-int launch_bwd_pair(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mdo, const CUtensorMap& mk64, BwdParams p,
+// Both kernels of one backward, with or without the caller's mask.  make_mk64 encodes the map of K in boxes of 64 rows, which the dQ kernel
+// of passed dS alone reads.
+template <int HD, bool SPLIT, bool MASKED, bool NARROW, typename MapK64>
+int launch_bwd_pair(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mdo, const MapK64& make_mk64, BwdParams p,
                     void* dq, void* dk, void* dv, int B, int H, int T, const DsRoom& room, cudaStream_t st) {
   using PL = BwdPlan<SPLIT ? 128 : HD, NARROW>;
   const size_t smem_kv = PL::BYTES_KV;
@@ -1141,6 +1142,8 @@ int launch_bwd_pair(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensor
       if ((e = mca_smem_once(done_kv, sdpa_bwd_dkdv_tc_kernel<HD, SPLIT, MASKED, NARROW, true>, smem_kv)) ||
           (e = mca_smem_once(done_dq, sdpa_bwd_dq_ds_tc_kernel<HD, SPLIT>, (size_t)PD::BYTES)))
         return e;
+      CUtensorMap mk64;
+      if ((e = make_mk64(&mk64))) return e;
       const int nt = mca_ceil_div(T, BLK), group = p.group;
       p.ds = room.ptr;
       for (int i = 0; i < plan.parts; ++i) {
@@ -1186,13 +1189,13 @@ int launch_bwd(const void* q, const void* k, const void* v, const void* dy, cons
   if (mask != nullptr && causal) return ERROR_ATTN_UNSUPPORTED_SHAPE;
   constexpr bool NARROW = HD <= 64;
   constexpr int BN = BwdPlan<HD, NARROW>::BN;
-  CUtensorMap mq, mk, mv, mdo, mk64;
+  CUtensorMap mq, mk, mv, mdo;
   int e;
   const McaStrides sin = mca_in_strides(layout, H, T, HD), sout = mca_out_strides(layout, H, T, HD);
   if ((e = make_map_bf16(&mq, q, B, H, T, HD, sin, BN)) || (e = make_map_bf16(&mk, k, B, H, T, HD, sin, BN)) ||
-      (e = make_map_bf16(&mv, v, B, H, T, HD, sin, BN)) || (e = make_map_bf16(&mdo, dy, B, H, T, HD, sout, BN)) ||
-      (e = make_map_bf16(&mk64, k, B, H, T, HD, sin, 64)))
+      (e = make_map_bf16(&mv, v, B, H, T, HD, sin, BN)) || (e = make_map_bf16(&mdo, dy, B, H, T, HD, sout, BN)))
     return e;
+  const auto mk64 = [&](CUtensorMap* m) { return make_map_bf16(m, k, B, H, T, HD, sin, 64); };
   BwdParams p;
   p.scales = nullptr;
   p.lse = lse; p.delta = delta; p.status = status; p.T = T; p.causal = causal; p.H = H;
@@ -1224,15 +1227,16 @@ int launch_bwd_split(const float* dy, const float* y_copy, const float* lse, flo
   // the kernel that splits dY also forms delta = rowsum(dY o Y) from the elements it holds
   int e = split::run<HD>(job, 1, sout, B, H, T, w, st, y_copy, delta);
   if (e) return e;
-  CUtensorMap mq, mk, mv, mdo, mk64;
+  CUtensorMap mq, mk, mv, mdo;
   const McaStrides sp{(int64_t)H * T * 128, (int64_t)T * 128, 128};
   const CUtensorMap* maps[4] = {&mq, &mk, &mv, &mdo};
   for (int i = 0; i < 4; ++i)
     if ((e = make_map_4d(const_cast<CUtensorMap*>(maps[i]), w.tensor[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, B, H, T, 128, sp,
                          CU_TENSOR_MAP_SWIZZLE_128B)))
       return e;
-  if ((e = make_map_4d(&mk64, w.tensor[split::TENSOR_K], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, B, H, T, 128, sp, CU_TENSOR_MAP_SWIZZLE_128B, 64)))
-    return e;
+  const auto mk64 = [&](CUtensorMap* m) {
+    return make_map_4d(m, w.tensor[split::TENSOR_K], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, B, H, T, 128, sp, CU_TENSOR_MAP_SWIZZLE_128B, 64);
+  };
   BwdParams p;
   p.scales = w.scale;
   p.lse = lse; p.delta = delta; p.status = status; p.T = T; p.causal = causal; p.H = H;
