@@ -20,6 +20,7 @@
 #include "common.cuh"
 #include "ds_rules.h"
 #include "kernels.h"
+#include "small_rules.h"
 
 namespace {
 
@@ -755,7 +756,7 @@ long attn_fwd_once(Kernel* k, long llInput, MCA_LONGLONG* pl, int layout) {
     // to the exact kernels, whose masked-row convention that backward shares.
     const bool tc_bwd = mca_sdpa_backward_f32_tc_supported(a.D) != 0;
     if ((e = look_up_mask(k, a, (long)pl[6], batch_mask, T, &mask, &mode))) return e;
-    if (!save && mca_sdpa_forward_small_takes(q, kk, v, y, a.B, a.H, T, a.D))   // applies the mask as it is: no class is needed
+    if (!save && small_rules::takes(q, kk, v, y, mask, batch_mask, packed, a.B, a.H, T, a.D))   // applies the mask as it is: no class is needed
       return mca_sdpa_forward_small(q, kk, v, mask, mode, a.B, a.H, T, a.D, y, layout, 0);
     const bool classify = mode == MCA_MASK_TT;
     McaClassifyJob job;

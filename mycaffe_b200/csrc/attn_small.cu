@@ -9,10 +9,13 @@
 // the chip: a lane has every 32nd key for the scores, and for P V four columns over every KG-th group of U keys.
 #include "kernels.h"
 #include "common.cuh"
+#include "small_rules.h"
 
 namespace {
 
-constexpr int WARPS = 8, THREADS = WARPS * 32, KEYS = 128, KPL = KEYS / 32;
+using small_rules::KEYS;
+using small_rules::WARPS;
+constexpr int THREADS = WARPS * 32, KPL = KEYS / 32;
 
 template <int D> struct Tile {
   static constexpr int CG = D / 4, KG = 32 / CG;             // 16-byte column groups of a row, key groups of a warp
@@ -174,18 +177,6 @@ template <int D> int pick(const SmallParams& p, int B, cudaStream_t st) {
 }
 
 }  // namespace
-
-// The keys of one tile, and no more rows than give every CTA an SM of its own.  A call, waited for / one of many, us, before (split operands)
-// and with this kernel: 4 heads of 128 x 16 under a (T,T) mask 20.5 -> 14.2 / 14.8 -> 5.2, 16 heads of 128 x 64 20.5 -> 17.9 / 9.1 -> 8.7,
-// 64 of 64 x 64 20.2 -> 17.8 / 11.3 -> 8.6, 15 of 77 x 64 under a key mask 25.2 -> 17.1 / 12.4 -> 7.6.  Beyond: 64 heads of 128 x 64 21.0 -> 23.8 /
-// 13.0 -> 12.5, of 128 x 32 19.8 -> 19.7 / 9.6 -> 12.3; and with a second tile 16 heads of 256 x 32 21.2 -> 20.0 / 10.8 -> 13.0, 8 of 256 x 64
-// 22.8 -> 21.8 / 11.8 -> 18.6.
-bool mca_sdpa_forward_small_takes(const void* q, const void* k, const void* v, const void* y, int B, int H, int T, int D) {
-  if (D != 16 && D != 32 && D != 64) return false;
-  if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(y)) & 15)
-    return false;
-  return T <= KEYS && (int64_t)B * H * mca_ceil_div(T, WARPS * 4) <= 148;
-}
 
 int mca_sdpa_forward_small(const float* q, const float* k, const float* v, const float* mask, int mode, int B, int H, int T, int D, float* y,
                            int layout, void* stream) {

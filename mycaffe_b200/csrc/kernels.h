@@ -31,8 +31,7 @@ int mca_sdpa_backward_f32_tc_ws(const float* dy, const float* y_copy, const floa
                                 int layout, const uint32_t* mask_bits, const uint32_t* mask_bits_t, int mask_mode, void* ds,
                                 int64_t ds_bytes, void* stream);
 
-// Internal: the fp32 forward of a short call that nothing is kept of, in one launch (attn_small.cu), and whether it takes a call.
-bool mca_sdpa_forward_small_takes(const void* q, const void* k, const void* v, const void* y, int B, int H, int T, int D);
+// Internal: the fp32 forward of a short call that nothing is kept of, in one launch (attn_small.cu); small_rules::takes says which.
 int mca_sdpa_forward_small(const float* q, const float* k, const float* v, const float* mask, int mode, int B, int H, int T, int D, float* y,
                            int layout, void* stream);
 

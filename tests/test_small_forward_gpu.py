@@ -48,3 +48,22 @@ def test_packed(T, H, D):
     q, k, v = (np.ascontiguousarray(x[:, :, i].transpose(0, 2, 1, 3)) for i in range(3))
     assert rel_err(y, oracle.sdpa_forward(q, k, v, None, 3, f64=True)) < TOL
     cuda.Dispose()
+
+
+@pytest.mark.parametrize("over", ["q", "k", "v", "mask"])
+@pytest.mark.parametrize("T,H,D", [(128, 4, 64), (100, 9, 32)])
+def test_output_over_an_input(T, H, D, over):
+    """y may be q's, k's, v's or the mask's memory: the split kernels take such a call, which read all of them before they write."""
+    cuda = CudaDnn(0)
+    rng = np.random.default_rng(T)
+    q, k, v = (rng.standard_normal((1, H, T, D)).astype(np.float32) for _ in range(3))
+    pairs = (rng.random((T, T)) > 0.3).astype(np.float32)
+    hc, ha = cuda.CreateCuDNN(), cuda.CreateAttn()
+    cuda.SetAttn(hc, ha, 0, False, 1, T, H, D, 0.0, 0, ids.MCA_DTYPE_F32, 0)
+    room = np.zeros(max(T * T, q.size), np.float32)
+    room[:T * T] = pairs.ravel()
+    h = {"q": cuda.AllocMemory(q), "k": cuda.AllocMemory(k), "v": cuda.AllocMemory(v), "mask": cuda.AllocMemory(room)}
+    cuda.AttnScaledDotProductForward(hc, ha, T, h["q"], h["k"], h["v"], h["mask"], h[over], False)
+    y = cuda.GetMemory(h[over], q.size).reshape(q.shape)
+    assert rel_err(y, oracle.sdpa_forward(q, k, v, pairs, 1, f64=True)) < 2e-5     # the split kernels' bound
+    cuda.Dispose()
