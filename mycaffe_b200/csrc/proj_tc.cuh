@@ -558,6 +558,7 @@ __global__ void __maxnreg__(Plan<WT>::CONVERT ? 72 : 112) proj_tc_kernel(const _
       }
       last = __shfl_sync(0xffffffffu, last, 0);
       if (!last) continue;
+      __syncwarp();   // what lane 0 has acquired is the other lanes' too: a shuffle orders no memory
       // all of a round's loads in flight together; the sums are taken in the parts' order whoever arrived last
       const float* p0 = g_partials + r;
       for (int c0 = col_first; c0 < p.Bp; c0 += 16) {
