@@ -201,8 +201,9 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) gemv_stream_k
   const bool residual = !GLU && p.accumulate && p.n_mats == 1;
   float first_res = 0.f;
   if (residual) {
-    const int o = S == 1 ? lane : lane % OUTS, r = (step_lo + (S == 1 ? 0 : lane / OUTS)) * STEP + o / NB, b = b0 + o % NB;
-    if (seg == 0 && o < OUTS && r < total_rows && b < p.B) first_res = p.out[0][(int64_t)b * total_rows + r];
+    const int o = S == 1 ? lane : lane % OUTS, st = S == 1 ? 0 : lane / OUTS, r = (step_lo + st) * STEP + o / NB, b = b0 + o % NB;
+    // of this group's own steps: another group's outputs may be on their way by now
+    if (seg == 0 && o < OUTS && st < n_steps && r < total_rows && b < p.B) first_res = p.out[0][(int64_t)b * total_rows + r];
   }
 
   // ---- phase 1: activations of this pass's sequences -> shared memory, RMS-normalised
