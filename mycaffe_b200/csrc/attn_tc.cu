@@ -811,18 +811,24 @@ template <int HD, int MODE, bool NARROW>
 int launch_shape(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const TcParams& p, int B, int H, int T,
                  bool masked, cudaStream_t st) {
   using SH = Shape<HD, MODE, NARROW>;
-  const size_t smem = SH::PL::BYTES;
   dim3 grid(mca_ceil_div(T, SH::QT * BLK), B * H);
+  // Two narrow CTAs fit an SM.  Behind the operand split they are launched while its CTAs are still there, and where the grid has an SM for
+  // each, pairs of them shared one while others stood idle: each then asks for more than half of an SM's memory (forwards alone, us, before /
+  // now: 12 heads of 1500 x 64 under a key mask 61.5 / 44.3, 8 of 2000 77.9 / 56.4, 12 of 1500 without a mask 44.5 / 38.0, causal 40.6 / 37.5; from 149
+  // CTAs on nothing changes).
+  constexpr bool alone = MODE == MODE_SPLIT && NARROW;
+  constexpr size_t smem_max = alone && SH::PL::BYTES < 116 * 1024 ? 116 * 1024 : SH::PL::BYTES;
+  const size_t smem = alone && (int64_t)grid.x * grid.y <= 148 ? smem_max : (size_t)SH::PL::BYTES;
   if constexpr (MODE != MODE_TF32) {
     if (masked) {
       static std::atomic<uint64_t> done{0};
-      const int e = mca_smem_once(done, sdpa_fwd_tc_kernel<HD, MODE, true, NARROW>, smem);
+      const int e = mca_smem_once(done, sdpa_fwd_tc_kernel<HD, MODE, true, NARROW>, smem_max);
       if (e) return e;
       return mca_launch_pdl(sdpa_fwd_tc_kernel<HD, MODE, true, NARROW>, grid, dim3(SH::THREADS), smem, st, mq, mk, mv, p);
     }
   }
   static std::atomic<uint64_t> done{0};
-  const int e = mca_smem_once(done, sdpa_fwd_tc_kernel<HD, MODE, false, NARROW>, smem);
+  const int e = mca_smem_once(done, sdpa_fwd_tc_kernel<HD, MODE, false, NARROW>, smem_max);
   if (e) return e;
   return mca_launch_pdl(sdpa_fwd_tc_kernel<HD, MODE, false, NARROW>, grid, dim3(SH::THREADS), smem, st, mq, mk, mv, p);
 }
