@@ -1077,10 +1077,9 @@ int mca_split_forward_main(int causal, int B, int H, int T, int D, float* y, flo
 // Rows are padded to whole 128-key tiles (mca_mask_bits_row_words(T) words).
 // ---------------------------------------------------------------------------------------------
 namespace {
-__global__ void __launch_bounds__(256) mask_pack_kernel(const float* mask, int rows, int T, int wpr, uint32_t* bits, uint32_t* bits_t) {
-  // The forward behind this kernel is not let go before it ends: its CTAs, launched at the top, took the SMs that were free, two to one where
-  // the grid has one for each (layers under a key mask, bf16, us: 8 heads of 1024 x 128 54.4, 45.7 so; 24 of 384 x 128 31.1, 26.9; 64 of 256 x 64 28.1,
-  // 25.2; launched ordinarily 47.7, 28.8, 26.7).
+__global__ void __launch_bounds__(256) mask_pack_kernel(const float* mask, int rows, int T, int wpr, uint32_t* bits, uint32_t* bits_t,
+                                                        int let_go) {
+  if (let_go) mca_pdl_launch_dependents();
   mca_pdl_wait();   // the mask may be the kernel before's, and the bits be read by it
   const int64_t word = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -1113,13 +1112,16 @@ int mca_mask_bits_view(const uint32_t* bits, const uint32_t* bits_t, int mask_mo
 }
 
 int mca_mask_pack(const float* mask, int mask_mode, int B, int T, uint32_t* bits, uint32_t* bits_t, void* stream) {
+  return mca_mask_pack_ahead(mask, mask_mode, B, T, bits, bits_t, 0, stream);
+}
+int mca_mask_pack_ahead(const float* mask, int mask_mode, int B, int T, uint32_t* bits, uint32_t* bits_t, int let_go, void* stream) {
   if (!mask || !bits) return ERROR_PARAM_NULL;
   if (T <= 0 || B <= 0) return ERROR_PARAM_OUT_OF_RANGE;
   if (mask_mode != MCA_MASK_TT && mask_mode != MCA_MASK_BATCH) return ERROR_PARAM_OUT_OF_RANGE;
   const int rows = mask_mode == MCA_MASK_TT ? T : B, wpr = mca_mask_bits_row_words(T);
   const int64_t words = (int64_t)rows * wpr;
   return mca_launch_pdl(mask_pack_kernel, dim3((unsigned)((words + 7) / 8)), dim3(256), 0, (cudaStream_t)stream, mask, rows, T, wpr, bits,
-                        mask_mode == MCA_MASK_TT ? bits_t : nullptr);
+                        mask_mode == MCA_MASK_TT ? bits_t : nullptr, let_go);
 }
 
 int mca_set_fail_words_fwd(int* words) { return (int)cudaMemcpyToSymbol(tc::g_fail_words, &words, sizeof(words)); }

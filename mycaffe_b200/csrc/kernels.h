@@ -42,6 +42,9 @@ int mca_split_forward_prepass(const float* q, const float* k, const float* v, in
 int mca_split_forward_main(int causal, int B, int H, int T, int D, float* y, float* row_max, float* row_sum, float* y_copy, float* lse,
                            void* workspace, int* status, int layout, const uint32_t* mask_bits, int mask_mode, void* stream);
 
+// Internal: mca_mask_pack whose forward may be let go at its top.
+int mca_mask_pack_ahead(const float* mask, int mask_mode, int B, int T, uint32_t* bits, uint32_t* bits_t, int let_go, void* stream);
+
 // Internal: hand the current device's kernels the address of their row of failure words (McaFailWord).
 int mca_set_fail_words_fwd(int* words);
 int mca_set_fail_words_bwd(int* words);
