@@ -16,10 +16,10 @@ inline bool overlap(const Range& a, const Range& b) {
 }
 
 // The keys of one tile, and no more rows than give every CTA an SM of its own.  A call, waited for / one of many, us, before (split operands)
-// and with this kernel: 4 heads of 128 x 16 under a (T,T) mask 20.5 -> 14.2 / 14.8 -> 5.2, 16 heads of 128 x 64 20.5 -> 17.9 / 9.1 -> 8.7,
-// 64 of 64 x 64 20.2 -> 17.8 / 11.3 -> 8.6, 15 of 77 x 64 under a key mask 25.2 -> 17.1 / 12.4 -> 7.6.  Beyond: 64 heads of 128 x 64 21.0 -> 23.8 /
-// 13.0 -> 12.5, of 128 x 32 19.8 -> 19.7 / 9.6 -> 12.3; and with a second tile 16 heads of 256 x 32 21.2 -> 20.0 / 10.8 -> 13.0, 8 of 256 x 64
-// 22.8 -> 21.8 / 11.8 -> 18.6.
+// and with this kernel: 4 heads of 128 x 16 under a (T,T) mask 20.5 -> 14.6 / 15.1 -> 5.4, 16 heads of 128 x 64 20.4 -> 18.3 / 8.3 -> 6.5,
+// 64 of 64 x 64 20.9 -> 18.3 / 11.1 -> 6.5, 15 of 77 x 64 under a key mask 25.2 -> 17.5 / 12.4 -> 5.8.  Beyond: 64 heads of 128 x 64 20.6 -> 24.5 /
+// 9.9 -> 12.6, of 128 x 32 19.5 -> 20.2 / 8.2 -> 8.3; and with a second tile, measured with an earlier launch of what follows, 16 heads of 256 x 32
+// 21.2 -> 20.0 / 10.8 -> 13.0, 8 of 256 x 64 22.8 -> 21.8 / 11.8 -> 18.6.
 inline bool fits(int B, int H, int T, int D) {
   return (D == 16 || D == 32 || D == 64) && T <= KEYS && (int64_t)B * H * ((T + WARPS * 4 - 1) / (WARPS * 4)) <= 148;
 }

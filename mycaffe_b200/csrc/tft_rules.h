@@ -45,8 +45,9 @@ inline Split backward_split(int B, int H, int tiles, int d = 64) {
 // Whether the backward runs two items to an SM, with one buffer for V and then each head's K in turn: where there are more items than SMs.
 // One's copies and barriers then stand beside the other's products, which one item's own second buffer does less well (forward and backward,
 // us: 256 items, 8 heads, 40 x 192, d 16 291 -> 260; 300, 4, 24 x 150, 32 154 -> 142; 200, 8, 192 x 192, 32 1414 -> 1366; 170, 6, 160 x 160, 16
-// 614 -> 548; 155, 1, 5 x 40, 16 22.6 -> 20.5).  64-wide heads have not the registers (128 a thread, 100 spilled): 256, 4, 24 x 192
-// 137.3 -> 136.6, 192 x 192 988 -> 1088.
+// 614 -> 548; 155, 1, 5 x 40, 16 22.6 -> 20.5; and just beyond a round or two of the SMs, over many row tiles, where V is read again for
+// each of them: 149, 4, 192 x 192, 16 526 -> 476, 32 760 -> 673; 149, 8, 160 x 160, 32 1020 -> 975; 223, 8, 160 x 160, 16 867 -> 776; 296, 1,
+// 192 x 192, 32 361 -> 339).  64-wide heads have not the registers (128 a thread, 100 spilled): 256, 4, 24 x 192 137.3 -> 136.6, 192 x 192 988 -> 1088.
 inline bool backward_pair(int B, int d) { return d <= 32 && B > 148; }
 
 // Into how many CTAs the forward of a row tile's heads goes: as long as every tile's cluster is resident at once, with an SM to each

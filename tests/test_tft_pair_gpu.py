@@ -11,3 +11,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("B,H,Nq,Nk,d", [(149, 2, 50, 61, 32), (151, 3, 24, 192, 16), (150, 1, 25, 33, 32), (149, 1, 1, 1, 16), (300, 4, 7, 130, 16)])
 def test_two_items_to_an_sm(cuda, B, H, Nq, Nk, d, with_attn_grad):  # noqa: F811
     forward_and_backward(cuda, B, H, Nq, Nk, d, with_attn_grad, with_mask=True)
+
+
+@pytest.mark.parametrize("B,H,Nq,Nk,d", [(149, 2, 30, 61, 32), (150, 3, 24, 190, 16)])
+def test_without_a_mask(cuda, B, H, Nq, Nk, d):  # noqa: F811
+    forward_and_backward(cuda, B, H, Nq, Nk, d, True, with_mask=False)
