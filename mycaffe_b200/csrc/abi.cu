@@ -20,6 +20,7 @@
 #include "common.cuh"
 #include "ds_rules.h"
 #include "kernels.h"
+#include "launch_rules.h"
 #include "small_rules.h"
 
 namespace {
@@ -632,12 +633,7 @@ long mask_bits_room(AttnHandle& a) {
 long pack_mask_bits(AttnHandle& a, const float* mask, int mode, int T) {
   const long e = mask_bits_room(a);
   if (e) return e;
-  // Is the forward let go at the top of the packing?  Its CTAs then take the SMs that are free, two to one where the grid has one for
-  // each: bf16 layers under a key mask, us, let go at the top / at the end / ordinary launches: 8 heads of 1024 x 128 54.4 / 45.7 / 47.7, 24 of 384 x 128
-  // 31.1 / 26.9 / 28.8, 64 of 256 x 64 28.1 / 25.2 / 26.7.  With few CTAs enough SMs are free, and the launch is hidden (layers of 64-wide heads, to 60
-  // CTAs, 3 to 6 %; of 128-wide ones, to 40, nothing or little; forwards alone, to 64, 3 %; 72 lose 25).  Split operands' CTAs ask for an SM of their own.
-  const int64_t ctas = (int64_t)a.B * a.H * ((T + 127) / 128);
-  const bool let_go = a.dtype != MCA_DTYPE_BF16 || ctas <= (!a.training ? 64 : a.D == 128 ? 40 : 60);
+  const bool let_go = a.dtype != MCA_DTYPE_BF16 || launch_rules::pack_lets_go((int64_t)a.B * a.H, T, a.D, a.training);
   return mca_mask_pack_ahead(mask, mode, a.B, T, a.mask_bits, a.mask_bits_t, let_go, 0);
 }
 

@@ -28,6 +28,7 @@
 
 #include "ds_rules.h"
 #include "kernels.h"
+#include "launch_rules.h"
 #include "tc_common.cuh"
 #include "split_prepass.cuh"
 
@@ -41,6 +42,7 @@ using namespace tc;
 // queries are what a thread that reads dS^T from TMEM has in four registers, so a warp writes 512 consecutive bytes an instruction without
 // a shuffle, and the dQ kernel reads a tile by plain bulk copies.
 constexpr int DS_GROUP_BYTES = 32 * 16, DS_BLOCK_BYTES = 16 * DS_GROUP_BYTES;
+static_assert(launch_rules::TILE == BLK);
 static_assert(ds_rules::TILE == BLK && ds_rules::tile_bytes(false) == 4 * DS_BLOCK_BYTES && ds_rules::tile_bytes(true) == 8 * DS_BLOCK_BYTES);
 template <bool SPLIT> __device__ __forceinline__ int64_t ds_tile_offset(int64_t head, int qt, int kt, int T, int causal) {
   const int nt = (T + BLK - 1) / BLK;
@@ -1078,18 +1080,6 @@ sdpa_bwd_dq_ds_tc_kernel(const __grid_constant__ CUtensorMap map_k, const BwdPar
 // dK/dV kernel, so dY (which the forward does not write) is asked for into L2 before the wait, and all of a thread's loads
 // are in flight together behind it: T = 7001, 16 heads x 128: 18 us behind the forward -> 15.
 constexpr int DELTA_STEPS = 4;
-// Is the dK/dV kernel let go only when the forward has left the SMs (late), not at the delta kernel's top?  Launched before, its CTAs take what
-// is free, two to one SM where the grid has one for each; late, its launch is no longer hidden.  Beyond three tiles a head late gains for
-// 128-wide heads (layers, us: 12 of 1024 41.6 -> 40.1; 24 and more of any length the same).  64-wide ones, two of whose CTAs an SM takes,
-// lose 3 to 8 % with fewer rows than 64 CTAs have.  With more, all as long, they gain (no mask, by CTAs: 64 3 to 6 %, 96 3.5 to 5, 128 0.4 to
-// 4.5, 144 3 to 4, from 192 0 to 1, but 64 of 8 heads of 900 lose 4.7; 8 of 2048 under a (T,T) mask 145 -> 132).  Causal CTAs are of all
-// lengths: 80 gain 6.7 and 3.8 %, 96 2.6 to 4.2, 160 2.2 and 3.7, 192 2.2 to 3.6, but 128 lose 5 to 7, 240 to 330 up to 6.
-inline bool delta_lets_go_late(int64_t heads, int T, int D, bool causal) {
-  const int64_t nt = (T + BLK - 1) / BLK, ctas = heads * nt;
-  if (nt <= 3) return false;
-  if (D == 128) return true;
-  return causal ? (ctas >= 72 && ctas <= 96) || (ctas >= 160 && ctas <= 224) : heads * T >= 64 * BLK;
-}
 __global__ void __launch_bounds__(256) bwd_delta_bf16_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* y, int64_t rows, int H, int T,
                                                              int D, const McaStrides ys, float* __restrict__ delta, int late) {
   if (!late) mca_pdl_launch_dependents();
@@ -1308,7 +1298,7 @@ int mca_sdpa_backward_tc_ws(const void* q, const void* k, const void* v, const v
     const int64_t rows_per_block = 8 * (256 / D) * DELTA_STEPS;   // eight warps, 256 / D rows each a step
     e = mca_launch_pdl(bwd_delta_bf16_kernel, dim3((unsigned)((rows + rows_per_block - 1) / rows_per_block)), dim3(256), 0, st,
                        (const __nv_bfloat16*)dy, (const __nv_bfloat16*)y, rows, H, T, D, mca_out_strides(layout, H, T, D), delta_scratch,
-                       (int)delta_lets_go_late((int64_t)B * H, T, D, causal != 0));
+                       (int)launch_rules::delta_lets_go_late((int64_t)B * H, T, D, causal != 0));
   }
   if (e) return e;
   const DsRoom room{static_cast<uint8_t*>(ds), ds_bytes};
